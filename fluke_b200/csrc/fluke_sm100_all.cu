@@ -6,5 +6,6 @@
 #include "lstm_sm100.cu"
 #include "lstm_persist_sm100.cu"
 #include "lstm_cluster_sm100.cu"
+#include "lstm_group_sm100.cu"
 #include "lstm_noalloc_sm100.cu"
 #include "stack_sm100.cu"

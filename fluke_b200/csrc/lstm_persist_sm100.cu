@@ -137,10 +137,9 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "memory");
 }
 
-// The cell update of two adjacent hidden units of one row, in packed f32x2 arithmetic where the
-// instruction set has it. gi..go: the accumulator bits (f32) of the four gates of units u, u+1;
-// bi..bo: their biases; c: the two cell values, updated in place. Returns the two int8 codes of
-// h in bits 0-7 and 8-15.
+// The update of two cells (adjacent hidden units of one row, or one unit of two rows), in packed
+// f32x2 arithmetic where the instruction set has it. gi..go: the accumulator bits (f32) of the two cells' four gates;
+// bi..bo: their biases; c: the two cell values, updated in place. Returns the two int8 codes of h.
 //   gates   i, f, o = clamp(0.2 (acc + b) + 0.5, 0, 1) as one saturating fma each,
 //           g = clamp(acc + b, -1, 1)
 //   cell    c = fma(f, c, i * g)
@@ -151,9 +150,9 @@ __device__ __forceinline__ float p_sat_fma(float x, float a, float b) {
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(x), "f"(a), "f"(b));
     return y;
 }
-__device__ __forceinline__ uint32_t lstm_cell_pair(uint32_t gi0, uint32_t gi1, uint32_t gf0, uint32_t gf1,
-                                                   uint32_t gg0, uint32_t gg1, uint32_t go0, uint32_t go1,
-                                                   float2 bi, float2 bf, float2 bg, float2 bo, float2 &c) {
+__device__ __forceinline__ int2 lstm_cell_codes(uint32_t gi0, uint32_t gi1, uint32_t gf0, uint32_t gf1,
+                                                uint32_t gg0, uint32_t gg1, uint32_t go0, uint32_t go1,
+                                                float2 bi, float2 bf, float2 bg, float2 bo, float2 &c) {
     const float2 pi = add2(make_float2(__uint_as_float(gi0), __uint_as_float(gi1)), bi);
     const float2 pf = add2(make_float2(__uint_as_float(gf0), __uint_as_float(gf1)), bf);
     const float2 pg = add2(make_float2(__uint_as_float(gg0), __uint_as_float(gg1)), bg);
@@ -176,7 +175,14 @@ __device__ __forceinline__ uint32_t lstm_cell_pair(uint32_t gi0, uint32_t gi1, u
     // (__fadd_rn: never fused with the multiplication before it)
     const float hx = __fadd_rn(hs.x, __uint_as_float(0x3F000000u | (__float_as_uint(hs.x) & 0x80000000u)));
     const float hy = __fadd_rn(hs.y, __uint_as_float(0x3F000000u | (__float_as_uint(hs.y) & 0x80000000u)));
-    return (uint32_t(__float2int_rz(hx)) & 0xFFu) | ((uint32_t(__float2int_rz(hy)) & 0xFFu) << 8);
+    return make_int2(__float2int_rz(hx), __float2int_rz(hy));
+}
+// The two codes in bits 0-7 and 8-15.
+__device__ __forceinline__ uint32_t lstm_cell_pair(uint32_t gi0, uint32_t gi1, uint32_t gf0, uint32_t gf1,
+                                                   uint32_t gg0, uint32_t gg1, uint32_t go0, uint32_t go1,
+                                                   float2 bi, float2 bf, float2 bg, float2 bo, float2 &c) {
+    const int2 h = lstm_cell_codes(gi0, gi1, gf0, gf1, gg0, gg1, go0, go1, bi, bf, bg, bo, c);
+    return (uint32_t(h.x) & 0xFFu) | ((uint32_t(h.y) & 0xFFu) << 8);
 }
 
 template <int UNITS, int WPT>

@@ -300,8 +300,9 @@ extern "C" int fluke_sm100_lstm_layer_persistent(const void *layer, const void *
                                                  void *flags, void *stream);
 extern "C" int fluke_sm100_lstm_layer_cluster(const void *layer, const void *x_down, int allow_waves,
                                               void *stream);
+extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_down, void *stream);
 // Form selection (see fluke_sm100_set_lstm_persistent in fluke_sm100.h) and the form the last
-// whole-layer call used: 0 per step, 1 cluster, 2 L2 exchange. Both are kept per host thread: a
+// whole-layer call used: 0 per step, 1 cluster, 2 L2 exchange, 3 small clusters. Both are kept per host thread: a
 // process that drives several GPUs from several threads sets and reads its own.
 static thread_local int g_lstm_last_form = -1;
 extern "C" int fluke_sm100_lstm_last_form(void) { return g_lstm_last_form; }
@@ -364,6 +365,7 @@ extern "C" int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, 
                 case 1: return fluke_sm100_lstm_layer_cluster(l, x_down, 0, stream);   // all tiles at once only
                 case 5: return fluke_sm100_lstm_layer_cluster(l, x_down, 1, stream);   // in rounds if need be
                 case 2: return fluke_sm100_lstm_layer_persistent(l, x_down, hh_down, flags, stream);
+                case 3: return fluke_sm100_lstm_layer_group(l, x_down, stream);
                 default: return -2;
             }
         };
@@ -371,13 +373,14 @@ extern "C" int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, 
         switch (g_lstm_persistent) {
             case 2: order[0] = 2; break;
             case 4: order[0] = 5; order[1] = 2; break;
-            default: order[0] = 1; order[1] = 2; order[2] = 5; break;
+            default: order[0] = 3; order[1] = 1; order[2] = 2; order[3] = 5; break;
         }
         rc = -2;
         for (int i = 0; i < 4 && rc == -2 && order[i]; ++i) {
             rc = run_form(order[i]);
             g_lstm_last_form = order[i] == 5 ? 1 : order[i];
         }
+        if (rc == 0 && g_lstm_last_form == 3) return 0;  // has written the final hidden state
         if (rc == 0) {
             const int t_last = l->reverse ? 0 : T - 1;
             return (int)cudaMemcpyAsync(l->h_i8, static_cast<int8_t *>(l->h_out_i8) + size_t(t_last) * B * H,

@@ -88,32 +88,46 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
                  "r"(bytes)
                  : "memory");
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t done;
-    asm volatile(
-        "{\n"
-        ".reg .pred P;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, P;\n"
-        "}\n"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
+    if constexpr (CLUSTER)
+        asm volatile(
+            "{\n"
+            ".reg .pred P;\n"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, P;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n"
+            ".reg .pred P;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, P;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
     return done != 0;
 }
 
 // Waits for the phase with the given parity to complete. Gives up after `limit` cycles
 // (kWaitCycleLimit in every kernel of the library): records `site` in the status word, raises
 // *abort_flag (shared memory, seen by the other roles of the CTA) and returns false. A raised
-// abort flag also ends the wait.
+// abort flag also ends the wait. CLUSTER: the phase is completed by other CTAs of the cluster, whose
+// stores the wait has to acquire.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
                                           unsigned int site, long long limit = kWaitCycleLimit) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
 #pragma unroll 1
         for (int i = 0; i < 64; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
+            if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > limit) {
             report_timeout(site);
@@ -287,6 +301,19 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
     }
 }
 
+// The same with the A operand in tensor memory: lane = row of A, a 32-bit column = the next 4 bytes
+// of K, so one instruction (32 bytes of K) reads 8 columns starting at a_tmem.
+template <int KIND>
+__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                          uint32_t idesc, uint32_t accumulate) {
+    static_assert(KIND == kKindF16, "only the f16 form is used");
+    asm volatile(
+        "{\n.reg .pred P;\nsetp.ne.b32 P, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, P;\n}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // Instruction descriptor for a dense, K-major x K-major MMA of shape M x N (x 32 bytes of K).
 //   bits [4,6) accumulator format, [7,10) A format, [10,13) B format, 15/16 A/B major
 //   (0 = K), [17,23) N/8, [24,29) M/16.
@@ -352,6 +379,28 @@ __device__ __forceinline__ void tmem_ld_16x256_x8(uint32_t taddr, uint32_t (&r)[
           "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Thread i of the warp writes columns [col, col+32) of row (lane base + i).
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+          "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+          "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+          "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+          "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
