@@ -827,7 +827,7 @@ def run_ours(args):
         flops = T * (2.0 * B * (2 * R) * (4 * H) + 2.0 * B * R * H)   # per 1024-chunk layer: f16 gate contraction + int8 hh projection
 
         def roofline_of(us_layer, us_xdown, form, batches):
-            kname = {1: "lstm_cluster_kernel", 2: "lstm_persist_kernel"}.get(form, "lstm_step_kernel")
+            kname = {1: "lstm_cluster_kernel", 2: "lstm_persist_kernel", 3: "lstm_group_kernel"}.get(form, "lstm_step_kernel")
             us_k = us_layer - us_xdown
             achieved = batches * flops / (us_k * 1e-6) / 1e12
             tr = recurrence_traffic(kname, batches * ((B + 127) // 128))
@@ -883,7 +883,7 @@ def run_ours(args):
                 sat[str(b)] = {"us_per_step": round(us, 3), "form": L.fluke_sm100_lstm_last_form(),
                                "chunk_timesteps_per_s": round(b / (us * 1e-6), 0)}
                 del xb, sb
-            line["saturation"] = {"note": "one layer, T=250, recurrence launch only; form 1 = cluster exchange, 2 = L2 exchange", "by_chunks": sat}
+            line["saturation"] = {"note": "one layer, T=250, recurrence launch only; form 3 = small clusters, 1 = cluster exchange, 2 = L2 exchange", "by_chunks": sat}
             del x_dev, xs_dev, bufs
             torch.cuda.empty_cache()
             tensor_peaks = measure_tensor_peaks(torch)

@@ -139,8 +139,9 @@ int fluke_sm100_lstm_layer(const void *layer /* const fluke_flstm_layer_t* */, v
 int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, void *stream);
 /* How the recurrence of a layer is run (a per-host-thread setting).
  * 1 (default): one launch, the fastest single-launch form the shape and the device allow: the
- *    cluster form while all row tiles of the layer run at once, else the L2-exchange form, else the
- *    cluster form in rounds;
+ *    small-cluster form (R = 128, H a multiple of 128 from 256 to 1024), else the cluster form
+ *    while all row tiles of the layer run at once, else the L2-exchange form, else the cluster
+ *    form in rounds;
  * 2: the L2-exchange form only (separate projection CTAs; R = 128, H a multiple of 128 up to 1024);
  * 4: the cluster form only, in rounds when the layer has more row tiles than clusters fit
  *    (exchange inside thread-block clusters; R = 128, H a multiple of 64 up to 768);
@@ -153,7 +154,8 @@ void fluke_sm100_set_lstm_persistent(int mode);
  * -1 (default): wide when the layer has more row tiles than a narrow launch holds; 0: never;
  * 1: whenever the shape allows it. */
 void fluke_sm100_set_lstm_wide(int mode);
-/* Which form the last whole-layer call used: 1 cluster exchange, 2 L2 exchange, 0 per step. */
+/* Which form the last whole-layer call used: 3 small clusters, 1 cluster exchange, 2 L2 exchange,
+ * 0 per step. */
 int fluke_sm100_lstm_last_form(void);
 /* Row tiles (clusters) of the cluster form that run at once for hidden size H; 0 = unavailable. */
 int fluke_sm100_lstm_cluster_capacity(int H);

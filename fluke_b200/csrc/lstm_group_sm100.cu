@@ -59,6 +59,8 @@ struct GroupDev {
     int reverse;
     int rows;                  // chunk rows per cluster (the last cluster may have fewer)
     int n_own, n_pad;          // rows a pair projects; the same rounded up to a multiple of 8
+    int dn_ts;                 // K blocks of the projection weights kept in tensor memory
+    const int8_t *dn;          // [R, H]
     const __half *w_up;        // [4H, 2R]
     const float *bias;         // [4H]
     const float *dn_scale;     // [R]
@@ -72,15 +74,21 @@ struct GroupDev {
 struct GroupLayout {
     int x, hh, dn, h, stage, bars, misc, dynamic;
 };
+// K blocks (128 hidden units, 32 columns) of the projection weights that fit in tensor memory beside
+// the gate weights and the accumulators.
+__host__ __device__ constexpr int group_dn_ts(int nb, int H, int n_pad) {
+    const int fit = (kGTmemW - 4 * nb - n_pad) / 32;
+    return fit < H / kGUnits ? fit : H / kGUnits;
+}
 __host__ __device__ constexpr GroupLayout group_layout(int nb, int H, int n_pad) {
     GroupLayout l = {};
-    l.x = kGWxBytes;                  // x_down rows: 2 K blocks [nb x 128 B]
-    l.hh = l.x + nb * 256;            // hh_down rows, the same shape
-    l.dn = l.hh + nb * 256;           // 64 projection rows: H/128 K blocks [64 x 128 B]
-    l.h = l.dn + 64 * H;              // hidden rows of the pair: H/128 K blocks [n_pad x 128 B]
+    l.x = kGWxBytes;                  // x_down rows of two steps: 2 K blocks [nb x 128 B] each
+    l.hh = l.x + 2 * nb * 256;        // hh_down rows, the same shape
+    l.dn = l.hh + nb * 256;           // 64 projection rows: the other K blocks [64 x 128 B]
+    l.h = l.dn + 64 * (H - 128 * group_dn_ts(nb, H, n_pad));              // hidden rows of the pair: H/128 K blocks [n_pad x 128 B]
     l.stage = l.h + n_pad * H;        // 16 warps x (nb/4 rows x 32 B)
     l.bars = l.stage + nb * 128;
-    l.misc = l.bars + 8 * 8;
+    l.misc = l.bars + 10 * 8;
     l.dynamic = l.misc + 16 + 1024;   // slack for the manual 1024-byte alignment
     return l;
 }
@@ -114,9 +122,9 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                   const __grid_constant__ CUtensorMap tm_h0,   // h_0 [H/128, B, 128] int8, boxes of n_pad rows
                   const GroupDev p) {
     constexpr int kCols = NB / 4;                    // rows an epilogue thread holds at most
-    constexpr int kSendH = (NB + 31) / 32;           // 16-byte stores per lane and step, hidden slices
-    constexpr int kSendP = 3;                        // the same, projections
-    static_assert(NB % 16 == 0 && 4 * NB + 48 <= kGTmemW, "accumulators beside the weights in tensor memory");
+    constexpr int kBatches = kCols / 4;              // it takes them four at a time
+    constexpr int kSendP = NB / 16;                  // 16-byte stores per lane and step, projections
+    static_assert(NB % 16 == 0 && 4 * NB + NB <= kGTmemW, "accumulators beside the weights in tensor memory");
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
     // shared-window offsets as this CTA's
@@ -125,13 +133,13 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     const GroupLayout L = group_layout(NB, p.H, p.n_pad);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
     uint64_t *bar_once = &bars[0];       // resident weights loaded
-    uint64_t *bar_x = &bars[1];          // x_down rows landed
-    uint64_t *bar_x_free = &bars[2];     // x half of the contraction has read them
-    uint64_t *bar_h = &bars[3];          // complete hidden rows of the pair arrived
-    uint64_t *bar_proj = &bars[4];       // projection accumulator complete
-    uint64_t *bar_hh = &bars[5];         // hh_down rows arrived
-    uint64_t *bar_acc = &bars[6];        // gate accumulators complete
-    uint64_t *bar_acc_free = &bars[7];   // epilogue has read them
+    uint64_t *bar_x = &bars[1];          // [2] x_down rows landed
+    uint64_t *bar_x_free = &bars[3];     // [2] x half of the contraction has read them
+    uint64_t *bar_h = &bars[5];          // complete hidden rows of the pair arrived
+    uint64_t *bar_proj = &bars[6];       // projection accumulator complete
+    uint64_t *bar_hh = &bars[7];         // hh_down rows arrived
+    uint64_t *bar_acc = &bars[8];        // gate accumulators complete
+    uint64_t *bar_acc_free = &bars[9];   // epilogue has read them
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
 
@@ -147,7 +155,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
 
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 7; ++b) mbar_init(&bars[b], 1);
+        for (int b = 0; b < 9; ++b) mbar_init(&bars[b], 1);
         mbar_init(bar_acc_free, kGEpiWarps);
         *abort_flag = 0;
         fence_barrier_init();
@@ -163,15 +171,16 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         const int q = warp & 3, g = (warp - 2) >> 2;
         const uint4 *src = reinterpret_cast<const uint4 *>(
             p.w_up + (size_t(g) * p.H + n0 + q * 32 + lane) * (2 * kGRank));
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-            uint32_t r[32];
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                const uint4 w = __ldg(src + part * 8 + v);
-                r[4 * v] = w.x; r[4 * v + 1] = w.y; r[4 * v + 2] = w.z; r[4 * v + 3] = w.w;
-            }
-            tmem_st_32x32(tmem + (uint32_t(q * 32) << 16) + kGTmemW + g * 64 + part * 32, r);
+        const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16) + kGTmemW;
+#pragma unroll 1
+        for (int v = 0; v < 8; ++v) tmem_st_32x8(t_lane + g * 64 + v * 8, __ldg(src + 2 * v), __ldg(src + 2 * v + 1));
+        if (projects) {
+            // and K blocks g, g + 4, .. of the projection rows (M = 64: row 16 q + i in lane 32 q + i)
+            const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(half * 64 + q * 16 + (lane & 15)) * p.H);
+            for (int kb = g; kb < p.dn_ts; kb += 4)
+#pragma unroll 1
+                for (int v = 0; v < 4; ++v)
+                    tmem_st_32x8(t_lane - 32 * (kb + 1) + v * 8, __ldg(dn + kb * 8 + 2 * v), __ldg(dn + kb * 8 + 2 * v + 1));
         }
         tmem_st_wait();
         tc_fence_before_sync();
@@ -184,23 +193,23 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     if (warp == 0) {
         // ------------------------------ loader (one thread) -----------------------------
         if (elect_one()) {
-            mbar_arrive_expect_tx(bar_once, kGWxBytes + (projects ? 64 * p.H : 0));
+            mbar_arrive_expect_tx(bar_once, kGWxBytes + (projects ? (C - p.dn_ts) * 8192 : 0));
             for (int g = 0; g < 4; ++g)
                 for (int kb = 0; kb < 2; ++kb)
                     tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * p.H + n0);
             if (projects) {
-                for (int kb = 0; kb < C; ++kb)
-                    tma_load_2d(smem + L.dn + kb * 8192, &tm_dn, bar_once, kb * 128, half * 64);
+                for (int kb = p.dn_ts; kb < C; ++kb)
+                    tma_load_2d(smem + L.dn + (kb - p.dn_ts) * 8192, &tm_dn, bar_once, kb * 128, half * 64);
                 // step 0 projects the layer's initial hidden state
                 mbar_arrive_expect_tx(bar_h, uint32_t(p.n_pad) * p.H);
                 tma_load_3d(smem + L.h, &tm_h0, bar_h, 0, m0 + pair * p.n_own, 0);
             }
             bool ok = true;
             for (int i = 0; i < p.T && ok; ++i) {
-                if (i > 0) ok = mbar_wait(bar_x_free, (i - 1) & 1, abort_flag, 96);
+                if (i > 1) ok = mbar_wait(&bar_x_free[i & 1], ((i >> 1) - 1) & 1, abort_flag, 96);
                 if (!ok) break;
-                mbar_arrive_expect_tx(bar_x, NB * 256);
-                tma_load_4d(smem + L.x, &tm_x, bar_x, 0, m0, 0, time_of(i));
+                mbar_arrive_expect_tx(&bar_x[i & 1], NB * 256);
+                tma_load_4d(smem + L.x + (i & 1) * (NB * 256), &tm_x, &bar_x[i & 1], 0, m0, 0, time_of(i));
             }
         }
         __syncwarp();
@@ -210,28 +219,36 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         // K loops unrolled, so an MMA is issued every few cycles.
         constexpr uint32_t kIdescGate = make_idesc<kKindF16>(128, NB);
         const uint32_t idesc_proj = make_idesc<kKindI8>(64, 0) | (uint32_t(p.n_pad >> 3) << 17);
-        const uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
-        const uint64_t d_x = make_smem_desc_sw128(smem_u32(smem + L.x));
-        const uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
-        const uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
-        const uint64_t d_h = make_smem_desc_sw128(smem_u32(smem + L.h));
+        uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
+        uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
+        uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
+        uint64_t d_h = make_smem_desc_sw128(smem_u32(smem + L.h));
+        uint64_t d_x = 0;
         const uint32_t t_proj = tmem + 4 * NB;
+        // The x half of gates [g0, g1). Its 32 MMAs read their A operand from shared memory (33
+        // cycles each, a third of a step in all) and the tensor pipe works in order: half of them go in front
+        // of the projection, while the hidden state is computed and travels, half behind it, while
+        // the projection is converted and travels.
+        auto x_half = [&](int g0, int g1) {
+#pragma unroll
+            for (int g = g0; g < g1; ++g)
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    tc_mma<kKindF16>(tmem + g * NB, d_wx + uint64_t((g * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
+                                     d_x + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescGate, k != 0);
+        };
         bool ok = mbar_wait(bar_once, 0, abort_flag, 97);
         for (int i = 0; i < p.T && ok; ++i) {
             if (i > 0) ok = mbar_wait(bar_acc_free, (i - 1) & 1, abort_flag, 98);
             if (!ok) break;
-            ok = mbar_wait(bar_x, i & 1, abort_flag, 99);
+            ok = mbar_wait(&bar_x[i & 1], (i >> 1) & 1, abort_flag, 99);
             if (!ok) break;
             tc_fence_after_sync();
-            if (elect_one()) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        tc_mma<kKindF16>(tmem + g * NB, d_wx + uint64_t((g * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                         d_x + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescGate, k != 0);
-                tc_commit(bar_x_free);
-            }
+            // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
+            // more registers than there are.
+            d_x = make_smem_desc_sw128(smem_u32(smem + L.x)) + uint64_t((i & 1) * (NB * 16));
+            asm volatile("" : "+l"(d_wx), "+l"(d_x), "+l"(d_hh), "+l"(d_dn), "+l"(d_h));
+            if (elect_one()) x_half(0, 2);
             __syncwarp();
             if (projects) {
                 ok = mbar_wait<true>(bar_h, i & 1, abort_flag, 100);
@@ -240,23 +257,33 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 tc_fence_after_sync();
                 FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + 3, clock64());
                 if (elect_one()) {
-                    if (i + 1 < p.T) mbar_arrive_expect_tx(bar_h, uint32_t(n_own) * p.H);  // arm the next step
-                    for (int kb = 0; kb < C; ++kb)
+                    // an MMA is 8 to 12 cycles with its weights in tensor memory, 24 from shared memory
+                    for (int kb = 0; kb < p.dn_ts; ++kb)
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
-                            tc_mma<kKindI8>(t_proj, d_dn + uint64_t(kb * 512 + 2 * k),
+                            tc_mma_ts<kKindI8>(t_proj, tmem + kGTmemW - 32 * (kb + 1) + 8 * k,
+                                               d_h + uint64_t(kb * p.n_pad * 8 + 2 * k), idesc_proj, (kb | k) != 0);
+                    for (int kb = p.dn_ts; kb < C; ++kb)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            tc_mma<kKindI8>(t_proj, d_dn + uint64_t((kb - p.dn_ts) * 512 + 2 * k),
                                             d_h + uint64_t(kb * p.n_pad * 8 + 2 * k), idesc_proj, (kb | k) != 0);
                     tc_commit(bar_proj);
+                    if (i + 1 < p.T) mbar_arrive_expect_tx(bar_h, uint32_t(n_own) * p.H);  // arm the next step
                 }
                 __syncwarp();
             }
+            if (elect_one()) {
+                x_half(2, 4);
+                tc_commit(&bar_x_free[i & 1]);
+            }
+            __syncwarp();
             ok = mbar_wait<true>(bar_hh, i & 1, abort_flag, 101);
             if (!ok) break;
             fence_proxy_async_smem();
             tc_fence_after_sync();
             FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + 6, clock64());
             if (elect_one()) {
-                if (i + 1 < p.T) mbar_arrive_expect_tx(bar_hh, uint32_t(n_rows) * 256);
 #pragma unroll
                 for (int g = 0; g < 4; ++g)
 #pragma unroll
@@ -264,6 +291,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                         tc_mma_ts<kKindF16>(tmem + g * NB, tmem + kGTmemW + g * 64 + k * 8,
                                             d_hh + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescGate, 1u);
                 tc_commit(bar_acc);
+                if (i + 1 < p.T) mbar_arrive_expect_tx(bar_hh, uint32_t(n_rows) * 256);
             }
             __syncwarp();
         }
@@ -295,33 +323,34 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         // The stores of every step go to the same places: addresses are worked out once. An item of
         // the hidden slice is (row, 16 units, projection half); of the projection (row, 8 columns, CTA).
         const uint32_t stage = smem_u32(smem + L.stage) + (warp - 2) * (kCols * 32);
-        uint32_t hs_src[kSendH], hs_dst[kSendH], hs_bar[kSendH];
+        // A destination is 16-byte aligned; its low bits hold the peer's rank (the peer's mbarrier
+        // address follows from it), 8 marks an item that exists.
+        uint32_t hs_dst[kBatches];   // lanes 0-15, one store per batch of four rows
 #pragma unroll
-        for (int s = 0; s < kSendH; ++s) {
-            const int id = lane + 32 * s, row = id >> 2, ch = (id >> 1) & 1;
+        for (int b = 0; b < kBatches; ++b) {
+            const int row = 4 * b + (lane >> 2), ch = (lane >> 1) & 1;
             const int pr = (r0 + row) / p.n_own, lr = (r0 + row) - pr * p.n_own;
-            hs_src[s] = 0; hs_dst[s] = 0; hs_bar[s] = 0;
-            if (row < my_rows) {
-                const uint32_t to = uint32_t(2 * pr + (id & 1));
-                hs_src[s] = stage + row * 32 + ch * 16;
-                hs_dst[s] = map_to_rank(smem_u32(smem + L.h + rank * (p.n_pad * 128)) + sw128_offset(lr, 2 * q + ch), to);
-                hs_bar[s] = map_to_rank(smem_u32(bar_h), to);
-            }
+            const uint32_t to = uint32_t(2 * pr + (lane & 1));
+            hs_dst[b] = lane < 16 && row < my_rows
+                ? map_to_rank(smem_u32(smem + L.h + rank * (p.n_pad * 128)) + sw128_offset(lr, 2 * q + ch), to) | 8u | to
+                : 0u;
         }
-        uint32_t ps_src[kSendP], ps_dst[kSendP], ps_bar[kSendP];
+        // ceil(ceil(NB / pairs) / 4) rows of 2 C items each: at most 24 items per 16 rows (C = 3)
+        uint32_t ps_src[kSendP], ps_dst[kSendP];
 #pragma unroll
         for (int s = 0; s < kSendP; ++s) {
             const int id = lane + 32 * s, row = id / (2 * C), rest = id - row * 2 * C, ch = rest >= C ? 1 : 0;
-            ps_src[s] = 0; ps_dst[s] = 0; ps_bar[s] = 0;
-            if (row < my_pr) {
-                int to = rest - ch * C + rank;   // start with a different peer in every CTA
-                if (to >= C) to -= C;
-                const int hh_row = pair * p.n_own + pr0 + row;
-                ps_src[s] = stage + row * 32 + ch * 16;
-                ps_dst[s] = map_to_rank(smem_u32(smem + L.hh + half * (NB * 128)) + sw128_offset(hh_row, 2 * q + ch), uint32_t(to));
-                ps_bar[s] = map_to_rank(smem_u32(bar_hh), uint32_t(to));
-            }
+            int to = rest - ch * C + rank;   // start with a different peer in every CTA
+            if (to >= C) to -= C;
+            ps_src[s] = stage + row * 32 + ch * 16;
+            ps_dst[s] = row < my_pr
+                ? map_to_rank(smem_u32(smem + L.hh + half * (NB * 128)) + sw128_offset(pair * p.n_own + pr0 + row, 2 * q + ch),
+                              uint32_t(to)) | 8u | uint32_t(to)
+                : 0u;
         }
+        auto send = [&](uint32_t dst, uint32_t src, uint64_t *bar) {
+            if (dst) store_to_peer(dst & ~15u, lds128(src), map_to_rank(smem_u32(bar), dst & 7u));
+        };
         // the hidden slice's 16-byte pieces in global memory: lane = (row, 16 units)
         const bool g_ok = (lane >> 1) < my_rows;
         const uint32_t g_src = stage + lane * 16;
@@ -351,7 +380,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 __syncwarp();
 #pragma unroll
                 for (int s = 0; s < kSendP; ++s)
-                    if (ps_src[s]) store_to_peer(ps_dst[s], lds128(ps_src[s]), ps_bar[s]);
+                    send(ps_dst[s], ps_src[s], bar_hh);
                 FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 5, clock64());
                 __syncwarp();
             }
@@ -360,36 +389,43 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             if (!ok) break;
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 0, clock64());
             tc_fence_after_sync();
-            uint32_t gi[kCols], gf[kCols], gg[kCols], go[kCols];
+            // Four rows at a time: the next four leave tensor memory while these are computed, and
+            // each batch is sent as soon as it is staged, so the exchange runs beside the arithmetic.
+            uint32_t a[2][4][4];
+            auto load4 = [&](int b) {
 #pragma unroll
-            for (int j = 0; j < kCols; j += 4) {
-                tmem_ld_32x4(t_lane + 0 * NB + r0 + j, *reinterpret_cast<uint32_t(*)[4]>(gi + j));
-                tmem_ld_32x4(t_lane + 1 * NB + r0 + j, *reinterpret_cast<uint32_t(*)[4]>(gf + j));
-                tmem_ld_32x4(t_lane + 2 * NB + r0 + j, *reinterpret_cast<uint32_t(*)[4]>(gg + j));
-                tmem_ld_32x4(t_lane + 3 * NB + r0 + j, *reinterpret_cast<uint32_t(*)[4]>(go + j));
-            }
-            tmem_ld_wait();
-            // all reads of the step are done: the x half of the next one may overwrite
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_acc_free);
+                for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_lane + g * NB + r0 + 4 * b, a[b & 1][g]);
+            };
+            load4(0);
 #pragma unroll
-            for (int j = 0; j < kCols; j += 2) {
-                if (j < share) {
-                    const int2 h = lstm_cell_codes(gi[j], gi[j + 1], gf[j], gf[j + 1], gg[j], gg[j + 1], go[j], go[j + 1],
-                                                   make_float2(b_i, b_i), make_float2(b_f, b_f), make_float2(b_g, b_g),
-                                                   make_float2(b_o, b_o), c2[j / 2]);
-                    sts8(stage + j * 32 + lane, h.x);
-                    sts8(stage + (j + 1) * 32 + lane, h.y);
+            for (int b = 0; b < kBatches; ++b) {
+                tmem_ld_wait();
+                if (b + 1 < kBatches) {
+                    load4(b + 1);
+                } else {
+                    // all reads of the step are done: the x half of the next one may overwrite
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_acc_free);
+                }
+                const auto &v = a[b & 1];
+                if (4 * b < my_rows) {
+                    int2 h[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        h[j] = lstm_cell_codes(v[0][2 * j], v[0][2 * j + 1], v[1][2 * j], v[1][2 * j + 1], v[2][2 * j], v[2][2 * j + 1],
+                                               v[3][2 * j], v[3][2 * j + 1], make_float2(b_i, b_i), make_float2(b_f, b_f),
+                                               make_float2(b_g, b_g), make_float2(b_o, b_o), c2[2 * b + j]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        sts8(stage + (4 * b + 2 * j) * 32 + lane, h[j].x);
+                        sts8(stage + (4 * b + 2 * j + 1) * 32 + lane, h[j].y);
+                    }
+                    __syncwarp();
+                    if (i + 1 < p.T) send(hs_dst[b], stage + b * 128 + (lane >> 1) * 16, bar_h);
                 }
             }
-            __syncwarp();
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 1, clock64());
-            if (i + 1 < p.T) {
-#pragma unroll
-                for (int s = 0; s < kSendH; ++s)
-                    if (hs_src[s]) store_to_peer(hs_dst[s], lds128(hs_src[s]), hs_bar[s]);
-            }
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 2, clock64());
             if (g_ok) {
                 const uint4 v = lds128(g_src);
@@ -511,7 +547,8 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
 
     GroupDev p;
     p.T = T; p.B = B; p.H = H; p.reverse = l->reverse;
-    p.rows = g.rows; p.n_own = g.n_own; p.n_pad = g.n_pad;
+    p.rows = g.rows; p.n_own = g.n_own; p.n_pad = g.n_pad; p.dn_ts = group_dn_ts(g.nb, H, g.n_pad);
+    p.dn = static_cast<const int8_t *>(l->dn_hh_i8);
     p.w_up = static_cast<const __half *>(l->w_up_f16);
     p.bias = static_cast<const float *>(l->bias_f32);
     p.dn_scale = static_cast<const float *>(l->dn_hh_scale);

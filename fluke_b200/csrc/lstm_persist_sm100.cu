@@ -143,8 +143,8 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
 //   gates   i, f, o = clamp(0.2 (acc + b) + 0.5, 0, 1) as one saturating fma each,
 //           g = clamp(acc + b, -1, 1)
 //   cell    c = fma(f, c, i * g)
-//   hidden  h = o * tanh(c), tanh as 1 - 2 / (exp(2c) + 1) with the fast exponential (absolute
-//           error ~1e-7, far below one int8 code); code = trunc(127 h +- 0.5)
+//   hidden  h = o * tanh(c), tanh as 1 - 2 / (exp(2c) + 1) with the fast exponential and reciprocal
+//           (absolute error ~1e-7, far below one int8 code); code = trunc(127 h +- 0.5)
 __device__ __forceinline__ float p_sat_fma(float x, float a, float b) {
     float y;
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(x), "f"(a), "f"(b));
@@ -168,8 +168,12 @@ __device__ __forceinline__ int2 lstm_cell_codes(uint32_t gi0, uint32_t gi1, uint
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(t.x));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ey) : "f"(t.y));
     const float2 den = add2(make_float2(ex, ey), make_float2(1.f, 1.f));
-    const float2 q = make_float2(__fdividef(2.0f, den.x), __fdividef(2.0f, den.y));
-    const float2 th = add2(make_float2(1.f, 1.f), make_float2(-q.x, -q.y));
+    // 1 - 2 r with r = 1 / (exp(2c) + 1), which is never below the smallest normal number's inverse:
+    // the flush-to-zero reciprocal needs no range check, and the doubling is exact
+    float rx, ry;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(den.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(den.y));
+    const float2 th = fma2(make_float2(rx, ry), make_float2(-2.f, -2.f), make_float2(1.f, 1.f));
     const float2 hs = mul2(mul2(o_a, th), make_float2(127.f, 127.f));
     // round half away from zero: add 0.5 with the sign of the value, then truncate
     // (__fadd_rn: never fused with the multiplication before it)

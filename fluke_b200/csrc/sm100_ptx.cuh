@@ -301,17 +301,25 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
     }
 }
 
-// The same with the A operand in tensor memory: lane = row of A, a 32-bit column = the next 4 bytes
-// of K, so one instruction (32 bytes of K) reads 8 columns starting at a_tmem.
+// The same with the A operand in tensor memory: a 32-bit column = the next 4 bytes of K, so one
+// instruction (32 bytes of K) reads 8 columns starting at a_tmem. M = 128: lane = row of A; M = 64:
+// row i in lane 32 (i / 16) + i % 16, as in the accumulator.
 template <int KIND>
 __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
                                           uint32_t idesc, uint32_t accumulate) {
-    static_assert(KIND == kKindF16, "only the f16 form is used");
-    asm volatile(
-        "{\n.reg .pred P;\nsetp.ne.b32 P, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, P;\n}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    static_assert(KIND == kKindF16 || KIND == kKindI8, "forms in use");
+    if constexpr (KIND == kKindI8)
+        asm volatile(
+            "{\n.reg .pred P;\nsetp.ne.b32 P, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, P;\n}\n"
+            ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n.reg .pred P;\nsetp.ne.b32 P, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, P;\n}\n"
+            ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 
 // Instruction descriptor for a dense, K-major x K-major MMA of shape M x N (x 32 bytes of K).
@@ -386,18 +394,11 @@ __device__ __forceinline__ void tmem_ld_32x4(uint32_t taddr, uint32_t (&r)[4]) {
                  : "r"(taddr)
                  : "memory");
 }
-// Thread i of the warp writes columns [col, col+32) of row (lane base + i).
-__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-          "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-          "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-          "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-          "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
+// Thread i of the warp writes columns [col, col+8) of row (lane base + i).
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, uint4 lo, uint4 hi) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

@@ -404,3 +404,29 @@ def test_wide_l2_configuration_matches_the_narrow_one(flib):
         he, ce, _ = _run_oracle_layer(layer, x, xs, False)
         d = np.abs(res[1][0].cpu().numpy().astype(np.int32) - he.astype(np.int32))
         assert d.max() <= 1 and (d != 0).mean() < 5e-3
+
+
+@pytest.mark.parametrize("H,B", [(768, 1), (768, 45), (768, 352), (768, 353), (768, 704), (768, 705), (768, 1056), (768, 1057),
+                                 (256, 300), (384, 47), (384, 700), (512, 1600), (640, 90), (896, 500), (1024, 33), (1024, 481)])
+def test_small_cluster_form_gives_the_bytes_of_the_l2_form(flib, H, B):
+    """The default form (few chunk rows per cluster, operands swapped) against the L2-exchange form,
+    which shares none of its data movement: same arithmetic in the same order, so equal bytes from a
+    non-zero state. Batches around the row counts where the kernel's column count (16, 32, 48) or the
+    number of waves changes on a B200, one row, ragged last clusters, an odd number of CTAs
+    (H = 384, 640, 896), one pair (256) and the largest cluster (1024)."""
+    T, R = 4, 128
+    layer, x, xs = _layer_case(T, B, H, R, H + B, B % 2 == 1)
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, h = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale,
+                                         layer.w_up, layer.bias, c, h, reverse=layer.reverse)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, h))
+    flib.fluke_set_lstm_persistent(1)
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
