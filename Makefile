@@ -50,7 +50,11 @@ SM100_DEPS = $(wildcard fluke_b200/csrc/*.cu fluke_b200/csrc/*.cuh fluke_b200/cs
 PROBELIB = $(BUILD_DIR)/libfluke_probe.so
 WAITPROBELIB = $(BUILD_DIR)/libfluke_waitprobe.so
 
-.PHONY: all shared probe waitprobe clean distclean
+# Python extension of fluke_b200.ops (argument checks, output allocation and the call in one step)
+NATIVEEXT = fluke_b200/_native.so
+PYTHON ?= python3
+
+.PHONY: all shared probe waitprobe pyext clean distclean
 
 all: $(STATICLIB)
 shared: $(SHAREDLIB)
@@ -65,6 +69,15 @@ $(WAITPROBELIB): tests/csrc/wait_probe.cu $(SM100_DEPS) | $(BUILD_DIR)
 
 $(PROBELIB): fluke_b200/csrc/mma_peak_sm100.cu $(SM100_DEPS) | $(BUILD_DIR)
 	$(NVCC) $(CUDA_CFLAGS) $(CPPFLAGS) -shared fluke_b200/csrc/mma_peak_sm100.cu -o $@ $(CUDA_LDFLAGS)
+
+pyext: $(NATIVEEXT)
+
+$(NATIVEEXT): fluke_b200/csrc/native_ops.cpp include/fluke/fluke.h
+	T=`$(PYTHON) -c "import os, torch; print(os.path.dirname(torch.__file__))"` && \
+	P=`$(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])"` && \
+	$(CXX) -O2 -g0 -std=c++17 -fPIC -shared -fvisibility=hidden -Wall -DHAVE_CUDA=1 -I include -I $$P -I $$T/include \
+	    -I $$T/include/torch/csrc/api/include -I $(CUDA_INC) $< -o $@ \
+	    -L$$T/lib -lc10 -lc10_cuda -ltorch_cpu -ltorch_cuda -ltorch -ltorch_python
 
 $(STATICLIB): $(OBJ) $(GPU_OBJ)
 	rm -f $@

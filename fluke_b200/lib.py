@@ -7,6 +7,7 @@ There is no fallback: if the library cannot be built or loaded, `load()` raises.
 import ctypes
 import os
 import subprocess
+import sys
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SO_PATH = os.path.join(ROOT, "lib", "libfluke.so")
@@ -108,9 +109,10 @@ PROBE_PATH = os.path.join(ROOT, "lib", "libfluke_probe.so")
 
 
 def build(verbose=False):
-    """`make shared probe waitprobe cuda=1` at the repository root (nvcc cross-compiles sm_100a
-    without a GPU): the library, the benchmark's issue-rate probe and the tests' wait probe."""
-    cmd = ["make", "shared", "probe", "waitprobe", "cuda=1"]
+    """`make shared probe waitprobe pyext cuda=1` at the repository root (nvcc cross-compiles sm_100a
+    without a GPU): the library, the benchmark's issue-rate probe, the tests' wait probe and the
+    extension module of fluke_b200.ops (for this interpreter)."""
+    cmd = ["make", "shared", "probe", "waitprobe", "pyext", "cuda=1", "PYTHON=" + sys.executable]
     res = subprocess.run(cmd, cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or res.returncode != 0:
         print(res.stdout)
@@ -136,6 +138,24 @@ def load(rebuild=False):
         fn.argtypes = argtypes
     _LIB = lib
     return lib
+
+
+NATIVE_PATH = os.path.join(ROOT, "fluke_b200", "_native.so")
+_NATIVE = None
+
+
+def native():
+    """The extension module behind fluke_b200.ops, bound to the library that load() returns."""
+    global _NATIVE
+    if _NATIVE is None:
+        lib = load()
+        if not os.path.isfile(NATIVE_PATH):
+            build()
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        from . import _native
+        _native.bind({n: ctypes.cast(getattr(lib, n), P).value for n in _native.names()})
+        _NATIVE = _native
+    return _NATIVE
 
 
 _PROBE = None
