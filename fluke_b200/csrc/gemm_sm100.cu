@@ -192,6 +192,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     const int m_first = blockIdx.x / p.num_n_tiles;
     const int n0 = n_tile * BN_OUT;
 
+    dependency_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full_bar[s], 1);
@@ -214,6 +215,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    dependency_wait();
     // The launch gives every thread 65536 / 384 registers; the loader and issuer need few, the
     // epilogue threads hold a whole row segment plus rotary tables: each role branch below
     // starts by resizing its warpgroup's share.
@@ -328,7 +330,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int row = m0 + q * 32 + g8 + 8 * k;
-                sa[k] = p.scale_a ? (row < p.M ? __ldg(p.scale_a + row) : 0.f) : p.const_scale_a;
+                sa[k] = p.scale_a ? (row < p.M ? p.scale_a[row] : 0.f) : p.const_scale_a;
             }
         };
 
@@ -387,13 +389,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             for (int h2 = 0; h2 < 2; ++h2)
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    sc[h2][j] = __ldg(reinterpret_cast<const float2 *>(p.scale_b + n0 + (2 * ch + h2) * 64 + 8 * j + 2 * t4));
+                    sc[h2][j] = *reinterpret_cast<const float2 *>(p.scale_b + n0 + (2 * ch + h2) * 64 + 8 * j + 2 * t4);
             float2 sn2[4][4], cs2[4][4];  // [row k][pair group j]
             auto load_tables = [&](int k, int pos) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    sn2[k][j] = __ldg(reinterpret_cast<const float2 *>(p.sin_tab + pos * 32 + 8 * j + 2 * t4));
-                    cs2[k][j] = __ldg(reinterpret_cast<const float2 *>(p.cos_tab + pos * 32 + 8 * j + 2 * t4));
+                    sn2[k][j] = *reinterpret_cast<const float2 *>(p.sin_tab + pos * 32 + 8 * j + 2 * t4);
+                    cs2[k][j] = *reinterpret_cast<const float2 *>(p.cos_tab + pos * 32 + 8 * j + 2 * t4);
                 }
             };
             // stmatrix: lane i gives the address of row i % 8 of matrix i / 8
@@ -505,11 +507,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int col = n0 + c0 + 8 * j + 2 * t4;
-                sc[j] = cols_ok ? __ldg(reinterpret_cast<const float2 *>(p.scale_b + col)) : make_float2(0.f, 0.f);
+                sc[j] = cols_ok ? *reinterpret_cast<const float2 *>(p.scale_b + col) : make_float2(0.f, 0.f);
                 if constexpr (kDual) {
                     // the epilogue works on gate/2: halving the scale is exact
                     sc[j] = make_float2(0.5f * sc[j].x, 0.5f * sc[j].y);
-                    sc_up[j] = cols_ok ? __ldg(reinterpret_cast<const float2 *>(p.scale_b2 + col)) : make_float2(0.f, 0.f);
+                    sc_up[j] = cols_ok ? *reinterpret_cast<const float2 *>(p.scale_b2 + col) : make_float2(0.f, 0.f);
                 }
             }
             float sa_next[4];
@@ -712,9 +714,8 @@ int plan_launch(const GemmPlan &plan, int a_plane, cudaStream_t stream) {
     if (plan.grid == 0) return 0;
     GemmDev p = plan.p;
     p.a_plane = a_plane;
-    kernel<<<plan.grid, kNumThreads, L::kDynamic, stream>>>(plan.tm_a, plan.tm_b, plan.tm_b2,
-                                                            plan.tm_out, p);
-    return (int)cudaGetLastError();
+    return launch_dependent(kernel, plan.grid, kNumThreads, L::kDynamic, stream, plan.tm_a, plan.tm_b, plan.tm_b2,
+                            plan.tm_out, p);
 }
 
 template <int KIND, int EPI, int BN_MMA, int STAGES>

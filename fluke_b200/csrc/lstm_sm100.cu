@@ -84,6 +84,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
     const int m0 = blockIdx.x * 128;
     const int n0 = blockIdx.y * UNITS;
 
+    dependency_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kLstmMaxKB; ++s) mbar_init(&full_bar[s], 1);
         mbar_init(tfull_bar, 1);
@@ -95,6 +96,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    dependency_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -154,10 +156,10 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
                     uint32_t hq[4];
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
-                        const float4 bi = __ldg(reinterpret_cast<const float4 *>(p.bias[0] + n0 + u0) + v);
-                        const float4 bf = __ldg(reinterpret_cast<const float4 *>(p.bias[1] + n0 + u0) + v);
-                        const float4 bg = __ldg(reinterpret_cast<const float4 *>(p.bias[2] + n0 + u0) + v);
-                        const float4 bo = __ldg(reinterpret_cast<const float4 *>(p.bias[3] + n0 + u0) + v);
+                        const float4 bi = reinterpret_cast<const float4 *>(p.bias[0] + n0 + u0)[v];
+                        const float4 bf = reinterpret_cast<const float4 *>(p.bias[1] + n0 + u0)[v];
+                        const float4 bg = reinterpret_cast<const float4 *>(p.bias[2] + n0 + u0)[v];
+                        const float4 bo = reinterpret_cast<const float4 *>(p.bias[3] + n0 + u0)[v];
                         const float bis[4] = {bi.x, bi.y, bi.z, bi.w}, bfs[4] = {bf.x, bf.y, bf.z, bf.w};
                         const float bgs[4] = {bg.x, bg.y, bg.z, bg.w}, bos[4] = {bo.x, bo.y, bo.z, bo.w};
                         uint32_t packed = 0;
@@ -264,9 +266,8 @@ int lstm_launch_units(const LstmPlan &plan, const LstmDev &p, cudaStream_t strea
         if (e != cudaSuccess) return (int)e;
         done[dev] = true;
     }
-    kernel<<<plan.grid, kLstmThreads, LstmSmem<UNITS>::kDynamic, stream>>>(
-        plan.tm_a_lo, plan.tm_a_hi, plan.tm_w[0], plan.tm_w[1], plan.tm_w[2], plan.tm_w[3], p);
-    return (int)cudaGetLastError();
+    return launch_dependent(kernel, plan.grid, kLstmThreads, LstmSmem<UNITS>::kDynamic, stream, plan.tm_a_lo, plan.tm_a_hi,
+                            plan.tm_w[0], plan.tm_w[1], plan.tm_w[2], plan.tm_w[3], p);
 }
 
 int lstm_plan_launch(const LstmPlan &plan, int plane_lo, int plane_hi, int8_t *h_out,

@@ -17,6 +17,7 @@
 // Other reductions of the path are maxima, which do not depend on order.
 #include "fluke_sm100.h"
 #include "sm100_ptx.cuh"
+#include "tma_host.cuh"
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -228,9 +229,11 @@ enum { kOutF16 = 0, kOutI8 = 1, kOutF8 = 2 };
 constexpr int kNormWarps = 4;
 template <int L, int MODE>
 __global__ void __launch_bounds__(kNormWarps * 32, (L <= 2 ? 16 : 1))
-rmsnorm_rows_kernel(const __half *__restrict__ in, const void *residual_in,
-                    const __half *__restrict__ weight, void *out, float *res_scale, int n_tokens,
+rmsnorm_rows_kernel(const __half * in, const void *residual_in,
+                    const __half * weight, void *out, float *res_scale, int n_tokens,
                     int hidden_dim, float alpha, float eps) {
+    dependency_trigger();
+    dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
     if (row >= n_tokens) return;
@@ -245,10 +248,10 @@ rmsnorm_rows_kernel(const __half *__restrict__ in, const void *residual_in,
     for (int q = 0; q < L; ++q) {
         const int off = (q * 32 + lane) * 8;
         float2 xf[4];
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(in + base + off)), xf);
+        unpack8(*(reinterpret_cast<const uint4 *>(in + base + off)), xf);
         if constexpr (MODE == kOutF16) {
             float2 rf[4];
-            unpack8(__ldg(reinterpret_cast<const uint4 *>(
+            unpack8(*(reinterpret_cast<const uint4 *>(
                         static_cast<const __half *>(residual_in) + base + off)), rf);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -289,7 +292,7 @@ rmsnorm_rows_kernel(const __half *__restrict__ in, const void *residual_in,
     for (int q = 0; q < L; ++q) {
         const int off = (q * 32 + lane) * 8;
         float2 wf[4];
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(weight + off)), wf);
+        unpack8(*(reinterpret_cast<const uint4 *>(weight + off)), wf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             val[q][k] = mul2(mul2(val[q][k], make_float2(rms_inv, rms_inv)), wf[k]);
@@ -377,10 +380,12 @@ __device__ __forceinline__ float block_max(float v, float *buf) {
 }
 
 template <int MODE>
-__global__ void rmsnorm_generic_kernel(const __half *__restrict__ in, const void *residual_in,
-                                       const __half *__restrict__ weight, void *out,
+__global__ void rmsnorm_generic_kernel(const __half * in, const void *residual_in,
+                                       const __half * weight, void *out,
                                        float *res_scale, int n_tokens, int hidden_dim, float alpha,
                                        float eps) {
+    dependency_trigger();
+    dependency_wait();
     __shared__ float buf[32];
     const int64_t row = blockIdx.x;
     const int t = threadIdx.x;
@@ -440,6 +445,7 @@ int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, 
                    float *res_scale, int n_tokens, int hidden_dim, float alpha, float eps,
                    cudaStream_t s) {
     if (n_tokens <= 0) return 0;
+    int rc;
     const __half *x = static_cast<const __half *>(in), *w = static_cast<const __half *>(weight);
     const bool aligned =
         ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weight) |
@@ -448,16 +454,16 @@ int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, 
         const int grid = (n_tokens + kNormWarps - 1) / kNormWarps;
         const int block = kNormWarps * 32;
         switch (hidden_dim / 256) {
-            case 1: rmsnorm_rows_kernel<1, MODE><<<grid, block, 0, s>>>(x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
-            case 2: rmsnorm_rows_kernel<2, MODE><<<grid, block, 0, s>>>(x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
-            case 3: rmsnorm_rows_kernel<3, MODE><<<grid, block, 0, s>>>(x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
-            default: rmsnorm_rows_kernel<4, MODE><<<grid, block, 0, s>>>(x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
+            case 1: rc = launch_dependent(rmsnorm_rows_kernel<1, MODE>, grid, block, 0, s, x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
+            case 2: rc = launch_dependent(rmsnorm_rows_kernel<2, MODE>, grid, block, 0, s, x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
+            case 3: rc = launch_dependent(rmsnorm_rows_kernel<3, MODE>, grid, block, 0, s, x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
+            default: rc = launch_dependent(rmsnorm_rows_kernel<4, MODE>, grid, block, 0, s, x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps); break;
         }
     } else {
         const int block = ((hidden_dim / 2 + 31) / 32) * 32;
-        rmsnorm_generic_kernel<MODE><<<n_tokens, block, 0, s>>>(x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps);
+        rc = launch_dependent(rmsnorm_generic_kernel<MODE>, n_tokens, block, 0, s, x, residual_in, w, out, res_scale, n_tokens, hidden_dim, alpha, eps);
     }
-    return (int)cudaGetLastError();
+    return rc;
 }
 
 // ---- per-token quantisers (nn_kernel_cuda.h:352-411), hidden_dim = 256*L: one warp per row, the
@@ -467,8 +473,10 @@ int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, 
 // the conversion instruction. CTA shape as for the RMSNorm kernels.
 template <int L, bool FP8>
 __global__ void __launch_bounds__(kNormWarps * 32, (L <= 2 ? 16 : 1))
-quant_rows_reg_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
-                      float *__restrict__ scale, int n_tokens) {
+quant_rows_reg_kernel(const __half * in, uint8_t * out,
+                      float * scale, int n_tokens) {
+    dependency_trigger();
+    dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
     if (row >= n_tokens) return;
@@ -477,7 +485,7 @@ quant_rows_reg_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
     float amax = 0.f;
 #pragma unroll
     for (int q = 0; q < L; ++q) {
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(in + base + (q * 32 + lane) * 8)), val[q]);
+        unpack8(*(reinterpret_cast<const uint4 *>(in + base + (q * 32 + lane) * 8)), val[q]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) amax = fmaxf(amax, fmaxf(fabsf(val[q][k].x), fabsf(val[q][k].y)));
     }
@@ -518,8 +526,10 @@ quant_rows_reg_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
 // The second pass re-reads the row (at most 4 KB, still in L1).
 template <bool FP8>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-quant_rows_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
-                  float *__restrict__ scale, int n_tokens, int hidden_dim, int vec_ok) {
+quant_rows_kernel(const __half * in, uint8_t * out,
+                  float * scale, int n_tokens, int hidden_dim, int vec_ok) {
+    dependency_trigger();
+    dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
     if (row >= n_tokens) return;
@@ -530,7 +540,7 @@ quant_rows_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
     if (vec_ok) {
         for (int c = lane; c < (hidden_dim >> 3); c += 32) {
             float2 f[4];
-            unpack8(__ldg(reinterpret_cast<const uint4 *>(x) + c), f);
+            unpack8(*(reinterpret_cast<const uint4 *>(x) + c), f);
 #pragma unroll
             for (int k = 0; k < 4; ++k) amax = fmaxf(amax, fmaxf(fabsf(f[k].x), fabsf(f[k].y)));
         }
@@ -552,7 +562,7 @@ quant_rows_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
     if (vec_ok) {
         for (int c = lane; c < (hidden_dim >> 3); c += 32) {
             float2 f[4];
-            unpack8(__ldg(reinterpret_cast<const uint4 *>(x) + c), f);
+            unpack8(*(reinterpret_cast<const uint4 *>(x) + c), f);
             uint2 raw;
             uint8_t *ob = reinterpret_cast<uint8_t *>(&raw);
 #pragma unroll
@@ -580,9 +590,11 @@ quant_rows_kernel(const __half *__restrict__ in, uint8_t *__restrict__ out,
 // more instructions than the rotation itself.
 template <bool SHIFTS>
 __global__ void __launch_bounds__(256)
-rotary_vec_kernel(__half *x, const float *__restrict__ sin_tab, const float *__restrict__ cos_tab,
+rotary_vec_kernel(__half *x, const float * sin_tab, const float * cos_tab,
                   int64_t total, int seq_len, int n_heads, int width, int64_t stride_batch,
                   int64_t stride_seq, int64_t stride_head, int cpw_log2, int heads_log2) {
+    dependency_trigger();
+    dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     int c, h, s;
@@ -611,7 +623,7 @@ rotary_vec_kernel(__half *x, const float *__restrict__ sin_tab, const float *__r
     unpack8(*reinterpret_cast<const uint4 *>(p1), bq);
     const float4 *cs4 = reinterpret_cast<const float4 *>(cos_tab + int64_t(s) * width + c * 8);
     const float4 *sn4 = reinterpret_cast<const float4 *>(sin_tab + int64_t(s) * width + c * 8);
-    const float4 c0 = __ldg(cs4), c1 = __ldg(cs4 + 1), s0 = __ldg(sn4), s1 = __ldg(sn4 + 1);
+    const float4 c0 = cs4[0], c1 = cs4[1], s0 = sn4[0], s1 = sn4[1];
     const float cosv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
     const float sinv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
     float2 o0[4], o1[4];
@@ -635,9 +647,11 @@ rotary_vec_kernel(__half *x, const float *__restrict__ sin_tab, const float *__r
 
 // Scalar path for widths or strides that are not multiples of 8 elements.
 __global__ void __launch_bounds__(256)
-rotary_scalar_kernel(__half *x, const float *__restrict__ sin_tab,
-                     const float *__restrict__ cos_tab, int64_t total, int seq_len, int n_heads,
+rotary_scalar_kernel(__half *x, const float * sin_tab,
+                     const float * cos_tab, int64_t total, int seq_len, int n_heads,
                      int width, int64_t stride_batch, int64_t stride_seq, int64_t stride_head) {
+    dependency_trigger();
+    dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int rot = int(idx % width);
@@ -669,8 +683,10 @@ __device__ __forceinline__ void split_index(int64_t idx, int64_t total, int per_
 // ---- SiLU-multiply (nn_kernel_cuda.h:71-90) -----------------------------------------------------
 template <int VEC>
 __global__ void __launch_bounds__(256)
-silu_mul_kernel(const __half *__restrict__ in, __half *__restrict__ out, int64_t total_vec,
+silu_mul_kernel(const __half * in, __half * out, int64_t total_vec,
                 int hidden_dim) {
+    dependency_trigger();
+    dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
     const int per_row = hidden_dim / VEC;
@@ -683,8 +699,8 @@ silu_mul_kernel(const __half *__restrict__ in, __half *__restrict__ out, int64_t
     __half *o = out + t * hidden_dim + k;
     if constexpr (VEC == 8) {
         float2 yf[4], gf[4], of[4];
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(y)), yf);
-        unpack8(__ldg(reinterpret_cast<const uint4 *>(g)), gf);
+        unpack8(*(reinterpret_cast<const uint4 *>(y)), yf);
+        unpack8(*(reinterpret_cast<const uint4 *>(g)), gf);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             of[j].x = (gf[j].x / (1.0f + __expf(-gf[j].x))) * yf[j].x;
@@ -713,8 +729,10 @@ __device__ __forceinline__ void flstm_gate(float gi, float gf, float gg, float g
 
 template <int VEC>
 __global__ void __launch_bounds__(256)
-flstm_step_kernel(const __half *__restrict__ scratch, const __half *__restrict__ ih_t,
-                  __half *cell, __half *__restrict__ hh_next, int64_t total_vec, int hidden_dim) {
+flstm_step_kernel(const __half * scratch, const __half * ih_t,
+                  __half *cell, __half * hh_next, int64_t total_vec, int hidden_dim) {
+    dependency_trigger();
+    dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
     const int per_row = hidden_dim / VEC;
@@ -727,8 +745,8 @@ flstm_step_kernel(const __half *__restrict__ scratch, const __half *__restrict__
         float2 a[4][4], b[4][4], cf[4], cn[4], hn[4];
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-            unpack8(__ldg(reinterpret_cast<const uint4 *>(scratch + gbase + g * hidden_dim)), a[g]);
-            unpack8(__ldg(reinterpret_cast<const uint4 *>(ih_t + gbase + g * hidden_dim)), b[g]);
+            unpack8(*(reinterpret_cast<const uint4 *>(scratch + gbase + g * hidden_dim)), a[g]);
+            unpack8(*(reinterpret_cast<const uint4 *>(ih_t + gbase + g * hidden_dim)), b[g]);
         }
         unpack8(*reinterpret_cast<const uint4 *>(cell + cbase), cf);
 #pragma unroll
@@ -755,9 +773,11 @@ flstm_step_kernel(const __half *__restrict__ scratch, const __half *__restrict__
 // ---- dequantise + transpose [T,N,C] -> [N,T,C] (nn_kernel_cuda.h:416-443) ---------------------
 template <bool FP8, int VEC>
 __global__ void __launch_bounds__(256)
-dequant_transpose_kernel(const uint8_t *__restrict__ in, __half *__restrict__ out,
+dequant_transpose_kernel(const uint8_t * in, __half * out,
                          int64_t total_vec, int n_timesteps, int batch_size, int n_channels,
                          float scale) {
+    dependency_trigger();
+    dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
     const int per_row = n_channels / VEC;
@@ -773,7 +793,7 @@ dequant_transpose_kernel(const uint8_t *__restrict__ in, __half *__restrict__ ou
         else return (float)(int8_t)b * scale;
     };
     if constexpr (VEC == 16) {
-        const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(src));
+        const uint4 raw = *reinterpret_cast<const uint4 *>(src);
         const uint8_t *rb = reinterpret_cast<const uint8_t *>(&raw);
         float2 f0[4], f1[4];
         if constexpr (FP8) {
@@ -844,6 +864,7 @@ extern "C" int fluke_sm100_rmsnorm_quant_fp8(const void *in, const void *weight,
 static int launch_quant(const void *in, void *out, void *scale, int n_tokens, int hidden_dim,
                         bool fp8, cudaStream_t s) {
     if (n_tokens <= 0) return 0;
+    int rc;
     const int vec_ok = (hidden_dim % 8 == 0) &&
                        ((reinterpret_cast<uintptr_t>(in) & 15u) == 0) &&
                        ((reinterpret_cast<uintptr_t>(out) & 7u) == 0);
@@ -853,27 +874,25 @@ static int launch_quant(const void *in, void *out, void *scale, int n_tokens, in
         float *sc = static_cast<float *>(scale);
         const int grid = (n_tokens + kNormWarps - 1) / kNormWarps, block = kNormWarps * 32;
         switch ((hidden_dim / 256) * 2 + (fp8 ? 1 : 0)) {
-            case 2: quant_rows_reg_kernel<1, false><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            case 3: quant_rows_reg_kernel<1, true><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            case 4: quant_rows_reg_kernel<2, false><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            case 5: quant_rows_reg_kernel<2, true><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            case 6: quant_rows_reg_kernel<3, false><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            case 7: quant_rows_reg_kernel<3, true><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            case 8: quant_rows_reg_kernel<4, false><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
-            default: quant_rows_reg_kernel<4, true><<<grid, block, 0, s>>>(x, o, sc, n_tokens); break;
+            case 2: rc = launch_dependent(quant_rows_reg_kernel<1, false>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            case 3: rc = launch_dependent(quant_rows_reg_kernel<1, true>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            case 4: rc = launch_dependent(quant_rows_reg_kernel<2, false>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            case 5: rc = launch_dependent(quant_rows_reg_kernel<2, true>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            case 6: rc = launch_dependent(quant_rows_reg_kernel<3, false>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            case 7: rc = launch_dependent(quant_rows_reg_kernel<3, true>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            case 8: rc = launch_dependent(quant_rows_reg_kernel<4, false>, grid, block, 0, s, x, o, sc, n_tokens); break;
+            default: rc = launch_dependent(quant_rows_reg_kernel<4, true>, grid, block, 0, s, x, o, sc, n_tokens); break;
         }
-        return (int)cudaGetLastError();
+        return rc;
     }
     const int grid = (n_tokens + kWarpsPerBlock - 1) / kWarpsPerBlock;
     if (fp8)
-        quant_rows_kernel<true><<<grid, kWarpsPerBlock * 32, 0, s>>>(
-            static_cast<const __half *>(in), static_cast<uint8_t *>(out), static_cast<float *>(scale),
+        rc = launch_dependent(quant_rows_kernel<true>, grid, kWarpsPerBlock * 32, 0, s, static_cast<const __half *>(in), static_cast<uint8_t *>(out), static_cast<float *>(scale),
             n_tokens, hidden_dim, vec_ok);
     else
-        quant_rows_kernel<false><<<grid, kWarpsPerBlock * 32, 0, s>>>(
-            static_cast<const __half *>(in), static_cast<uint8_t *>(out), static_cast<float *>(scale),
+        rc = launch_dependent(quant_rows_kernel<false>, grid, kWarpsPerBlock * 32, 0, s, static_cast<const __half *>(in), static_cast<uint8_t *>(out), static_cast<float *>(scale),
             n_tokens, hidden_dim, vec_ok);
-    return (int)cudaGetLastError();
+    return rc;
 }
 
 extern "C" int fluke_sm100_quant_int8(const void *in, void *out, void *scale, int n_tokens,
@@ -891,20 +910,21 @@ extern "C" int fluke_sm100_dequant_transpose(const void *in, void *out, int n_ti
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t rows = int64_t(n_timesteps) * batch_size;
     if (rows <= 0 || n_channels <= 0) return 0;
+    int rc;
     const bool vec = (n_channels % 16 == 0) &&
                      (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0);
     const uint8_t *src = static_cast<const uint8_t *>(in);
     __half *dst = static_cast<__half *>(out);
     if (vec) {
         const int64_t total = rows * (n_channels / 16);
-        if (is_fp8) dequant_transpose_kernel<true, 16><<<grid_for(total, 256), 256, 0, s>>>(src, dst, total, n_timesteps, batch_size, n_channels, scale);
-        else dequant_transpose_kernel<false, 16><<<grid_for(total, 256), 256, 0, s>>>(src, dst, total, n_timesteps, batch_size, n_channels, scale);
+        if (is_fp8) rc = launch_dependent(dequant_transpose_kernel<true, 16>, grid_for(total, 256), 256, 0, s, src, dst, total, n_timesteps, batch_size, n_channels, scale);
+        else rc = launch_dependent(dequant_transpose_kernel<false, 16>, grid_for(total, 256), 256, 0, s, src, dst, total, n_timesteps, batch_size, n_channels, scale);
     } else {
         const int64_t total = rows * n_channels;
-        if (is_fp8) dequant_transpose_kernel<true, 1><<<grid_for(total, 256), 256, 0, s>>>(src, dst, total, n_timesteps, batch_size, n_channels, scale);
-        else dequant_transpose_kernel<false, 1><<<grid_for(total, 256), 256, 0, s>>>(src, dst, total, n_timesteps, batch_size, n_channels, scale);
+        if (is_fp8) rc = launch_dependent(dequant_transpose_kernel<true, 1>, grid_for(total, 256), 256, 0, s, src, dst, total, n_timesteps, batch_size, n_channels, scale);
+        else rc = launch_dependent(dequant_transpose_kernel<false, 1>, grid_for(total, 256), 256, 0, s, src, dst, total, n_timesteps, batch_size, n_channels, scale);
     }
-    return (int)cudaGetLastError();
+    return rc;
 }
 
 extern "C" int fluke_sm100_rotary_emb(void *x, const void *sin_tab, const void *cos_tab,
@@ -915,6 +935,7 @@ extern "C" int fluke_sm100_rotary_emb(void *x, const void *sin_tab, const void *
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int W = sincos_width;
     if (batch_size <= 0 || seq_len <= 0 || n_heads <= 0 || W <= 0) return 0;
+    int rc;
     const bool vec = (W % 8 == 0) && (stride_batch % 8 == 0) && (stride_seq % 8 == 0) &&
                      (stride_head % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) &&
                      (((reinterpret_cast<uintptr_t>(sin_tab) | reinterpret_cast<uintptr_t>(cos_tab)) & 15u) == 0);
@@ -924,57 +945,56 @@ extern "C" int fluke_sm100_rotary_emb(void *x, const void *sin_tab, const void *
         auto log2_of = [](int v) { int l = 0; while ((1 << l) < v) ++l; return (1 << l) == v ? l : -1; };
         const int cl = log2_of(cpw), hl = log2_of(n_heads);
         if (cl >= 0 && hl >= 0 && total < (int64_t(1) << 31)) {
-            rotary_vec_kernel<true><<<grid_for(total, 256), 256, 0, s>>>(
-                static_cast<__half *>(x), static_cast<const float *>(sin_tab),
+            rc = launch_dependent(rotary_vec_kernel<true>, grid_for(total, 256), 256, 0, s, static_cast<__half *>(x), static_cast<const float *>(sin_tab),
                 static_cast<const float *>(cos_tab), total, seq_len, n_heads, W, stride_batch,
                 stride_seq, stride_head, cl, hl);
         } else {
-            rotary_vec_kernel<false><<<grid_for(total, 256), 256, 0, s>>>(
-                static_cast<__half *>(x), static_cast<const float *>(sin_tab),
+            rc = launch_dependent(rotary_vec_kernel<false>, grid_for(total, 256), 256, 0, s, static_cast<__half *>(x), static_cast<const float *>(sin_tab),
                 static_cast<const float *>(cos_tab), total, seq_len, n_heads, W, stride_batch,
                 stride_seq, stride_head, 0, 0);
         }
     } else {
         const int64_t total = int64_t(batch_size) * seq_len * n_heads * W;
-        rotary_scalar_kernel<<<grid_for(total, 256), 256, 0, s>>>(
-            static_cast<__half *>(x), static_cast<const float *>(sin_tab),
+        rc = launch_dependent(rotary_scalar_kernel, grid_for(total, 256), 256, 0, s, static_cast<__half *>(x), static_cast<const float *>(sin_tab),
             static_cast<const float *>(cos_tab), total, seq_len, n_heads, W, stride_batch,
             stride_seq, stride_head);
     }
-    return (int)cudaGetLastError();
+    return rc;
 }
 
 extern "C" int fluke_sm100_silu_mul(const void *in, void *out, int n_tokens, int hidden_dim,
                                     void *stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (n_tokens <= 0 || hidden_dim <= 0) return 0;
+    int rc;
     const bool vec = (hidden_dim % 8 == 0) &&
                      (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0);
     if (vec) {
         const int64_t total = int64_t(n_tokens) * (hidden_dim / 8);
-        silu_mul_kernel<8><<<grid_for(total, 256), 256, 0, s>>>(static_cast<const __half *>(in), static_cast<__half *>(out), total, hidden_dim);
+        rc = launch_dependent(silu_mul_kernel<8>, grid_for(total, 256), 256, 0, s, static_cast<const __half *>(in), static_cast<__half *>(out), total, hidden_dim);
     } else {
         const int64_t total = int64_t(n_tokens) * hidden_dim;
-        silu_mul_kernel<1><<<grid_for(total, 256), 256, 0, s>>>(static_cast<const __half *>(in), static_cast<__half *>(out), total, hidden_dim);
+        rc = launch_dependent(silu_mul_kernel<1>, grid_for(total, 256), 256, 0, s, static_cast<const __half *>(in), static_cast<__half *>(out), total, hidden_dim);
     }
-    return (int)cudaGetLastError();
+    return rc;
 }
 
 extern "C" int fluke_sm100_flstm_step(const void *scratch, const void *ih_t, void *cell,
                                       void *hh_next, int batch_size, int hidden_dim, void *stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (batch_size <= 0 || hidden_dim <= 0) return 0;
+    int rc;
     const bool vec = (hidden_dim % 8 == 0) &&
                      (((reinterpret_cast<uintptr_t>(scratch) | reinterpret_cast<uintptr_t>(ih_t) |
                         reinterpret_cast<uintptr_t>(cell) | reinterpret_cast<uintptr_t>(hh_next)) & 15u) == 0);
     if (vec) {
         const int64_t total = int64_t(batch_size) * (hidden_dim / 8);
-        flstm_step_kernel<8><<<grid_for(total, 256), 256, 0, s>>>(static_cast<const __half *>(scratch), static_cast<const __half *>(ih_t), static_cast<__half *>(cell), static_cast<__half *>(hh_next), total, hidden_dim);
+        rc = launch_dependent(flstm_step_kernel<8>, grid_for(total, 256), 256, 0, s, static_cast<const __half *>(scratch), static_cast<const __half *>(ih_t), static_cast<__half *>(cell), static_cast<__half *>(hh_next), total, hidden_dim);
     } else {
         const int64_t total = int64_t(batch_size) * hidden_dim;
-        flstm_step_kernel<1><<<grid_for(total, 256), 256, 0, s>>>(static_cast<const __half *>(scratch), static_cast<const __half *>(ih_t), static_cast<__half *>(cell), static_cast<__half *>(hh_next), total, hidden_dim);
+        rc = launch_dependent(flstm_step_kernel<1>, grid_for(total, 256), 256, 0, s, static_cast<const __half *>(scratch), static_cast<const __half *>(ih_t), static_cast<__half *>(cell), static_cast<__half *>(hh_next), total, hidden_dim);
     }
-    return (int)cudaGetLastError();
+    return rc;
 }
 
 extern "C" int fluke_sm100_fp8_unshuffle(void *dst_nk, const void *src, int N, int K, void *stream) {

@@ -74,6 +74,23 @@ __device__ __forceinline__ void fence_barrier_init() {
 }
 
 // ---------------------------------------------------------------------------------------
+// Programmatic dependent launch (the kernels launched with launch_dependent() of tma_host.cuh)
+// ---------------------------------------------------------------------------------------
+// Lets the next kernel of the stream be set up on the device as soon as every block of this one has
+// started; what it does before its own dependency_wait() runs beside this kernel.
+__device__ __forceinline__ void dependency_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Returns when the kernels before this one in the stream have completed and their writes are
+// visible. Every block executes it before its first access to global memory (reads of weights
+// included: the kernel before may have written them), so that a kernel never completes before its
+// predecessors. Data that an earlier kernel may have written is read with ordinary loads, not through the
+// read-only path, whose contents are only coherent from kernel start to kernel start.
+__device__ __forceinline__ void dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t arrivals) {

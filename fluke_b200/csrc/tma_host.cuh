@@ -4,7 +4,9 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <new>
 #include <stdint.h>
+#include <string.h>
 
 namespace fluke_sm100 {
 
@@ -26,6 +28,67 @@ inline encode_tiled_fn get_encode_tiled() {
     return fn;
 }
 
+// cuTensorMapEncodeTiled with the options every map of the library shares (no interleave, unit
+// element strides, 256-byte L2 promotion, zero fill). An encoded map depends on nothing but these
+// arguments, so each host thread keeps the last kMapSlots of them: an encode takes the driver 0.5 us,
+// a GEMM call needs three or four, and a program that calls with the same buffers again finds them here.
+constexpr int kMapSlots = 64;
+struct TmapKey {
+    const void *base;
+    cuuint64_t dims[5], strides[4];
+    cuuint32_t box[5];
+    int rank, dt, swizzle;
+};
+inline int encode_tmap(CUtensorMap *m, const TmapKey &k) {
+    struct Slot { TmapKey key; CUtensorMap map; bool used; };
+    struct Table {
+        Slot *slots = nullptr;
+        ~Table() { delete[] slots; }
+    };
+    static thread_local Table table;
+    if (!table.slots) table.slots = new (std::nothrow) Slot[kMapSlots]();
+    uint64_t h = reinterpret_cast<uintptr_t>(k.base) >> 4;
+    h = (h ^ k.dims[0] ^ (k.dims[1] << 20) ^ (uint64_t(k.box[1]) << 44) ^ (uint64_t(k.box[0]) << 52)) * 0x9E3779B97F4A7C15ull;
+    static_assert(kMapSlots == 64, "six bits of the hash");
+    Slot *s = table.slots ? &table.slots[h >> 58] : nullptr;
+    if (s && s->used && memcmp(&s->key, &k, sizeof(k)) == 0) {
+        *m = s->map;
+        return 0;
+    }
+    encode_tiled_fn fn = get_encode_tiled();
+    if (!fn) return (int)cudaErrorNotSupported;
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = fn(m, static_cast<CUtensorMapDataType>(k.dt), (cuuint32_t)k.rank, const_cast<void *>(k.base), k.dims,
+                          k.strides, k.box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, static_cast<CUtensorMapSwizzle>(k.swizzle),
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
+    if (s) {
+        s->key = k;
+        s->map = *m;
+        s->used = true;
+    }
+    return 0;
+}
+
+// Launches a kernel that begins with dependency_trigger() / dependency_wait(): its launch and set-up
+// overlap the end of the kernel before it in the stream.
+template <typename... P, typename... A>
+int launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();  // returned here: it must not linger as the thread's last error
+    return (int)e;
+}
+
 // Row-major 2-D tensor [rows, cols] with `row_stride_bytes` between rows (multiple of 16),
 // copied in boxes of box_rows x box_cols elements; box_cols * elem_bytes must be 128 when the
 // 128-byte swizzle is used. Out-of-range parts of a box read as zero and are not written.
@@ -33,18 +96,15 @@ inline encode_tiled_fn get_encode_tiled() {
 inline int make_tmap_2d_sw(CUtensorMap *m, CUtensorMapDataType dt, const void *base, uint64_t rows,
                            uint64_t cols, uint64_t row_stride_bytes, uint32_t box_rows,
                            uint32_t box_cols, CUtensorMapSwizzle swizzle) {
-    encode_tiled_fn fn = get_encode_tiled();
-    if (!fn) return (int)cudaErrorNotSupported;
     if ((reinterpret_cast<uintptr_t>(base) & 15u) || (row_stride_bytes & 15u))
         return (int)cudaErrorMisalignedAddress;
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {row_stride_bytes};
-    cuuint32_t box[2] = {box_cols, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(m, dt, 2, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+    TmapKey k;
+    memset(&k, 0, sizeof(k));  // compared byte by byte
+    k.base = base; k.rank = 2; k.dt = dt; k.swizzle = swizzle;
+    k.dims[0] = cols; k.dims[1] = rows;
+    k.strides[0] = row_stride_bytes;
+    k.box[0] = box_cols; k.box[1] = box_rows;
+    return encode_tmap(m, k);
 }
 
 inline int make_tmap_2d(CUtensorMap *m, CUtensorMapDataType dt, uint32_t elem_bytes,
@@ -60,19 +120,16 @@ inline int make_tmap_3d_sw(CUtensorMap *m, CUtensorMapDataType dt, const void *b
                            uint64_t rows, uint64_t cols, uint64_t row_stride_bytes,
                            uint64_t plane_stride_bytes, uint32_t box_rows, uint32_t box_cols,
                            CUtensorMapSwizzle swizzle) {
-    encode_tiled_fn fn = get_encode_tiled();
-    if (!fn) return (int)cudaErrorNotSupported;
     if ((reinterpret_cast<uintptr_t>(base) & 15u) || (row_stride_bytes & 15u) ||
         (plane_stride_bytes & 15u))
         return (int)cudaErrorMisalignedAddress;
-    cuuint64_t dims[3] = {cols, rows, planes};
-    cuuint64_t strides[2] = {row_stride_bytes, plane_stride_bytes};
-    cuuint32_t box[3] = {box_cols, box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(m, dt, 3, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+    TmapKey k;
+    memset(&k, 0, sizeof(k));
+    k.base = base; k.rank = 3; k.dt = dt; k.swizzle = swizzle;
+    k.dims[0] = cols; k.dims[1] = rows; k.dims[2] = planes;
+    k.strides[0] = row_stride_bytes; k.strides[1] = plane_stride_bytes;
+    k.box[0] = box_cols; k.box[1] = box_rows; k.box[2] = 1;
+    return encode_tmap(m, k);
 }
 
 inline int make_tmap_3d(CUtensorMap *m, CUtensorMapDataType dt, const void *base, uint64_t planes,
@@ -91,21 +148,17 @@ inline int make_tmap_3d(CUtensorMap *m, CUtensorMapDataType dt, const void *base
 inline int make_tmap_nd(CUtensorMap *m, CUtensorMapDataType dt, const void *base, int rank,
                         const uint64_t *dims, const uint64_t *strides_bytes, const uint32_t *box,
                         CUtensorMapSwizzle swizzle) {
-    encode_tiled_fn fn = get_encode_tiled();
-    if (!fn) return (int)cudaErrorNotSupported;
     if (rank < 2 || rank > 5) return (int)cudaErrorInvalidValue;
     if (reinterpret_cast<uintptr_t>(base) & 15u) return (int)cudaErrorMisalignedAddress;
-    cuuint64_t d[5], st[4];
-    cuuint32_t b[5], estr[5];
-    for (int i = 0; i < rank; ++i) { d[i] = dims[i]; b[i] = box[i]; estr[i] = 1; }
+    TmapKey k;
+    memset(&k, 0, sizeof(k));
+    k.base = base; k.rank = rank; k.dt = dt; k.swizzle = swizzle;
+    for (int i = 0; i < rank; ++i) { k.dims[i] = dims[i]; k.box[i] = box[i]; }
     for (int i = 0; i + 1 < rank; ++i) {
         if (strides_bytes[i] & 15u) return (int)cudaErrorMisalignedAddress;
-        st[i] = strides_bytes[i];
+        k.strides[i] = strides_bytes[i];
     }
-    CUresult r = fn(m, dt, (cuuint32_t)rank, const_cast<void *>(base), d, st, b, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+    return encode_tmap(m, k);
 }
 
 }  // namespace fluke_sm100
