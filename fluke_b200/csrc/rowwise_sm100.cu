@@ -111,6 +111,12 @@ __device__ __forceinline__ float2 div_by_scale2(float2 x, float s, float r) {
                        __uint_as_float((__float_as_uint(q.y) & 0x7FFFFFFFu) | (__float_as_uint(x.y) & 0x80000000u)));
 }
 
+// ---- launching ----------------------------------------------------------------------------
+// Every kernel here is launched as a dependent of the one before it and starts with
+// dependency_wait(). None calls dependency_trigger(): with thousands of short-lived CTAs the next
+// kernel's first wave would only take slots from this one's last ([128000, 512] int8 quantiser: 33.8 us
+// with the call, 29.3 without).
+
 // ---- small helpers -----------------------------------------------------------------------
 __device__ __forceinline__ void unpack8(const uint4 &raw, float2 (&f)[4]) {
     const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
@@ -232,7 +238,6 @@ __global__ void __launch_bounds__(kNormWarps * 32, (L <= 2 ? 16 : 1))
 rmsnorm_rows_kernel(const __half * in, const void *residual_in,
                     const __half * weight, void *out, float *res_scale, int n_tokens,
                     int hidden_dim, float alpha, float eps) {
-    dependency_trigger();
     dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
@@ -279,6 +284,16 @@ rmsnorm_rows_kernel(const __half * in, const void *residual_in,
         for (int k = 0; k < 4; ++k) sq[q][k] = val[q][k].x * val[q][k].x + val[q][k].y * val[q][k].y;
     }
 
+    // The weights are read in front of the first store (the compiler may not move them across it), and
+    // in front of the reduction except where the f16 residual leaves no registers for them.
+    uint4 wraw[L];
+    auto load_weight = [&](int q0, int q1) {
+#pragma unroll
+        for (int q = q0; q < q1; ++q) wraw[q] = *reinterpret_cast<const uint4 *>(weight + (q * 32 + lane) * 8);
+    };
+    constexpr int kEarly = MODE == kOutF16 ? 0 : L;
+    load_weight(0, kEarly);
+
     float sum_sq;
     if constexpr (L == 2) sum_sq = row_sum_sq_2(sq, lane);
     else sum_sq = row_sum_sq<L>(sq);
@@ -287,12 +302,14 @@ rmsnorm_rows_kernel(const __half * in, const void *residual_in,
     const float mean_sq = (L == 1 || L == 2 || L == 4) ? sum_sq * (1.0f / (256.0f * L)) : sum_sq / hidden_dim;
     const float rms_inv = rsqrtf(mean_sq + eps);
 
+    load_weight(kEarly, L);
+
     float amax = 0.f;
 #pragma unroll
     for (int q = 0; q < L; ++q) {
         const int off = (q * 32 + lane) * 8;
         float2 wf[4];
-        unpack8(*(reinterpret_cast<const uint4 *>(weight + off)), wf);
+        unpack8(wraw[q], wf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             val[q][k] = mul2(mul2(val[q][k], make_float2(rms_inv, rms_inv)), wf[k]);
@@ -384,7 +401,6 @@ __global__ void rmsnorm_generic_kernel(const __half * in, const void *residual_i
                                        const __half * weight, void *out,
                                        float *res_scale, int n_tokens, int hidden_dim, float alpha,
                                        float eps) {
-    dependency_trigger();
     dependency_wait();
     __shared__ float buf[32];
     const int64_t row = blockIdx.x;
@@ -475,7 +491,6 @@ template <int L, bool FP8>
 __global__ void __launch_bounds__(kNormWarps * 32, (L <= 2 ? 16 : 1))
 quant_rows_reg_kernel(const __half * in, uint8_t * out,
                       float * scale, int n_tokens) {
-    dependency_trigger();
     dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
@@ -528,7 +543,6 @@ template <bool FP8>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 quant_rows_kernel(const __half * in, uint8_t * out,
                   float * scale, int n_tokens, int hidden_dim, int vec_ok) {
-    dependency_trigger();
     dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -593,7 +607,6 @@ __global__ void __launch_bounds__(256)
 rotary_vec_kernel(__half *x, const float * sin_tab, const float * cos_tab,
                   int64_t total, int seq_len, int n_heads, int width, int64_t stride_batch,
                   int64_t stride_seq, int64_t stride_head, int cpw_log2, int heads_log2) {
-    dependency_trigger();
     dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total) return;
@@ -650,7 +663,6 @@ __global__ void __launch_bounds__(256)
 rotary_scalar_kernel(__half *x, const float * sin_tab,
                      const float * cos_tab, int64_t total, int seq_len, int n_heads,
                      int width, int64_t stride_batch, int64_t stride_seq, int64_t stride_head) {
-    dependency_trigger();
     dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total) return;
@@ -685,7 +697,6 @@ template <int VEC>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __half * in, __half * out, int64_t total_vec,
                 int hidden_dim) {
-    dependency_trigger();
     dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
@@ -731,7 +742,6 @@ template <int VEC>
 __global__ void __launch_bounds__(256)
 flstm_step_kernel(const __half * scratch, const __half * ih_t,
                   __half *cell, __half * hh_next, int64_t total_vec, int hidden_dim) {
-    dependency_trigger();
     dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
@@ -776,7 +786,6 @@ __global__ void __launch_bounds__(256)
 dequant_transpose_kernel(const uint8_t * in, __half * out,
                          int64_t total_vec, int n_timesteps, int batch_size, int n_channels,
                          float scale) {
-    dependency_trigger();
     dependency_wait();
     const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
