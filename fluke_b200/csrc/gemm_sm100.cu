@@ -727,6 +727,14 @@ int launch(const fluke_sm100_gemm_t *g, cudaStream_t stream) {
     return plan_launch<KIND, EPI, BN_MMA, STAGES>(plan, 0, stream);
 }
 
+}  // namespace
+}  // namespace fluke_sm100
+
+#include "gemm_tile_sm100.cu"
+
+namespace fluke_sm100 {
+namespace {
+
 // Tile shapes: 128 x 128 (K up to 1024 resident) for the plain GEMMs; 128 x 256 (one UMMA of
 // N = 256 per K step, K up to 512 resident) for the two fused transformer kernels. Beside the
 // resident weight tile and 32 KB of store staging there is room for a ring of four 16 KB
@@ -734,8 +742,46 @@ int launch(const fluke_sm100_gemm_t *g, cudaStream_t stream) {
 constexpr int kPlainBN = 128, kFusedBN = 256;
 constexpr int kPlainStages = 4, kFusedStages = 4, kSiluStages = 4;
 
+// Problems whose tiles are all resident at once go to the one-tile-per-CTA kernel (gemm_tile_sm100.cu);
+// with more of them its CTAs would run in rounds, each paying the whole latency again, and the
+// persistent kernel is the faster one. Measured in us, tile kernel against persistent, at K = 512:
+// rotary 125 rows 2.96 : 5.55, 900 rows (192 tiles of 296 resident) 4.41 : 5.87, 1803 rows (360)
+// 6.7 : 6.1; gated (one CTA per SM) 125 rows 3.6 : 5.3, 500 rows (128 tiles of 148) 3.8 : 5.5, 900 rows
+// (256) 7.3 : 5.8; plain 125 rows 2.5 : 3.9, 1803 rows 3.4 : 4.1. The plain form takes 32-column tiles
+// while those are all resident, then 64. Returns the tile width, 0 for the persistent kernel.
+int tile_width(const fluke_sm100_gemm_t *g) {
+    const bool aligned = (reinterpret_cast<uintptr_t>(g->out) & 15u) == 0 && g->ld_out % 8 == 0;
+    if (!aligned || g->K % 128 != 0) return 0;
+    const int64_t m_tiles = (g->M + 127) / 128, sms = device_sm_count();
+    const bool dual = g->epilogue == FLUKE_SM100_EPI_SILU, plain = !dual && g->epilogue != FLUKE_SM100_EPI_ROTARY;
+    for (int bn = plain ? 32 : 64; bn <= 64; bn *= 2) {
+        const int per_sm = 2 * tile_smem(g->K, dual ? 2 * bn : bn) <= 227 * 1024 ? 2 : 1;
+        if (m_tiles * (g->N / bn) <= sms * per_sm) return bn;
+    }
+    return 0;
+}
+
+template <int KIND, int EPI>
+int tile_dispatch(const fluke_sm100_gemm_t *g, int width, cudaStream_t s) {
+    if constexpr (EPI == FLUKE_SM100_EPI_DEQUANT || EPI == FLUKE_SM100_EPI_DEQUANT2)
+        if (width == 32) return tile_launch<KIND, EPI, 32>(g, s);
+    return tile_launch<KIND, EPI, 64>(g, s);
+}
+
 template <int KIND>
 int dispatch(const fluke_sm100_gemm_t *g, cudaStream_t s) {
+    if (g->M == 0) return 0;
+    if (g->epilogue != FLUKE_SM100_EPI_RAW) {
+        const int width = tile_width(g);
+        if (width)
+            switch (g->epilogue) {
+                case FLUKE_SM100_EPI_DEQUANT: return tile_dispatch<KIND, FLUKE_SM100_EPI_DEQUANT>(g, width, s);
+                case FLUKE_SM100_EPI_DEQUANT2: return tile_dispatch<KIND, FLUKE_SM100_EPI_DEQUANT2>(g, width, s);
+                case FLUKE_SM100_EPI_ROTARY: return tile_dispatch<KIND, FLUKE_SM100_EPI_ROTARY>(g, width, s);
+                case FLUKE_SM100_EPI_SILU: return tile_dispatch<KIND, FLUKE_SM100_EPI_SILU>(g, width, s);
+                default: break;
+            }
+    }
     switch (g->epilogue) {
         case FLUKE_SM100_EPI_RAW:
             return launch<KIND, FLUKE_SM100_EPI_RAW, kPlainBN, kPlainStages>(g, s);

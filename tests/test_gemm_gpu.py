@@ -418,3 +418,42 @@ def test_transformer_ops_are_shard_invariant(be, be8):
         for full, pa, pb in zip(whole, a, b):
             assert torch.equal(full, torch.cat([pa, pb], dim=0))
     assert L.read_status() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 31, 128, 129, 300, 512, 1664, 1665, 2304, 2305, 4736, 4737])
+def test_few_tiles_give_the_bits_of_many(be, be8, rows):
+    """The kernel for few output tiles and the persistent one compute an element in the same order, so
+    the first rows of a large call and a call of those rows alone have equal bits: int8 and fp8, the
+    three fused or plain forms. Row counts at the edges of a 128-row tile and on both sides of the
+    tile counts where a B200 (148 SMs, one or two CTAs each) changes kernel or tile width."""
+    g, m, seqlen = torch.Generator().manual_seed(rows), 6016, 64
+    sin, cos = (t.to(DEV) for t in prep.rotary_tables(seqlen, 64))
+    w16 = [torch.randn(n, 512, generator=g) * 0.02 for n in (1536, 2048, 2048, 512)]
+    x = torch.randn(m, 512, generator=g)
+    for fp8 in (False, True):
+        def quantise(t):
+            q, s = prep.quantize_fp8_rows(t) if fp8 else prep.quantize_int8_rows(t)
+            return (q.view(torch.uint8) if fp8 else q).contiguous().to(DEV), s.contiguous().to(DEV)
+        (wq, sq), (wg, sg), (wu, su), (wo, so) = map(quantise, w16)
+        a, sa = quantise(x)
+        def run(a, sa):
+            if fp8:
+                return (ops.qkv_rotary_fp8(be8, a, wq, sa, sq, sin, cos, seqlen, plain=True),
+                        ops.gated_mlp_fp8(be8, a, wg, wu, sa, sg, su, plain=True), ops.gemm_fp8(a, wo, sa, so))
+            return (ops.qkv_rotary_i8(be, a, wq, sa, sq, sin, cos, seqlen), ops.gated_mlp_i8(be, a, wg, wu, sa, sg, su),
+                    ops.gemm_i8(a, wo, sa, so))
+        for big, small in zip(run(a, sa), run(a[:rows], sa[:rows])):
+            assert torch.equal(big[:rows], small)
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 128, 768), (500, 128, 1024), (1, 64, 128), (130, 64, 384), (77, 128, 896), (40, 64, 144)])
+def test_down_projection_of_few_rows_vs_oracle(m, n, k):
+    """K from one 128-byte block to eight, odd numbers of blocks (a half-empty second load) and one that
+    is no whole number of blocks (persistent kernel), into a wider buffer: bit for bit."""
+    g = torch.Generator().manual_seed(m + k)
+    a, sa = prep.quantize_int8_rows(torch.randn(m, k, generator=g))
+    b, sb = prep.quantize_int8_rows(torch.randn(n, k, generator=g) * 0.1)
+    wide = torch.full((m, 2 * n), 7.0, dtype=torch.float16, device=DEV)
+    ops.down_proj_i8(a.to(DEV), b.to(DEV), sa.to(DEV), sb.to(DEV), out=wide[:, n:])
+    assert np.array_equal(wide[:, n:].cpu().numpy(), port.gemm_i8(a.numpy(), b.numpy(), sa.numpy(), sb.numpy()))
+    assert bool((wide[:, :n] == 7.0).all())
