@@ -203,12 +203,10 @@ PyObject *rotary_qkv(Args a) {
     const at::Tensor *sin = input(a[1]), *cos = input(a[2]);
     const int width = integer(a[3]);
     TORCH_CHECK(qkv.dim() == 5, "rotary_qkv_ needs [N, seq, 3, heads, head_dim]");
-    char *x = static_cast<char *>(ptr(qkv));
+    // the q and k heads lie side by side: one call rotates both
     unlocked([&] {
-        for (int chunk = 0; chunk < 2; ++chunk)
-            L.fluke_rotary_emb_gpu(x + chunk * qkv.stride(2) * qkv.element_size(), ptr(sin), ptr(cos), int(qkv.size(0)),
-                                   int(qkv.size(1)), int(qkv.size(3)), int(qkv.size(4)), width, int(qkv.stride(0)),
-                                   int(qkv.stride(1)), int(qkv.stride(3)));
+        L.fluke_rotary_emb_gpu(ptr(qkv), ptr(sin), ptr(cos), int(qkv.size(0)), int(qkv.size(1)), 2 * int(qkv.size(3)),
+                               int(qkv.size(4)), width, int(qkv.stride(0)), int(qkv.stride(1)), int(qkv.stride(3)));
     });
     Py_INCREF(a[0]);
     return a[0];

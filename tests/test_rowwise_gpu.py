@@ -241,3 +241,47 @@ def test_empty_inputs_are_noops():
     assert ops.quant_int8(z)[0].shape == (0, 512)
     assert ops.rmsnorm(z, z, torch.ones(512, dtype=torch.float16, device=DEV), 1.0, 1e-5).shape == (0, 512)
     assert ops.silu_mul(torch.zeros(0, 64, dtype=torch.float16, device=DEV)).shape == (0, 32)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 301])
+def test_row512_forms_give_the_bits_of_the_unaligned_ones(n):
+    """Rows of 512 elements: the 256-bit kernels (32-byte aligned tensors) against the same call on
+    tensors that start 16 bytes further on, which the 128-bit kernels take. Rows that do not fill a CTA,
+    zero rows, signed zeros and large values among them."""
+    g = torch.Generator().manual_seed(n)
+    def shifted(t):
+        raw = torch.empty(t.numel() * t.element_size() + 64, dtype=torch.uint8, device=DEV)
+        v = raw[16:16 + t.numel() * t.element_size()].view(t.dtype).view(t.shape)
+        v.copy_(t)
+        assert v.data_ptr() % 32 == 16
+        return v
+    x = torch.randn(n, 512, generator=g) * 3
+    x[0, ::2] = -0.0
+    x[n // 2] = 0.0 if n > 1 else x[0]
+    x[-1, 7] = 6e4
+    x, res, w = x.half().to(DEV), torch.randn(n, 512, generator=g).half().to(DEV), torch.randn(512, generator=g).half().to(DEV)
+    assert torch.equal(ops.rmsnorm(x, res, w, 2.0, 1e-5).view(torch.int16), ops.rmsnorm(shifted(x), res, w, 2.0, 1e-5).view(torch.int16))
+    for quant in (ops.quant_int8, ops.quant_fp8):
+        (q, s), (q2, s2) = quant(x), quant(shifted(x))
+        assert torch.equal(q, q2) and torch.equal(s, s2)
+    for norm, dt in ((ops.rmsnorm_quant_int8, torch.int8), (ops.rmsnorm_quant_fp8, torch.uint8)):
+        r = torch.randint(0, 127, (n, 512), generator=g, dtype=dt).to(DEV); rs = (torch.rand(n, generator=g) * 0.02).to(DEV)
+        r2, rs2 = r.clone(), rs.clone()
+        norm(x, w, r, rs, 2.0, 1e-5)
+        norm(shifted(x), w, r2, rs2, 2.0, 1e-5)
+        assert torch.equal(r, r2) and torch.equal(rs, rs2)
+
+
+@pytest.mark.parametrize("rows", [2367, 2368, 2369])
+def test_wide_elementwise_forms_give_the_bits_of_narrow_ones(rows):
+    """SiLU product and rotary around the row count where a thread takes sixteen elements instead of
+    eight (148 * 2048 threads): equal to the same rows in small calls."""
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    x = torch.randn(rows, 4096, generator=g, device=DEV).half()
+    assert torch.equal(ops.silu_mul(x), torch.cat([ops.silu_mul(p.contiguous()) for p in x.split(500)]))
+    from fluke_b200 import prep
+    seq, n = 100, 94 + rows % 5  # 16 heads x 2 threads per position: 9472 positions fill the device
+    sin, cos = prep.rotary_tables(seq, 64, device=DEV)
+    qkv = torch.randn(n, seq, 3, 8, 64, generator=g, device=DEV).half()
+    want = torch.cat([ops.rotary_qkv_(p.clone(), sin, cos, 32) for p in qkv.split(20)])
+    assert torch.equal(ops.rotary_qkv_(qkv, sin, cos, 32), want) and torch.equal(qkv, want)
