@@ -7,8 +7,8 @@
 // contractions that amount does not shrink with the batch; here the operands are swapped. The
 // WEIGHTS are the M dimension (128 hidden units per CTA, one accumulator block per gate) and the
 // chunk rows are N = 16, 32 or 48 columns, and the recurrent half of the gate weights lives in
-// TENSOR MEMORY as the A operand: an MMA then costs N/2 cycles (8 for N = 16) instead of the 33 that
-// reading a 128-row A operand from shared memory takes whatever N is.
+// TENSOR MEMORY as the A operand: an MMA then costs 12 to 20 cycles instead of the 40 that reading a
+// 128-row A operand from shared memory takes whatever N is.
 //
 // A cluster has C = H / 128 CTAs (2 to 8). CTA j
 //   * owns units 128 j .. 128 j + 127: their four gate weight blocks (hh half in tensor memory, x
@@ -18,7 +18,9 @@
 //     int8 rows. With an odd C the last CTA projects nothing.
 // Per step two exchanges inside the cluster, both of 16-byte st.async stores that complete on an
 // mbarrier of the receiver: the int8 hidden slices go to the pair that owns the row, the
-// f16 projections back to every CTA. The x half of the next step's contraction runs meanwhile.
+// f16 projections back to every CTA. The x half of the contraction runs meanwhile. With more than
+// some twenty rows the cluster treats them as two groups, so that one is computed while the
+// other travels.
 //
 //   warp 0       loader: resident weights, x_down rows of every step
 //   warp 1       MMA issuer
@@ -26,10 +28,16 @@
 //                of the rows each (gates, cell update, int8 code); the same warps turn the
 //                projection accumulators into f16 and send them
 //
-// A buffer is only overwritten after its reader has provably finished: a CTA sends h_t after its
-// gate contraction of step t, which needs hh_t from every pair, which a pair sends after its
+// A buffer is only overwritten after its reader has provably finished: a CTA sends h_t (of a group) after
+// its gate contraction of step t, which needs hh_t from every pair, which a pair sends after its
 // projection of h_{t-1} is complete; and the other way round for hh. Nobody leaves before the final
 // cluster barrier. Clusters never wait for one another, so any number of them may run in waves.
+//
+// What bounds a step (B200, H = 768, cycles at 1.93 GHz): with few rows (3 per cluster, 2900 cycles = 1.5 us)
+// the chain: h exchange 600, projection 500 + read-back 250, hh exchange 500, contraction 450,
+// cell update 400; with 47 (6360 cycles = 3.5 us for 1024 chunks) the tensor pipe (x half 1450,
+// projections 1300, hh half 1150) and the epilogue warps (3200) one after the other: the accumulators
+// leave no tensor memory for a second set.
 //
 // Arithmetic and its order are those of the other single-launch forms (x_down half first, then the
 // hh_down half in K steps of 16; int32 sums scaled by (1/127)*scale and rounded to f16): the bytes
@@ -53,13 +61,13 @@ constexpr int kGMaxCtas = 8;       // portable cluster size: H <= 1024
 constexpr int kGTmemCols = 512;
 constexpr int kGTmemW = 256;       // first column of the hh half of the gate weights: 4 gates x 64
 constexpr int kGWxBytes = 4 * kGUnits * 256;  // x half of the gate weights in shared memory
+constexpr int kGMaxSmem = 232448;
 
 struct GroupDev {
-    int T, B, H;
+    int T, B;
     int reverse;
-    int rows;                  // chunk rows per cluster (the last cluster may have fewer)
-    int n_own, n_pad;          // rows a pair projects; the same rounded up to a multiple of 8
-    int dn_ts;                 // K blocks of the projection weights kept in tensor memory
+    int rows;                  // chunk rows per cluster (the last one may have fewer)
+    int n_own[2];              // rows of a group a pair projects
     const int8_t *dn;          // [R, H]
     const __half *w_up;        // [4H, 2R]
     const float *bias;         // [4H]
@@ -70,27 +78,40 @@ struct GroupDev {
     long long *trace;          // trace builds only: [T][8] SM-clock stamps of CTA 0
 };
 
-// Shared-memory layout; the row-dependent parts are sized at launch.
+// All of the following depends on the cluster size C = H / 128, which the kernel is compiled for: with
+// operand addresses at fixed distances the issuer needs few instructions between MMAs (the 24 of a
+// projection took 800 cycles to issue with C a variable).
+// Rows of a group's hidden tile (and columns of its projection): what a pair projects of the group's n rows, as
+// a multiple of 8.
+__host__ __device__ constexpr int group_h_rows(int n, int C) { return ((n + C / 2 - 1) / (C / 2) + 7) / 8 * 8; }
+// K blocks (128 hidden units, 32 columns) of the projection weights that fit in tensor memory beside
+// the gate weights, the gate accumulators and the projections.
+__host__ __device__ constexpr int group_dn_ts(int n0, int n1, int C) {
+    const int fit = (kGTmemW - 4 * (n0 + n1) - group_h_rows(n0, C) - group_h_rows(n1, C)) / 32;
+    return fit < C ? fit : C;
+}
 struct GroupLayout {
     int x, hh, dn, h, stage, bars, misc, dynamic;
 };
-// K blocks (128 hidden units, 32 columns) of the projection weights that fit in tensor memory beside
-// the gate weights and the accumulators.
-__host__ __device__ constexpr int group_dn_ts(int nb, int H, int n_pad) {
-    const int fit = (kGTmemW - 4 * nb - n_pad) / 32;
-    return fit < H / kGUnits ? fit : H / kGUnits;
-}
-__host__ __device__ constexpr GroupLayout group_layout(int nb, int H, int n_pad) {
+__host__ __device__ constexpr GroupLayout group_layout_slots(int n0, int n1, int C, int x_slots) {
     GroupLayout l = {};
-    l.x = kGWxBytes;                  // x_down rows of two steps: 2 K blocks [nb x 128 B] each
-    l.hh = l.x + 2 * nb * 256;        // hh_down rows, the same shape
-    l.dn = l.hh + nb * 256;           // 64 projection rows: the other K blocks [64 x 128 B]
-    l.h = l.dn + 64 * (H - 128 * group_dn_ts(nb, H, n_pad));              // hidden rows of the pair: H/128 K blocks [n_pad x 128 B]
-    l.stage = l.h + n_pad * H;        // 16 warps x (nb/4 rows x 32 B)
-    l.bars = l.stage + nb * 128;
-    l.misc = l.bars + 10 * 8;
-    l.dynamic = l.misc + 16 + 1024;   // slack for the manual 1024-byte alignment
+    const int n = n0 + n1;
+    l.x = kGWxBytes;                            // x_down rows: 2 K blocks [n x 128 B] per slot
+    l.hh = l.x + x_slots * n * 256;             // hh_down rows, the same shape
+    l.dn = l.hh + n * 256;                      // 64 projection rows: the K blocks not in tensor memory [64 x 128 B]
+    l.h = l.dn + 8192 * (C - group_dn_ts(n0, n1, C));  // hidden rows of the pair, per group: C K blocks
+    l.stage = l.h + (group_h_rows(n0, C) + group_h_rows(n1, C)) * C * kGUnits;  // 16 warps x (n0/4 rows x 32 B)
+    l.bars = l.stage + n0 * 128;
+    l.misc = l.bars + 15 * 8;
+    l.dynamic = l.misc + 16 + 1024;             // slack for the manual 1024-byte alignment
     return l;
+}
+// x tiles of two steps where shared memory allows it, else of one.
+__host__ __device__ constexpr int group_x_slots(int n0, int n1, int C) {
+    return group_layout_slots(n0, n1, C, 2).dynamic <= kGMaxSmem ? 2 : 1;
+}
+__host__ __device__ constexpr GroupLayout group_layout(int n0, int n1, int C) {
+    return group_layout_slots(n0, n1, C, group_x_slots(n0, n1, C));
 }
 
 // 16 bytes into a CTA of the cluster; completes 16 bytes of the transaction count of an mbarrier
@@ -114,52 +135,67 @@ __device__ __forceinline__ void sts16(uint32_t addr, unsigned short v) {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
 }
 
-template <int NB>
+template <int V>
+struct Int { static constexpr int value = V; };  // a number that a lambda receives as a type
+
+// N0 + N1: accumulator columns, i.e. chunk rows of a cluster at most. With N1 = 0 they are one group: the chain
+// of a step is all there is to run. Otherwise the first N0 rows and the others are two groups that share the
+// x part of the contraction (its MMAs read their A operand from shared memory, 40 cycles each whatever
+// N is up to 64, so one for both) and go through the rest of the step one after the other: while
+// one is exchanged, the other is projected or computed.
+template <int N0, int N1, int C>
 __global__ void __launch_bounds__(kGThreads, 1)
 lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] f16, boxes 128 x 64
                   const __grid_constant__ CUtensorMap tm_x,    // x_down [T, 2, B, 64] f16, boxes of NB rows
                   const __grid_constant__ CUtensorMap tm_dn,   // dn_hh [R, H] int8, boxes 64 x 128
-                  const __grid_constant__ CUtensorMap tm_h0,   // h_0 [H/128, B, 128] int8, boxes of n_pad rows
+                  const __grid_constant__ CUtensorMap tm_h0,   // h_0 [H/128, B, 128] int8, boxes of the first group's tile
+                  const __grid_constant__ CUtensorMap tm_h1,   // and of the second's
                   const GroupDev p) {
-    constexpr int kCols = NB / 4;                    // rows an epilogue thread holds at most
+    constexpr int G = N1 > 0 ? 2 : 1, NB = N0 + N1;
+    constexpr int kXSlots = group_x_slots(N0, N1, C);
+    constexpr int H = C * kGUnits;
+    constexpr int kPad0 = group_h_rows(N0, C), kPad1 = group_h_rows(N1, C);
+    constexpr int kDnTs = group_dn_ts(N0, N1, C);
+    constexpr GroupLayout L = group_layout(N0, N1, C);
+    constexpr int kCols = N0 / 4;                    // rows of the first group that an epilogue thread holds at most
     constexpr int kBatches = kCols / 4;              // it takes them four at a time
-    constexpr int kSendP = NB / 16;                  // 16-byte stores per lane and step, projections
-    static_assert(NB % 16 == 0 && 4 * NB + NB <= kGTmemW, "accumulators beside the weights in tensor memory");
+    constexpr int kSendP = N0 / 16;                  // 16-byte stores per lane and step, projections
+    static_assert(N0 % 16 == 0 && N1 % 16 == 0 && N1 <= N0 && 5 * NB <= kGTmemW, "accumulators beside the weights in tensor memory");
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
     // shared-window offsets as this CTA's
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const GroupLayout L = group_layout(NB, p.H, p.n_pad);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
     uint64_t *bar_once = &bars[0];       // resident weights loaded
-    uint64_t *bar_x = &bars[1];          // [2] x_down rows landed
-    uint64_t *bar_x_free = &bars[3];     // [2] x half of the contraction has read them
-    uint64_t *bar_h = &bars[5];          // complete hidden rows of the pair arrived
-    uint64_t *bar_proj = &bars[6];       // projection accumulator complete
-    uint64_t *bar_hh = &bars[7];         // hh_down rows arrived
-    uint64_t *bar_acc = &bars[8];        // gate accumulators complete
-    uint64_t *bar_acc_free = &bars[9];   // epilogue has read them
+    uint64_t *bar_x = &bars[1];          // [slots] x_down rows landed
+    uint64_t *bar_x_free = &bars[3];     // [slots] x half of the contraction has read them
+    uint64_t *bar_h = &bars[5];          // [G] complete hidden rows of the pair arrived
+    uint64_t *bar_proj = &bars[7];       // [G] projection accumulator complete
+    uint64_t *bar_hh = &bars[9];         // [G] hh_down rows arrived
+    uint64_t *bar_acc = &bars[11];       // [G] gate accumulators complete
+    uint64_t *bar_acc_free = &bars[13];  // [G] epilogue has read them
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
-    const int C = p.H / kGUnits;
     const int rank = int(cluster_ctarank());
     const int pair = rank >> 1, half = rank & 1;
     const bool projects = rank < (C & ~1);
     const int m0 = (blockIdx.x / C) * p.rows;          // first chunk row of the cluster
     const int n_rows = min(p.rows, p.B - m0);          // and how many it has
-    const int n_own = min(max(n_rows - pair * p.n_own, 0), p.n_own);  // rows this CTA projects
     const int n0 = rank * kGUnits;
+    // of group e: rows it has, rows of them this CTA projects
+    auto rows_of = [&](int e) { return G == 1 ? n_rows : e == 0 ? min(n_rows, N0) : max(n_rows - N0, 0); };
+    auto own_of = [&](int e) { return min(max(rows_of(e) - pair * p.n_own[e], 0), p.n_own[e]); };
+    constexpr int h_group1 = kPad0 * H;                // byte offset of the second group's hidden rows
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
-
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 9; ++b) mbar_init(&bars[b], 1);
-        mbar_init(bar_acc_free, kGEpiWarps);
+        for (int b = 0; b < 13; ++b) mbar_init(&bars[b], 1);
+        for (int b = 13; b < 15; ++b) mbar_init(&bars[b], kGEpiWarps);
         *abort_flag = 0;
         fence_barrier_init();
-        mbar_arrive_expect_tx(bar_hh, uint32_t(n_rows) * 256);
+        for (int e = 0; e < G; ++e) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
     }
     if (warp == 1) tmem_alloc(tmem_slot, kGTmemCols);
     tc_fence_before_sync();
@@ -170,14 +206,14 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         // the hh half of the gate weights: warp = (lane quadrant, gate), thread = row of the block
         const int q = warp & 3, g = (warp - 2) >> 2;
         const uint4 *src = reinterpret_cast<const uint4 *>(
-            p.w_up + (size_t(g) * p.H + n0 + q * 32 + lane) * (2 * kGRank));
+            p.w_up + (size_t(g) * H + n0 + q * 32 + lane) * (2 * kGRank));
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16) + kGTmemW;
 #pragma unroll 1
         for (int v = 0; v < 8; ++v) tmem_st_32x8(t_lane + g * 64 + v * 8, __ldg(src + 2 * v), __ldg(src + 2 * v + 1));
         if (projects) {
             // and K blocks g, g + 4, .. of the projection rows (M = 64: row 16 q + i in lane 32 q + i)
-            const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(half * 64 + q * 16 + (lane & 15)) * p.H);
-            for (int kb = g; kb < p.dn_ts; kb += 4)
+            const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(half * 64 + q * 16 + (lane & 15)) * H);
+            for (int kb = g; kb < kDnTs; kb += 4)
 #pragma unroll 1
                 for (int v = 0; v < 4; ++v)
                     tmem_st_32x8(t_lane - 32 * (kb + 1) + v * 8, __ldg(dn + kb * 8 + 2 * v), __ldg(dn + kb * 8 + 2 * v + 1));
@@ -193,23 +229,26 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     if (warp == 0) {
         // ------------------------------ loader (one thread) -----------------------------
         if (elect_one()) {
-            mbar_arrive_expect_tx(bar_once, kGWxBytes + (projects ? (C - p.dn_ts) * 8192 : 0));
+            mbar_arrive_expect_tx(bar_once, kGWxBytes + (projects ? (C - kDnTs) * 8192 : 0));
             for (int g = 0; g < 4; ++g)
                 for (int kb = 0; kb < 2; ++kb)
-                    tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * p.H + n0);
+                    tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
             if (projects) {
-                for (int kb = p.dn_ts; kb < C; ++kb)
-                    tma_load_2d(smem + L.dn + (kb - p.dn_ts) * 8192, &tm_dn, bar_once, kb * 128, half * 64);
+                for (int kb = kDnTs; kb < C; ++kb)
+                    tma_load_2d(smem + L.dn + (kb - kDnTs) * 8192, &tm_dn, bar_once, kb * 128, half * 64);
                 // step 0 projects the layer's initial hidden state
-                mbar_arrive_expect_tx(bar_h, uint32_t(p.n_pad) * p.H);
-                tma_load_3d(smem + L.h, &tm_h0, bar_h, 0, m0 + pair * p.n_own, 0);
+                for (int e = 0; e < G; ++e) {
+                    mbar_arrive_expect_tx(&bar_h[e], uint32_t(e ? kPad1 : kPad0) * H);
+                    tma_load_3d(smem + L.h + e * h_group1, e ? &tm_h1 : &tm_h0, &bar_h[e], 0, m0 + e * N0 + pair * p.n_own[e], 0);
+                }
             }
             bool ok = true;
             for (int i = 0; i < p.T && ok; ++i) {
-                if (i > 1) ok = mbar_wait(&bar_x_free[i & 1], ((i >> 1) - 1) & 1, abort_flag, 96);
+                const int s = i % kXSlots, u = i / kXSlots;
+                if (u > 0) ok = mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
                 if (!ok) break;
-                mbar_arrive_expect_tx(&bar_x[i & 1], NB * 256);
-                tma_load_4d(smem + L.x + (i & 1) * (NB * 256), &tm_x, &bar_x[i & 1], 0, m0, 0, time_of(i));
+                mbar_arrive_expect_tx(&bar_x[s], NB * 256);
+                tma_load_4d(smem + L.x + s * (NB * 256), &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
             }
         }
         __syncwarp();
@@ -217,157 +256,195 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         // ------------------------------ MMA issuer --------------------------------------
         // The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
         // K loops unrolled, so an MMA is issued every few cycles.
-        constexpr uint32_t kIdescGate = make_idesc<kKindF16>(128, NB);
-        const uint32_t idesc_proj = make_idesc<kKindI8>(64, 0) | (uint32_t(p.n_pad >> 3) << 17);
+        constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, NB);
         uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
-        uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
+        uint64_t d_x0 = make_smem_desc_sw128(smem_u32(smem + L.x));
+        uint64_t d_hh0 = make_smem_desc_sw128(smem_u32(smem + L.hh));
         uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
-        uint64_t d_h = make_smem_desc_sw128(smem_u32(smem + L.h));
-        uint64_t d_x = 0;
-        const uint32_t t_proj = tmem + 4 * NB;
-        // The x half of gates [g0, g1). Its 32 MMAs read their A operand from shared memory (33
-        // cycles each, a third of a step in all) and the tensor pipe works in order: half of them go in front
-        // of the projection, while the hidden state is computed and travels, half behind it, while
-        // the projection is converted and travels.
-        auto x_half = [&](int g0, int g1) {
-#pragma unroll
-            for (int g = g0; g < g1; ++g)
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    tc_mma<kKindF16>(tmem + g * NB, d_wx + uint64_t((g * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                     d_x + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescGate, k != 0);
-        };
+        uint64_t d_h0 = make_smem_desc_sw128(smem_u32(smem + L.h));
         bool ok = mbar_wait(bar_once, 0, abort_flag, 97);
-        for (int i = 0; i < p.T && ok; ++i) {
-            if (i > 0) ok = mbar_wait(bar_acc_free, (i - 1) & 1, abort_flag, 98);
-            if (!ok) break;
-            ok = mbar_wait(&bar_x[i & 1], (i >> 1) & 1, abort_flag, 99);
-            if (!ok) break;
-            tc_fence_after_sync();
-            // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
-            // more registers than there are.
-            d_x = make_smem_desc_sw128(smem_u32(smem + L.x)) + uint64_t((i & 1) * (NB * 16));
-            asm volatile("" : "+l"(d_wx), "+l"(d_x), "+l"(d_hh), "+l"(d_dn), "+l"(d_h));
-            if (elect_one()) x_half(0, 2);
-            __syncwarp();
-            if (projects) {
-                ok = mbar_wait<true>(bar_h, i & 1, abort_flag, 100);
-                if (!ok) break;
-                fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
-                tc_fence_after_sync();
-                FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + 3, clock64());
-                if (elect_one()) {
-                    // an MMA is 8 to 12 cycles with its weights in tensor memory, 24 from shared memory
-                    for (int kb = 0; kb < p.dn_ts; ++kb)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            tc_mma_ts<kKindI8>(t_proj, tmem + kGTmemW - 32 * (kb + 1) + 8 * k,
-                                               d_h + uint64_t(kb * p.n_pad * 8 + 2 * k), idesc_proj, (kb | k) != 0);
-                    for (int kb = p.dn_ts; kb < C; ++kb)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            tc_mma<kKindI8>(t_proj, d_dn + uint64_t((kb - p.dn_ts) * 512 + 2 * k),
-                                            d_h + uint64_t(kb * p.n_pad * 8 + 2 * k), idesc_proj, (kb | k) != 0);
-                    tc_commit(bar_proj);
-                    if (i + 1 < p.T) mbar_arrive_expect_tx(bar_h, uint32_t(n_own) * p.H);  // arm the next step
-                }
-                __syncwarp();
-            }
+        int i = 0;
+        // The x half of gates [g0, g1). Its 32 MMAs read their A operand from shared memory (40 cycles
+        // each, a third of a one-group step in all) and the tensor pipe works in order, so they are
+        // issued in pieces for the times when it would wait.
+        auto x_half = [&](auto from, auto to) {
+            constexpr int g0 = decltype(from)::value, g1 = decltype(to)::value;
+            const uint64_t d_x = d_x0 + uint64_t((i % kXSlots) * (NB * 16));
             if (elect_one()) {
-                x_half(2, 4);
-                tc_commit(&bar_x_free[i & 1]);
+#pragma unroll
+                for (int g = g0; g < g1; ++g)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma<kKindF16>(tmem + g * NB, d_wx + uint64_t((g * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
+                                         d_x + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+                if (g1 == 4) tc_commit(&bar_x_free[i % kXSlots]);
             }
             __syncwarp();
-            ok = mbar_wait<true>(bar_hh, i & 1, abort_flag, 101);
-            if (!ok) break;
+        };
+        auto wait_x = [&]() {
+            if (i > 0)
+                for (int e = 0; e < G; ++e) ok = ok && mbar_wait(&bar_acc_free[e], (i - 1) & 1, abort_flag, 98);
+            ok = ok && mbar_wait(&bar_x[i % kXSlots], (i / kXSlots) & 1, abort_flag, 99);
+            tc_fence_after_sync();
+            return ok;
+        };
+        auto project = [&](auto group) {
+            constexpr int e = decltype(group)::value;
+            if (!projects) return true;
+            ok = ok && mbar_wait<true>(&bar_h[e], i & 1, abort_flag, 100);
+            if (!ok) return false;
+            fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
+            tc_fence_after_sync();
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + (e ? 2 : 3), clock64());
+            if (elect_one()) {
+                constexpr int kPad = e ? kPad1 : kPad0;
+                constexpr uint32_t kIdesc = make_idesc<kKindI8>(64, kPad);
+                const uint32_t t_proj = tmem + 4 * NB + (e ? kPad0 : 0);
+                const uint64_t d_h = d_h0 + uint64_t(e * (h_group1 >> 4));
+                // an MMA is 8 to 12 cycles with its weights in tensor memory, 27 from shared memory
+#pragma unroll
+                for (int kb = 0; kb < C; ++kb)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint64_t rows = d_h + uint64_t(kb * kPad * 8 + 2 * k);
+                        if (kb < kDnTs)
+                            tc_mma_ts<kKindI8>(t_proj, tmem + kGTmemW - 32 * (kb + 1) + 8 * k, rows, kIdesc, (kb | k) != 0);
+                        else
+                            tc_mma<kKindI8>(t_proj, d_dn + uint64_t((kb - kDnTs) * 512 + 2 * k), rows, kIdesc, (kb | k) != 0);
+                    }
+                tc_commit(&bar_proj[e]);
+                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_h[e], uint32_t(own_of(e)) * H);  // arm the next step
+            }
+            __syncwarp();
+            return true;
+        };
+        auto hh_half = [&](auto group) {
+            constexpr int e = decltype(group)::value;
+            constexpr uint32_t kIdesc = make_idesc<kKindF16>(128, e ? N1 : N0);
+            ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
+            if (!ok) return false;
             fence_proxy_async_smem();
             tc_fence_after_sync();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + 6, clock64());
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + (e ? 7 : 6), clock64());
             if (elect_one()) {
+                const uint64_t d_hh = d_hh0 + uint64_t(e * (N0 * 8));
 #pragma unroll
                 for (int g = 0; g < 4; ++g)
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        tc_mma_ts<kKindF16>(tmem + g * NB, tmem + kGTmemW + g * 64 + k * 8,
-                                            d_hh + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescGate, 1u);
-                tc_commit(bar_acc);
-                if (i + 1 < p.T) mbar_arrive_expect_tx(bar_hh, uint32_t(n_rows) * 256);
+                        tc_mma_ts<kKindF16>(tmem + g * NB + e * N0, tmem + kGTmemW + g * 64 + k * 8,
+                                            d_hh + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdesc, 1u);
+                tc_commit(&bar_acc[e]);
+                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
             }
             __syncwarp();
+            return true;
+        };
+        for (; i < p.T && ok; ++i) {
+            // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
+            // more registers than there are.
+            asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh0), "+l"(d_dn), "+l"(d_h0));
+            if constexpr (G == 1) {
+                // half of the x part while the hidden state is computed and travels, half while the
+                // projection is converted and travels
+                if (!wait_x()) break;
+                x_half(Int<0>{}, Int<2>{});
+                if (!project(Int<0>{})) break;
+                x_half(Int<2>{}, Int<4>{});
+                if (!hh_half(Int<0>{})) break;
+            } else {
+                // pieces of the x part while the hidden rows of the groups travel, the rest while their
+                // projections are converted and travel
+                if (!wait_x()) break;
+                x_half(Int<0>{}, Int<1>{});
+                if (!project(Int<0>{})) break;
+                x_half(Int<1>{}, Int<2>{});
+                if (!project(Int<1>{})) break;
+                x_half(Int<2>{}, Int<4>{});
+                if (!hh_half(Int<0>{})) break;
+                if (!hh_half(Int<1>{})) break;
+            }
         }
     } else {
         // ------------------------------ epilogues ---------------------------------------
         const int q = warp & 3, ug = (warp - 2) >> 2;
-        // gates: this warp's rows of the cluster (an even share, so that rows pair up)
-        const int share = ((p.rows + 3) / 4 + 1) & ~1;
-        const int r0 = ug * share;
-        const int my_rows = min(max(n_rows - r0, 0), share);
+        // gates: this warp's rows of a group (an even share, so that rows pair up)
+        auto share_of = [&](int e) {
+            const int most = G == 1 ? p.rows : e == 0 ? min(p.rows, N0) : p.rows - N0;
+            return max((most + 3) / 4 + 1, 0) & ~1;
+        };
+        auto r0_of = [&](int e) { return e * N0 + ug * share_of(e); };   // in the cluster's rows
+        auto my_rows_of = [&](int e) { return min(max(rows_of(e) - ug * share_of(e), 0), share_of(e)); };
         // projection: its columns (= rows) of the pair's accumulator
-        const int p_share = (p.n_own + 3) / 4;
-        const int pr0 = ug * p_share;
-        const int my_pr = projects ? min(max(n_own - pr0, 0), p_share) : 0;
+        auto pr0_of = [&](int e) { return ug * ((p.n_own[e] + 3) / 4); };
+        auto my_pr_of = [&](int e) { return projects ? min(max(own_of(e) - pr0_of(e), 0), (p.n_own[e] + 3) / 4) : 0; };
 
         const int unit = n0 + q * 32 + lane;
-        const float b_i = __ldg(p.bias + unit), b_f = __ldg(p.bias + p.H + unit);
-        const float b_g = __ldg(p.bias + 2 * p.H + unit), b_o = __ldg(p.bias + 3 * p.H + unit);
+        const float b_i = __ldg(p.bias + unit), b_f = __ldg(p.bias + H + unit);
+        const float b_g = __ldg(p.bias + 2 * H + unit), b_o = __ldg(p.bias + 3 * H + unit);
         // one projection column per lane (16 lanes of a quadrant hold rows of an M = 64 accumulator)
         const int r_col = half * 64 + q * 16 + (lane & 15);
         const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + r_col);  // operand order of the dequant GEMM: sa * sb
-        float2 c2[kCols / 2];
+        float2 c2[G][kCols / 2];
 #pragma unroll
-        for (int j = 0; j < kCols / 2; ++j) {
-            const float *cp = p.c + int64_t(m0 + r0 + 2 * j) * p.H + unit;
-            c2[j] = make_float2(2 * j < my_rows ? cp[0] : 0.f, 2 * j + 1 < my_rows ? cp[p.H] : 0.f);
-        }
+        for (int e = 0; e < G; ++e)
+#pragma unroll
+            for (int j = 0; j < kCols / 2; ++j) {
+                const float *cp = p.c + int64_t(m0 + r0_of(e) + 2 * j) * H + unit;
+                const int n = my_rows_of(e);
+                c2[e][j] = make_float2(2 * j < n ? cp[0] : 0.f, 2 * j + 1 < n ? cp[H] : 0.f);
+            }
 
-        // The stores of every step go to the same places: addresses are worked out once. An item of
-        // the hidden slice is (row, 16 units, projection half); of the projection (row, 8 columns, CTA).
+        // The stores of every step go to the same places: addresses are worked out once. An item of the
+        // hidden slice is (row, 16 units, projection half); of the projection (row, 8 columns, CTA).
         const uint32_t stage = smem_u32(smem + L.stage) + (warp - 2) * (kCols * 32);
         // A destination is 16-byte aligned; its low bits hold the peer's rank (the peer's mbarrier
         // address follows from it), 8 marks an item that exists.
-        uint32_t hs_dst[kBatches];   // lanes 0-15, one store per batch of four rows
+        uint32_t hs_dst[G][kBatches];   // lanes 0-15, one store per batch of four rows
 #pragma unroll
-        for (int b = 0; b < kBatches; ++b) {
-            const int row = 4 * b + (lane >> 2), ch = (lane >> 1) & 1;
-            const int pr = (r0 + row) / p.n_own, lr = (r0 + row) - pr * p.n_own;
-            const uint32_t to = uint32_t(2 * pr + (lane & 1));
-            hs_dst[b] = lane < 16 && row < my_rows
-                ? map_to_rank(smem_u32(smem + L.h + rank * (p.n_pad * 128)) + sw128_offset(lr, 2 * q + ch), to) | 8u | to
-                : 0u;
-        }
-        // ceil(ceil(NB / pairs) / 4) rows of 2 C items each: at most 24 items per 16 rows (C = 3)
-        uint32_t ps_src[kSendP], ps_dst[kSendP];
+        for (int e = 0; e < G; ++e)
+#pragma unroll
+            for (int b = 0; b < (e ? N1 / 16 : kBatches); ++b) {
+                const int row = 4 * b + (lane >> 2), ch = (lane >> 1) & 1, at = ug * share_of(e) + row;
+                const int pr = at / p.n_own[e], lr = at - pr * p.n_own[e];
+                const uint32_t to = uint32_t(2 * pr + (lane & 1));
+                hs_dst[e][b] = lane < 16 && row < my_rows_of(e)
+                    ? map_to_rank(smem_u32(smem + L.h + e * h_group1 + rank * ((e ? kPad1 : kPad0) * 128)) + sw128_offset(lr, 2 * q + ch), to) | 8u | to
+                    : 0u;
+            }
+        // ceil(ceil(N / pairs) / 4) rows of 2 C items each: at most 24 items per 16 rows (C = 3)
+        uint32_t ps_src[kSendP], ps_dst[G][kSendP];
 #pragma unroll
         for (int s = 0; s < kSendP; ++s) {
             const int id = lane + 32 * s, row = id / (2 * C), rest = id - row * 2 * C, ch = rest >= C ? 1 : 0;
             int to = rest - ch * C + rank;   // start with a different peer in every CTA
             if (to >= C) to -= C;
             ps_src[s] = stage + row * 32 + ch * 16;
-            ps_dst[s] = row < my_pr
-                ? map_to_rank(smem_u32(smem + L.hh + half * (NB * 128)) + sw128_offset(pair * p.n_own + pr0 + row, 2 * q + ch),
-                              uint32_t(to)) | 8u | uint32_t(to)
-                : 0u;
+#pragma unroll
+            for (int e = 0; e < G; ++e)
+                ps_dst[e][s] = row < my_pr_of(e)
+                    ? map_to_rank(smem_u32(smem + L.hh + half * (NB * 128)) +
+                                      sw128_offset(e * N0 + pair * p.n_own[e] + pr0_of(e) + row, 2 * q + ch), uint32_t(to)) | 8u | uint32_t(to)
+                    : 0u;
         }
         auto send = [&](uint32_t dst, uint32_t src, uint64_t *bar) {
             if (dst) store_to_peer(dst & ~15u, lds128(src), map_to_rank(smem_u32(bar), dst & 7u));
         };
-        // the hidden slice's 16-byte pieces in global memory: lane = (row, 16 units)
-        const bool g_ok = (lane >> 1) < my_rows;
-        const uint32_t g_src = stage + lane * 16;
-        const int64_t g_off = int64_t(m0 + r0 + (lane >> 1)) * p.H + n0 + q * 32 + (lane & 1) * 16;
-
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
-        bool ok = true;
-        for (int i = 0; i < p.T && ok; ++i) {
+        int i = 0;
+
+        // ---- projection of group e's h_{i-1}: int32 -> f16, to every CTA of the cluster ----
+        auto project_epilogue = [&](auto group) {
+            constexpr int e = decltype(group)::value;
+            const int my_pr = my_pr_of(e);
             if (my_pr > 0) {
-                // ---- projection of h_{i-1}: int32 -> f16, to every CTA of the cluster ----
-                ok = mbar_wait(bar_proj, i & 1, abort_flag, 102);
-                if (!ok) break;
-                FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 4, clock64());
+                if (!mbar_wait(&bar_proj[e], i & 1, abort_flag, 102)) return false;
+                FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 4, clock64());
                 tc_fence_after_sync();
+                const uint32_t t_proj = t_lane + 4 * NB + (e ? kPad0 : 0) + pr0_of(e);
                 for (int c = 0; c < my_pr; c += 4) {
                     uint32_t a[4];
-                    tmem_ld_32x4(t_lane + 4 * NB + pr0 + c, a);
+                    tmem_ld_32x4(t_proj + c, a);
                     tmem_ld_wait();
                     if (lane < 16) {
 #pragma unroll
@@ -379,15 +456,20 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 tc_fence_before_sync();
                 __syncwarp();
 #pragma unroll
-                for (int s = 0; s < kSendP; ++s)
-                    send(ps_dst[s], ps_src[s], bar_hh);
-                FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 5, clock64());
+                for (int s = 0; s < (e ? N1 / 16 : kSendP); ++s) send(ps_dst[e][s], ps_src[s], &bar_hh[e]);
+                FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 5, clock64());
                 __syncwarp();
             }
-            // ---- gates, cell update, hidden code ----
-            ok = mbar_wait(bar_acc, i & 1, abort_flag, 103);
-            if (!ok) break;
-            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 0, clock64());
+            return true;
+        };
+
+        // ---- gates, cell update, hidden code of group e ----
+        auto gate_epilogue = [&](auto group) {
+            constexpr int e = decltype(group)::value;
+            constexpr int kB = e ? N1 / 16 : kBatches;
+            const int my_rows = my_rows_of(e), r0 = r0_of(e);
+            if (!mbar_wait(&bar_acc[e], i & 1, abort_flag, 103)) return false;
+            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 0, clock64());
             tc_fence_after_sync();
             // Four rows at a time: the next four leave tensor memory while these are computed, and
             // each batch is sent as soon as it is staged, so the exchange runs beside the arithmetic.
@@ -398,15 +480,15 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             };
             load4(0);
 #pragma unroll
-            for (int b = 0; b < kBatches; ++b) {
+            for (int b = 0; b < kB; ++b) {
                 tmem_ld_wait();
-                if (b + 1 < kBatches) {
+                if (b + 1 < kB) {
                     load4(b + 1);
                 } else {
                     // all reads of the step are done: the x half of the next one may overwrite
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_acc_free);
+                    if (lane == 0) mbar_arrive(&bar_acc_free[e]);
                 }
                 const auto &v = a[b & 1];
                 if (4 * b < my_rows) {
@@ -415,31 +497,45 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     for (int j = 0; j < 2; ++j)
                         h[j] = lstm_cell_codes(v[0][2 * j], v[0][2 * j + 1], v[1][2 * j], v[1][2 * j + 1], v[2][2 * j], v[2][2 * j + 1],
                                                v[3][2 * j], v[3][2 * j + 1], make_float2(b_i, b_i), make_float2(b_f, b_f),
-                                               make_float2(b_g, b_g), make_float2(b_o, b_o), c2[2 * b + j]);
+                                               make_float2(b_g, b_g), make_float2(b_o, b_o), c2[e][2 * b + j]);
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         sts8(stage + (4 * b + 2 * j) * 32 + lane, h[j].x);
                         sts8(stage + (4 * b + 2 * j + 1) * 32 + lane, h[j].y);
                     }
                     __syncwarp();
-                    if (i + 1 < p.T) send(hs_dst[b], stage + b * 128 + (lane >> 1) * 16, bar_h);
+                    if (i + 1 < p.T) send(hs_dst[e][b], stage + b * 128 + (lane >> 1) * 16, &bar_h[e]);
                 }
             }
-            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 1, clock64());
-            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64, i * 8 + 2, clock64());
-            if (g_ok) {
-                const uint4 v = lds128(g_src);
-                *reinterpret_cast<uint4 *>(p.h_out + int64_t(time_of(i)) * p.B * p.H + g_off) = v;
-                if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + g_off) = v;
+            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 1, clock64());
+            // the slice's 16-byte pieces in global memory: lane = (row, 16 units)
+            if ((lane >> 1) < my_rows) {
+                const int64_t off = int64_t(m0 + r0 + (lane >> 1)) * H + n0 + q * 32 + (lane & 1) * 16;
+                const uint4 v = lds128(stage + lane * 16);
+                *reinterpret_cast<uint4 *>(p.h_out + int64_t(time_of(i)) * p.B * H + off) = v;
+                if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + off) = v;
             }
             __syncwarp();
+            return true;
+        };
+
+        for (; i < p.T; ++i) {
+            if (!project_epilogue(Int<0>{})) break;
+            if constexpr (G > 1)
+                if (!project_epilogue(Int<1>{})) break;
+            if (!gate_epilogue(Int<0>{})) break;
+            if constexpr (G > 1)
+                if (!gate_epilogue(Int<1>{})) break;
         }
 #pragma unroll
-        for (int j = 0; j < kCols / 2; ++j) {
-            float *cp = p.c + int64_t(m0 + r0 + 2 * j) * p.H + unit;
-            if (2 * j < my_rows) cp[0] = c2[j].x;
-            if (2 * j + 1 < my_rows) cp[p.H] = c2[j].y;
-        }
+        for (int e = 0; e < G; ++e)
+#pragma unroll
+            for (int j = 0; j < kCols / 2; ++j) {
+                float *cp = p.c + int64_t(m0 + r0_of(e) + 2 * j) * H + unit;
+                const int n = my_rows_of(e);
+                if (2 * j < n) cp[0] = c2[e][j].x;
+                if (2 * j + 1 < n) cp[H] = c2[e][j].y;
+            }
     }
 
     // Nobody leaves (and frees shared memory that a peer's store may still target) before every
@@ -459,41 +555,56 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 constexpr int kGMinRows = 2;  // fewer rows than this per cluster do not make a step shorter
 
 struct GroupPlan {
-    int nb;       // row columns of the kernel (16, 32 or 48)
-    int rows;     // rows per cluster
-    int tiles;    // clusters
-    int n_own, n_pad;
+    int kernel;       // index in kGroupKernels
+    int rows;         // rows per cluster
+    int tiles;        // clusters
 };
 
-constexpr int group_pad8(int v) { return (v + 7) / 8 * 8; }
+using group_kernel_fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GroupDev);
+struct GroupKernel { int n0, n1; group_kernel_fn fn[kGMaxCtas + 1]; };
+template <int N0, int N1, int C>
+constexpr group_kernel_fn group_kernel_fits() {
+    if constexpr (group_layout(N0, N1, C).dynamic <= kGMaxSmem) return lstm_group_kernel<N0, N1, C>;
+    else return nullptr;
+}
+template <int N0, int N1>
+constexpr GroupKernel group_kernels() {
+    return {N0, N1, {nullptr, nullptr, group_kernel_fits<N0, N1, 2>(), group_kernel_fits<N0, N1, 3>(), group_kernel_fits<N0, N1, 4>(),
+                     group_kernel_fits<N0, N1, 5>(), group_kernel_fits<N0, N1, 6>(), group_kernel_fits<N0, N1, 7>(),
+                     group_kernel_fits<N0, N1, 8>()}};
+}
+const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0>(), group_kernels<48, 0>(),
+                                     group_kernels<16, 16>(), group_kernels<32, 16>()};
 
-inline int group_smem(int nb, int rows, int H) {
-    const int n_pairs = H / kGUnits / 2;
-    return group_layout(nb, H, group_pad8((rows + n_pairs - 1) / n_pairs)).dynamic;
+// The kernel for `rows` rows per cluster of hidden size H, or -1: the narrowest that holds them, as two groups
+// when the second is at least half full. Step of one group against two at H = 768, in us: 20 rows per
+// cluster 2.47 : 2.53, 24 rows 2.65 : 2.59, 32 rows 3.04 : 2.59; 39 rows 3.36 : 3.51, 47 rows 3.63 : 3.51; at
+// H = 384 and 42 rows 3.87 : 3.27.
+inline int group_kernel_for(int rows, int H) {
+    const int C = H / kGUnits;
+    if (rows > 48) return -1;
+    const int one = rows <= 16 ? 0 : rows <= 32 ? 1 : 2, two = rows <= 32 ? 3 : 4;
+    const int want = one > 0 && rows - kGroupKernels[two].n0 >= kGroupKernels[two].n1 / 2 ? two : one;
+    return kGroupKernels[want].fn[C] ? want : kGroupKernels[one].fn[C] ? one : -1;
 }
 
-using group_kernel_fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GroupDev);
-inline group_kernel_fn group_kernel(int nb) {
-    return nb == 16 ? lstm_group_kernel<16> : nb == 32 ? lstm_group_kernel<32> : lstm_group_kernel<48>;
-}
-
-// Clusters of C CTAs of the NB-row kernel that the device runs at once with the largest shared
-// memory a CTA can have (0: the form is not available).
-int group_capacity(int nb, int C) {
-    static int known[64][3][kGMaxCtas + 1];  // n + 1, or -1
+// Clusters of C CTAs of kernel k that the device runs at once with the largest shared memory a CTA can
+// have (0: the form is not available).
+int group_capacity(int k, int C) {
+    static int known[64][sizeof(kGroupKernels) / sizeof(kGroupKernels[0])][kGMaxCtas + 1];  // n + 1, or -1
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return 0;
-    int &slot = known[dev][nb / 16 - 1][C];
+    int &slot = known[dev][k][C];
     if (slot == 0) {
         int n = 0;
-        const void *fn = reinterpret_cast<const void *>(group_kernel(nb));
-        bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448) == cudaSuccess;
+        const void *fn = reinterpret_cast<const void *>(kGroupKernels[k].fn[C]);
+        bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGMaxSmem) == cudaSuccess;
         if (ok) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(C);
             cfg.blockDim = dim3(kGThreads);
-            cfg.dynamicSmemBytes = 232448;
+            cfg.dynamicSmemBytes = kGMaxSmem;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = C;
@@ -515,21 +626,18 @@ bool group_plan(int B, int H, GroupPlan *g) {
     if (H % kGUnits) return false;
     const int C = H / kGUnits;
     if (C < 2 || C > kGMaxCtas) return false;
-    int max_nb = 48;
-    while (max_nb >= 16 && group_smem(max_nb, max_nb, H) > 232448) max_nb -= 16;
-    if (max_nb < 16) return false;
-    const int cap = group_capacity(max_nb, C);
+    int max_rows = 48;
+    while (max_rows > 0 && (g->kernel = group_kernel_for(max_rows, H)) < 0) max_rows -= 16;
+    if (max_rows < 16) return false;
+    const int cap = group_capacity(g->kernel, C);
     if (cap < 1) return false;
-    const int waves = (B + cap * max_nb - 1) / (cap * max_nb);
+    const int waves = (B + cap * max_rows - 1) / (cap * max_rows);
     int tiles = cap * waves;
     if (tiles > (B + kGMinRows - 1) / kGMinRows) tiles = (B + kGMinRows - 1) / kGMinRows;
     g->rows = (B + tiles - 1) / tiles;
     g->tiles = (B + g->rows - 1) / g->rows;
-    g->nb = (g->rows + 15) / 16 * 16;
-    if (group_capacity(g->nb, C) < 1) return false;
-    g->n_own = (g->rows + C / 2 - 1) / (C / 2);
-    g->n_pad = group_pad8(g->n_own);
-    return true;
+    g->kernel = group_kernel_for(g->rows, H);
+    return g->kernel >= 0 && group_capacity(g->kernel, C) > 0;
 }
 
 }  // namespace
@@ -543,11 +651,14 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     const int T = l->T, B = l->B, H = l->H, R = l->R;
     GroupPlan g;
     if (R != kGRank || !group_plan(B, H, &g)) return -2;
+    const GroupKernel &kn = kGroupKernels[g.kernel];
     const int C = H / kGUnits;
 
     GroupDev p;
-    p.T = T; p.B = B; p.H = H; p.reverse = l->reverse;
-    p.rows = g.rows; p.n_own = g.n_own; p.n_pad = g.n_pad; p.dn_ts = group_dn_ts(g.nb, H, g.n_pad);
+    p.T = T; p.B = B; p.reverse = l->reverse;
+    p.rows = g.rows;
+    const int in_group[2] = {kn.n1 ? min(g.rows, kn.n0) : g.rows, kn.n1 ? max(g.rows - kn.n0, 0) : 0};
+    for (int e = 0; e < 2; ++e) p.n_own[e] = max((in_group[e] + C / 2 - 1) / (C / 2), 1);
     p.dn = static_cast<const int8_t *>(l->dn_hh_i8);
     p.w_up = static_cast<const __half *>(l->w_up_f16);
     p.bias = static_cast<const float *>(l->bias_f32);
@@ -557,7 +668,7 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     p.h_state = static_cast<int8_t *>(l->h_i8);
     p.trace = trace_buffer();
 
-    CUtensorMap tm_w, tm_x, tm_dn, tm_h0;
+    CUtensorMap tm_w, tm_x, tm_dn, tm_h[2];
     int rc = make_tmap_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, l->w_up_f16, 4 * uint64_t(H), 2 * R, uint64_t(2 * R) * 2,
                           kGUnits, 64, true);
     if (rc) return rc;
@@ -565,24 +676,24 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
         // both K blocks of a row range in one box: the 128-byte blocks of a row are a dimension
         const uint64_t dims[4] = {64, uint64_t(B), 2, uint64_t(T)};
         const uint64_t strides[3] = {uint64_t(R) * 2, 128, uint64_t(B) * R * 2};
-        const uint32_t box[4] = {64, uint32_t(g.nb), 2, 1};
+        const uint32_t box[4] = {64, uint32_t(kn.n0 + kn.n1), 2, 1};
         rc = make_tmap_nd(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_down, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
     rc = make_tmap_2d(&tm_dn, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, l->dn_hh_i8, R, H, H, 64, 128, true);
     if (rc) return rc;
-    {
+    for (int e = 0; e < 2; ++e) {
         const uint64_t dims[3] = {128, uint64_t(B), uint64_t(C)};
         const uint64_t strides[2] = {uint64_t(H), 128};
-        const uint32_t box[3] = {128, uint32_t(g.n_pad), uint32_t(C)};
-        rc = make_tmap_nd(&tm_h0, CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_i8, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+        const uint32_t box[3] = {128, uint32_t(group_h_rows(e && kn.n1 ? kn.n1 : kn.n0, C)), uint32_t(C)};
+        rc = make_tmap_nd(&tm_h[e], CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_i8, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.tiles * C);
     cfg.blockDim = dim3(kGThreads);
-    cfg.dynamicSmemBytes = group_layout(g.nb, H, g.n_pad).dynamic;
+    cfg.dynamicSmemBytes = group_layout(kn.n0, kn.n1, C).dynamic;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -591,5 +702,5 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, group_kernel(g.nb), tm_w, tm_x, tm_dn, tm_h0, p);
+    return (int)cudaLaunchKernelEx(&cfg, kn.fn[C], tm_w, tm_x, tm_dn, tm_h[0], tm_h[1], p);
 }

@@ -406,14 +406,16 @@ def test_wide_l2_configuration_matches_the_narrow_one(flib):
         assert d.max() <= 1 and (d != 0).mean() < 5e-3
 
 
-@pytest.mark.parametrize("H,B", [(768, 1), (768, 45), (768, 352), (768, 353), (768, 704), (768, 705), (768, 1056), (768, 1057),
-                                 (256, 300), (384, 47), (384, 700), (512, 1600), (640, 90), (896, 500), (1024, 33), (1024, 481)])
+@pytest.mark.parametrize("H,B", [(768, 1), (768, 45), (768, 352), (768, 353), (768, 506), (768, 507), (768, 704), (768, 705),
+                                 (768, 858), (768, 859), (768, 1056), (768, 1057), (256, 300), (256, 2900), (384, 47), (384, 1600),
+                                 (384, 2048), (512, 1000), (512, 1600), (640, 90), (640, 1200), (896, 500), (896, 800), (1024, 33),
+                                 (1024, 470), (1024, 481)])
 def test_small_cluster_form_gives_the_bytes_of_the_l2_form(flib, H, B):
     """The default form (few chunk rows per cluster, operands swapped) against the L2-exchange form,
     which shares none of its data movement: same arithmetic in the same order, so equal bytes from a
-    non-zero state. Batches around the row counts where the kernel's column count (16, 32, 48) or the
-    number of waves changes on a B200, one row, ragged last clusters, an odd number of CTAs
-    (H = 384, 640, 896), one pair (256) and the largest cluster (1024)."""
+    non-zero state. Batches around the row counts per cluster where the kernel's column count (16, 32, 48),
+    the number of groups or the number of waves changes on a B200, one row, ragged last clusters (an
+    empty second group among them), every cluster size from 2 to 8 CTAs."""
     T, R = 4, 128
     layer, x, xs = _layer_case(T, B, H, R, H + B, B % 2 == 1)
     g = torch.Generator().manual_seed(B)
