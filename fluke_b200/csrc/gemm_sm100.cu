@@ -79,31 +79,40 @@ struct GemmDev {
 struct TrueTag { static constexpr bool value = true; };
 struct FalseTag { static constexpr bool value = false; };
 
-// The work list of a CTA: items w_begin, w_begin + w_step, ... < w_end; item -> first row.
-struct TileIter {
-    int w_begin, w_end, w_step;
-    __device__ __forceinline__ TileIter(const GemmDev &p, int m_first) {
+// Walks the work list of a CTA. The position is advanced, never recomputed from the item number: the integer
+// divisions of that lay on the path of every role (QKV + rotary [32000] 30.4 -> 28.8 us, gated MLP 52.3 -> 51.0).
+struct TileCursor {
+    int left;        // items still to do, this one included
+    int row;         // first row of the item's tile
+    int seq, s;      // sequence and tile in the sequence (whole sequences only)
+    __device__ __forceinline__ TileCursor(const GemmDev &p, int m_first) {
         if (p.seq_tiles > 0) {
-            w_begin = m_first * p.items_per_cta;
-            w_end = min(p.seq_tiles * p.n_seq, w_begin + p.items_per_cta);
-            w_step = 1;
+            const int w = m_first * p.items_per_cta;
+            left = min(p.seq_tiles * p.n_seq - w, p.items_per_cta);
+            s = w / p.n_seq;
+            seq = w - s * p.n_seq;
+            row = seq * p.seqlen + seq_pos0(p);
         } else {
-            w_begin = m_first;
-            w_end = p.num_m_tiles;
-            w_step = p.ctas_per_n;
+            left = (p.num_m_tiles - m_first + p.ctas_per_n - 1) / p.ctas_per_n;
+            seq = s = 0;
+            row = m_first * kBlockM;
         }
     }
-    // tile-in-sequence index (seq mode only)
-    __device__ __forceinline__ static int seq_index(const GemmDev &p, int w) { return w / p.n_seq; }
-    __device__ __forceinline__ static int seq_pos0(const GemmDev &p, int s) {
-        return min(s * kBlockM, p.seqlen - kBlockM);
-    }
-    __device__ __forceinline__ static int row0(const GemmDev &p, int w) {
+    __device__ __forceinline__ bool valid() const { return left > 0; }
+    // first position of the tile in its sequence
+    __device__ __forceinline__ int seq_pos0(const GemmDev &p) const { return min(s * kBlockM, p.seqlen - kBlockM); }
+    __device__ __forceinline__ void next(const GemmDev &p) {
+        --left;
         if (p.seq_tiles > 0) {
-            const int s = w / p.n_seq;
-            return (w - s * p.n_seq) * p.seqlen + seq_pos0(p, s);
+            row += p.seqlen;
+            if (++seq == p.n_seq) {
+                seq = 0;
+                ++s;
+                row = seq_pos0(p);
+            }
+        } else {
+            row += p.ctas_per_n * kBlockM;
         }
-        return w * kBlockM;
     }
 };
 
@@ -237,28 +246,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const TileIter it(p, m_first);
             // The CTAs that share an activation tile reach it at about the same time, so without
-            // help every tile load would pay the HBM latency. One of them (chosen by the tile
-            // index) asks for the tile kPrefetchTiles steps ahead to be brought into L2. With a
+            // help every tile load would pay the HBM latency. One of them (they take turns)
+            // asks for the tile kPrefetchTiles steps ahead to be brought into L2. With a
             // single N tile nothing is shared and the ring alone covers the latency.
-            auto prefetch_tile = [&](int w) {
-                if (p.num_n_tiles > 1 && w < it.w_end && (w % p.num_n_tiles) == n_tile) {
-                    const int m0 = TileIter::row0(p, w);
+            TileCursor ahead(p, m_first);
+            int turn = n_tile;
+            auto prefetch_tile = [&]() {
+                if (p.num_n_tiles > 1 && ahead.valid() && turn == 0)
                     for (int kb = 0; kb < p.num_k_blocks; ++kb)
-                        tma_prefetch_l2_3d(&tm_a, kb * kBlockKBytes, m0, p.a_plane);
-                }
+                        tma_prefetch_l2_3d(&tm_a, kb * kBlockKBytes, ahead.row, p.a_plane);
+                ahead.next(p);
+                if (++turn == p.num_n_tiles) turn = 0;
             };
-            for (int d = 0; d < kPrefetchTiles; ++d) prefetch_tile(it.w_begin + d * it.w_step);
-            for (int w = it.w_begin; w < it.w_end && ok; w += it.w_step) {
-                const int m0 = TileIter::row0(p, w);
-                prefetch_tile(w + kPrefetchTiles * it.w_step);
+            for (int d = 0; d < kPrefetchTiles; ++d) prefetch_tile();
+            for (TileCursor it(p, m_first); it.valid() && ok; it.next(p)) {
+                prefetch_tile();
                 for (int kb = 0; kb < p.num_k_blocks; ++kb) {
                     ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, 1);
                     if (!ok) break;
                     mbar_arrive_expect_tx(&full_bar[stage], L::kABytes);
                     tma_load_3d(smem + L::kOffA + stage * L::kABytes, &tm_a, &full_bar[stage],
-                                kb * kBlockKBytes, m0, p.a_plane);
+                                kb * kBlockKBytes, it.row, p.a_plane);
                     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -277,8 +286,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             uint32_t phase = 0;
             int local = 0;
             bool ok = mbar_wait(w_bar, 0, abort_flag, 6);
-            const TileIter it(p, m_first);
-            for (int w = it.w_begin; w < it.w_end && ok; w += it.w_step, ++local) {
+            for (TileCursor it(p, m_first); it.valid() && ok; it.next(p), ++local) {
                 const int acc = local & 1;
                 const uint32_t acc_phase = (local >> 1) & 1;
                 ok = mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag, 2);
@@ -321,7 +329,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         const int ch = (warp - kEpilogueWarp0) >> 2;      // which of the quadrant's two warps
         const int g8 = lane >> 2, t4 = lane & 3;
         uint8_t *staging = smem + L::kOffStaging + (warp - kEpilogueWarp0) * kStagingBytes;
-        const TileIter it(p, m_first);
+        TileCursor it(p, m_first);
         int local = 0;
         bool ok = true;
 
@@ -336,14 +344,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
 
         if constexpr (EPI == FLUKE_SM100_EPI_RAW) {
             // 32-bit accumulators, no scaling: thread = row, 32 columns per store
-            for (int w = it.w_begin; w < it.w_end && ok; w += it.w_step, ++local) {
-                const int m0 = TileIter::row0(p, w);
+            for (; it.valid() && ok; ++local) {
+                const int m0 = it.row;
                 const int acc = local & 1;
                 const uint32_t acc_phase = (local >> 1) & 1;
                 ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 4);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN_MMA;
+                it.next(p);
                 constexpr int kChunks = kWarpCols / 32;
 #pragma unroll 1
                 for (int chunk = 0; chunk < kChunks; ++chunk) {
@@ -403,23 +412,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             const bool seq_mode = p.seq_tiles > 0;
             int cur_s = -1;
             float sa_next[4];
-            if (it.w_begin < it.w_end) load_sa(TileIter::row0(p, it.w_begin), sa_next);
-            for (int w = it.w_begin; w < it.w_end && ok; w += it.w_step, ++local) {
-                const int m0 = TileIter::row0(p, w);
+            if (it.valid()) load_sa(it.row, sa_next);
+            for (; it.valid() && ok; ++local) {
+                const int m0 = it.row;
                 const int acc = local & 1;
                 const uint32_t acc_phase = (local >> 1) & 1;
                 float2 sa2[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) sa2[k] = make_float2(sa_next[k], sa_next[k]);
-                if (w + it.w_step < it.w_end) load_sa(TileIter::row0(p, w + it.w_step), sa_next);
+                const int s_idx = it.s, pos0 = it.seq_pos0(p);
+                it.next(p);
+                if (it.valid()) load_sa(it.row, sa_next);
                 if (rotate) {
                     if (seq_mode) {
                         // the positions only change when the tile-in-sequence index does
-                        const int s_idx = TileIter::seq_index(p, w);
                         if (s_idx != cur_s) {
                             cur_s = s_idx;
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) load_tables(k, TileIter::seq_pos0(p, s_idx) + q * 32 + g8 + 8 * k);
+                            for (int k = 0; k < 4; ++k) load_tables(k, pos0 + q * 32 + g8 + 8 * k);
                         }
                     } else {
 #pragma unroll
@@ -515,15 +525,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 }
             }
             float sa_next[4];
-            if (it.w_begin < it.w_end) load_sa(TileIter::row0(p, it.w_begin), sa_next);
-            for (int w = it.w_begin; w < it.w_end && ok; w += it.w_step, ++local) {
-                const int m0 = TileIter::row0(p, w);
+            if (it.valid()) load_sa(it.row, sa_next);
+            for (; it.valid() && ok; ++local) {
+                const int m0 = it.row;
                 const int acc = local & 1;
                 const uint32_t acc_phase = (local >> 1) & 1;
                 float2 sa2[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) sa2[k] = make_float2(sa_next[k], sa_next[k]);
-                if (w + it.w_step < it.w_end) load_sa(TileIter::row0(p, w + it.w_step), sa_next);
+                it.next(p);
+                if (it.valid()) load_sa(it.row, sa_next);
 
                 ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, 4);
                 if (!ok) break;
