@@ -100,8 +100,8 @@ __host__ __device__ constexpr GroupLayout group_layout_slots(int n0, int n1, int
     l.hh = l.x + x_slots * n * 256;             // hh_down rows, the same shape
     l.dn = l.hh + n * 256;                      // 64 projection rows: the K blocks not in tensor memory [64 x 128 B]
     l.h = l.dn + 8192 * (C - group_dn_ts(n0, n1, C));  // hidden rows of the pair, per group: C K blocks
-    l.stage = l.h + (group_h_rows(n0, C) + group_h_rows(n1, C)) * C * kGUnits;  // 16 warps x (n0/4 rows x 32 B)
-    l.bars = l.stage + n0 * 128;
+    l.stage = l.h + (group_h_rows(n0, C) + group_h_rows(n1, C)) * C * kGUnits;  // 16 warps x (a quarter of the larger group x 32 B)
+    l.bars = l.stage + (n0 > n1 ? n0 : n1) * 128;
     l.misc = l.bars + 15 * 8;
     l.dynamic = l.misc + 16 + 1024;             // slack for the manual 1024-byte alignment
     return l;
@@ -157,10 +157,10 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     constexpr int kPad0 = group_h_rows(N0, C), kPad1 = group_h_rows(N1, C);
     constexpr int kDnTs = group_dn_ts(N0, N1, C);
     constexpr GroupLayout L = group_layout(N0, N1, C);
-    constexpr int kCols = N0 / 4;                    // rows of the first group that an epilogue thread holds at most
+    constexpr int kCols = (N0 > N1 ? N0 : N1) / 4;   // rows of a group that an epilogue thread holds at most
     constexpr int kBatches = kCols / 4;              // it takes them four at a time
-    constexpr int kSendP = N0 / 16;                  // 16-byte stores per lane and step, projections
-    static_assert(N0 % 16 == 0 && N1 % 16 == 0 && N1 <= N0 && 5 * NB <= kGTmemW, "accumulators beside the weights in tensor memory");
+    constexpr int kSendP = kCols / 4;                // 16-byte stores per lane and step, projections
+    static_assert(N0 % 16 == 0 && N1 % 16 == 0 && 5 * NB <= kGTmemW, "accumulators beside the weights in tensor memory");
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
     // shared-window offsets as this CTA's
@@ -358,9 +358,9 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (!wait_x()) break;
                 x_half(Int<0>{}, Int<1>{});
                 if (!project(Int<0>{})) break;
-                x_half(Int<1>{}, Int<2>{});
+                x_half(Int<1>{}, Int<3>{});
                 if (!project(Int<1>{})) break;
-                x_half(Int<2>{}, Int<4>{});
+                x_half(Int<3>{}, Int<4>{});
                 if (!hh_half(Int<0>{})) break;
                 if (!hh_half(Int<1>{})) break;
             }
@@ -404,7 +404,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 #pragma unroll
         for (int e = 0; e < G; ++e)
 #pragma unroll
-            for (int b = 0; b < (e ? N1 / 16 : kBatches); ++b) {
+            for (int b = 0; b < (e ? N1 : N0) / 16; ++b) {
                 const int row = 4 * b + (lane >> 2), ch = (lane >> 1) & 1, at = ug * share_of(e) + row;
                 const int pr = at / p.n_own[e], lr = at - pr * p.n_own[e];
                 const uint32_t to = uint32_t(2 * pr + (lane & 1));
@@ -456,7 +456,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 tc_fence_before_sync();
                 __syncwarp();
 #pragma unroll
-                for (int s = 0; s < (e ? N1 / 16 : kSendP); ++s) send(ps_dst[e][s], ps_src[s], &bar_hh[e]);
+                for (int s = 0; s < (e ? N1 : N0) / 16; ++s) send(ps_dst[e][s], ps_src[s], &bar_hh[e]);
                 FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 5, clock64());
                 __syncwarp();
             }
@@ -466,29 +466,33 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         // ---- gates, cell update, hidden code of group e ----
         auto gate_epilogue = [&](auto group) {
             constexpr int e = decltype(group)::value;
-            constexpr int kB = e ? N1 / 16 : kBatches;
+            constexpr int kB = (e ? N1 : N0) / 16;
             const int my_rows = my_rows_of(e), r0 = r0_of(e);
             if (!mbar_wait(&bar_acc[e], i & 1, abort_flag, 103)) return false;
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 0, clock64());
             tc_fence_after_sync();
-            // Four rows at a time: the next four leave tensor memory while these are computed, and
-            // each batch is sent as soon as it is staged, so the exchange runs beside the arithmetic.
+            // Four rows at a time, and each batch is sent as soon as it is staged, so that the exchange runs
+            // beside the arithmetic. Two batches are read at the start, which hands the accumulators back
+            // before the arithmetic; a third while the first is computed.
             uint32_t a[2][4][4];
             auto load4 = [&](int b) {
 #pragma unroll
                 for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_lane + g * NB + r0 + 4 * b, a[b & 1][g]);
             };
+            auto hand_back = [&]() {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_acc_free[e]);
+            };
             load4(0);
+            if (kB > 1) load4(1);
+            tmem_ld_wait();
+            if (kB <= 2) hand_back();
 #pragma unroll
             for (int b = 0; b < kB; ++b) {
-                tmem_ld_wait();
-                if (b + 1 < kB) {
-                    load4(b + 1);
-                } else {
-                    // all reads of the step are done: the x half of the next one may overwrite
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_acc_free[e]);
+                if (b == 2) {
+                    tmem_ld_wait();
+                    hand_back();
                 }
                 const auto &v = a[b & 1];
                 if (4 * b < my_rows) {
@@ -506,6 +510,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     __syncwarp();
                     if (i + 1 < p.T) send(hs_dst[e][b], stage + b * 128 + (lane >> 1) * 16, &bar_h[e]);
                 }
+                if (b == 0 && kB > 2) load4(2);
             }
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 1, clock64());
             // the slice's 16-byte pieces in global memory: lane = (row, 16 units)
@@ -574,7 +579,7 @@ constexpr GroupKernel group_kernels() {
                      group_kernel_fits<N0, N1, 8>()}};
 }
 const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0>(), group_kernels<48, 0>(),
-                                     group_kernels<16, 16>(), group_kernels<32, 16>()};
+                                     group_kernels<16, 16>(), group_kernels<16, 32>()};
 
 // The kernel for `rows` rows per cluster of hidden size H, or -1: the narrowest that holds them, as two groups
 // when the second is at least half full. Step of one group against two at H = 768, in us: 20 rows per
@@ -584,7 +589,7 @@ inline int group_kernel_for(int rows, int H) {
     const int C = H / kGUnits;
     if (rows > 48) return -1;
     const int one = rows <= 16 ? 0 : rows <= 32 ? 1 : 2, two = rows <= 32 ? 3 : 4;
-    const int want = one > 0 && rows - kGroupKernels[two].n0 >= kGroupKernels[two].n1 / 2 ? two : one;
+    const int want = one > 0 && rows >= (rows <= 32 ? 24 : 40) ? two : one;
     return kGroupKernels[want].fn[C] ? want : kGroupKernels[one].fn[C] ? one : -1;
 }
 
