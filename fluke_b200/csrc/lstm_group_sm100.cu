@@ -473,27 +473,21 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             tc_fence_after_sync();
             // Four rows at a time, and each batch is sent as soon as it is staged, so that the exchange runs
             // beside the arithmetic. Two batches are read at the start, which hands the accumulators back
-            // before the arithmetic; a third while the first is computed.
+            // before the arithmetic.
+            static_assert(kB <= 2, "two batches are in registers");
             uint32_t a[2][4][4];
             auto load4 = [&](int b) {
 #pragma unroll
                 for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_lane + g * NB + r0 + 4 * b, a[b & 1][g]);
             };
-            auto hand_back = [&]() {
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_acc_free[e]);
-            };
             load4(0);
             if (kB > 1) load4(1);
             tmem_ld_wait();
-            if (kB <= 2) hand_back();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_acc_free[e]);
 #pragma unroll
             for (int b = 0; b < kB; ++b) {
-                if (b == 2) {
-                    tmem_ld_wait();
-                    hand_back();
-                }
                 const auto &v = a[b & 1];
                 if (4 * b < my_rows) {
                     int2 h[2];
@@ -510,7 +504,6 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     __syncwarp();
                     if (i + 1 < p.T) send(hs_dst[e][b], stage + b * 128 + (lane >> 1) * 16, &bar_h[e]);
                 }
-                if (b == 0 && kB > 2) load4(2);
             }
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 1, clock64());
             // the slice's 16-byte pieces in global memory: lane = (row, 16 units)
@@ -578,19 +571,16 @@ constexpr GroupKernel group_kernels() {
                      group_kernel_fits<N0, N1, 5>(), group_kernel_fits<N0, N1, 6>(), group_kernel_fits<N0, N1, 7>(),
                      group_kernel_fits<N0, N1, 8>()}};
 }
-const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0>(), group_kernels<48, 0>(),
-                                     group_kernels<16, 16>(), group_kernels<16, 32>()};
+const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0>(), group_kernels<16, 16>(), group_kernels<16, 32>()};
 
-// The kernel for `rows` rows per cluster of hidden size H, or -1: the narrowest that holds them, as two groups
-// when the second is at least half full. Step of one group against two at H = 768, in us: 20 rows per
-// cluster 2.47 : 2.53, 24 rows 2.65 : 2.59, 32 rows 3.04 : 2.59; 39 rows 3.36 : 3.51, 47 rows 3.63 : 3.51; at
-// H = 384 and 42 rows 3.87 : 3.27.
+// The kernel for `rows` rows per cluster of hidden size H, or -1. Two groups from 24 rows on, with few CTAs per
+// cluster (short exchanges) from 17. Step of one group against two, in us: H = 768, 20 rows per cluster 2.42 : 2.51,
+// 23 rows 2.58 : 2.56, 32 rows 3.03 : 2.59, 39 rows 3.36 : 2.93, 48 rows 3.66 : 3.11; H = 384, 17 rows
+// 2.34 : 2.22, 40 rows 3.77 : 3.04; H = 1024, 22 rows 2.66 : 2.77, 32 rows 3.09 : 2.85.
 inline int group_kernel_for(int rows, int H) {
     const int C = H / kGUnits;
-    if (rows > 48) return -1;
-    const int one = rows <= 16 ? 0 : rows <= 32 ? 1 : 2, two = rows <= 32 ? 3 : 4;
-    const int want = one > 0 && rows >= (rows <= 32 ? 24 : 40) ? two : one;
-    return kGroupKernels[want].fn[C] ? want : kGroupKernels[one].fn[C] ? one : -1;
+    const int k = rows <= 16 ? 0 : rows <= 32 ? (rows < 24 && C >= 4 ? 1 : 2) : 3;
+    return rows <= 48 && kGroupKernels[k].fn[C] ? k : -1;
 }
 
 // Clusters of C CTAs of kernel k that the device runs at once with the largest shared memory a CTA can
