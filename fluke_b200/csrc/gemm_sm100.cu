@@ -178,6 +178,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             const GemmDev p) {
     using L = SmemLayout<EPI, BN_MMA, STAGES>;
     constexpr bool kDual = (EPI == FLUKE_SM100_EPI_SILU);
+    constexpr bool kRotary = (EPI == FLUKE_SM100_EPI_ROTARY);
     constexpr int BN_OUT = kDual ? BN_MMA / 2 : BN_MMA;  // output columns per tile
     constexpr int kWarpCols = BN_OUT / 2;                // output columns per epilogue warp
     constexpr uint32_t kTmemCols = 2 * BN_MMA;  // two accumulator buffers (256 or 512)
@@ -380,8 +381,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     }
                 }
             }
-        } else if constexpr (EPI == FLUKE_SM100_EPI_ROTARY) {
-            // A tile is four heads; warp `ch` owns heads 2*ch and 2*ch+1. Accumulators come in the
+        } else if constexpr (BN_OUT == 256) {
+            // The rotary form, and the plain ones where their tiles are as wide (columns in blocks of 64 for
+            // heads, nothing rotated). A tile is four heads; warp `ch` owns heads 2*ch and 2*ch+1. Accumulators come in the
             // 16-lane x 256-bit layout: a thread holds columns 8j + 2t, +1 (j = 0..7) of a head for
             // rows g + 8k (k = 0..3) of its quadrant, so both halves of a rotation pair (columns i
             // and i + 32: j and j + 4) are its own, its 32 column scales never change (registers),
@@ -391,8 +393,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
             // tile. The epilogue reads nothing from shared memory; its outputs, which are 8 x 8
             // matrix fragments in this layout, go to the staging tile four matrices per
             // instruction (stmatrix).
-            static_assert(BN_OUT == 256, "two heads per epilogue warp");
-            const bool rotate = n0 < p.qk_cols;
+            const bool rotate = kRotary && n0 < p.qk_cols;
+            auto scaled = [](float2 v, float2 sa, float2 sb) {
+                return EPI == FLUKE_SM100_EPI_DEQUANT ? mul2(v, mul2(sa, sb)) : mul2(mul2(v, sa), sb);
+            };
             float2 sc[2][8];
 #pragma unroll
             for (int h2 = 0; h2 < 2; ++h2)
@@ -476,9 +480,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                                 // (acc*sa)*sb, then the rotation in a fixed operation order (no
                                 // compiler-chosen contraction): lo' = fma(x0, cos, -(x1*sin)),
                                 // hi' = fma(x0, sin, x1*cos)
-                                const float2 x0 = mul2(mul2(acc_to_float2<KIND>(a[4 * j + 2 * k2], a[4 * j + 2 * k2 + 1]), sa2[k]), sc[h2][j]);
-                                const float2 x1 = mul2(mul2(acc_to_float2<KIND>(a[4 * (j + 4) + 2 * k2], a[4 * (j + 4) + 2 * k2 + 1]), sa2[k]),
-                                                       sc[h2][j + 4]);
+                                const float2 x0 = scaled(acc_to_float2<KIND>(a[4 * j + 2 * k2], a[4 * j + 2 * k2 + 1]), sa2[k], sc[h2][j]);
+                                const float2 x1 = scaled(acc_to_float2<KIND>(a[4 * (j + 4) + 2 * k2], a[4 * (j + 4) + 2 * k2 + 1]), sa2[k],
+                                                         sc[h2][j + 4]);
                                 float2 o_lo = x0, o_hi = x1;
                                 if constexpr (kRot) {
                                     const float2 m = mul2(x1, sn2[k][j]);
@@ -502,8 +506,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 };
 #pragma unroll
                 for (int h2 = 0; h2 < 2; ++h2) {
-                    if (rotate) head_math(TrueTag{}, h2);
-                    else head_math(FalseTag{}, h2);
+                    if constexpr (kRotary) {
+                        if (rotate) head_math(TrueTag{}, h2);
+                        else head_math(FalseTag{}, h2);
+                    } else {
+                        head_math(FalseTag{}, h2);
+                    }
                 }
             }
         } else {
@@ -747,7 +755,8 @@ namespace fluke_sm100 {
 namespace {
 
 // Tile shapes: 128 x 128 (K up to 1024 resident) for the plain GEMMs; 128 x 256 (one UMMA of
-// N = 256 per K step, K up to 512 resident) for the two fused transformer kernels. Beside the
+// N = 256 per K step, K up to 512 resident) for the two fused transformer kernels and plain ones of
+// many rows. Beside the
 // resident weight tile and 32 KB of store staging there is room for a ring of four 16 KB
 // activation stages.
 constexpr int kPlainBN = 128, kFusedBN = 256;
@@ -770,6 +779,15 @@ int tile_width(const fluke_sm100_gemm_t *g) {
         if (m_tiles * (g->N / bn) <= sms * per_sm) return bn;
     }
     return 0;
+}
+
+// Plain GEMMs of many rows take 256 columns per CTA like the fused ones, which halves how often the
+// activations are read (each item of work moves 64 KB of them into its SM). [M, 512] x [512, 512]: 128000 rows
+// 50.5 -> 41 us, 64000 24.0 -> 21.8, 20000 11.5 -> 10.4, 32000 even; with two rounds or less of wide tiles the
+// coarser items cost more (9331 rows 5.4 -> 5.7).
+bool wide_tiles(const fluke_sm100_gemm_t *g) {
+    if (g->N % kFusedBN != 0 || g->K > 512) return false;
+    return (g->M + 127) / 128 > 2 * (device_sm_count() / (g->N / kFusedBN));
 }
 
 template <int KIND, int EPI>
@@ -797,8 +815,10 @@ int dispatch(const fluke_sm100_gemm_t *g, cudaStream_t s) {
         case FLUKE_SM100_EPI_RAW:
             return launch<KIND, FLUKE_SM100_EPI_RAW, kPlainBN, kPlainStages>(g, s);
         case FLUKE_SM100_EPI_DEQUANT:
+            if (wide_tiles(g)) return launch<KIND, FLUKE_SM100_EPI_DEQUANT, kFusedBN, kFusedStages>(g, s);
             return launch<KIND, FLUKE_SM100_EPI_DEQUANT, kPlainBN, kPlainStages>(g, s);
         case FLUKE_SM100_EPI_DEQUANT2:
+            if (wide_tiles(g)) return launch<KIND, FLUKE_SM100_EPI_DEQUANT2, kFusedBN, kFusedStages>(g, s);
             return launch<KIND, FLUKE_SM100_EPI_DEQUANT2, kPlainBN, kPlainStages>(g, s);
         case FLUKE_SM100_EPI_ROTARY:
             return launch<KIND, FLUKE_SM100_EPI_ROTARY, kFusedBN, kFusedStages>(g, s);

@@ -457,3 +457,19 @@ def test_down_projection_of_few_rows_vs_oracle(m, n, k):
     ops.down_proj_i8(a.to(DEV), b.to(DEV), sa.to(DEV), sb.to(DEV), out=wide[:, n:])
     assert np.array_equal(wide[:, n:].cpu().numpy(), port.gemm_i8(a.numpy(), b.numpy(), sa.numpy(), sb.numpy()))
     assert bool((wide[:, :n] == 7.0).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(18944, 512, 512), (18945, 512, 512), (9473, 1024, 384), (38000, 256, 80)])
+def test_wide_plain_tiles_give_the_bits_of_narrow_ones(m, n, k):
+    """Both sides of the row count where a plain GEMM takes 256 columns per CTA on a B200, a K that ends
+    inside a 128-byte block, one N tile: equal to calls over a few rows each, int8 and fp8."""
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x, w = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV) * 0.05
+    for fp8 in (False, True):
+        quantise = prep.quantize_fp8_rows if fp8 else prep.quantize_int8_rows
+        (a, sa), (b, sb) = quantise(x), quantise(w)
+        run = (lambda a, sa: ops.gemm_fp8(a.view(torch.uint8), b.view(torch.uint8), sa, sb)) if fp8 else \
+              (lambda a, sa: ops.gemm_i8(a, b, sa, sb))
+        got = run(a, sa)
+        for r0 in (0, 127, m // 2, m - 300):
+            assert torch.equal(got[r0:r0 + 300], run(a[r0:r0 + 300].contiguous(), sa[r0:r0 + 300].contiguous()))
