@@ -90,6 +90,11 @@ __host__ __device__ constexpr int group_dn_ts(int n0, int n1, int C) {
     const int fit = (kGTmemW - 4 * (n0 + n1) - group_h_rows(n0, C) - group_h_rows(n1, C)) / 32;
     return fit < C ? fit : C;
 }
+// Rows of a staging slot: a batch of four hidden rows, or the projected rows of a quarter of the warps.
+__host__ __device__ constexpr int group_stage_rows(int n0, int n1, int C) {
+    const int r = group_h_rows(n0 > n1 ? n0 : n1, C) / 4;
+    return r > 4 ? r : 4;
+}
 struct GroupLayout {
     int x, hh, dn, h, stage, bars, misc, dynamic;
 };
@@ -100,8 +105,8 @@ __host__ __device__ constexpr GroupLayout group_layout_slots(int n0, int n1, int
     l.hh = l.x + x_slots * n * 256;             // hh_down rows, the same shape
     l.dn = l.hh + n * 256;                      // 64 projection rows: the K blocks not in tensor memory [64 x 128 B]
     l.h = l.dn + 8192 * (C - group_dn_ts(n0, n1, C));  // hidden rows of the pair, per group: C K blocks
-    l.stage = l.h + (group_h_rows(n0, C) + group_h_rows(n1, C)) * C * kGUnits;  // 16 warps x (a quarter of the larger group x 32 B)
-    l.bars = l.stage + (n0 > n1 ? n0 : n1) * 128;
+    l.stage = l.h + (group_h_rows(n0, C) + group_h_rows(n1, C)) * C * kGUnits;  // 2 slots x 4 x [rows x 128 B]
+    l.bars = l.stage + 8 * group_stage_rows(n0, n1, C) * 128;
     l.misc = l.bars + 15 * 8;
     l.dynamic = l.misc + 16 + 1024;             // slack for the manual 1024-byte alignment
     return l;
@@ -135,6 +140,19 @@ __device__ __forceinline__ void sts16(uint32_t addr, unsigned short v) {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
 }
 
+// Barrier of the four warps that share a staging slot. True if all four say so: a warp whose wait ran out
+// takes the others along instead of leaving them at the barrier.
+__device__ __forceinline__ bool quad_agree(int id, bool mine) {
+    int all;
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "setp.ne.s32 p, %2, 0;\n"
+        "barrier.cta.red.and.pred q, %1, 128, p;\n"
+        "selp.s32 %0, 1, 0, q;\n}"
+        : "=r"(all) : "r"(id), "r"(int(mine)) : "memory");
+    return all != 0;
+}
+
 template <int V>
 struct Int { static constexpr int value = V; };  // a number that a lambda receives as a type
 
@@ -160,6 +178,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     constexpr int kCols = (N0 > N1 ? N0 : N1) / 4;   // rows of a group that an epilogue thread holds at most
     constexpr int kBatches = kCols / 4;              // it takes them four at a time
     constexpr int kSendP = kCols / 4;                // 16-byte stores per lane and step, projections
+    constexpr int kStageRows = group_stage_rows(N0, N1, C);
     static_assert(N0 % 16 == 0 && N1 % 16 == 0 && 5 * NB <= kGTmemW, "accumulators beside the weights in tensor memory");
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
@@ -395,40 +414,48 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 c2[e][j] = make_float2(2 * j < n ? cp[0] : 0.f, 2 * j + 1 < n ? cp[H] : 0.f);
             }
 
-        // The stores of every step go to the same places: addresses are worked out once. An item of the
-        // hidden slice is (row, 16 units, projection half); of the projection (row, 8 columns, CTA).
-        const uint32_t stage = smem_u32(smem + L.stage) + (warp - 2) * (kCols * 32);
-        // A destination is 16-byte aligned; its low bits hold the peer's rank (the peer's mbarrier
-        // address follows from it), 8 marks an item that exists.
-        uint32_t hs_dst[G][kBatches];   // lanes 0-15, one store per batch of four rows
+        // What a CTA sends leaves in rows of 128 bytes, eight lanes each: the network between the SMs moves 64
+        // contiguous bytes to one CTA in the time of 16 (20.7 against 9.5 B per cycle and SM, measured with
+        // six CTAs sending to each other). A warp holds 32 bytes of a row, so the four warps of a quarter stage
+        // together, in two slots in turn: the barrier after one batch is staged also says that the slot of
+        // the batch before has been read.
+        const uint32_t stage = smem_u32(smem + L.stage) + ug * (kStageRows * 128);
+        uint32_t slot = 0;
+        auto next_slot = [&]() { slot ^= 4 * kStageRows * 128; };
+        // The stores of every step go to the same places: addresses are worked out once. A destination is
+        // 16-byte aligned; its low bits hold the peer's rank (the peer's mbarrier address follows from
+        // it), 8 marks one that exists. Lane 8 j + c stores piece c of the swizzled row.
+        uint32_t hs_dst[G][kBatches];   // lanes 0-15: row q of a batch of four, to both CTAs of the pair
 #pragma unroll
         for (int e = 0; e < G; ++e)
 #pragma unroll
             for (int b = 0; b < (e ? N1 : N0) / 16; ++b) {
-                const int row = 4 * b + (lane >> 2), ch = (lane >> 1) & 1, at = ug * share_of(e) + row;
+                const int row = 4 * b + q, at = ug * share_of(e) + row;
                 const int pr = at / p.n_own[e], lr = at - pr * p.n_own[e];
-                const uint32_t to = uint32_t(2 * pr + (lane & 1));
+                const uint32_t to = uint32_t(2 * pr + (lane >> 3));
                 hs_dst[e][b] = lane < 16 && row < my_rows_of(e)
-                    ? map_to_rank(smem_u32(smem + L.h + e * h_group1 + rank * ((e ? kPad1 : kPad0) * 128)) + sw128_offset(lr, 2 * q + ch), to) | 8u | to
+                    ? map_to_rank(smem_u32(smem + L.h + e * h_group1 + rank * ((e ? kPad1 : kPad0) * 128)) + lr * 128 + (lane & 7) * 16, to) | 8u | to
                     : 0u;
             }
-        // ceil(ceil(N / pairs) / 4) rows of 2 C items each: at most 24 items per 16 rows (C = 3)
+        // ceil(ceil(N / pairs) / 4) rows to C CTAs each: at most 12 (row, CTA) per 16 rows (C = 3), 16 per store
         uint32_t ps_src[kSendP], ps_dst[G][kSendP];
 #pragma unroll
         for (int s = 0; s < kSendP; ++s) {
-            const int id = lane + 32 * s, row = id / (2 * C), rest = id - row * 2 * C, ch = rest >= C ? 1 : 0;
-            int to = rest - ch * C + rank;   // start with a different peer in every CTA
+            const int id = 16 * s + 4 * q + (lane >> 3), row = id / C;
+            int to = id - row * C + rank;   // start with a different peer in every CTA
             if (to >= C) to -= C;
-            ps_src[s] = stage + row * 32 + ch * 16;
+            ps_src[s] = row * 128;
 #pragma unroll
             for (int e = 0; e < G; ++e)
                 ps_dst[e][s] = row < my_pr_of(e)
                     ? map_to_rank(smem_u32(smem + L.hh + half * (NB * 128)) +
-                                      sw128_offset(e * N0 + pair * p.n_own[e] + pr0_of(e) + row, 2 * q + ch), uint32_t(to)) | 8u | uint32_t(to)
+                                      (e * N0 + pair * p.n_own[e] + pr0_of(e) + row) * 128 + (lane & 7) * 16, uint32_t(to)) | 8u | uint32_t(to)
                     : 0u;
         }
-        auto send = [&](uint32_t dst, uint32_t src, uint64_t *bar) {
-            if (dst) store_to_peer(dst & ~15u, lds128(src), map_to_rank(smem_u32(bar), dst & 7u));
+        // the piece of a staged row that belongs at a destination of the 128-byte swizzle
+        auto piece = [&](uint32_t dst) { return (uint32_t(lane) ^ (dst >> 7)) & 7u; };
+        auto send = [&](uint32_t dst, uint4 v, uint64_t *bar) {
+            store_to_peer(dst & ~15u, v, map_to_rank(smem_u32(bar), dst & 7u));
         };
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
         int i = 0;
@@ -438,11 +465,12 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             constexpr int e = decltype(group)::value;
             const int my_pr = my_pr_of(e);
             if (my_pr > 0) {
-                if (!mbar_wait(&bar_proj[e], i & 1, abort_flag, 102)) return false;
+                const bool ok = mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
+                next_slot();
                 FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 4, clock64());
                 tc_fence_after_sync();
                 const uint32_t t_proj = t_lane + 4 * NB + (e ? kPad0 : 0) + pr0_of(e);
-                for (int c = 0; c < my_pr; c += 4) {
+                for (int c = 0; c < my_pr && ok; c += 4) {
                     uint32_t a[4];
                     tmem_ld_32x4(t_proj + c, a);
                     tmem_ld_wait();
@@ -450,15 +478,15 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
                             if (c + j < my_pr)
-                                sts16(stage + (c + j) * 32 + lane * 2, __half_as_ushort(__float2half_rn(float(int(a[j])) * sc)));
+                                sts16(stage + slot + (c + j) * 128 + q * 32 + lane * 2, __half_as_ushort(__float2half_rn(float(int(a[j])) * sc)));
                     }
                 }
                 tc_fence_before_sync();
-                __syncwarp();
+                if (!quad_agree(1 + ug, ok)) return false;
 #pragma unroll
-                for (int s = 0; s < (e ? N1 : N0) / 16; ++s) send(ps_dst[e][s], ps_src[s], &bar_hh[e]);
+                for (int s = 0; s < (e ? N1 : N0) / 16; ++s)
+                    if (const uint32_t dst = ps_dst[e][s]) send(dst, lds128(stage + slot + ps_src[s] + piece(dst) * 16), &bar_hh[e]);
                 FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 5, clock64());
-                __syncwarp();
             }
             return true;
         };
@@ -468,11 +496,11 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             constexpr int e = decltype(group)::value;
             constexpr int kB = (e ? N1 : N0) / 16;
             const int my_rows = my_rows_of(e), r0 = r0_of(e);
-            if (!mbar_wait(&bar_acc[e], i & 1, abort_flag, 103)) return false;
+            const bool ok = mbar_wait(&bar_acc[e], i & 1, abort_flag, 103);
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 0, clock64());
             tc_fence_after_sync();
-            // Four rows at a time, and each batch is sent as soon as it is staged, so that the exchange runs
-            // beside the arithmetic. Two batches are read at the start, which hands the accumulators back
+            // Four rows at a time, and each batch is sent as soon as it is staged (and stored, 128 bytes of a
+            // row by eight lanes), so that the exchange runs beside the arithmetic. Two batches are read at the start, which hands the accumulators back
             // before the arithmetic.
             static_assert(kB <= 2, "two batches are in registers");
             uint32_t a[2][4][4];
@@ -489,6 +517,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 #pragma unroll
             for (int b = 0; b < kB; ++b) {
                 const auto &v = a[b & 1];
+                if (b > 0 && 4 * b >= my_rows) break;
+                next_slot();
                 if (4 * b < my_rows) {
                     auto codes = [&](int j) {
                         return lstm_cell_codes(v[0][2 * j], v[0][2 * j + 1], v[1][2 * j], v[1][2 * j + 1], v[2][2 * j], v[2][2 * j + 1],
@@ -496,8 +526,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                                                make_float2(b_g, b_g), make_float2(b_o, b_o), c2[e][2 * b + j]);
                     };
                     auto stage_codes = [&](int j, int2 h) {
-                        sts8(stage + (4 * b + 2 * j) * 32 + lane, h.x);
-                        sts8(stage + (4 * b + 2 * j + 1) * 32 + lane, h.y);
+                        sts8(stage + slot + 2 * j * 128 + q * 32 + lane, h.x);
+                        sts8(stage + slot + (2 * j + 1) * 128 + q * 32 + lane, h.y);
                     };
                     // Both pairs side by side: two chains. The second is left out where its rows do not exist
                     // (300 chunks 1.94 -> 1.87 us per step) in the kernels that gain from the branch.
@@ -508,19 +538,19 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     } else {
                         stage_codes(0, codes(0));
                     }
-                    __syncwarp();
-                    if (i + 1 < p.T) send(hs_dst[e][b], stage + b * 128 + (lane >> 1) * 16, &bar_h[e]);
+                }
+                if (!quad_agree(1 + ug, ok)) return false;
+                if (const uint32_t dst = hs_dst[e][b]) {
+                    const uint4 v = lds128(stage + slot + q * 128 + piece(dst) * 16);
+                    if (i + 1 < p.T) send(dst, v, &bar_h[e]);
+                    if (lane < 8) {
+                        const int64_t off = int64_t(m0 + r0 + 4 * b + q) * H + n0 + piece(dst) * 16;
+                        *reinterpret_cast<uint4 *>(p.h_out + int64_t(time_of(i)) * p.B * H + off) = v;
+                        if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + off) = v;
+                    }
                 }
             }
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 1, clock64());
-            // the slice's 16-byte pieces in global memory: lane = (row, 16 units)
-            if ((lane >> 1) < my_rows) {
-                const int64_t off = int64_t(m0 + r0 + (lane >> 1)) * H + n0 + q * 32 + (lane & 1) * 16;
-                const uint4 v = lds128(stage + lane * 16);
-                *reinterpret_cast<uint4 *>(p.h_out + int64_t(time_of(i)) * p.B * H + off) = v;
-                if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + off) = v;
-            }
-            __syncwarp();
             return true;
         };
 
