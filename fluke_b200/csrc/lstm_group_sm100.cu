@@ -140,18 +140,8 @@ __device__ __forceinline__ void sts16(uint32_t addr, unsigned short v) {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
 }
 
-// Barrier of the four warps that share a staging slot. True if all four say so: a warp whose wait ran out
-// takes the others along instead of leaving them at the barrier.
-__device__ __forceinline__ bool quad_agree(int id, bool mine) {
-    int all;
-    asm volatile(
-        "{\n.reg .pred p, q;\n"
-        "setp.ne.s32 p, %2, 0;\n"
-        "barrier.cta.red.and.pred q, %1, 128, p;\n"
-        "selp.s32 %0, 1, 0, q;\n}"
-        : "=r"(all) : "r"(id), "r"(int(mine)) : "memory");
-    return all != 0;
-}
+// Barrier of the four warps that share a staging slot.
+__device__ __forceinline__ void quad_sync(int id) { asm volatile("barrier.cta.sync %0, 128;" ::"r"(id) : "memory"); }
 
 template <int V>
 struct Int { static constexpr int value = V; };  // a number that a lambda receives as a type
@@ -301,17 +291,18 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             __syncwarp();
         };
         auto wait_x = [&]() {
-            if (i > 0)
-                for (int e = 0; e < G; ++e) ok = ok && mbar_wait(&bar_acc_free[e], (i - 1) & 1, abort_flag, 98);
             ok = ok && mbar_wait(&bar_x[i % kXSlots], (i / kXSlots) & 1, abort_flag, 99);
+            if (i > 0) ok = ok && mbar_wait(bar_acc_free, (i - 1) & 1, abort_flag, 98);
             tc_fence_after_sync();
+            return ok;
+        };
+        auto wait_h = [&](int e) {
+            if (projects) ok = ok && mbar_wait<true>(&bar_h[e], i & 1, abort_flag, 100);
             return ok;
         };
         auto project = [&](auto group) {
             constexpr int e = decltype(group)::value;
             if (!projects) return true;
-            ok = ok && mbar_wait<true>(&bar_h[e], i & 1, abort_flag, 100);
-            if (!ok) return false;
             fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
             tc_fence_after_sync();
             FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + (e ? 2 : 3), clock64());
@@ -368,7 +359,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 // projection is converted and travels
                 if (!wait_x()) break;
                 x_half(Int<0>{}, Int<2>{});
-                if (!project(Int<0>{})) break;
+                if (!wait_h(0) || !project(Int<0>{})) break;
                 x_half(Int<2>{}, Int<4>{});
                 if (!hh_half(Int<0>{})) break;
             } else {
@@ -376,9 +367,11 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 // projections are converted and travel
                 if (!wait_x()) break;
                 x_half(Int<0>{}, Int<1>{});
-                if (!project(Int<0>{})) break;
+                if (!wait_h(0)) break;
+                project(Int<0>{});
                 x_half(Int<1>{}, Int<3>{});
-                if (!project(Int<1>{})) break;
+                if (!wait_h(1)) break;
+                project(Int<1>{});
                 x_half(Int<3>{}, Int<4>{});
                 if (!hh_half(Int<0>{})) break;
                 if (!hh_half(Int<1>{})) break;
@@ -459,18 +452,23 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         };
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
         int i = 0;
+        // A warp whose wait ran out walks the remaining steps without waiting, sending or storing: the
+        // three it shares a slot with meet it at every barrier until their own waits give up.
+        bool ok = true;
+        const int64_t plane = int64_t(p.reverse ? -p.B : p.B) * H;
+        int8_t *h_out = p.h_out + int64_t(time_of(0)) * p.B * H;
 
         // ---- projection of group e's h_{i-1}: int32 -> f16, to every CTA of the cluster ----
         auto project_epilogue = [&](auto group) {
             constexpr int e = decltype(group)::value;
             const int my_pr = my_pr_of(e);
             if (my_pr > 0) {
-                const bool ok = mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
+                ok = ok && mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
                 next_slot();
                 FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 4, clock64());
                 tc_fence_after_sync();
                 const uint32_t t_proj = t_lane + 4 * NB + (e ? kPad0 : 0) + pr0_of(e);
-                for (int c = 0; c < my_pr && ok; c += 4) {
+                for (int c = 0; c < my_pr; c += 4) {
                     uint32_t a[4];
                     tmem_ld_32x4(t_proj + c, a);
                     tmem_ld_wait();
@@ -482,13 +480,12 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     }
                 }
                 tc_fence_before_sync();
-                if (!quad_agree(1 + ug, ok)) return false;
+                quad_sync(1 + ug);
 #pragma unroll
                 for (int s = 0; s < (e ? N1 : N0) / 16; ++s)
-                    if (const uint32_t dst = ps_dst[e][s]) send(dst, lds128(stage + slot + ps_src[s] + piece(dst) * 16), &bar_hh[e]);
+                    if (const uint32_t dst = ok ? ps_dst[e][s] : 0u) send(dst, lds128(stage + slot + ps_src[s] + piece(dst) * 16), &bar_hh[e]);
                 FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 5, clock64());
             }
-            return true;
         };
 
         // ---- gates, cell update, hidden code of group e ----
@@ -496,12 +493,12 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             constexpr int e = decltype(group)::value;
             constexpr int kB = (e ? N1 : N0) / 16;
             const int my_rows = my_rows_of(e), r0 = r0_of(e);
-            const bool ok = mbar_wait(&bar_acc[e], i & 1, abort_flag, 103);
+            ok = ok && mbar_wait(&bar_acc[e], i & 1, abort_flag, 103);
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 0, clock64());
             tc_fence_after_sync();
             // Four rows at a time, and each batch is sent as soon as it is staged (and stored, 128 bytes of a
-            // row by eight lanes), so that the exchange runs beside the arithmetic. Two batches are read at the start, which hands the accumulators back
-            // before the arithmetic.
+            // row by eight lanes), so that the exchange runs beside the arithmetic. Two batches are read at the
+            // start, which hands the accumulators back before the arithmetic.
             static_assert(kB <= 2, "two batches are in registers");
             uint32_t a[2][4][4];
             auto load4 = [&](int b) {
@@ -513,7 +510,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             tmem_ld_wait();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_acc_free[e]);
+            if (e == G - 1 && lane == 0) mbar_arrive(bar_acc_free);
 #pragma unroll
             for (int b = 0; b < kB; ++b) {
                 const auto &v = a[b & 1];
@@ -539,28 +536,25 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                         stage_codes(0, codes(0));
                     }
                 }
-                if (!quad_agree(1 + ug, ok)) return false;
-                if (const uint32_t dst = hs_dst[e][b]) {
+                quad_sync(1 + ug);
+                if (const uint32_t dst = ok ? hs_dst[e][b] : 0u) {
                     const uint4 v = lds128(stage + slot + q * 128 + piece(dst) * 16);
                     if (i + 1 < p.T) send(dst, v, &bar_h[e]);
                     if (lane < 8) {
-                        const int64_t off = int64_t(m0 + r0 + 4 * b + q) * H + n0 + piece(dst) * 16;
-                        *reinterpret_cast<uint4 *>(p.h_out + int64_t(time_of(i)) * p.B * H + off) = v;
+                        const size_t off = size_t(m0 + r0 + 4 * b + q) * H + n0 + piece(dst) * 16;
+                        *reinterpret_cast<uint4 *>(h_out + off) = v;
                         if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + off) = v;
                     }
                 }
             }
             FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 1, clock64());
-            return true;
         };
 
-        for (; i < p.T; ++i) {
-            if (!project_epilogue(Int<0>{})) break;
-            if constexpr (G > 1)
-                if (!project_epilogue(Int<1>{})) break;
-            if (!gate_epilogue(Int<0>{})) break;
-            if constexpr (G > 1)
-                if (!gate_epilogue(Int<1>{})) break;
+        for (; i < p.T; ++i, h_out += plane) {
+            project_epilogue(Int<0>{});
+            if constexpr (G > 1) project_epilogue(Int<1>{});
+            gate_epilogue(Int<0>{});
+            if constexpr (G > 1) gate_epilogue(Int<1>{});
         }
 #pragma unroll
         for (int e = 0; e < G; ++e)
@@ -610,13 +604,14 @@ constexpr GroupKernel group_kernels() {
 }
 const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0>(), group_kernels<16, 16>(), group_kernels<16, 32>()};
 
-// The kernel for `rows` rows per cluster of hidden size H, or -1. Two groups from 24 rows on, with few CTAs per
-// cluster (short exchanges) from 17. Step of one group against two, in us: H = 768, 20 rows per cluster 2.42 : 2.51,
-// 23 rows 2.58 : 2.56, 32 rows 3.03 : 2.59, 39 rows 3.36 : 2.93, 48 rows 3.66 : 3.11; H = 384, 17 rows
-// 2.34 : 2.22, 40 rows 3.77 : 3.04; H = 1024, 22 rows 2.66 : 2.77, 32 rows 3.09 : 2.85.
+// The kernel for `rows` rows per cluster of hidden size H, or -1. One group has the shorter chain, two hide
+// half of it: the longer the exchanges (more CTAs), the more rows it takes for two to be the faster. Step of one
+// group against two, in us: H = 256, 20 rows 2.09 : 2.16, 28 rows 2.30 : 2.22; H = 384 (one pair of CTAs
+// projects all rows), 17 rows 2.19 : 2.19, 20 rows 2.40 : 2.21; H = 512, 26 rows 2.36 : 2.35, 32 rows 2.52 : 2.36;
+// H = 768, 28 rows 2.52 : 2.56, 32 rows 2.65 : 2.56; H = 1024, 32 rows 2.75 : 2.80.
 inline int group_kernel_for(int rows, int H) {
-    const int C = H / kGUnits;
-    const int k = rows <= 16 ? 0 : rows <= 32 ? (rows < 24 && C >= 4 ? 1 : 2) : 3;
+    const int C = H / kGUnits, two_from = C == 3 ? 17 : 18 + 2 * C;
+    const int k = rows <= 16 ? 0 : rows <= 32 ? (rows < two_from ? 1 : 2) : 3;
     return rows <= 48 && kGroupKernels[k].fn[C] ? k : -1;
 }
 
