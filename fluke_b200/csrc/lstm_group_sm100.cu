@@ -16,10 +16,10 @@
 //   * projects: the CTAs form pairs (2p, 2p+1); pair p owns a contiguous part of the rows, CTA
 //     2p + s computes projection columns 64 s .. 64 s + 63 of them (M = 64) from the complete
 //     int8 rows. With an odd C the last CTA projects nothing.
-// Per step two exchanges inside the cluster, both of 16-byte st.async stores that complete on an
-// mbarrier of the receiver: the int8 hidden slices go to the pair that owns the row, the
-// f16 projections back to every CTA. The x half of the contraction runs meanwhile. With more than
-// some twenty rows the cluster treats them as two groups, so that one is computed while the
+// Per step two exchanges inside the cluster, both of 16-byte st.async stores (eight lanes write 128
+// contiguous bytes) that complete on an mbarrier of the receiver: the int8 hidden slices go to the pair that
+// owns the row, the f16 projections back to every CTA. The x half of the contraction runs meanwhile. With
+// more than some thirty rows the cluster treats them as two groups, so that one is computed while the
 // other travels.
 //
 //   warp 0       loader: resident weights, x_down rows of every step
@@ -33,11 +33,11 @@
 // projection of h_{t-1} is complete; and the other way round for hh. Nobody leaves before the final
 // cluster barrier. Clusters never wait for one another, so any number of them may run in waves.
 //
-// What bounds a step (B200, H = 768, cycles at 1.93 GHz): with few rows (3 per cluster, 2900 cycles = 1.5 us)
-// the chain: h exchange 600, projection 500 + read-back 250, hh exchange 500, contraction 450,
-// cell update 400; with 47 (6360 cycles = 3.5 us for 1024 chunks) the tensor pipe (x half 1450,
-// projections 1300, hh half 1150) and the epilogue warps (3200) one after the other: the accumulators
-// leave no tensor memory for a second set.
+// What bounds a step (B200, H = 768, cycles at 1.93 GHz): with few rows (3 per cluster, 2790 cycles = 1.48 us)
+// the chain: h exchange 600, projection 450 + read-back 250, hh exchange 500, contraction 500,
+// cell update 430; with 47 (5500 cycles = 2.86 us for 1024 chunks, 3.08 while the exchanges left in 16-byte
+// pieces) the tensor pipe (x half 1450, projections 1400, hh half 1150), which waits for the second
+// group's accumulators to be read and its hidden rows to arrive: the accumulators leave no tensor memory for a second set.
 //
 // Arithmetic and its order are those of the other single-launch forms (x_down half first, then the
 // hh_down half in K steps of 16; int32 sums scaled by (1/127)*scale and rounded to f16): the bytes
@@ -363,8 +363,9 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 x_half(Int<2>{}, Int<4>{});
                 if (!hh_half(Int<0>{})) break;
             } else {
-                // pieces of the x part while the hidden rows of the groups travel, the rest while their
-                // projections are converted and travel
+                // Pieces of the x part while the hidden rows of the groups travel, one gate while the second
+                // projection is converted. 1024 chunks, gates in front of the first projection, between and
+                // behind: 1-2-1 2.87 us per step, 1-1-2 3.02, 0-3-1 2.94, 1-3-0 3.02, 0-4-0 3.00.
                 if (!wait_x()) break;
                 x_half(Int<0>{}, Int<1>{});
                 if (!wait_h(0)) break;
