@@ -26,7 +26,8 @@
 namespace fluke_sm100 {
 namespace {
 
-constexpr int kLstmThreads = 192;
+constexpr int kLstmEpiThreads = 512;  // four warps per tensor-memory lane quadrant, a quarter of the units each
+constexpr int kLstmThreads = 64 + kLstmEpiThreads;
 constexpr int kLstmMaxKB = 4;  // K blocks of 64 f16 kept resident: Kc <= 256
 
 struct LstmDev {
@@ -44,7 +45,8 @@ struct LstmSmem {
     static constexpr int kWBytes = 4 * UNITS * 128;
     static constexpr int kOffA = 0;
     static constexpr int kOffW = kLstmMaxKB * kABytes;
-    static constexpr int kOffBars = kOffW + kLstmMaxKB * kWBytes;
+    static constexpr int kOffBias = kOffW + kLstmMaxKB * kWBytes;   // f32 [4][UNITS]
+    static constexpr int kOffBars = kOffBias + 4 * UNITS * 4;
     static constexpr int kOffMisc = kOffBars + (kLstmMaxKB + 1) * 8;
     static constexpr int kDynamic = kOffMisc + 16 + 1024;
 };
@@ -119,7 +121,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
             ok = mbar_wait(&full_bar[kb], 0, abort_flag, 16);
             if (!ok) break;
             tc_fence_after_sync();
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint64_t adesc = make_smem_desc_sw128(smem_u32(smem + L::kOffA + kb * L::kABytes));
                 const uint64_t bdesc = make_smem_desc_sw128(smem_u32(smem + L::kOffW + kb * L::kWBytes));
 #pragma unroll
@@ -131,58 +133,63 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
             __syncwarp();
         }
     } else {
-        const int q = warp & 3;
+        // Thread = (row, a quarter of the units). The cell states and biases are loaded while the contraction
+        // runs. With one warp per quadrant, which did both for all units of its rows after the contraction, this
+        // part was most of the kernel: 500 chunks, H = 1024 5.7 us then, 4.3 now.
+        constexpr int kOwn = UNITS / 4;
+        const int q = warp & 3, u0 = ((warp - 2) >> 2) * kOwn;
         const int row = m0 + q * 32 + lane;
         const bool row_ok = row < p.B;
+        const int64_t off = int64_t(row) * p.H + n0 + u0;
+        float *s_bias = reinterpret_cast<float *>(smem + L::kOffBias);
+        const int t = threadIdx.x - 64;
+        if (t < 4 * UNITS) {
+            const int g = t / UNITS;
+            s_bias[t] = (g == 0 ? p.bias[0] : g == 1 ? p.bias[1] : g == 2 ? p.bias[2] : p.bias[3])[n0 + t - g * UNITS];
+        }
+        float4 cv[kOwn / 4];
+#pragma unroll
+        for (int v = 0; v < kOwn / 4; ++v)
+            cv[v] = row_ok ? reinterpret_cast<const float4 *>(p.c + off)[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+        asm volatile("barrier.cta.sync 1, %0;" ::"n"(kLstmEpiThreads) : "memory");
         if (mbar_wait(tfull_bar, 0, abort_flag, 17)) {
             tc_fence_after_sync();
-            const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16);
-#pragma unroll 1
-            for (int u0 = 0; u0 < UNITS; u0 += 16) {
-                uint32_t gi[16], gf[16], gg[16], go[16];
-                tmem_ld_32x16(t_row + 0 * UNITS + u0, gi);
-                tmem_ld_32x16(t_row + 1 * UNITS + u0, gf);
-                tmem_ld_32x16(t_row + 2 * UNITS + u0, gg);
-                tmem_ld_32x16(t_row + 3 * UNITS + u0, go);
+            const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + u0;
+            uint32_t hq[kOwn / 4];
+#pragma unroll
+            for (int v = 0; v < kOwn / 4; ++v) {
+                uint32_t a[4][4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_row + g * UNITS + 4 * v, a[g]);
                 tmem_ld_wait();
-                if (row_ok) {
-                    const int64_t off = int64_t(row) * p.H + n0 + u0;
-                    float cv[16];
+                float bs[4][4], cc[4] = {cv[v].x, cv[v].y, cv[v].z, cv[v].w};
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        const float4 c4 = *reinterpret_cast<const float4 *>(p.c + off + 4 * v);
-                        cv[4 * v] = c4.x; cv[4 * v + 1] = c4.y; cv[4 * v + 2] = c4.z; cv[4 * v + 3] = c4.w;
-                    }
-                    uint32_t hq[4];
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        const float4 bi = reinterpret_cast<const float4 *>(p.bias[0] + n0 + u0)[v];
-                        const float4 bf = reinterpret_cast<const float4 *>(p.bias[1] + n0 + u0)[v];
-                        const float4 bg = reinterpret_cast<const float4 *>(p.bias[2] + n0 + u0)[v];
-                        const float4 bo = reinterpret_cast<const float4 *>(p.bias[3] + n0 + u0)[v];
-                        const float bis[4] = {bi.x, bi.y, bi.z, bi.w}, bfs[4] = {bf.x, bf.y, bf.z, bf.w};
-                        const float bgs[4] = {bg.x, bg.y, bg.z, bg.w}, bos[4] = {bo.x, bo.y, bo.z, bo.w};
-                        uint32_t packed = 0;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int e = 4 * v + j;
-                            const float i_a = hard_sigmoid(__uint_as_float(gi[e]) + bis[j]);
-                            const float f_a = hard_sigmoid(__uint_as_float(gf[e]) + bfs[j]);
-                            const float o_a = hard_sigmoid(__uint_as_float(go[e]) + bos[j]);
-                            const float g_a = fmaxf(-1.f, fminf(1.f, __uint_as_float(gg[e]) + bgs[j]));
-                            const float c_new = __fmaf_rn(f_a, cv[e], __fmul_rn(i_a, g_a));
-                            cv[e] = c_new;
-                            const float h_new = o_a * tanhf(c_new);
-                            packed |= (uint32_t(quant_h(h_new)) & 0xFFu) << (8 * j);
-                        }
-                        hq[v] = packed;
-                    }
-#pragma unroll
-                    for (int v = 0; v < 4; ++v)
-                        *reinterpret_cast<float4 *>(p.c + off + 4 * v) =
-                            make_float4(cv[4 * v], cv[4 * v + 1], cv[4 * v + 2], cv[4 * v + 3]);
-                    *reinterpret_cast<uint4 *>(p.h_out + off) = make_uint4(hq[0], hq[1], hq[2], hq[3]);
+                for (int g = 0; g < 4; ++g) {
+                    const float4 b4 = *reinterpret_cast<const float4 *>(s_bias + g * UNITS + u0 + 4 * v);
+                    bs[g][0] = b4.x; bs[g][1] = b4.y; bs[g][2] = b4.z; bs[g][3] = b4.w;
                 }
+                hq[v] = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float i_a = hard_sigmoid(__uint_as_float(a[0][j]) + bs[0][j]);
+                    const float f_a = hard_sigmoid(__uint_as_float(a[1][j]) + bs[1][j]);
+                    const float g_a = fmaxf(-1.f, fminf(1.f, __uint_as_float(a[2][j]) + bs[2][j]));
+                    const float o_a = hard_sigmoid(__uint_as_float(a[3][j]) + bs[3][j]);
+                    cc[j] = __fmaf_rn(f_a, cc[j], __fmul_rn(i_a, g_a));
+                    const float h_new = o_a * tanhf(cc[j]);
+                    hq[v] |= (uint32_t(quant_h(h_new)) & 0xFFu) << (8 * j);
+                }
+                cv[v] = make_float4(cc[0], cc[1], cc[2], cc[3]);
+            }
+            if (row_ok) {
+#pragma unroll
+                for (int v = 0; v < kOwn / 4; ++v) reinterpret_cast<float4 *>(p.c + off)[v] = cv[v];
+                int8_t *h = p.h_out + off;
+                if constexpr (kOwn == 16) *reinterpret_cast<uint4 *>(h) = make_uint4(hq[0], hq[1], hq[2], hq[3]);
+                else if constexpr (kOwn == 8) *reinterpret_cast<uint2 *>(h) = make_uint2(hq[0], hq[1]);
+                else
+#pragma unroll
+                    for (int v = 0; v < kOwn / 4; ++v) reinterpret_cast<uint32_t *>(h)[v] = hq[v];
             }
         }
     }
@@ -204,14 +211,18 @@ struct LstmPlan {
     dim3 grid;
 };
 
+// Units per CTA: the fewest with which all CTAs run at once, because a CTA's epilogue grows with them and a
+// second round costs the whole latency again (1024 rows, H = 768: 32 units in 192 CTAs 9.3 us, 48 in 128 7.5).
+// Sixteen only up to two thirds of the SMs: with more CTAs fetching the same rows, 32 are the faster (300 rows,
+// H = 768: 144 CTAs 5.28 us, 72 CTAs 4.99). With more rows than one round takes, as many as there are.
 inline int pick_units(int B, int H) {
-    const int row_tiles = (B + 127) / 128;
+    const int row_tiles = (B + 127) / 128, sms = device_sm_count();
     const int cand[4] = {64, 48, 32, 16};
     int best = 0;
     for (int i = 0; i < 4; ++i) {
         if (H % cand[i]) continue;
+        if (best && row_tiles * (H / cand[i]) > (cand[i] == 16 ? sms * 2 / 3 : sms)) break;
         best = cand[i];
-        if (row_tiles * (H / cand[i]) >= 128) break;  // enough CTAs to fill the GPU
     }
     return best;
 }

@@ -44,6 +44,22 @@ def test_step_vs_oracle(B, H, Kc):
     assert d.max() <= 1 and (d != 0).mean() < 1e-3
 
 
+@pytest.mark.parametrize("B,H", [(1, 768), (129, 768), (257, 768), (641, 768), (769, 768), (1281, 512), (2000, 768), (640, 96), (300, 48)])
+def test_step_of_every_unit_width_vs_oracle(B, H):
+    """Rows and hidden sizes on either side of where the kernel changes between 16, 32, 48 and 64 units per
+    block on a B200, ragged last row tiles. Cells: 256 products of f16 values summed in f32, then one
+    fma, 2^-24 * 256 relative to sums of order 1; a code differs where 127 h lies at a rounding boundary."""
+    g = torch.Generator().manual_seed(B + H)
+    A = (torch.randn(B, 256, generator=g) * 0.3).half(); W = (torch.randn(4 * H, 256, generator=g) * 0.1).half()
+    bias = torch.randn(4 * H, generator=g) * 0.1; c = torch.randn(B, H, generator=g) * 0.1
+    cg = c.clone().to(DEV)
+    hg = ops.factored_lstm_step_i8(A.to(DEV), W.to(DEV), bias.to(DEV), cg)
+    ce, he = port.lstm_step(A.numpy(), W.numpy(), bias.numpy(), c.numpy())
+    assert np.abs(cg.cpu().numpy() - ce).max() < 1e-4
+    d = np.abs(hg.cpu().numpy().astype(np.int32) - he.astype(np.int32))
+    assert d.max() <= 1 and (d != 0).mean() < 1e-3
+
+
 def test_step_golden_from_reference_test(golden_tests):
     g = golden_tests
     H = g["lstm_c"].shape[1]
