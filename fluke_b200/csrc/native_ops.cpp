@@ -211,10 +211,12 @@ PyObject *rotary_qkv(Args a) {
     const at::Tensor *sin = input(a[1]), *cos = input(a[2]);
     const int width = integer(a[3]);
     TORCH_CHECK(qkv.dim() == 5, "rotary_qkv_ needs [N, seq, 3, heads, head_dim]");
-    // the q and k heads lie side by side: one call rotates both
+    // The q and k heads lie side by side: one call rotates both. The strides follow from the sizes: those of
+    // a contiguous tensor say nothing in a dimension of one element, and with one head q and k are two.
+    const int64_t heads = qkv.size(3), head_dim = qkv.size(4), position = qkv.size(2) * heads * head_dim;
     unlocked([&] {
-        L.fluke_rotary_emb_gpu(ptr(qkv), ptr(sin), ptr(cos), int(qkv.size(0)), int(qkv.size(1)), 2 * int(qkv.size(3)),
-                               int(qkv.size(4)), width, int(qkv.stride(0)), int(qkv.stride(1)), int(qkv.stride(3)));
+        L.fluke_rotary_emb_gpu(ptr(qkv), ptr(sin), ptr(cos), int(qkv.size(0)), int(qkv.size(1)), 2 * int(heads), int(head_dim),
+                               width, int(qkv.size(1) * position), int(position), int(head_dim));
     });
     Py_INCREF(a[0]);
     return a[0];

@@ -236,6 +236,22 @@ def test_rotary_config_size_round_trip():
     assert np.array_equal(sub.view(np.uint16), fwd[:2].cpu().numpy().ravel().view(np.uint16))
 
 
+@pytest.mark.parametrize("n,s", [(3, 5), (2, 1), (1, 7)])
+def test_rotary_qkv_of_one_head_with_a_stride_of_its_own(n, s):
+    """[N, seq, 3, 1, D] seen through a transposed view is contiguous, whatever the stride of the one head:
+    the bits of the same values in a plain tensor, and nothing past the end is written."""
+    g = torch.Generator().manual_seed(n * 10 + s)
+    sin, cos = (t.to(DEV) for t in prep.rotary_tables(s, 64))
+    raw = torch.full((n * s * 192 + 256,), 3.0, dtype=torch.float16, device=DEV)
+    base = raw[:n * s * 192].view(n, s, 1, 3, 64)
+    base.copy_(torch.randn(n, s, 1, 3, 64, generator=g).half())
+    qkv = base.transpose(2, 3)
+    assert qkv.is_contiguous() and qkv.stride(3) != 64
+    want = ops.rotary_qkv_(qkv.reshape(-1).clone().view(n, s, 3, 1, 64), sin, cos, 32)
+    assert torch.equal(ops.rotary_qkv_(qkv, sin, cos, 32), want)
+    assert bool((raw[n * s * 192:] == 3.0).all())
+
+
 def test_empty_inputs_are_noops():
     z = torch.zeros(0, 512, dtype=torch.float16, device=DEV)
     assert ops.quant_int8(z)[0].shape == (0, 512)
