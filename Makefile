@@ -25,10 +25,11 @@ ifdef asan
 	LDFLAGS += -fsanitize=address -fno-omit-frame-pointer
 endif
 
+CUDA_ROOT ?= /usr/local/cuda
+CUDA_INC ?= $(CUDA_ROOT)/include
+
 ifdef cuda
-	CUDA_ROOT ?= /usr/local/cuda
 	CUDA_LIB ?= $(CUDA_ROOT)/lib64
-	CUDA_INC ?= $(CUDA_ROOT)/include
 	NVCC ?= $(CUDA_ROOT)/bin/nvcc
 	SM100_ARCH = -gencode arch=compute_100a,code=sm_100a
 	CUDA_CFLAGS += -O3 -std=c++17 -lineinfo $(SM100_ARCH) -Xcompiler -Wall -Xcompiler -fPIC

@@ -4,6 +4,7 @@ the oracle and with the reference's own nn_cpu.c (when oracle/_ref is built)."""
 import ctypes
 import os
 import re
+import subprocess
 
 import numpy as np
 import pytest
@@ -65,6 +66,15 @@ def test_ops_refuse_cpu_tensors():
     from fluke_b200 import ops
     with pytest.raises(RuntimeError):
         ops.quant_int8(torch.zeros(4, 8, dtype=torch.float16))
+
+
+def test_extension_target_needs_no_other_variable():
+    """`make pyext` on its own compiles the extension's source: no include path is left empty, which
+    would take the next word of the command, the source, for its directory."""
+    res = subprocess.run(["make", "-n", "-B", "pyext"], cwd=ROOT, stdout=subprocess.PIPE, text=True, check=True)
+    words = res.stdout.split()
+    assert "fluke_b200/csrc/native_ops.cpp" in words
+    assert not any(a == "-I" and (b.startswith("-") or b.endswith(".cpp")) for a, b in zip(words, words[1:]))
 
 
 def _tables(seq, w):
