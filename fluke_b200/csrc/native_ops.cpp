@@ -66,6 +66,15 @@ const at::Tensor &required(PyObject *o) {
     if (!t) tensor(o);  // raises
     return *t;
 }
+// The same with the dimensions that the operator's sizes are read from.
+const at::Tensor &required(PyObject *o, int64_t dims) {
+    const at::Tensor &t = required(o);
+    if (t.dim() != dims) {
+        PyErr_Format(PyExc_ValueError, "fluke_b200.ops: a tensor of %lld dimensions where %lld are needed", (long long)t.dim(), (long long)dims);
+        throw Failed();
+    }
+    return t;
+}
 void *ptr(const at::Tensor *t) { return t ? t->data_ptr() : nullptr; }
 void *ptr(const at::Tensor &t) { return t.data_ptr(); }
 int integer(PyObject *o) {
@@ -186,7 +195,7 @@ PyObject *quant(Args a) {
 
 // x, scale, fp8
 PyObject *dequant_transpose(Args a) {
-    const at::Tensor &x = required(a[0]);
+    const at::Tensor &x = required(a[0], 3);
     const float scale = real(a[1]);
     auto fn = truth(a[2]) ? L.fluke_dequant_fp8_transpose_gpu : L.fluke_dequant_int8_transpose_gpu;
     const int64_t t = x.size(0), n = x.size(1), c = x.size(2);
@@ -207,10 +216,9 @@ PyObject *rotary_emb(Args a) {
 
 // qkv, sin, cos, width
 PyObject *rotary_qkv(Args a) {
-    const at::Tensor &qkv = required(a[0]);
+    const at::Tensor &qkv = required(a[0], 5);
     const at::Tensor *sin = input(a[1]), *cos = input(a[2]);
     const int width = integer(a[3]);
-    TORCH_CHECK(qkv.dim() == 5, "rotary_qkv_ needs [N, seq, 3, heads, head_dim]");
     // The q and k heads lie side by side: one call rotates both. The strides follow from the sizes: those of
     // a contiguous tensor say nothing in a dimension of one element, and with one head q and k are two.
     const int64_t heads = qkv.size(3), head_dim = qkv.size(4), position = qkv.size(2) * heads * head_dim;
@@ -284,7 +292,7 @@ PyObject *gated_mlp(Args a) {
 
 // a, b, scale_a, scale_b, const_scale_a
 PyObject *gemm_i8(Args a) {
-    const at::Tensor &x = required(a[0]), &w = required(a[1]);
+    const at::Tensor &x = required(a[0], 2), &w = required(a[1]);
     const at::Tensor *sa = input(a[2]), *sb = input(a[3]);
     const float csa = real(a[4]);
     const int m = int(x.size(0)), k = int(x.size(1)), n = int(w.size(0));
@@ -295,7 +303,7 @@ PyObject *gemm_i8(Args a) {
 
 // a, b, scale_a, scale_b
 PyObject *gemm_fp8(Args a) {
-    const at::Tensor &x = required(a[0]), &w = required(a[1]);
+    const at::Tensor &x = required(a[0], 2), &w = required(a[1]);
     const at::Tensor *sa = input(a[2]), *sb = input(a[3]);
     const int m = int(x.size(0)), k = int(x.size(1)), n = int(w.size(0));
     at::Tensor out = empty_on(x, {m, n}, at::kHalf);
@@ -305,7 +313,7 @@ PyObject *gemm_fp8(Args a) {
 
 // a, w, scale_a, scale_b, out, fp8
 PyObject *down_proj(Args a) {
-    const at::Tensor &x = required(a[0]), &w = required(a[1]);
+    const at::Tensor &x = required(a[0], 2), &w = required(a[1]);
     const at::Tensor *sa = input(a[2]), *sb = input(a[3]);
     const bool fp8 = truth(a[5]);
     const int m = int(x.size(0)), k = int(x.size(1)), n = int(w.size(0));
@@ -319,7 +327,7 @@ PyObject *down_proj(Args a) {
 
 // A, W4, bias4, c, h_out, fp8_export_name
 PyObject *lstm_step(Args a) {
-    const at::Tensor &x = required(a[0]), &w4 = required(a[1]), &b4 = required(a[2]), &c = required(a[3]);
+    const at::Tensor &x = required(a[0], 2), &w4 = required(a[1]), &b4 = required(a[2]), &c = required(a[3]);
     const int b = int(x.size(0)), kc = int(x.size(1)), h = int(c.size(1));
     at::Tensor out = output(a[4], x, {b, h}, at::kChar);
     const char *w = static_cast<const char *>(ptr(w4));

@@ -473,3 +473,19 @@ def test_wide_plain_tiles_give_the_bits_of_narrow_ones(m, n, k):
         got = run(a, sa)
         for r0 in (0, 127, m // 2, m - 300):
             assert torch.equal(got[r0:r0 + 300], run(a[r0:r0 + 300].contiguous(), sa[r0:r0 + 300].contiguous()))
+
+
+def test_operators_refuse_tensors_of_other_ranks():
+    """Operators that read two, three or five sizes off a tensor take no tensor of another rank (a [T, B, K]
+    batch would pass for its first two sizes); nothing is launched."""
+    z = lambda *shape, dtype=torch.int8: torch.zeros(*shape, dtype=dtype, device=DEV)
+    w, s, f16 = z(64, 128), z(64, dtype=torch.float32), torch.float16
+    for a in (z(4, 128, 128), z(128)):
+        u8 = a.view(torch.uint8)
+        for call in (lambda: ops.gemm_i8(a, w, s, s), lambda: ops.gemm_fp8(u8, w.view(torch.uint8), s, s),
+                     lambda: ops.down_proj_i8(a, w, None, s), lambda: ops.down_proj_fp8(u8, w.view(torch.uint8), s, s),
+                     lambda: ops.factored_lstm_step_i8(a.to(f16), z(256, 128, dtype=f16), z(256, dtype=torch.float32), z(4, 64, dtype=torch.float32)),
+                     lambda: ops.dequant_transpose(z(2, 2, 4, 8), 1.0), lambda: ops.dequant_transpose(z(4, 8), 1.0),
+                     lambda: ops.rotary_qkv_(z(2, 4, 3, 64, dtype=f16), s, s, 32)):
+            with pytest.raises(ValueError):
+                call()
