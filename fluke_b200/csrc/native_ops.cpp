@@ -77,25 +77,44 @@ const at::Tensor &required(PyObject *o, int64_t dims) {
 }
 void *ptr(const at::Tensor *t) { return t ? t->data_ptr() : nullptr; }
 void *ptr(const at::Tensor &t) { return t.data_ptr(); }
+// Numbers and addresses are taken as ctypes takes them for the same C arguments: an int of any size
+// by its low bits (the stride of a dimension of one element may be anything), a ctypes integer by its value,
+// an address also as a ctypes pointer or array; a real number as float() converts it.
 int integer(PyObject *o) {
-    const long v = PyLong_AsLong(o);
-    if (v == -1 && PyErr_Occurred()) throw Failed();
-    if (v != int(v)) {
-        PyErr_SetString(PyExc_OverflowError, "integer argument out of range");
+    if (PyLong_Check(o)) return int(PyLong_AsUnsignedLongMask(o));
+    PyObject *v = PyIndex_Check(o) ? PyNumber_Index(o) : PyObject_GetAttrString(o, "value");
+    if (!v || !PyLong_Check(v)) {
+        Py_XDECREF(v);
+        PyErr_Format(PyExc_TypeError, "fluke_b200.ops: an integer is needed, got %s", Py_TYPE(o)->tp_name);
         throw Failed();
     }
-    return int(v);
+    const int r = int(PyLong_AsUnsignedLongMask(v));
+    Py_DECREF(v);
+    return r;
 }
 void *address(PyObject *o) {
     if (o == Py_None) return nullptr;
-    void *p = PyLong_AsVoidPtr(o);
-    if (!p && PyErr_Occurred()) throw Failed();
+    if (PyLong_Check(o)) return reinterpret_cast<void *>(uintptr_t(PyLong_AsUnsignedLongLongMask(o)));
+    PyObject *ctypes = PyImport_ImportModule("ctypes");
+    PyObject *type = ctypes ? PyObject_GetAttrString(ctypes, "c_void_p") : nullptr;
+    PyObject *cast = type ? PyObject_CallMethod(ctypes, "cast", "OO", o, type) : nullptr;
+    PyObject *v = cast ? PyObject_GetAttrString(cast, "value") : nullptr;
+    void *p = v && v != Py_None ? PyLong_AsVoidPtr(v) : nullptr;
+    const bool ok = v && !PyErr_Occurred();
+    Py_XDECREF(v);
+    Py_XDECREF(cast);
+    Py_XDECREF(type);
+    Py_XDECREF(ctypes);
+    if (!ok) throw Failed();
     return p;
 }
 float real(PyObject *o) {
-    const double v = PyFloat_AsDouble(o);
-    if (v == -1.0 && PyErr_Occurred()) throw Failed();
-    return float(v);
+    if (PyFloat_Check(o)) return float(PyFloat_AS_DOUBLE(o));
+    PyObject *v = PyNumber_Float(o);
+    if (!v) throw Failed();
+    const double r = PyFloat_AS_DOUBLE(v);
+    Py_DECREF(v);
+    return float(r);
 }
 bool truth(PyObject *o) {
     const int v = PyObject_IsTrue(o);

@@ -68,6 +68,24 @@ def test_ops_refuse_cpu_tensors():
         ops.quant_int8(torch.zeros(4, 8, dtype=torch.float16))
 
 
+def test_ops_take_numbers_and_addresses_as_ctypes_does():
+    """The extension's arguments: an address as an int, None, a ctypes pointer or array; an int beyond 32 bits (the
+    stride of a dimension of one element) by its low bits, a ctypes int, an index; nothing else. An empty batch
+    returns before anything is launched."""
+    from fluke_b200 import ops
+    def call(x=0, batch=0, stride=64):
+        ops.rotary_emb_(x, None, None, batch, 1, 1, 64, 32, stride, 64, 64)
+    for x in (0, None, 1 << 63, ctypes.c_void_p(256), ctypes.c_void_p(None), (ctypes.c_char * 4)(), ctypes.pointer(ctypes.c_int(3))):
+        call(x=x)
+    for stride in (1 << 31, -5, 1 << 40, ctypes.c_int(7), np.int64(7)):
+        call(stride=stride)
+    call(batch=ctypes.c_int(0))
+    call(batch=1 << 32)   # low bits: 0
+    for bad in (dict(x=1.5), dict(x=object()), dict(stride=1.5), dict(stride="4"), dict(stride=None), dict(batch=ctypes.c_float(0))):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            call(**bad)
+
+
 def test_extension_target_needs_no_other_variable():
     """`make pyext` on its own compiles the extension's source: no include path is left empty, which
     would take the next word of the command, the source, for its directory."""
