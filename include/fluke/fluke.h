@@ -428,7 +428,7 @@ typedef struct {
     const void *bias_f32;       /* [4*H] f32, gate order i,f,g,o                        */
     void *c_f32;                /* [B,H] f32 cell state, in/out                         */
     void *h_i8;                 /* [B,H] int8 hidden state @1/127, in (h_0) / out (h_T) */
-    void *h_out_i8;             /* [T,B,H] int8 hidden outputs @1/127                   */
+    void *h_out_i8;             /* [T,B,H] int8 hidden outputs @1/127, 16-byte aligned  */
     void *workspace;            /* fluke_factored_lstm_layer_workspace() bytes          */
     size_t workspace_bytes;
 } fluke_flstm_layer_t;

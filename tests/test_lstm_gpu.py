@@ -263,6 +263,25 @@ def test_stack_entry_point_equals_layer_by_layer(flib):
     assert flib.fluke_factored_lstm_stack_i8_gpu(None, 0, T, B, H, R, 0, 0, 0, 0, 0, 0, 0, 0) != 0  # bad arguments: refused
 
 
+@pytest.mark.parametrize("mode", [0, 1, 2, 4])
+def test_hidden_output_that_is_not_16_byte_aligned_is_refused(flib, mode):
+    """No form launches for an h_out that its 16-byte stores could not write: the call returns an error,
+    the buffer and the state stay as they are."""
+    T, B, H, R = 2, 200, 768, 128
+    layer, x, xs = _layer_case(T, B, H, R, 3, False)
+    raw = torch.full((T * B * H + 16,), 5, dtype=torch.int8, device=DEV)
+    c = torch.zeros(B, H, device=DEV); h = torch.zeros(B, H, dtype=torch.int8, device=DEV)
+    flib.fluke_set_lstm_persistent(mode)
+    try:
+        for off in (1, 4, 8):
+            with pytest.raises(RuntimeError, match="misaligned"):
+                ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale,
+                                           layer.w_up, layer.bias, c, h, h_out=raw[off:off + T * B * H].view(T, B, H))
+    finally:
+        flib.fluke_set_lstm_persistent(1)
+    assert bool((raw == 5).all()) and not c.any() and not h.any()
+
+
 def test_persistent_and_per_step_layers_agree(flib):
     """Same layer through all three drivers: the only difference is the accumulation order of the two
     K halves, so codes differ by at most one, rarely. Also other hidden sizes (1024, 384 with an odd
