@@ -202,7 +202,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     const int m_first = blockIdx.x / p.num_n_tiles;
     const int n0 = n_tile * BN_OUT;
 
-    dependency_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full_bar[s], 1);
@@ -225,6 +224,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    dependency_trigger();
     dependency_wait();
     // The launch gives every thread 65536 / 384 registers; the loader and issuer need few, the
     // epilogue threads hold a whole row segment plus rotary tables: each role branch below

@@ -68,7 +68,6 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     const int pieces = p.nkb > p.half_kb ? 2 : 1;
     uint8_t *sa = smem, *sb = smem + 2 * p.half_kb * kABytes;
 
-    dependency_trigger();
     if (threadIdx.x == 0) {
         mbar_init(&full_bar[0], 1);
         mbar_init(&full_bar[1], 1);
@@ -84,6 +83,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = tmem_slot;
+    dependency_trigger();
     dependency_wait();
 
     if (warp == 0) {

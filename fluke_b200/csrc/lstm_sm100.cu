@@ -86,7 +86,6 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
     const int m0 = blockIdx.x * 128;
     const int n0 = blockIdx.y * UNITS;
 
-    dependency_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kLstmMaxKB; ++s) mbar_init(&full_bar[s], 1);
         mbar_init(tfull_bar, 1);
@@ -98,6 +97,7 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    dependency_trigger();
     dependency_wait();
 
     if (warp == 0) {

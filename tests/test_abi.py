@@ -2,6 +2,7 @@
 declares, keeps the reference loader's contract, and its CPU functions agree bit for bit with
 the oracle and with the reference's own nn_cpu.c (when oracle/_ref is built)."""
 import ctypes
+import glob
 import os
 import re
 import subprocess
@@ -84,6 +85,22 @@ def test_ops_take_numbers_and_addresses_as_ctypes_does():
     for bad in (dict(x=1.5), dict(x=object()), dict(stride=1.5), dict(stride="4"), dict(stride=None), dict(batch=ctypes.c_float(0))):
         with pytest.raises((TypeError, ctypes.ArgumentError)):
             call(**bad)
+
+
+def test_kernels_trigger_their_dependents_behind_the_tensor_memory_allocation():
+    """In a kernel that lets its dependents start early, the allocation of tensor memory and a barrier of the
+    block come first: otherwise a dependent block could take the columns that a block of this kernel still
+    has to get, and wait for that block while holding them."""
+    found = 0
+    for path in glob.glob(os.path.join(ROOT, "fluke_b200", "csrc", "*.cu")):
+        for body in open(path).read().split("__global__")[1:]:
+            at = body.find("dependency_trigger();")
+            if at < 0 or "tmem_alloc(" not in body:
+                continue
+            found += 1
+            alloc = body.index("tmem_alloc(")
+            assert 0 <= alloc < body.find("__syncthreads();", alloc) < at < body.index("dependency_wait();"), path
+    assert found >= 3
 
 
 def test_extension_target_needs_no_other_variable():
