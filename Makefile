@@ -51,9 +51,12 @@ SM100_DEPS = $(wildcard fluke_b200/csrc/*.cu fluke_b200/csrc/*.cuh fluke_b200/cs
 PROBELIB = $(BUILD_DIR)/libfluke_probe.so
 WAITPROBELIB = $(BUILD_DIR)/libfluke_waitprobe.so
 
-# Python extension of fluke_b200.ops (argument checks, output allocation and the call in one step)
-NATIVEEXT = fluke_b200/_native.so
+# Python extension of fluke_b200.ops (argument checks, output allocation and the call in one step), for the
+# interpreter and torch of PYTHON: their versions are part of its name
 PYTHON ?= python3
+ifneq ($(filter pyext,$(MAKECMDGOALS)),)
+NATIVEEXT := fluke_b200/$(shell $(PYTHON) -c "from fluke_b200 import lib; print(lib.native_name())")
+endif
 
 .PHONY: all shared probe waitprobe pyext clean distclean
 
@@ -71,14 +74,17 @@ $(WAITPROBELIB): tests/csrc/wait_probe.cu $(SM100_DEPS) | $(BUILD_DIR)
 $(PROBELIB): fluke_b200/csrc/mma_peak_sm100.cu $(SM100_DEPS) | $(BUILD_DIR)
 	$(NVCC) $(CUDA_CFLAGS) $(CPPFLAGS) -shared fluke_b200/csrc/mma_peak_sm100.cu -o $@ $(CUDA_LDFLAGS)
 
+ifdef NATIVEEXT
 pyext: $(NATIVEEXT)
 
+# linked under another name first: a process that finds the file finds all of it
 $(NATIVEEXT): fluke_b200/csrc/native_ops.cpp include/fluke/fluke.h
 	T=`$(PYTHON) -c "import os, torch; print(os.path.dirname(torch.__file__))"` && \
 	P=`$(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])"` && \
 	$(CXX) -O2 -g0 -std=c++17 -fPIC -shared -fvisibility=hidden -Wall -DHAVE_CUDA=1 -I include -I $$P -I $$T/include \
-	    -I $$T/include/torch/csrc/api/include -I $(CUDA_INC) $< -o $@ \
-	    -L$$T/lib -lc10 -lc10_cuda -ltorch_cpu -ltorch_cuda -ltorch -ltorch_python
+	    -I $$T/include/torch/csrc/api/include -I $(CUDA_INC) $< -o $@.$$$$ \
+	    -L$$T/lib -lc10 -lc10_cuda -ltorch_cpu -ltorch_cuda -ltorch -ltorch_python && mv -f $@.$$$$ $@
+endif
 
 $(STATICLIB): $(OBJ) $(GPU_OBJ)
 	rm -f $@

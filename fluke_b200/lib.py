@@ -5,6 +5,9 @@ fly/common.py:96-107 for the fused fp8 signatures, include/fluke/fluke.h for the
 There is no fallback: if the library cannot be built or loaded, `load()` raises.
 """
 import ctypes
+import fcntl
+import importlib.metadata
+import importlib.util
 import os
 import subprocess
 import sys
@@ -111,9 +114,13 @@ PROBE_PATH = os.path.join(ROOT, "lib", "libfluke_probe.so")
 def build(verbose=False):
     """`make shared probe waitprobe pyext cuda=1` at the repository root (nvcc cross-compiles sm_100a
     without a GPU): the library, the benchmark's issue-rate probe, the tests' wait probe and the
-    extension module of fluke_b200.ops (for this interpreter)."""
+    extension module of fluke_b200.ops (for this interpreter and its torch). One process at a time: the ranks of
+    a multi-process start that all find a file missing wait for the first."""
     cmd = ["make", "shared", "probe", "waitprobe", "pyext", "cuda=1", "PYTHON=" + sys.executable]
-    res = subprocess.run(cmd, cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    os.makedirs(os.path.dirname(SO_PATH), exist_ok=True)
+    with open(os.path.join(os.path.dirname(SO_PATH), ".build.lock"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        res = subprocess.run(cmd, cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or res.returncode != 0:
         print(res.stdout)
     if res.returncode != 0:
@@ -137,11 +144,23 @@ def load(rebuild=False):
         fn.restype = restype
         fn.argtypes = argtypes
     _LIB = lib
+    if _NATIVE is not None:
+        _bind(_NATIVE, lib)
     return lib
 
 
-NATIVE_PATH = os.path.join(ROOT, "fluke_b200", "_native.so")
+def native_name():
+    """File name of the extension module: it is built against the C++ interface of one torch for one
+    interpreter, so a program that runs with others looks for another file."""
+    return f"_native.{sys.implementation.cache_tag}-torch{importlib.metadata.version('torch')}.so"
+
+
 _NATIVE = None
+
+
+def _bind(module, lib):
+    """Makes the operators call `lib`: its entry points, stream setting, last error and prepared weights."""
+    module.bind({n: ctypes.cast(getattr(lib, n), P).value for n in module.names()})
 
 
 def native():
@@ -149,12 +168,15 @@ def native():
     global _NATIVE
     if _NATIVE is None:
         lib = load()
-        if not os.path.isfile(NATIVE_PATH):
+        path = os.path.join(ROOT, "fluke_b200", native_name())
+        if not os.path.isfile(path):
             build()
         import torch  # noqa: F401  (its libraries must be loaded first)
-        from . import _native
-        _native.bind({n: ctypes.cast(getattr(lib, n), P).value for n in _native.names()})
-        _NATIVE = _native
+        spec = importlib.util.spec_from_file_location("fluke_b200._native", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _bind(module, lib)
+        _NATIVE = module
     return _NATIVE
 
 

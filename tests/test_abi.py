@@ -5,7 +5,9 @@ import ctypes
 import glob
 import os
 import re
+import shutil
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -85,6 +87,35 @@ def test_ops_take_numbers_and_addresses_as_ctypes_does():
     for bad in (dict(x=1.5), dict(x=object()), dict(stride=1.5), dict(stride="4"), dict(stride=None), dict(batch=ctypes.c_float(0))):
         with pytest.raises((TypeError, ctypes.ArgumentError)):
             call(**bad)
+
+
+def test_operators_follow_a_reloaded_library(monkeypatch, tmp_path):
+    """load(rebuild=True) may bring another copy of the library, with a stream setting and prepared weights of
+    its own: the extension module is bound to it, not left on the first."""
+    from fluke_b200 import lib as L
+    first, bound = L.load(), []
+    class Module:
+        names = staticmethod(lambda: ["fluke_gemm_i8_gpu", "fluke_last_error"])
+        bind = staticmethod(bound.append)
+    copy = shutil.copy(L.SO_PATH, tmp_path / "other.so")
+    monkeypatch.setattr(L, "_LIB", first)
+    monkeypatch.setattr(L, "_NATIVE", Module)
+    monkeypatch.setattr(L, "SO_PATH", str(copy))
+    monkeypatch.setattr(L, "build", lambda: None)
+    again = L.load(rebuild=True)
+    address = lambda lib, n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value
+    assert again is not first and address(again, "fluke_last_error") != address(first, "fluke_last_error")
+    assert bound == [{n: address(again, n) for n in Module.names()}]
+
+
+def test_extension_is_built_for_this_interpreter_and_torch():
+    from fluke_b200 import lib as L
+    import torch
+    L.native()
+    assert sys.implementation.cache_tag in L.native_name() and torch.__version__ in L.native_name()
+    assert os.path.isfile(os.path.join(ROOT, "fluke_b200", L.native_name()))
+    out = subprocess.run(["make", "-n", "-B", "pyext", "PYTHON=" + sys.executable], cwd=ROOT, stdout=subprocess.PIPE, text=True, check=True)
+    assert L.native_name() in out.stdout
 
 
 def test_kernels_trigger_their_dependents_behind_the_tensor_memory_allocation():
