@@ -252,6 +252,20 @@ def test_rotary_qkv_of_one_head_with_a_stride_of_its_own(n, s):
     assert bool((raw[n * s * 192:] == 3.0).all())
 
 
+@pytest.mark.parametrize("h", [8, 40, 248, 264, 520, 776, 1032, 1280, 1544, 1800, 2040, 2048, 2046])
+@pytest.mark.parametrize("n", [1, 9])
+def test_quantisers_of_every_width_vs_oracle(n, h):
+    """Rows of one to eight 16-byte chunks per lane, with a last chunk that only some lanes have, and a width that
+    is no whole number of chunks: the oracle's codes and scales, bit for bit."""
+    x = (torch.randn(n, h, generator=torch.Generator().manual_seed(h)) * 3).half()
+    x[0, -1], x[0, 0] = 700.0, -0.0   # the row's maximum in the last chunk
+    x[-1, 1::7] = 0.0
+    for fp8, op in ((False, ops.quant_int8), (True, ops.quant_fp8)):
+        q, s = op(x.to(DEV))
+        want, ws = port.quant(x.numpy(), fp8)
+        assert np.array_equal(q.cpu().numpy(), want) and np.array_equal(s.cpu().numpy(), ws)
+
+
 def test_empty_inputs_are_noops():
     z = torch.zeros(0, 512, dtype=torch.float16, device=DEV)
     assert ops.quant_int8(z)[0].shape == (0, 512)
