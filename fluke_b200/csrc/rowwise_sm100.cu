@@ -846,9 +846,8 @@ quant_rows_kernel(const __half * in, uint8_t * out,
 // SHIFTS: the thread index decomposes with shifts and one 32-bit division (chunks per head and
 // heads both powers of two, fewer than 2^31 threads); otherwise with 64-bit divisions, which cost
 // more instructions than the rotation itself.
-// VEC: pairs per thread, 16 (256-bit accesses) where alignment allows it and the threads still fill the
-// device, else 8.
-template <bool SHIFTS, int VEC>
+// Sixteen pairs per thread in 256-bit accesses were slower: q and k of 128000 positions 82.7 us, 78.9 this way.
+template <bool SHIFTS>
 __global__ void __launch_bounds__(256)
 rotary_vec_kernel(__half *x, const float *sin_tab, const float *cos_tab,
                   int64_t total, int seq_len, int n_heads, int width, int64_t stride_batch,
@@ -867,7 +866,7 @@ rotary_vec_kernel(__half *x, const float *sin_tab, const float *cos_tab,
         s = int(row - bq * uint32_t(seq_len));
         b = bq;
     } else {
-        const int cpw = width / VEC;
+        const int cpw = width >> 3;
         c = int(idx % cpw);
         int64_t r = idx / cpw;
         h = int(r % n_heads); r /= n_heads;
@@ -875,21 +874,15 @@ rotary_vec_kernel(__half *x, const float *sin_tab, const float *cos_tab,
         b = r / seq_len;
     }
 
-    __half *p0 = x + b * stride_batch + s * stride_seq + h * stride_head + c * VEC;
+    __half *p0 = x + b * stride_batch + s * stride_seq + h * stride_head + c * 8;
     __half *p1 = p0 + width;
-    uint32_t a[VEC / 2], bq[VEC / 2], o0[VEC / 2], o1[VEC / 2];
-    if constexpr (VEC == 16) {
-        load32(p0, a);
-        load32(p1, bq);
-    } else {
-        const uint4 v0 = *reinterpret_cast<const uint4 *>(p0), v1 = *reinterpret_cast<const uint4 *>(p1);
-        a[0] = v0.x; a[1] = v0.y; a[2] = v0.z; a[3] = v0.w;
-        bq[0] = v1.x; bq[1] = v1.y; bq[2] = v1.z; bq[3] = v1.w;
-    }
-    const float4 *cs4 = reinterpret_cast<const float4 *>(cos_tab + int64_t(s) * width + c * VEC);
-    const float4 *sn4 = reinterpret_cast<const float4 *>(sin_tab + int64_t(s) * width + c * VEC);
+    const uint4 v0 = *reinterpret_cast<const uint4 *>(p0), v1 = *reinterpret_cast<const uint4 *>(p1);
+    const uint32_t a[4] = {v0.x, v0.y, v0.z, v0.w}, bq[4] = {v1.x, v1.y, v1.z, v1.w};
+    uint32_t o0[4], o1[4];
+    const float4 *cs4 = reinterpret_cast<const float4 *>(cos_tab + int64_t(s) * width + c * 8);
+    const float4 *sn4 = reinterpret_cast<const float4 *>(sin_tab + int64_t(s) * width + c * 8);
 #pragma unroll
-    for (int v = 0; v < VEC / 4; ++v) {
+    for (int v = 0; v < 2; ++v) {
         const float4 cv = cs4[v], sv = sn4[v];
         const float2 cs[2] = {make_float2(cv.x, cv.y), make_float2(cv.z, cv.w)};
         const float2 sn[2] = {make_float2(sv.x, sv.y), make_float2(sv.z, sv.w)};
@@ -902,13 +895,8 @@ rotary_vec_kernel(__half *x, const float *sin_tab, const float *cos_tab,
         }
     }
     // the paired conversion rounds to nearest even, as __float2half does
-    if constexpr (VEC == 16) {
-        store32(p0, o0);
-        store32(p1, o1);
-    } else {
-        *reinterpret_cast<uint4 *>(p0) = make_uint4(o0[0], o0[1], o0[2], o0[3]);
-        *reinterpret_cast<uint4 *>(p1) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
-    }
+    *reinterpret_cast<uint4 *>(p0) = make_uint4(o0[0], o0[1], o0[2], o0[3]);
+    *reinterpret_cast<uint4 *>(p1) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
 }
 
 // Scalar path for widths or strides that are not multiples of 8 elements.
@@ -1223,16 +1211,12 @@ extern "C" int fluke_sm100_rotary_emb(void *x, const void *sin_tab, const void *
                      (stride_head % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) &&
                      (((reinterpret_cast<uintptr_t>(sin_tab) | reinterpret_cast<uintptr_t>(cos_tab)) & 15u) == 0);
     if (vec) {
-        const int64_t units = int64_t(batch_size) * seq_len * n_heads;
-        const bool wide = W % 16 == 0 && stride_batch % 16 == 0 && stride_seq % 16 == 0 && stride_head % 16 == 0 &&
-                          aligned32(x) && units * (W / 16) >= kFullDeviceThreads;
-        const int vec_pairs = wide ? 16 : 8, cpw = W / vec_pairs;
-        const int64_t total = units * cpw;
+        const int cpw = W / 8;
+        const int64_t total = int64_t(batch_size) * seq_len * n_heads * cpw;
         auto log2_of = [](int v) { int l = 0; while ((1 << l) < v) ++l; return (1 << l) == v ? l : -1; };
         const int cl = log2_of(cpw), hl = log2_of(n_heads);
         const bool shifts = cl >= 0 && hl >= 0 && total < (int64_t(1) << 31);
-        auto kernel = shifts ? (wide ? rotary_vec_kernel<true, 16> : rotary_vec_kernel<true, 8>)
-                             : (wide ? rotary_vec_kernel<false, 16> : rotary_vec_kernel<false, 8>);
+        auto kernel = shifts ? rotary_vec_kernel<true> : rotary_vec_kernel<false>;
         rc = launch_dependent(kernel, grid_for(total, 256), 256, 0, s, static_cast<__half *>(x), static_cast<const float *>(sin_tab),
                               static_cast<const float *>(cos_tab), total, seq_len, n_heads, W, stride_batch, stride_seq, stride_head, cl, hl);
     } else {

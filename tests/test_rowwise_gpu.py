@@ -304,13 +304,13 @@ def test_row512_forms_give_the_bits_of_the_unaligned_ones(n):
 
 @pytest.mark.parametrize("rows", [2367, 2368, 2369])
 def test_wide_elementwise_forms_give_the_bits_of_narrow_ones(rows):
-    """SiLU product and rotary around the row count where a thread takes sixteen elements instead of
-    eight (148 * 2048 threads): equal to the same rows in small calls."""
+    """SiLU product around the row count where a thread takes sixteen elements instead of eight (2048 threads on
+    each of 148 SMs), and the rotation of a batch that large: equal to the same rows in small calls."""
     g = torch.Generator(device=DEV).manual_seed(rows)
     x = torch.randn(rows, 4096, generator=g, device=DEV).half()
     assert torch.equal(ops.silu_mul(x), torch.cat([ops.silu_mul(p.contiguous()) for p in x.split(500)]))
     from fluke_b200 import prep
-    seq, n = 100, 94 + rows % 5  # 16 heads x 2 threads per position: 9472 positions fill the device
+    seq, n = 100, 94 + rows % 5
     sin, cos = prep.rotary_tables(seq, 64, device=DEV)
     qkv = torch.randn(n, seq, 3, 8, 64, generator=g, device=DEV).half()
     want = torch.cat([ops.rotary_qkv_(p.clone(), sin, cos, 32) for p in qkv.split(20)])
