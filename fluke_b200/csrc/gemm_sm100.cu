@@ -787,6 +787,7 @@ int tile_width(const fluke_sm100_gemm_t *g) {
 // coarser items cost more (9331 rows 5.4 -> 5.7).
 bool wide_tiles(const fluke_sm100_gemm_t *g) {
     if (g->N % kFusedBN != 0 || g->K > 512) return false;
+    if (g->N > kPlainBN * device_sm_count()) return false;  // refused below, whatever the number of rows
     return (g->M + 127) / 128 > 2 * (device_sm_count() / (g->N / kFusedBN));
 }
 

@@ -489,3 +489,13 @@ def test_operators_refuse_tensors_of_other_ranks():
                      lambda: ops.rotary_qkv_(z(2, 4, 3, 64, dtype=f16), s, s, 32)):
             with pytest.raises(ValueError):
                 call()
+
+
+def test_more_columns_than_resident_weight_tiles_are_refused_for_any_number_of_rows():
+    """A weight of more 128-row tiles than the device has SMs is an error, few rows or many (the wide form could
+    hold it, but only from some number of rows on)."""
+    n = 128 * (torch.cuda.get_device_properties(0).multi_processor_count // 2 * 2 + 2)
+    b, sb = torch.zeros(n, 128, dtype=torch.int8, device=DEV), torch.zeros(n, device=DEV)
+    for m in (64, 128, 1024, 3000):
+        with pytest.raises(RuntimeError):
+            ops.gemm_i8(torch.zeros(m, 128, dtype=torch.int8, device=DEV), b, torch.zeros(m, device=DEV), sb)
