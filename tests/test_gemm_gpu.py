@@ -420,13 +420,16 @@ def test_transformer_ops_are_shard_invariant(be, be8):
     assert L.read_status() == 0
 
 
-@pytest.mark.parametrize("rows", [1, 31, 128, 129, 300, 512, 1664, 1665, 2304, 2305, 4736, 4737])
-def test_few_tiles_give_the_bits_of_many(be, be8, rows):
+@pytest.mark.parametrize("rows", [1, 31, 128, 129, 300, 512, 513, 1536, 1537, 2304, 2305, 4736, 4737])
+@pytest.mark.parametrize("seqlen", [64, 188])
+def test_few_tiles_give_the_bits_of_many(be, be8, rows, seqlen):
     """The kernel for few output tiles and the persistent one compute an element in the same order, so
     the first rows of a large call and a call of those rows alone have equal bits: int8 and fp8, the
     three fused or plain forms. Row counts at the edges of a 128-row tile and on both sides of the
-    tile counts where a B200 (148 SMs, one or two CTAs each) changes kernel or tile width."""
-    g, m, seqlen = torch.Generator().manual_seed(rows), 6016, 64
+    tile counts where a B200 (148 SMs, one or two CTAs each) changes kernel or tile width: 512 gated, 1536
+    rotary, 2304 and 4736 plain. The large call is 94 sequences of 64 positions, or 32 of 188, whose tiles follow the
+    sequences."""
+    g, m = torch.Generator().manual_seed(rows), 6016
     sin, cos = (t.to(DEV) for t in prep.rotary_tables(seqlen, 64))
     w16 = [torch.randn(n, 512, generator=g) * 0.02 for n in (1536, 2048, 2048, 512)]
     x = torch.randn(m, 512, generator=g)
@@ -473,6 +476,26 @@ def test_wide_plain_tiles_give_the_bits_of_narrow_ones(m, n, k):
         got = run(a, sa)
         for r0 in (0, 127, m // 2, m - 300):
             assert torch.equal(got[r0:r0 + 300], run(a[r0:r0 + 300].contiguous(), sa[r0:r0 + 300].contiguous()))
+
+
+def test_kept_tensor_maps_follow_address_and_shape():
+    """A host thread keeps the tensor maps it has encoded: operands that begin at one address in several shapes,
+    more addresses than it keeps, and the same ones again with other contents give the oracle's results."""
+    g = torch.Generator().manual_seed(5)
+    shapes = [(5, 128, 64), (130, 64, 64), (3, 256, 128), (64, 128, 128)]   # m, k, n
+    weights = {(n, k): prep.quantize_int8_rows(torch.randn(n, k, generator=g)) for _, k, n in shapes}
+    on_gpu = {key: (w.to(DEV), s.to(DEV)) for key, (w, s) in weights.items()}
+    buf = torch.empty(1 << 15, dtype=torch.int8, device=DEV)
+    for _ in range(2):
+        host = torch.randint(-127, 128, buf.shape, generator=g, dtype=torch.int8)
+        buf.copy_(host)
+        for i in range(200):
+            m, k, n = shapes[i % 4]
+            off = 16 * ((i // 4) * 29)
+            sa = torch.rand(m, generator=g) * 0.01
+            got = ops.gemm_i8(buf[off:off + m * k].view(m, k), on_gpu[n, k][0], sa.to(DEV), on_gpu[n, k][1])
+            want = port.gemm_i8(host[off:off + m * k].view(m, k).numpy(), weights[n, k][0].numpy(), sa.numpy(), weights[n, k][1].numpy())
+            assert np.array_equal(got.cpu().numpy(), want), (i, off, m, k, n)
 
 
 def test_operators_refuse_tensors_of_other_ranks():

@@ -19,13 +19,14 @@ DEV = "cuda"
 
 
 # name -> (mode for fluke_set_lstm_persistent, form fluke_sm100_lstm_last_form then reports)
-LSTM_MODES = {"cluster": (4, 1), "persistent_l2": (2, 2), "per_step": (0, 0)}
+LSTM_MODES = {"small_clusters": (1, 3), "cluster": (4, 1), "persistent_l2": (2, 2), "per_step": (0, 0)}
 
 
 @pytest.fixture(params=list(LSTM_MODES))
 def lstm_mode(request, flib):
-    """Runs a test with each form of the layer recurrence: one launch with the exchange inside
-    thread-block clusters, one launch with the exchange through L2, and two launches per step."""
+    """Runs a test with each form of the layer recurrence: one launch with few chunk rows per thread-block cluster
+    (the default), one with the exchange inside larger clusters, one with the exchange through L2, and two
+    launches per step."""
     flib.fluke_set_lstm_persistent(LSTM_MODES[request.param][0])
     yield request.param
     flib.fluke_set_lstm_persistent(1)
@@ -445,13 +446,15 @@ def test_wide_l2_configuration_matches_the_narrow_one(flib):
                                  (768, 858), (768, 859), (768, 1056), (768, 1057), (256, 300), (256, 2900), (384, 47), (384, 1600),
                                  (384, 2048), (512, 1000), (512, 1600), (640, 90), (640, 1200), (896, 500), (896, 800), (1024, 33),
                                  (1024, 470), (1024, 481)])
-def test_small_cluster_form_gives_the_bytes_of_the_l2_form(flib, H, B):
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+def test_small_cluster_form_gives_the_bytes_of_the_l2_form(flib, H, B, T):
     """The default form (few chunk rows per cluster, operands swapped) against the L2-exchange form,
     which shares none of its data movement: same arithmetic in the same order, so equal bytes from a
     non-zero state. Batches around the row counts per cluster where the kernel's column count (16, 32, 48),
     the number of groups or the number of waves changes on a B200, one row, ragged last clusters (an
-    empty second group among them), every cluster size from 2 to 8 CTAs."""
-    T, R = 4, 128
+    empty second group among them), every cluster size from 2 to 8 CTAs; one step (no barrier is armed again, the
+    final state leaves at once) to four."""
+    R = 128
     layer, x, xs = _layer_case(T, B, H, R, H + B, B % 2 == 1)
     g = torch.Generator().manual_seed(B)
     c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
