@@ -620,7 +620,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
 }
 
 // ------------------------------------------------------------------------------------------
-// ------------------------------------------------------------------------------------------
 // Host side: a GemmPlan holds the tensor maps and kernel parameters of one problem; building
 // it costs four cuTensorMapEncodeTiled calls, launching it costs one kernel launch. Loops that
 // re-run the same GEMM on another plane of a 3-D A tensor (the LSTM down-projection per
@@ -632,15 +631,6 @@ struct GemmPlan {
     GemmDev p;
     int grid;
 };
-
-inline int device_sm_count() {
-    static int cached[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev);
-    return cached[dev];
-}
 
 // Raises the dynamic shared-memory limit of KERNEL once per device. The kernel is a template
 // argument so that every instantiation keeps its own "done" flags.

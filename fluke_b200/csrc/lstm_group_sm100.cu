@@ -33,9 +33,9 @@
 // projection of h_{t-1} is complete; and the other way round for hh. Nobody leaves before the final
 // cluster barrier. Clusters never wait for one another, so any number of them may run in waves.
 //
-// What bounds a step (B200, H = 768, cycles at 1.93 GHz): with few rows (3 per cluster, 2790 cycles = 1.48 us)
+// What bounds a step (B200, H = 768, cycles): with few rows (3 per cluster, 2790 cycles, 1.46 us)
 // the chain: h exchange 600, projection 450 + read-back 250, hh exchange 500, contraction 500,
-// cell update 430; with 47 (5500 cycles = 2.86 us for 1024 chunks, 3.08 while the exchanges left in 16-byte
+// cell update 430; with 47 (5500 cycles, 2.8 us for 1024 chunks; 0.2 more while the exchanges left in 16-byte
 // pieces) the tensor pipe (x half 1450, projections 1400, hh half 1150), which waits for the second
 // group's accumulators to be read and its hidden rows to arrive: the accumulators leave no tensor memory for a second set.
 //
@@ -527,8 +527,11 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                         sts8(stage + slot + 2 * j * 128 + q * 32 + lane, h.x);
                         sts8(stage + slot + (2 * j + 1) * 128 + q * 32 + lane, h.y);
                     };
-                    // Both pairs side by side: two chains. The second is left out where its rows do not exist
-                    // (300 chunks 1.94 -> 1.87 us per step) in the kernels that gain from the branch.
+                    // Both pairs side by side: two chains. The second is left out where its rows do not exist.
+                    // With the branch against without, us per step, x_down included: C = 6 7 rows per cluster 1.53 :
+                    // 1.62, 14 rows 1.67 : 1.70, 20 rows 2.25 : 2.37; C = 7 and 8 alike (7 rows 1.57 : 1.67, 1.63 :
+                    // 1.70), 10 rows 1 % slower. Two groups, 47 rows: 3.02 : 2.98, so not there. C = 2 and 3 go without:
+                    // between -5 % (7 rows 1.47 : 1.55) and +1 % (10 and 16 rows).
                     if (G > 1 || C < 4 || 4 * b + 2 < my_rows) {
                         const int2 h0 = codes(0), h1 = codes(1);
                         stage_codes(0, h0);
@@ -592,9 +595,12 @@ struct GroupPlan {
 
 using group_kernel_fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GroupDev);
 struct GroupKernel { int n0, n1; group_kernel_fn fn[kGMaxCtas + 1]; };
+// Rows per cluster from which two groups are the faster: see group_kernel_for.
+constexpr int group_two_from(int C) { return C == 3 ? 17 : 18 + 2 * C; }
 template <int N0, int N1, int C>
 constexpr group_kernel_fn group_kernel_fits() {
-    if constexpr (group_layout(N0, N1, C).dynamic <= kGMaxSmem) return lstm_group_kernel<N0, N1, C>;
+    constexpr bool kUsed = N1 == 0 || N0 + N1 > 32 || group_two_from(C) <= N0 + N1;
+    if constexpr (kUsed && group_layout(N0, N1, C).dynamic <= kGMaxSmem) return lstm_group_kernel<N0, N1, C>;
     else return nullptr;
 }
 template <int N0, int N1>
@@ -611,8 +617,8 @@ const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0
 // projects all rows), 17 rows 2.19 : 2.19, 20 rows 2.40 : 2.21; H = 512, 26 rows 2.36 : 2.35, 32 rows 2.52 : 2.36;
 // H = 768, 28 rows 2.52 : 2.56, 32 rows 2.65 : 2.56; H = 1024, 32 rows 2.75 : 2.80.
 inline int group_kernel_for(int rows, int H) {
-    const int C = H / kGUnits, two_from = C == 3 ? 17 : 18 + 2 * C;
-    const int k = rows <= 16 ? 0 : rows <= 32 ? (rows < two_from ? 1 : 2) : 3;
+    const int C = H / kGUnits;
+    const int k = rows <= 16 ? 0 : rows <= 32 ? (rows < group_two_from(C) ? 1 : 2) : 3;
     return rows <= 48 && kGroupKernels[k].fn[C] ? k : -1;
 }
 

@@ -168,8 +168,8 @@ __device__ __forceinline__ int2 lstm_cell_codes(uint32_t gi0, uint32_t gi1, uint
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(t.x));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ey) : "f"(t.y));
     const float2 den = add2(make_float2(ex, ey), make_float2(1.f, 1.f));
-    // 1 - 2 r with r = 1 / (exp(2c) + 1), which is never below the smallest normal number's inverse:
-    // the flush-to-zero reciprocal needs no range check, and the doubling is exact
+    // 1 - 2 r with r = 1 / (exp(2c) + 1). The denominator is at least 1; where it is so large (or infinite) that
+    // the reciprocal is flushed to zero, 1 - 2 r rounds to 1 either way. The doubling is exact.
     float rx, ry;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(den.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(den.y));

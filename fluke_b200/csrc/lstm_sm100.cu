@@ -213,8 +213,10 @@ struct LstmPlan {
 
 // Units per CTA: the fewest with which all CTAs run at once, because a CTA's epilogue grows with them and a
 // second round costs the whole latency again (1024 rows, H = 768: 32 units in 192 CTAs 9.3 us, 48 in 128 7.5).
-// Sixteen only up to two thirds of the SMs: with more CTAs fetching the same rows, 32 are the faster (300 rows,
-// H = 768: 144 CTAs 5.28 us, 72 CTAs 4.99). With more rows than one round takes, as many as there are.
+// Sixteen only up to two thirds of the SMs: with more CTAs fetching the same rows, 32 are the faster. 16 units
+// against 32, us: 32 to 64 CTAs of 16 units 3.7-4.1 : 4.2-4.3 (H = 384, 48: 4.3 : 4.9), 96 CTAs 4.80 : 4.29 at H = 512,
+// 4.93 : 5.02 at H = 768, 4.81 : 4.92 at H = 384, 120 to 144 CTAs 5.1-5.4 : 4.3-5.1 at every H. With more rows than
+// one round takes, as many as there are.
 inline int pick_units(int B, int H) {
     const int row_tiles = (B + 127) / 128, sms = device_sm_count();
     const int cand[4] = {64, 48, 32, 16};

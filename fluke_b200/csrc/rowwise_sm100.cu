@@ -1095,7 +1095,7 @@ fp8_unshuffle_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src,
     reinterpret_cast<uint2 *>(dst)[idx] = __ldg(reinterpret_cast<const uint2 *>(src) + src_run);
 }
 
-constexpr int64_t kFullDeviceThreads = 148 * 2048;
+inline int64_t full_device_threads() { return int64_t(device_sm_count()) * 2048; }
 inline int grid_for(int64_t total, int block) { return int((total + block - 1) / block); }
 
 }  // namespace
@@ -1238,7 +1238,7 @@ extern "C" int fluke_sm100_silu_mul(const void *in, void *out, int n_tokens, int
     // Sixteen elements per thread once those threads fill the device ([32000, 4096]: 72.8 -> 62.8 us, 0.95 of
     // the copy bandwidth); below that twice as many threads with eight each finish sooner (125 rows:
     // 1.84 against 2.27 us, 1803 rows 4.85 against 5.0).
-    if (vec && hidden_dim % 16 == 0 && aligned32(in, out) && int64_t(n_tokens) * (hidden_dim / 16) >= kFullDeviceThreads) {
+    if (vec && hidden_dim % 16 == 0 && aligned32(in, out) && int64_t(n_tokens) * (hidden_dim / 16) >= full_device_threads()) {
         const int64_t total = int64_t(n_tokens) * (hidden_dim / 16);
         rc = launch_dependent(silu_mul_kernel<16>, grid_for(total, 256), 256, 0, s, static_cast<const __half *>(in), static_cast<__half *>(out), total, hidden_dim);
     } else if (vec) {
