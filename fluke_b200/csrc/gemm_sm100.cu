@@ -219,12 +219,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         if (kDual) tma_prefetch_desc(&tm_b2);
         tma_prefetch_desc(&tm_out);
     }
-    if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemCols);
+        dependency_trigger();
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    dependency_trigger();
     dependency_wait();
     // The launch gives every thread 65536 / 384 registers; the loader and issuer need few, the
     // epilogue threads hold a whole row segment plus rotary tables: each role branch below

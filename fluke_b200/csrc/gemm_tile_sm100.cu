@@ -78,12 +78,14 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         tma_prefetch_desc(&tm_b);
         if (kDual) tma_prefetch_desc(&tm_b2);
     }
-    if (warp == 1) tmem_alloc(&tmem_slot, kTmemCols);
+    if (warp == 1) {
+        tmem_alloc(&tmem_slot, kTmemCols);
+        dependency_trigger();
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    dependency_trigger();
     dependency_wait();
 
     if (warp == 0) {

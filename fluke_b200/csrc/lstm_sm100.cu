@@ -92,12 +92,14 @@ lstm_step_kernel(const __grid_constant__ CUtensorMap tm_a_lo,
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemCols);
+        dependency_trigger();
+    }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    dependency_trigger();
     dependency_wait();
 
     if (warp == 0) {

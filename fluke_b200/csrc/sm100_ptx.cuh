@@ -77,10 +77,10 @@ __device__ __forceinline__ void fence_barrier_init() {
 // Programmatic dependent launch (the kernels launched with launch_dependent() of tma_host.cuh)
 // ---------------------------------------------------------------------------------------
 // Lets the next kernel of the stream be set up on the device as soon as every block of this one has
-// come here; what it does before its own dependency_wait() runs beside this kernel. A block that uses tensor
-// memory comes here behind the barrier that follows its tmem_alloc(): the next kernel's blocks take their
-// columns while this one runs and keep them until it ends, so a block of this one that had yet to allocate could
-// wait for them for ever.
+// come here (one thread of it is enough); what it does before its own dependency_wait() runs beside this kernel.
+// In a block that uses tensor memory only the warp that allocates comes here, behind its tmem_alloc(): the next
+// kernel's blocks take their columns while this one runs and keep them until it ends, so a block of this one that
+// had yet to allocate could wait for them for ever.
 __device__ __forceinline__ void dependency_trigger() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

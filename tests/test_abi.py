@@ -119,9 +119,9 @@ def test_extension_is_built_for_this_interpreter_and_torch():
 
 
 def test_kernels_trigger_their_dependents_behind_the_tensor_memory_allocation():
-    """In a kernel that lets its dependents start early, the allocation of tensor memory and a barrier of the
-    block come first: otherwise a dependent block could take the columns that a block of this kernel still
-    has to get, and wait for that block while holding them."""
+    """In a kernel that lets its dependents start early, the warp that allocates tensor memory does so behind the
+    allocation, and no other thread does: otherwise a dependent block could take the columns that a block of this
+    kernel still has to get, and wait for that block while holding them."""
     found = 0
     for path in glob.glob(os.path.join(ROOT, "fluke_b200", "csrc", "*.cu")):
         for body in open(path).read().split("__global__")[1:]:
@@ -129,8 +129,8 @@ def test_kernels_trigger_their_dependents_behind_the_tensor_memory_allocation():
             if at < 0 or "tmem_alloc(" not in body:
                 continue
             found += 1
-            alloc = body.index("tmem_alloc(")
-            assert 0 <= alloc < body.find("__syncthreads();", alloc) < at < body.index("dependency_wait();"), path
+            assert re.search(r"if \(warp == 1\) \{\s*tmem_alloc\([^;]*;\s*dependency_trigger\(\);\s*\}", body), path
+            assert body.count("dependency_trigger();") == 1 and at < body.index("dependency_wait();"), path
     assert found >= 3
 
 
