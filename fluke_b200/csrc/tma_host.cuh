@@ -40,10 +40,9 @@ inline int device_sm_count() {
 
 // cuTensorMapEncodeTiled with the options every map of the library shares (no interleave, unit
 // element strides, 256-byte L2 promotion, zero fill). An encoded map depends on nothing but these
-// arguments, so each host thread keeps up to kMapSlots of them, one per value of the hash: an encode takes the
-// driver 0.5 us, a GEMM call needs three or four, and a program that calls with the same buffers again finds those
-// whose slots no other map has taken. Operands at new addresses are encoded on every call. One LSTM step of 64
-// chunks, nine maps: 12.3 us with all of them found.
+// arguments, so each host thread keeps up to kMapSlots of them, one per value of the hash. A program that calls
+// with the same buffers again finds those whose slots no other map has taken; operands at new addresses are encoded in
+// every call. Host time of an LSTM step, nine maps: 8.5 us with all of them found, 8.95 with none kept.
 constexpr int kMapSlots = 64;
 struct TmapKey {
     const void *base;

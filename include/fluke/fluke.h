@@ -437,8 +437,11 @@ size_t fluke_factored_lstm_layer_workspace(int T, int B, int H, int R);
 int fluke_factored_lstm_layer_i8_gpu(const fluke_flstm_layer_t *layer);
 
 /* How fluke_factored_lstm_layer_i8_gpu runs the recurrence (a per-thread setting).
- *   1 (default): one launch per layer -- gate weights in shared memory and the cell state in
- *      registers for all T timesteps -- in the fastest form the shape and the device allow.
+ *   1 (default): one launch per layer -- gate weights on chip and the cell state in registers for
+ *      all T timesteps -- in the fastest form the shape and the device allow: the batch spread over
+ *      many small thread-block clusters (R = 128, H a multiple of 128 from 256 to 1024; the recurrent
+ *      half of the gate weights in tensor memory), else the form of mode 4 while all row tiles run
+ *      at once, else that of mode 2, else that of mode 4 in rounds.
  *   2: exchange through L2 with separate projection thread blocks (R = 128, H a multiple of 128
  *      up to 1024).
  *   4: exchange inside thread-block clusters through distributed shared memory (R = 128, H a
