@@ -772,7 +772,7 @@ def run_ours(args):
     ms_copy = timed(copy_only, args.steps, after=copy_done)
     torch.cuda.empty_cache()
 
-    # the recurrence kernel of the timed region (the wide configuration: 16 row tiles in one launch):
+    # the recurrence kernel of the timed region (both steps of a pair, 2048 chunks, in one launch):
     # layer minus x_down GEMM, both from CUDA events
     lay0 = layers[0]
     st2 = (torch.zeros(2 * B, H, dtype=torch.float32, device=dev), torch.zeros(2 * B, H, dtype=torch.int8, device=dev))
@@ -854,7 +854,7 @@ def run_ours(args):
                                    f"{B} chunks per GPU per step", "l2": "inputs larger than L2 (786 MB per layer input)",
                        "parallelism": f"dp{world} (independent chunks, no collective)",
                        "steps_per_launch": "2: the K independent steps run two at a time, side by side in one [T, 2048, H] "
-                                           "layer launch (16 row tiles); one_pass_per_launch is the figure with one step per launch"},
+                                           "layer launch ; one_pass_per_launch is the figure with one step per launch"},
             "timesteps_per_sec_per_gpu_per_layer": T * NL / (ms * 1e-3),
             "one_pass_per_launch": {"value": units / (ms_single * 1e-3), "unit": UNIT, "ms_per_step": ms_single,
                                     "roofline": roofline_single},

@@ -34,8 +34,8 @@ def _call_noalloc(layer, x, xs, c, h, reverse):
 
 @pytest.fixture(params=[1, 4, 2, 0], ids=["default", "cluster", "l2_exchange", "per_step"])
 def form(request):
-    """Every way the layer can run keeps different intermediates in the shared array: the cluster
-    form only x_down, the L2-exchange form also hh_down and its exchange counters, the per-step
+    """Every way the layer can run keeps different intermediates in the shared array: the default and
+    the cluster form only x_down, the L2-exchange form also hh_down and its exchange counters, the per-step
     kernels hh_down. The leftovers of the previous call must be harmless in each."""
     L.load().fluke_set_lstm_persistent(request.param)
     yield request.param
