@@ -6,38 +6,45 @@
 // to move and compute for its own rows. With the rows as the M = 128 dimension of the
 // contractions that amount does not shrink with the batch; here the operands are swapped. The
 // WEIGHTS are the M dimension (128 hidden units per CTA, one accumulator block per gate) and the
-// chunk rows are N = 16, 32 or 48 columns, and the recurrent half of the gate weights lives in
-// TENSOR MEMORY as the A operand: an MMA then costs 12 to 20 cycles instead of the 40 that reading a
-// 128-row A operand from shared memory takes whatever N is.
+// chunk rows the columns, and the recurrent half of the gate weights lives in
+// TENSOR MEMORY as the A operand: an MMA of 16 columns then costs 12 cycles instead of the 42 that reading a
+// 128-row A operand from shared memory takes (32 columns 18 against 44, 48 columns 24 against 48).
 //
-// A cluster has C = H / 128 CTAs (2 to 8). CTA j
-//   * owns units 128 j .. 128 j + 127: their four gate weight blocks (hh half in tensor memory, x
-//     half in shared memory) and, in registers, their cell state for the cluster's rows;
-//   * projects: the CTAs form pairs (2p, 2p+1); pair p owns a contiguous part of the rows, CTA
-//     2p + s computes projection columns 64 s .. 64 s + 63 of them (M = 64) from the complete
-//     int8 rows. With an odd C the last CTA projects nothing.
-// Per step two exchanges inside the cluster, both of 16-byte st.async stores (eight lanes write 128
-// contiguous bytes) that complete on an mbarrier of the receiver: the int8 hidden slices go to the pair that
-// owns the row, the f16 projections back to every CTA. The x half of the contraction runs meanwhile. With
-// more than some thirty rows the cluster treats them as two groups, so that one is computed while the
-// other travels.
+// A cluster has C = H / 128 CTAs (2 to 8). CTA j owns units 128 j .. 128 j + 127: their four gate weight
+// blocks (hh half in tensor memory, x half in shared memory) and, in registers, their cell state for the
+// cluster's rows. What is exchanged for the projection of the hidden rows depends on how many rows there are:
 //
-//   warp 0       loader: resident weights, x_down rows of every step
+//   GATHER, up to 16 rows: every CTA sends the int8 codes of its units to all CTAs and projects the complete
+//   rows itself (M = 128 projection columns, K = H). One exchange per step.
+//
+//   SPLIT, two groups of up to 16 or 24 rows: a CTA projects only its own units (K = 128), so hidden codes do not
+//   leave it. Its int32 partial sums go, four rows at a time, to the CTA that adds up those rows (integer sums,
+//   exact in any order), which sends the f16 result to all. Projecting complete rows takes 24 MMAs per group
+//   at H = 768 and 96 KB of weights, this 4 and 16 KB; what one group waits for is the other's time.
+//
+// All exchanges are 16-byte st.async stores that complete on an mbarrier of the receiver.
+//
+//   warp 0       loader: resident weights, x_down rows of every step; SPLIT: also the TMA stores of h_out
 //   warp 1       MMA issuer
-//   warps 2-17   epilogues, four per tensor-memory lane quadrant: thread = hidden unit, a quarter
-//                of the rows each (gates, cell update, int8 code); the same warps turn the
-//                projection accumulators into f16 and send them
+//   warps 2-17   four per tensor-memory lane quadrant: thread = hidden unit and projection column. GATHER: each has a quarter
+//                of the rows; SPLIT: eight warps per group, each half of its rows. They turn the projections into f16 (SPLIT:
+//                send, add up, send) and compute gates, cell update and int8 codes
 //
-// A buffer is only overwritten after its reader has provably finished: a CTA sends h_t (of a group) after
-// its gate contraction of step t, which needs hh_t from every pair, which a pair sends after its
-// projection of h_{t-1} is complete; and the other way round for hh. Nobody leaves before the final
-// cluster barrier. Clusters never wait for one another, so any number of them may run in waves.
+// A buffer is only overwritten after its reader has provably finished. SPLIT: a CTA sends partial sums of step t + 1
+// after its gate contraction of step t, for which every owner of rows has read its partial sums of step t; an owner
+// sends hh_{t+1} after every CTA's projection of h_t, i.e. after every CTA's contraction of step t. GATHER: a
+// CTA sends h_t after it has received h_{t-1} of every CTA, which each sent after its projection of h_{t-2}: two
+// slots of hidden rows. Nobody leaves before the final cluster barrier. Clusters never wait for one
+// another, so any number of them may run in waves.
 //
-// What bounds a step (B200, H = 768, cycles): with few rows (3 per cluster, 2790 cycles, 1.46 us)
-// the chain: h exchange 600, projection 450 + read-back 250, hh exchange 500, contraction 500,
-// cell update 430; with 47 (5500 cycles, 2.8 us for 1024 chunks; 0.2 more while the exchanges left in 16-byte
-// pieces) the tensor pipe (x half 1450, projections 1400, hh half 1150), which waits for the second
-// group's accumulators to be read and its hidden rows to arrive: the accumulators leave no tensor memory for a second set.
+// What bounds a step (B200, H = 768, cycles). 2 rows per cluster, 2100: the chain of exchange (490 from the first
+// store to the last arrival), projection 500, its conversion 220, hh half 460, cell update and staging 450. 14 rows, 2900: the
+// same with 950 for the cell updates and 600 for the exchange. 47 rows, 4930: tensor pipe (x part 1540, hh half 1460,
+// projections 370), idle from the end of a step's contractions to the first group's codes (900: 24 rows x 128 units of
+// cell updates share the special-function units with the other group's).
+//
+// The operand rows that are zero (see group_form) add zero times a weight to another group's or step's accumulators: with
+// finite weights nothing.
 //
 // Arithmetic and its order are those of the other single-launch forms (x_down half first, then the
 // hh_down half in K steps of 16; int32 sums scaled by (1/127)*scale and rounded to f16): the bytes
@@ -53,11 +60,11 @@
 namespace fluke_sm100 {
 namespace {
 
-constexpr int kGThreads = 576;
-constexpr int kGEpiWarps = 16;
 constexpr int kGUnits = 128;       // hidden units per CTA = tensor-memory lanes
 constexpr int kGRank = 128;        // factor rank the kernel is built for
 constexpr int kGMaxCtas = 8;       // portable cluster size: H <= 1024
+constexpr int kGEpiWarps = 16;
+constexpr int kGThreads = 32 * (2 + kGEpiWarps);
 constexpr int kGTmemCols = 512;
 constexpr int kGTmemW = 256;       // first column of the hh half of the gate weights: 4 gates x 64
 constexpr int kGWxBytes = 4 * kGUnits * 256;  // x half of the gate weights in shared memory
@@ -67,7 +74,6 @@ struct GroupDev {
     int T, B;
     int reverse;
     int rows;                  // chunk rows per cluster (the last one may have fewer)
-    int n_own[2];              // rows of a group a pair projects
     const int8_t *dn;          // [R, H]
     const __half *w_up;        // [4H, 2R]
     const float *bias;         // [4H]
@@ -75,48 +81,68 @@ struct GroupDev {
     float *c;                  // [B,H]
     int8_t *h_out;             // [T,B,H]
     int8_t *h_state;           // [B,H]: final hidden state
-    long long *trace;          // trace builds only: [T][8] SM-clock stamps of CTA 0
+    long long *trace;          // trace builds only: [T][16] SM-clock stamps of CTA 0
 };
 
-// All of the following depends on the cluster size C = H / 128, which the kernel is compiled for: with
-// operand addresses at fixed distances the issuer needs few instructions between MMAs (the 24 of a
-// projection took 800 cycles to issue with C a variable).
-// Rows of a group's hidden tile (and columns of its projection): what a pair projects of the group's n rows, as
-// a multiple of 8.
-__host__ __device__ constexpr int group_h_rows(int n, int C) { return ((n + C / 2 - 1) / (C / 2) + 7) / 8 * 8; }
-// K blocks (128 hidden units, 32 columns) of the projection weights that fit in tensor memory beside
-// the gate weights, the gate accumulators and the projections.
-__host__ __device__ constexpr int group_dn_ts(int n0, int n1, int C) {
-    const int fit = (kGTmemW - 4 * (n0 + n1) - group_h_rows(n0, C) - group_h_rows(n1, C)) / 32;
-    return fit < C ? fit : C;
+// The forms of the kernel: chunk rows per cluster up to 8, 16, 32 and 48. GATHER is one group of rows, SPLIT two. Step of the
+// kernel of one and two groups that exchanged hidden rows between pairs of CTAs and projected them there, against
+// these, in us, x_down included: H = 768 32 chunks (2 rows per cluster) 1.45 : 1.14, 170 (8 rows) 1.56 : 1.30, 300 (14 rows) 1.66 :
+// 1.61, 500 (23 rows) 2.40 : 2.05, 700 (32 rows) 2.62 : 2.13, 1024 (47 rows) 2.97 : 2.89; H = 384, 32 chunks (2 rows) 1.37 : 1.07;
+// H = 1024, where it took two waves from 577 chunks on, 700 (39 rows) 4.85 : 2.92.
+// Everything below depends on the form V and the cluster size C = H / 128, which the kernel is compiled
+// for: with operand addresses at fixed distances the issuer needs few instructions between MMAs.
+constexpr int kGForms = 4;
+struct GroupForm {
+    int most;           // rows per cluster
+    bool gather;
+    int groups, rows;   // groups, and chunk rows of each at most
+    int n;              // columns of the MMAs of one group: M = 128 takes multiples of 16
+    int stride;         // accumulator columns from gate to gate
+    int proj;           // columns of projection accumulators
+    int x_slots;        // steps whose x_down rows are in shared memory
+};
+// 8 rows: the sixteen columns that an MMA has at least are two steps' rows, see x_half. Two groups of 24 rows: an MMA of
+// the first group also covers the first columns of the second, with operand rows that are zero, before that
+// group's own MMAs; the second group's covers unused columns. They take turns with one projection accumulator.
+__host__ __device__ constexpr GroupForm group_form(int V) {
+    return V == 0   ? GroupForm{8, true, 1, 8, 16, 16, 16, 5}
+           : V == 1 ? GroupForm{16, true, 1, 16, 16, 16, 16, 2}
+           : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32, 2}
+                    : GroupForm{48, false, 2, 24, 32, 56, 32, 2};
 }
-// Rows of a staging slot: a batch of four hidden rows, or the projected rows of a quarter of the warps.
-__host__ __device__ constexpr int group_stage_rows(int n0, int n1, int C) {
-    const int r = group_h_rows(n0 > n1 ? n0 : n1, C) / 4;
-    return r > 4 ? r : 4;
+// K steps (32 units, 8 columns) of the projection weights that fit in tensor memory beside the gate weights, the gate
+// accumulators and the projections.
+__host__ __device__ constexpr int group_dn_ts(int V, int C) {
+    const GroupForm f = group_form(V);
+    const int fit = (kGTmemW - 4 * f.stride - f.proj) / 8, all = f.gather ? 4 * C : 4;
+    return fit < all ? fit : all;
+}
+// Four rows of a group are projected as one piece (16 bytes per projection column). The pieces of all groups are dealt to
+// the C CTAs in turn; the owner adds up what the C CTAs have of it.
+__host__ __device__ constexpr int group_own_pieces(int V, int C) {
+    return (group_form(V).groups * group_form(V).rows / 4 + C - 1) / C;
 }
 struct GroupLayout {
-    int x, hh, dn, h, stage, bars, misc, dynamic;
+    int x, hh, dn, h, recv, stage, bars, misc, dynamic;
 };
-__host__ __device__ constexpr GroupLayout group_layout_slots(int n0, int n1, int C, int x_slots) {
+__host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
+    const GroupForm f = group_form(V);
     GroupLayout l = {};
-    const int n = n0 + n1;
-    l.x = kGWxBytes;                            // x_down rows: 2 K blocks [n x 128 B] per slot
-    l.hh = l.x + x_slots * n * 256;             // hh_down rows, the same shape
-    l.dn = l.hh + n * 256;                      // 64 projection rows: the K blocks not in tensor memory [64 x 128 B]
-    l.h = l.dn + 8192 * (C - group_dn_ts(n0, n1, C));  // hidden rows of the pair, per group: C K blocks
-    l.stage = l.h + (group_h_rows(n0, C) + group_h_rows(n1, C)) * C * kGUnits;  // 2 slots x 4 x [rows x 128 B]
-    l.bars = l.stage + 8 * group_stage_rows(n0, n1, C) * 128;
-    l.misc = l.bars + 15 * 8;
-    l.dynamic = l.misc + 16 + 1024;             // slack for the manual 1024-byte alignment
+    l.x = kGWxBytes;                              // x_down rows, see x_half
+    l.hh = l.x + f.x_slots * f.groups * f.rows * 256;
+    // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
+    l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
+    // projection weights [128 x 128 B] of the K blocks that are not all in tensor memory
+    l.h = l.dn + 16384 * ((f.gather ? C : 1) - group_dn_ts(V, C) / 4);
+    // int8 hidden rows. GATHER: two slots of C K blocks [rows x 128 B]; else this CTA's units, per group [rows x 128 B].
+    // An MMA of more columns reads on behind them
+    l.recv = l.h + (f.gather ? 2 * C : f.groups) * f.rows * 128;
+    // partial sums of the CTA's own pieces: per piece and source CTA [128 columns][4 rows] int32
+    l.stage = l.recv + (f.gather ? 0 : group_own_pieces(V, C) * C * 2048);
+    l.bars = l.stage + 2048;                      // GATHER: two slots x four quarters x [2 rows x 128 B]; else per warp [2 rows x 64 B]
+    l.misc = l.bars + 24 * 8;
+    l.dynamic = l.misc + 16 + 1024;               // slack for the manual 1024-byte alignment
     return l;
-}
-// x tiles of two steps where shared memory allows it, else of one.
-__host__ __device__ constexpr int group_x_slots(int n0, int n1, int C) {
-    return group_layout_slots(n0, n1, C, 2).dynamic <= kGMaxSmem ? 2 : 1;
-}
-__host__ __device__ constexpr GroupLayout group_layout(int n0, int n1, int C) {
-    return group_layout_slots(n0, n1, C, group_x_slots(n0, n1, C));
 }
 
 // 16 bytes into a CTA of the cluster; completes 16 bytes of the transaction count of an mbarrier
@@ -133,6 +159,16 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ int2 lds64(uint32_t addr) {
+    int2 v;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ int lds8(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
 __device__ __forceinline__ void sts8(uint32_t addr, int v) {
     asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
@@ -146,65 +182,92 @@ __device__ __forceinline__ void quad_sync(int id) { asm volatile("barrier.cta.sy
 template <int V>
 struct Int { static constexpr int value = V; };  // a number that a lambda receives as a type
 
-// N0 + N1: accumulator columns, i.e. chunk rows of a cluster at most. With N1 = 0 they are one group: the chain
-// of a step is all there is to run. Otherwise the first N0 rows and the others are two groups that share the
-// x part of the contraction (its MMAs read their A operand from shared memory, 40 cycles each whatever
-// N is up to 64, so one for both) and go through the rest of the step one after the other: while
-// one is exchanged, the other is projected or computed.
-template <int N0, int N1, int C>
+// The groups of chunk rows share the x part of the contraction (its MMAs read their A operand from shared memory, so
+// one for both) and go through the rest of the step one after the other: while one is exchanged, the other
+// is projected or computed.
+template <int V, int C>
 __global__ void __launch_bounds__(kGThreads, 1)
 lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] f16, boxes 128 x 64
-                  const __grid_constant__ CUtensorMap tm_x,    // x_down [T, 2, B, 64] f16, boxes of NB rows
-                  const __grid_constant__ CUtensorMap tm_dn,   // dn_hh [R, H] int8, boxes 64 x 128
-                  const __grid_constant__ CUtensorMap tm_h0,   // h_0 [H/128, B, 128] int8, boxes of the first group's tile
-                  const __grid_constant__ CUtensorMap tm_h1,   // and of the second's
+                  const __grid_constant__ CUtensorMap tm_x,    // x_down [T, 2, B, 64] f16, boxes of all rows
+                  const __grid_constant__ CUtensorMap tm_dn,   // dn_hh [R, H] int8, boxes 128 x 128
+                  const __grid_constant__ CUtensorMap tm_h0,   // h_0 [H/128, B, 128] int8, boxes of a group's rows; GATHER: of all K blocks
+                  const __grid_constant__ CUtensorMap tm_o,    // SPLIT: h_out [T, B, H], boxes of the first group's rows x 128
+                  const __grid_constant__ CUtensorMap tm_ol,   // and of the second's
                   const GroupDev p) {
-    constexpr int G = N1 > 0 ? 2 : 1, NB = N0 + N1;
-    constexpr int kXSlots = group_x_slots(N0, N1, C);
-    constexpr int H = C * kGUnits;
-    constexpr int kPad0 = group_h_rows(N0, C), kPad1 = group_h_rows(N1, C);
-    constexpr int kDnTs = group_dn_ts(N0, N1, C);
-    constexpr GroupLayout L = group_layout(N0, N1, C);
-    constexpr int kCols = (N0 > N1 ? N0 : N1) / 4;   // rows of a group that an epilogue thread holds at most
-    constexpr int kBatches = kCols / 4;              // it takes them four at a time
-    constexpr int kSendP = kCols / 4;                // 16-byte stores per lane and step, projections
-    constexpr int kStageRows = group_stage_rows(N0, N1, C);
-    static_assert(N0 % 16 == 0 && N1 % 16 == 0 && 5 * NB <= kGTmemW, "accumulators beside the weights in tensor memory");
+    constexpr GroupForm F = group_form(V);
+    constexpr bool kGather = F.gather;
+    constexpr int G = F.groups, NB = G * F.rows, S = F.stride, H = C * kGUnits;
+    constexpr bool kTwoSteps = F.rows == 8;            // an x MMA covers two steps
+    constexpr int kXSlots = kTwoSteps ? 4 : F.x_slots;
+    constexpr int kTile = F.rows * 128;                // bytes of a group's hidden rows in one K block
+    constexpr int kHhTile = (kTwoSteps ? 24 : F.n) * 128;   // and of its hh_down rows
+    constexpr int kPieces = F.rows / 4;                // pieces of a group
+    constexpr int kPairs = kGather ? F.rows / 8 : F.rows / 4;   // pairs of rows of a gate thread
+    constexpr int kDnTs = group_dn_ts(V, C);
+    constexpr int kDnCol = kGTmemW - 8 * kDnTs;        // first column of the projection weights in tensor memory
+    constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
+    constexpr GroupLayout L = group_layout(V, C);
+    static_assert(4 * S + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
+    static_assert(L.dynamic <= kGMaxSmem, "shared memory of a CTA");
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
     // shared-window offsets as this CTA's
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *bar_once = &bars[0];       // resident weights loaded
+    uint64_t *bar_once = &bars[0];       // resident weights and the initial hidden rows loaded
     uint64_t *bar_x = &bars[1];          // [slots] x_down rows landed
-    uint64_t *bar_x_free = &bars[3];     // [slots] x half of the contraction has read them
-    uint64_t *bar_h = &bars[5];          // [G] complete hidden rows of the pair arrived
-    uint64_t *bar_proj = &bars[7];       // [G] projection accumulator complete
-    uint64_t *bar_hh = &bars[9];         // [G] hh_down rows arrived
-    uint64_t *bar_acc = &bars[11];       // [G] gate accumulators complete
-    uint64_t *bar_acc_free = &bars[13];  // [G] epilogue has read them
+    uint64_t *bar_x_free = &bars[5];     // [slots] the x part of the contraction has read them
+    uint64_t *bar_acc_free = &bars[9];   // the gate warps have read all accumulators
+    uint64_t *bar_proj = &bars[10];      // [G] projection accumulator complete
+    uint64_t *bar_acc = &bars[12];       // [G] gate accumulators complete
+    uint64_t *bar_hh = &bars[14];        // [G] hh_down rows in place
+    uint64_t *bar_code = &bars[16];      // SPLIT [G]: hidden codes of this CTA's units in place
+    uint64_t *bar_sum = &bars[18];       // SPLIT [G]: partial sums of the CTA's own pieces arrived
+    uint64_t *bar_sent = &bars[20];      // SPLIT: the projection accumulator has been read
+    uint64_t *bar_stored = &bars[21];    // SPLIT: the TMA stores have read the hidden codes
+    uint64_t *bar_h = &bars[16];         // GATHER [2]: hidden rows of all CTAs arrived
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0), lane = threadIdx.x & 31;
     const int rank = int(cluster_ctarank());
-    const int pair = rank >> 1, half = rank & 1;
-    const bool projects = rank < (C & ~1);
     const int m0 = (blockIdx.x / C) * p.rows;          // first chunk row of the cluster
     const int n_rows = min(p.rows, p.B - m0);          // and how many it has
     const int n0 = rank * kGUnits;
-    // of group e: rows it has, rows of them this CTA projects
-    auto rows_of = [&](int e) { return G == 1 ? n_rows : e == 0 ? min(n_rows, N0) : max(n_rows - N0, 0); };
-    auto own_of = [&](int e) { return min(max(rows_of(e) - pair * p.n_own[e], 0), p.n_own[e]); };
-    constexpr int h_group1 = kPad0 * H;                // byte offset of the second group's hidden rows
+    auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
+    // whether this CTA adds up piece k of group e, and how many pieces of the group it adds up
+    auto own_piece = [&](int e, int k) { return (kPieces * e + k) % C == rank && 4 * k < rows_of(e); };
+    auto own_pieces = [&](int e) {
+        int n = 0;
+#pragma unroll
+        for (int k = 0; k < kPieces; ++k) n += own_piece(e, k);
+        return n;
+    };
+    const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 13; ++b) mbar_init(&bars[b], 1);
-        for (int b = 13; b < 15; ++b) mbar_init(&bars[b], kGEpiWarps);
+        for (int b = 0; b < 24; ++b) mbar_init(&bars[b], 1);
+        mbar_init(bar_acc_free, kGather || both ? kGEpiWarps : kGEpiWarps / 2);
+        if (kGather) mbar_init(bar_hh, kGEpiWarps);
+        else for (int e = 0; e < G; ++e) mbar_init(&bar_code[e], kGEpiWarps / 2);
+        if (!kGather) mbar_init(bar_sent, kGEpiWarps / 2);
         *abort_flag = 0;
         fence_barrier_init();
-        for (int e = 0; e < G; ++e) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+        if constexpr (kGather) {
+            for (int s = 0; s < 2; ++s)
+                if (s + 1 < p.T) mbar_arrive_expect_tx(&bar_h[s], uint32_t(n_rows) * H);
+        } else {
+            for (int e = 0; e < (both ? 2 : 1); ++e) {
+                mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+                if (const int n = own_pieces(e)) mbar_arrive_expect_tx(&bar_sum[e], uint32_t(n) * C * 2048);
+            }
+        }
+    }
+    if (kHhTile > F.rows * 128) {   // the operand rows that are zero
+        for (int o = threadIdx.x * 16; o < L.dn - L.hh; o += kGThreads * 16)
+            *reinterpret_cast<uint4 *>(smem + L.hh + o) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_smem();
     }
     if (warp == 1) tmem_alloc(tmem_slot, kGTmemCols);
     tc_fence_before_sync();
@@ -216,17 +279,13 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         const int q = warp & 3, g = (warp - 2) >> 2;
         const uint4 *src = reinterpret_cast<const uint4 *>(
             p.w_up + (size_t(g) * H + n0 + q * 32 + lane) * (2 * kGRank));
-        const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16) + kGTmemW;
+        const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
 #pragma unroll 1
-        for (int v = 0; v < 8; ++v) tmem_st_32x8(t_lane + g * 64 + v * 8, __ldg(src + 2 * v), __ldg(src + 2 * v + 1));
-        if (projects) {
-            // and K blocks g, g + 4, .. of the projection rows (M = 64: row 16 q + i in lane 32 q + i)
-            const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(half * 64 + q * 16 + (lane & 15)) * H);
-            for (int kb = g; kb < kDnTs; kb += 4)
+        for (int v = 0; v < 8; ++v) tmem_st_32x8(t_lane + kGTmemW + g * 64 + v * 8, __ldg(src + 2 * v), __ldg(src + 2 * v + 1));
+        // and K steps g, g + 4, .. of the projection rows, of all units or this CTA's
+        const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(q * 32 + lane) * H + (kGather ? 0 : n0));
 #pragma unroll 1
-                for (int v = 0; v < 4; ++v)
-                    tmem_st_32x8(t_lane - 32 * (kb + 1) + v * 8, __ldg(dn + kb * 8 + 2 * v), __ldg(dn + kb * 8 + 2 * v + 1));
-        }
+        for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
         tmem_st_wait();
         tc_fence_before_sync();
     }
@@ -238,26 +297,48 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     if (warp == 0) {
         // ------------------------------ loader (one thread) -----------------------------
         if (elect_one()) {
-            mbar_arrive_expect_tx(bar_once, kGWxBytes + (projects ? (C - kDnTs) * 8192 : 0));
+            constexpr int kDnTiles = (L.h - L.dn) / 16384;   // the last K blocks
+            mbar_arrive_expect_tx(bar_once, kGWxBytes + kDnTiles * 16384 + (kGather ? C : 1) * NB * 128);
             for (int g = 0; g < 4; ++g)
                 for (int kb = 0; kb < 2; ++kb)
                     tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
-            if (projects) {
-                for (int kb = kDnTs; kb < C; ++kb)
-                    tma_load_2d(smem + L.dn + (kb - kDnTs) * 8192, &tm_dn, bar_once, kb * 128, half * 64);
-                // step 0 projects the layer's initial hidden state
-                for (int e = 0; e < G; ++e) {
-                    mbar_arrive_expect_tx(&bar_h[e], uint32_t(e ? kPad1 : kPad0) * H);
-                    tma_load_3d(smem + L.h + e * h_group1, e ? &tm_h1 : &tm_h0, &bar_h[e], 0, m0 + e * N0 + pair * p.n_own[e], 0);
-                }
-            }
+            for (int b = 0; b < kDnTiles; ++b)
+                tma_load_2d(smem + L.dn + b * 16384, &tm_dn, bar_once, kGather ? (kDnTs / 4 + b) * kGUnits : n0, 0);
+            // step 0 projects the layer's initial hidden state
+            for (int e = 0; e < G; ++e)
+                tma_load_3d(smem + L.h + (kGather ? C : e) * kTile, &tm_h0, bar_once, 0, m0 + F.rows * e, kGather ? 0 : rank);
             bool ok = true;
-            for (int i = 0; i < p.T && ok; ++i) {
-                const int s = i % kXSlots, u = i / kXSlots;
-                if (u > 0) ok = mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
-                if (!ok) break;
-                mbar_arrive_expect_tx(&bar_x[s], NB * 256);
-                tma_load_4d(smem + L.x + s * (NB * 256), &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
+            auto load_x = [&](int i) {
+                const int s = i & (kXSlots - 1), u = i / kXSlots;
+                if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
+                if (!ok) return;
+                if constexpr (kTwoSteps) {
+                    const bool twice = s == 0;   // the fifth slot repeats the first
+                    mbar_arrive_expect_tx(&bar_x[s], NB * 256 * (twice ? 2 : 1));
+                    for (int kb = 0; kb < 2; ++kb)
+                        for (int n = 0; n < (twice ? 2 : 1); ++n)
+                            tma_load_4d(smem + L.x + (kb * 5 + s + 4 * n) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
+                } else {
+                    mbar_arrive_expect_tx(&bar_x[s], NB * 256);
+                    tma_load_4d(smem + L.x + s * (NB * 256), &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
+                }
+            };
+            if constexpr (kGather) {
+                for (int i = 0; i < p.T && ok; ++i) load_x(i);
+            } else {
+                // between the loads the stores of the hidden rows
+                for (int i = 0; i < min(p.T, kXSlots); ++i) load_x(i);
+                for (int i = 0; i < p.T && ok; ++i) {
+                    for (int e = 0; e < (both ? 2 : 1) && ok; ++e) {
+                        ok = mbar_wait(&bar_code[e], i & 1, abort_flag, 107);
+                        if (ok) tma_store_3d(e > 0 ? &tm_ol : &tm_o, smem + L.h + e * kTile, n0, m0 + F.rows * e, time_of(i));
+                    }
+                    tma_store_commit();
+                    if (i + kXSlots < p.T) load_x(i + kXSlots);
+                    tma_store_wait_read<0>();
+                    mbar_arrive(bar_stored);
+                }
+                tma_store_wait_all<0>();
             }
         }
         __syncwarp();
@@ -265,310 +346,370 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         // ------------------------------ MMA issuer --------------------------------------
         // The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
         // K loops unrolled, so an MMA is issued every few cycles.
-        constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, NB);
+        constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, kTwoSteps ? 16 : NB);
+        constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
+        constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
         uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
         uint64_t d_x0 = make_smem_desc_sw128(smem_u32(smem + L.x));
-        uint64_t d_hh0 = make_smem_desc_sw128(smem_u32(smem + L.hh));
+        uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
         uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
         uint64_t d_h0 = make_smem_desc_sw128(smem_u32(smem + L.h));
         bool ok = mbar_wait(bar_once, 0, abort_flag, 97);
         int i = 0;
-        // The x half of gates [g0, g1). Its 32 MMAs read their A operand from shared memory (40 cycles
-        // each, a third of a one-group step in all) and the tensor pipe works in order, so they are
-        // issued in pieces for the times when it would wait.
-        auto x_half = [&](auto from, auto to) {
-            constexpr int g0 = decltype(from)::value, g1 = decltype(to)::value;
-            const uint64_t d_x = d_x0 + uint64_t((i % kXSlots) * (NB * 16));
+        // MMAs [from, to) of the x part of a step. They read their A operand from shared memory (42 cycles
+        // each, 48 with 48 columns) and the tensor pipe works in order, so they are issued in pieces for the times when it
+        // would wait. With up to 8 rows, where the 32 MMAs of a step would take longer than all of its waits, an MMA covers
+        // the rows of two steps: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
+        // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones.
+        constexpr int kX = kTwoSteps ? 16 : 32;
+        auto x_half = [&](auto from, auto to, int i) {
+            constexpr int m0 = decltype(from)::value, m1 = decltype(to)::value;
+            const uint64_t d_x = d_x0 + uint64_t((i & (kXSlots - 1)) * (kTwoSteps ? NB * 8 : NB * 16));
+            const int g0 = kTwoSteps ? 2 * (i & 1) : 0;
             if (elect_one()) {
 #pragma unroll
-                for (int g = g0; g < g1; ++g)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        tc_mma<kKindF16>(tmem + g * NB, d_wx + uint64_t((g * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                         d_x + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
-                if (g1 == 4) tc_commit(&bar_x_free[i % kXSlots]);
+                for (int m = m0; m < m1; ++m) {
+                    const int g = m >> 3, k = m & 7;
+                    tc_mma<kKindF16>(tmem + (g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
+                                     d_x + uint64_t((k >> 2) * ((kTwoSteps ? 5 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+                }
+                if (m1 == kX && i >= 0) tc_commit(&bar_x_free[i & (kXSlots - 1)]);
             }
             __syncwarp();
         };
-        auto wait_x = [&]() {
-            ok = ok && mbar_wait(&bar_x[i % kXSlots], (i / kXSlots) & 1, abort_flag, 99);
+        auto wait_x = [&](int step) {
+            if (step < p.T) ok = ok && mbar_wait(&bar_x[step & (kXSlots - 1)], (step / kXSlots) & 1, abort_flag, 99);
+            return ok;
+        };
+        auto wait_acc = [&]() {
             if (i > 0) ok = ok && mbar_wait(bar_acc_free, (i - 1) & 1, abort_flag, 98);
             tc_fence_after_sync();
             return ok;
         };
-        auto wait_h = [&](int e) {
-            if (projects) ok = ok && mbar_wait<true>(&bar_h[e], i & 1, abort_flag, 100);
+        // projection u overwrites what projection u - 1 left
+        auto wait_sent = [&](int u) {
+            if (kOneProj && u > 0) ok = ok && mbar_wait(bar_sent, (u - 1) & 1, abort_flag, 106);
             return ok;
         };
-        auto project = [&](auto group) {
+        // projection of h_{i-1}. SPLIT: this CTA's K block for the rows of a group
+        auto project = [&](auto group, int i) {
             constexpr int e = decltype(group)::value;
-            if (!projects) return true;
+            if (e > 0 && !both) return true;
+            if (i > 0) ok = ok && mbar_wait(&bar_code[e], (i - 1) & 1, abort_flag, 100);
+            if (!ok) return false;
+            tc_fence_after_sync();
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + e, clock64());
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t rows = d_h0 + uint64_t(e * (kTile >> 4) + 2 * k);
+                    constexpr int kTo = 4 * S + (kOneProj ? 0 : e * F.n);
+                    if (k < kDnTs) tc_mma_ts<kKindI8>(tmem + kTo, tmem + kDnCol + 8 * k, rows, kIdescP, k != 0);
+                    else tc_mma<kKindI8>(tmem + kTo, d_dn + uint64_t(2 * k), rows, kIdescP, k != 0);
+                }
+                tc_commit(&bar_proj[e]);
+            }
+            __syncwarp();
+            return true;
+        };
+        // GATHER: all K blocks
+        auto project_all = [&]() {
+            if (i > 0) ok = ok && mbar_wait<true>(&bar_h[(i + 1) & 1], ((i - 1) >> 1) & 1, abort_flag, 100);
+            if (!ok) return false;
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 11, clock64());
             fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
             tc_fence_after_sync();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + (e ? 2 : 3), clock64());
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 0, clock64());
             if (elect_one()) {
-                constexpr int kPad = e ? kPad1 : kPad0;
-                constexpr uint32_t kIdesc = make_idesc<kKindI8>(64, kPad);
-                const uint32_t t_proj = tmem + 4 * NB + (e ? kPad0 : 0);
-                const uint64_t d_h = d_h0 + uint64_t(e * (h_group1 >> 4));
-                // an MMA is 8 to 12 cycles with its weights in tensor memory, 27 from shared memory
+                const uint64_t d_h = d_h0 + uint64_t(((i + 1) & 1) * (C * kTile >> 4));
 #pragma unroll
                 for (int kb = 0; kb < C; ++kb)
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const uint64_t rows = d_h + uint64_t(kb * kPad * 8 + 2 * k);
-                        if (kb < kDnTs)
-                            tc_mma_ts<kKindI8>(t_proj, tmem + kGTmemW - 32 * (kb + 1) + 8 * k, rows, kIdesc, (kb | k) != 0);
-                        else
-                            tc_mma<kKindI8>(t_proj, d_dn + uint64_t((kb - kDnTs) * 512 + 2 * k), rows, kIdesc, (kb | k) != 0);
+                        const uint64_t rows = d_h + uint64_t(kb * (kTile >> 4) + 2 * k);
+                        if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + 4 * S, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdescP, (kb | k) != 0);
+                        else tc_mma<kKindI8>(tmem + 4 * S, d_dn + uint64_t((kb - kDnTs / 4) * 1024 + 2 * k), rows, kIdescP, (kb | k) != 0);
                     }
-                tc_commit(&bar_proj[e]);
-                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_h[e], uint32_t(own_of(e)) * H);  // arm the next step
+                tc_commit(&bar_proj[0]);
+                if (i > 0 && i + 2 < p.T) mbar_arrive_expect_tx(&bar_h[(i + 1) & 1], uint32_t(n_rows) * H);  // for h_{i+1}
             }
             __syncwarp();
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 1, clock64());
             return true;
         };
         auto hh_half = [&](auto group) {
             constexpr int e = decltype(group)::value;
-            constexpr uint32_t kIdesc = make_idesc<kKindF16>(128, e ? N1 : N0);
+            if (e > 0 && !both) return true;
             ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
             if (!ok) return false;
-            fence_proxy_async_smem();
+            if (!kGather) fence_proxy_async_smem();
             tc_fence_after_sync();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 8 + (e ? 7 : 6), clock64());
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 3 + e, clock64());
             if (elect_one()) {
-                const uint64_t d_hh = d_hh0 + uint64_t(e * (N0 * 8));
+                // two steps per MMA: the other step's columns get rows that are zero
+                const uint64_t rows[2] = {d_hh + uint64_t(kTwoSteps && !(i & 1) ? 64 : 0), d_hh + uint64_t(kTwoSteps && (i & 1) ? 64 : 0)};
 #pragma unroll
                 for (int g = 0; g < 4; ++g)
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        tc_mma_ts<kKindF16>(tmem + g * NB + e * N0, tmem + kGTmemW + g * 64 + k * 8,
-                                            d_hh + uint64_t((k >> 2) * (NB * 8) + 2 * (k & 3)), kIdesc, 1u);
+                        tc_mma_ts<kKindF16>(tmem + g * S + F.rows * e, tmem + kGTmemW + g * 64 + k * 8,
+                                            rows[g >> 1] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
                 tc_commit(&bar_acc[e]);
-                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+                if (!kGather && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
             }
             __syncwarp();
             return true;
         };
+        if constexpr (kTwoSteps) {
+            // gates 2 and 3 of step 0: as the second step of the one before it
+            if (ok) ok = mbar_wait(&bar_x[0], 0, abort_flag, 99);
+            if (ok) x_half(Int<0>{}, Int<16>{}, -1);
+        }
         for (; i < p.T && ok; ++i) {
             // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
             // more registers than there are.
-            asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh0), "+l"(d_dn), "+l"(d_h0));
-            if constexpr (G == 1) {
-                // half of the x part while the hidden state is computed and travels, half while the
-                // projection is converted and travels
-                if (!wait_x()) break;
-                x_half(Int<0>{}, Int<2>{});
-                if (!wait_h(0) || !project(Int<0>{})) break;
-                x_half(Int<2>{}, Int<4>{});
+            asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
+            constexpr int kFirstX = kTwoSteps ? 10 : kGather ? 24 : 4;
+            if constexpr (kGather) {
+                // Most of the x part while the hidden state is computed and travels, the rest while the
+                // projection is converted. 300 chunks, 20 / 24 / 28 of 32 in front: 1.63 / 1.60 / 1.63 us per step; 32 chunks, 8 / 10 /
+                // 12 of 16: 1.18 / 1.18 / 1.22.
+                if (!wait_x(kTwoSteps ? i + 1 : i) || !wait_acc()) break;
+                FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
+                x_half(Int<0>{}, Int<kFirstX>{}, i);
+                FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 10, clock64());
+                if (!project_all()) break;
+                x_half(Int<kFirstX>{}, Int<kX>{}, i);
                 if (!hh_half(Int<0>{})) break;
             } else {
-                // Pieces of the x part while the hidden rows of the groups travel, one gate while the second
-                // projection is converted. 1024 chunks, gates in front of the first projection, between and
-                // behind: 1-2-1 2.87 us per step, 1-1-2 3.02, 0-3-1 2.94, 1-3-0 3.02, 0-4-0 3.00.
-                if (!wait_x()) break;
-                x_half(Int<0>{}, Int<1>{});
-                if (!wait_h(0)) break;
-                project(Int<0>{});
-                x_half(Int<1>{}, Int<3>{});
-                if (!wait_h(1)) break;
-                project(Int<1>{});
-                x_half(Int<3>{}, Int<4>{});
+                // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
+                // what has long been there takes 100 cycles and more while the gate warps keep the units of the SM busy that
+                // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step).
+                // MMAs in front of the second projection, 1024 chunks: 2 2.88, 4 2.89, 8 2.99; 700 chunks 2.15, 2.13, 2.17.
+                // Four in front of the first as well 2.93 and 2.20.
+                if (!wait_x(i) || !wait_sent(both ? 2 * i : i)) break;
+                if (!project(Int<0>{}, i)) break;
+                if (!wait_acc()) break;
+                x_half(Int<0>{}, Int<kFirstX>{}, i);
+                if (both && !wait_sent(2 * i + 1)) break;
+                if (!project(Int<1>{}, i)) break;
+                x_half(Int<kFirstX>{}, Int<24>{}, i);
+                // the gate warps overwrite the hidden codes once the hh half is complete
+                if (i > 0) ok = ok && mbar_wait(bar_stored, (i - 1) & 1, abort_flag, 104);
+                x_half(Int<24>{}, Int<32>{}, i);
                 if (!hh_half(Int<0>{})) break;
                 if (!hh_half(Int<1>{})) break;
             }
         }
     } else {
-        // ------------------------------ epilogues ---------------------------------------
-        const int q = warp & 3, ug = (warp - 2) >> 2;
-        // gates: this warp's rows of a group (an even share, so that rows pair up)
-        auto share_of = [&](int e) {
-            const int most = G == 1 ? p.rows : e == 0 ? min(p.rows, N0) : p.rows - N0;
-            return max((most + 3) / 4 + 1, 0) & ~1;
-        };
-        auto r0_of = [&](int e) { return e * N0 + ug * share_of(e); };   // in the cluster's rows
-        auto my_rows_of = [&](int e) { return min(max(rows_of(e) - ug * share_of(e), 0), share_of(e)); };
-        // projection: its columns (= rows) of the pair's accumulator
-        auto pr0_of = [&](int e) { return ug * ((p.n_own[e] + 3) / 4); };
-        auto my_pr_of = [&](int e) { return projects ? min(max(own_of(e) - pr0_of(e), 0), (p.n_own[e] + 3) / 4) : 0; };
-
+        // ------------------------------ gates -------------------------------------------
+        // thread = hidden unit. GATHER: a quarter of the rows; SPLIT: half of the rows of one group, eight warps each, so
+        // that one group's waits are the other's time (a share is even, so that rows pair up)
+        const int q = warp & 3;
+        const int e = kGather ? 0 : (warp - 2) >> 3, part = ((warp - 2) >> 2) & (kGather ? 3 : 1);
+        constexpr int kParts = kGather ? 4 : 2;
+        const int share = ((min(p.rows - F.rows * e, F.rows) + kParts - 1) / kParts + 1) & ~1;
+        const int r0 = part * share, my_rows = min(max(rows_of(e) - r0, 0), share);
         const int unit = n0 + q * 32 + lane;
         const float b_i = __ldg(p.bias + unit), b_f = __ldg(p.bias + H + unit);
         const float b_g = __ldg(p.bias + 2 * H + unit), b_o = __ldg(p.bias + 3 * H + unit);
-        // one projection column per lane (16 lanes of a quadrant hold rows of an M = 64 accumulator)
-        const int r_col = half * 64 + q * 16 + (lane & 15);
-        const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + r_col);  // operand order of the dequant GEMM: sa * sb
-        float2 c2[G][kCols / 2];
+        float *c_at = p.c + int64_t(m0 + F.rows * e + r0) * H + unit;
+        float2 c2[kPairs];
 #pragma unroll
-        for (int e = 0; e < G; ++e)
-#pragma unroll
-            for (int j = 0; j < kCols / 2; ++j) {
-                const float *cp = p.c + int64_t(m0 + r0_of(e) + 2 * j) * H + unit;
-                const int n = my_rows_of(e);
-                c2[e][j] = make_float2(2 * j < n ? cp[0] : 0.f, 2 * j + 1 < n ? cp[H] : 0.f);
-            }
-
-        // What a CTA sends leaves in rows of 128 bytes, eight lanes each: the network between the SMs moves 64
-        // contiguous bytes to one CTA in the time of 16 (20.7 against 9.5 B per cycle and SM, measured with
-        // six CTAs sending to each other). A warp holds 32 bytes of a row, so the four warps of a quarter stage
-        // together, in two slots in turn: the barrier after one batch is staged also says that the slot of
-        // the batch before has been read.
-        const uint32_t stage = smem_u32(smem + L.stage) + ug * (kStageRows * 128);
-        uint32_t slot = 0;
-        auto next_slot = [&]() { slot ^= 4 * kStageRows * 128; };
-        // The stores of every step go to the same places: addresses are worked out once. A destination is
-        // 16-byte aligned; its low bits hold the peer's rank (the peer's mbarrier address follows from
-        // it), 8 marks one that exists. Lane 8 j + c stores piece c of the swizzled row.
-        uint32_t hs_dst[G][kBatches];   // lanes 0-15: row q of a batch of four, to both CTAs of the pair
-#pragma unroll
-        for (int e = 0; e < G; ++e)
-#pragma unroll
-            for (int b = 0; b < (e ? N1 : N0) / 16; ++b) {
-                const int row = 4 * b + q, at = ug * share_of(e) + row;
-                const int pr = at / p.n_own[e], lr = at - pr * p.n_own[e];
-                const uint32_t to = uint32_t(2 * pr + (lane >> 3));
-                hs_dst[e][b] = lane < 16 && row < my_rows_of(e)
-                    ? map_to_rank(smem_u32(smem + L.h + e * h_group1 + rank * ((e ? kPad1 : kPad0) * 128)) + lr * 128 + (lane & 7) * 16, to) | 8u | to
-                    : 0u;
-            }
-        // ceil(ceil(N / pairs) / 4) rows to C CTAs each: at most 12 (row, CTA) per 16 rows (C = 3), 16 per store
-        uint32_t ps_src[kSendP], ps_dst[G][kSendP];
-#pragma unroll
-        for (int s = 0; s < kSendP; ++s) {
-            const int id = 16 * s + 4 * q + (lane >> 3), row = id / C;
-            int to = id - row * C + rank;   // start with a different peer in every CTA
-            if (to >= C) to -= C;
-            ps_src[s] = row * 128;
-#pragma unroll
-            for (int e = 0; e < G; ++e)
-                ps_dst[e][s] = row < my_pr_of(e)
-                    ? map_to_rank(smem_u32(smem + L.hh + half * (NB * 128)) +
-                                      (e * N0 + pair * p.n_own[e] + pr0_of(e) + row) * 128 + (lane & 7) * 16, uint32_t(to)) | 8u | uint32_t(to)
-                    : 0u;
-        }
-        // the piece of a staged row that belongs at a destination of the 128-byte swizzle
-        auto piece = [&](uint32_t dst) { return (uint32_t(lane) ^ (dst >> 7)) & 7u; };
-        auto send = [&](uint32_t dst, uint4 v, uint64_t *bar) {
-            store_to_peer(dst & ~15u, v, map_to_rank(smem_u32(bar), dst & 7u));
-        };
+        for (int j = 0; j < kPairs; ++j)
+            c2[j] = make_float2(2 * j < my_rows ? c_at[int64_t(2 * j) * H] : 0.f, 2 * j + 1 < my_rows ? c_at[int64_t(2 * j + 1) * H] : 0.f);
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
-        int i = 0;
-        // A warp whose wait ran out walks the remaining steps without waiting, sending or storing: the
-        // three it shares a slot with meet it at every barrier until their own waits give up.
         bool ok = true;
-        const int64_t plane = int64_t(p.reverse ? -p.B : p.B) * H;
-        int8_t *h_out = p.h_out + int64_t(time_of(0)) * p.B * H;
+        using Acc = uint32_t[4][4];   // [gate][row] of two pairs
+        auto codes = [&](const Acc &a, int k, float2 &c) {
+            return lstm_cell_codes(a[0][2 * k], a[0][2 * k + 1], a[1][2 * k], a[1][2 * k + 1], a[2][2 * k], a[2][2 * k + 1],
+                                   a[3][2 * k], a[3][2 * k + 1], make_float2(b_i, b_i), make_float2(b_f, b_f),
+                                   make_float2(b_g, b_g), make_float2(b_o, b_o), c);
+        };
 
-        // ---- projection of group e's h_{i-1}: int32 -> f16, to every CTA of the cluster ----
-        auto project_epilogue = [&](auto group) {
-            constexpr int e = decltype(group)::value;
-            const int my_pr = my_pr_of(e);
-            if (my_pr > 0) {
-                ok = ok && mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
-                next_slot();
-                FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 4, clock64());
-                tc_fence_after_sync();
-                const uint32_t t_proj = t_lane + 4 * NB + (e ? kPad0 : 0) + pr0_of(e);
-                for (int c = 0; c < my_pr; c += 4) {
-                    uint32_t a[4];
-                    tmem_ld_32x4(t_proj + c, a);
+        if constexpr (kGather) {
+            // Two rows at a time leave as rows of 128 bytes, eight lanes each: the network between the SMs moves 64
+            // contiguous bytes to one CTA in the time of 16 (20.7 against 9.5 B per cycle and SM, measured with
+            // six CTAs sending to each other). A warp holds 32 bytes of a row, so the four warps of a quarter stage
+            // together, in two slots in turn: the barrier after one batch is staged also says that the slot of
+            // the batch before has been read.
+            const uint32_t stage = smem_u32(smem + L.stage) + part * 256;
+            uint32_t slot = 0;
+            // lanes 0-15 send to the CTA q behind this one, 16-31 to that q + 4 behind; the last sixteen of the four warps store
+            const int s_row = (lane >> 3) & 1, s_to = q + 4 * (lane >> 4);
+            const uint32_t to = uint32_t((s_to + rank) % C);
+            const uint32_t dst = map_to_rank(smem_u32(smem + L.h) + rank * kTile + (lane & 7) * 16, to);
+            const uint32_t dst_bar = map_to_rank(smem_u32(bar_h), to);
+            const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + q * 32 + lane);   // operand order of the dequant GEMM: sa * sb
+            const uint32_t hh = smem_u32(smem + L.hh) + (q >> 1) * kHhTile + (kTwoSteps ? 1024 : 0) + (lane & 7) * 2;
+            int8_t *h_out = p.h_out + (int64_t(time_of(0)) * p.B + m0) * H + n0;
+            const int64_t plane = int64_t(p.reverse ? -p.B : p.B) * H;
+            // A warp whose wait ran out walks the remaining steps without waiting, sending or storing: the
+            // three it shares a slot with meet it at every barrier until their own waits give up.
+            for (int i = 0; i < p.T; ++i, h_out += plane) {
+                // ---- projection of h_{i-1}: int32 -> f16, into the operand of the hh half ----
+                ok = ok && mbar_wait(&bar_proj[0], i & 1, abort_flag, 102);
+                FLUKE_STAMP(blockIdx.x == 0 && warp == 2 && lane == 0, i * 16 + 6, clock64());
+                if (my_rows > 0) {
+                    tc_fence_after_sync();
+                    uint32_t v[4];
+                    tmem_ld_32x4(t_lane + 4 * S + r0, v);
                     tmem_ld_wait();
-                    if (lane < 16) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (c + j < my_pr)
-                                sts16(stage + slot + (c + j) * 128 + q * 32 + lane * 2, __half_as_ushort(__float2half_rn(float(int(a[j])) * sc)));
+                    for (int j = 0; j < 2 * kPairs; ++j)
+                        if (j < my_rows)
+                            sts16(hh + (r0 + j) * 128 + ((((q & 1) * 4 + (lane >> 3)) ^ ((r0 + j) & 7)) << 4),
+                                  __half_as_ushort(__float2half_rn(float(int(v[j])) * sc)));
+                    tc_fence_before_sync();
+                    fence_proxy_async_smem();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_hh);
+                FLUKE_STAMP(blockIdx.x == 0 && warp == 2 && lane == 0, i * 16 + 7, clock64());
+                // ---- gates, cell update, hidden codes ----
+                ok = ok && mbar_wait(&bar_acc[0], i & 1, abort_flag, 103);
+                FLUKE_STAMP(blockIdx.x == 0 && warp == 2 && lane == 0, i * 16 + 12, clock64());
+                Acc a;
+                if (my_rows > 0) {
+                    tc_fence_after_sync();
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const uint32_t col = t_lane + g * S + r0 + (kTwoSteps ? ((i ^ (g >> 1)) & 1) * 8 : 0);
+                        if (kPairs > 1) tmem_ld_32x4(col, a[g]);
+                        else tmem_ld_32x2(col, a[g][0], a[g][1]);
+                    }
+                    tmem_ld_wait();
+                    tc_fence_before_sync();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_acc_free);
+#pragma unroll
+                for (int j = 0; j < kPairs; ++j) {
+                    if (2 * j >= my_rows) break;
+                    slot ^= 1024;
+                    const int2 h = codes(a, j, c2[j]);
+                    sts8(stage + slot + q * 32 + lane, h.x);
+                    sts8(stage + slot + 128 + q * 32 + lane, h.y);
+                    quad_sync(1 + part);
+                    const int row = r0 + 2 * j + s_row;
+                    if (ok && 2 * j + s_row < my_rows) {
+                        const int piece = (lane ^ row) & 7;   // that belongs at place lane & 7 of the 128-byte swizzle
+                        const uint4 v = lds128(stage + slot + s_row * 128 + piece * 16);
+                        if (s_to < C && i + 1 < p.T) store_to_peer(dst + (i & 1) * (C * kTile) + row * 128, v, dst_bar + (i & 1) * 8);
+                        if (s_to == 7) {
+                            const int64_t off = int64_t(row) * H + piece * 16;
+                            *reinterpret_cast<uint4 *>(h_out + off) = v;
+                            if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + int64_t(m0) * H + n0 + off) = v;
+                        }
                     }
                 }
+                FLUKE_STAMP(blockIdx.x == 0 && warp == 2 && lane == 0, i * 16 + 8, clock64());
+            }
+        } else if (e == 0 || both) {
+            // The codes go straight into the operand of the projection (128-byte swizzle), from where the issuer also stores them.
+            const uint32_t code = smem_u32(smem + L.h) + e * kTile + (lane & 15);
+            const uint32_t t_acc = t_lane + F.rows * e + r0;
+            const uint32_t t_proj = t_lane + 4 * S + (kOneProj ? 0 : e * F.n) + part * 4;
+            const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + q * 32 + lane);   // operand order of the dequant GEMM: sa * sb
+            const uint32_t recv = smem_u32(smem + L.recv) + uint32_t(q * 32 + lane) * 16;
+            const uint32_t bar_sum_e = smem_u32(&bar_sum[e]), bar_hh_e = smem_u32(&bar_hh[e]);
+            const uint32_t stage = smem_u32(smem + L.stage) + (warp - 2) * 128;
+            const uint32_t hh = smem_u32(smem + L.hh) + (2 * e + (q >> 1)) * kHhTile;
+            const int s_row = 2 * part + ((lane >> 2) & 1), s_piece = (q & 1) * 4 + (lane & 3);
+            const int own = own_pieces(e);
+            for (int i = 0; i < p.T && ok; ++i) {
+                // ---- projection of this CTA's h_{i-1}: every other piece to its owner ----
+                ok = mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
+                if (!ok) break;
+                tc_fence_after_sync();
+                uint32_t v[kPieces / 2][4];
+#pragma unroll
+                for (int k = 0; k < kPieces / 2; ++k) tmem_ld_32x4(t_proj + 8 * k, v[k]);
+                tmem_ld_wait();
                 tc_fence_before_sync();
-                quad_sync(1 + ug);
+                if (kOneProj) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_sent);
+                }
+                FLUKE_STAMP(blockIdx.x == 0 && (warp == 2 || warp == 10) && lane == 0, i * 16 + 6 + e, clock64());
 #pragma unroll
-                for (int s = 0; s < (e ? N1 : N0) / 16; ++s)
-                    if (const uint32_t dst = ok ? ps_dst[e][s] : 0u) send(dst, lds128(stage + slot + ps_src[s] + piece(dst) * 16), &bar_hh[e]);
-                FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 5, clock64());
-            }
-        };
-
-        // ---- gates, cell update, hidden code of group e ----
-        auto gate_epilogue = [&](auto group) {
-            constexpr int e = decltype(group)::value;
-            constexpr int kB = (e ? N1 : N0) / 16;
-            const int my_rows = my_rows_of(e), r0 = r0_of(e);
-            ok = ok && mbar_wait(&bar_acc[e], i & 1, abort_flag, 103);
-            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 0, clock64());
-            tc_fence_after_sync();
-            // Four rows at a time, and each batch is sent as soon as it is staged (and stored, 128 bytes of a
-            // row by eight lanes), so that the exchange runs beside the arithmetic. Two batches are read at the
-            // start, which hands the accumulators back before the arithmetic.
-            static_assert(kB <= 2, "two batches are in registers");
-            uint32_t a[2][4][4];
-            auto load4 = [&](int b) {
+                for (int k = 0; k < kPieces / 2; ++k) {
+                    const uint32_t n = uint32_t(kPieces * e + 2 * k + part), to = n % C;
+                    if (4 * (2 * k + part) < rows_of(e))
+                        store_to_peer(map_to_rank(recv + ((n / C) * C + rank) * 2048, to), make_uint4(v[k][0], v[k][1], v[k][2], v[k][3]),
+                                      map_to_rank(bar_sum_e, to));
+                }
+                // ---- the CTA's own pieces: summed, converted, to every CTA (two of the four rows) ----
+                if (own > 0) {
+                    ok = mbar_wait<true>(&bar_sum[e], i & 1, abort_flag, 105);
+                    if (!ok) break;
+                    if (q == 0 && part == 0 && lane == 0 && i + 1 < p.T)   // for the next step
+                        mbar_arrive_expect_tx(&bar_sum[e], uint32_t(own) * C * 2048);
+                    FLUKE_STAMP(blockIdx.x == 0 && (warp == 2 || warp == 10) && lane == 0, i * 16 + 9 + e, clock64());
+#pragma unroll 1
+                    for (int n = rank; n < kPieces * G; n += C) {
+                        const int k = n - kPieces * e;
+                        if (k < 0 || k >= kPieces || 4 * k >= rows_of(e)) continue;
+                        int s0 = 0, s1 = 0;
 #pragma unroll
-                for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_lane + g * NB + r0 + 4 * b, a[b & 1][g]);
-            };
-            load4(0);
-            if (kB > 1) load4(1);
-            tmem_ld_wait();
-            tc_fence_before_sync();
-            __syncwarp();
-            if (e == G - 1 && lane == 0) mbar_arrive(bar_acc_free);
+                        for (int j = 0; j < C; ++j) {
+                            const int2 w = lds64(recv + ((n / C) * C + j) * 2048 + part * 8);
+                            s0 += w.x;
+                            s1 += w.y;
+                        }
+                        __syncwarp();   // the piece before has left the staging rows
+                        sts16(stage + lane * 2, __half_as_ushort(__float2half_rn(float(s0) * sc)));
+                        sts16(stage + 64 + lane * 2, __half_as_ushort(__float2half_rn(float(s1) * sc)));
+                        __syncwarp();
+                        const uint4 w = lds128(stage + (lane & 7) * 16);
+                        const int row = 4 * k + s_row;
+                        const uint32_t at = hh + row * 128 + ((s_piece ^ (row & 7)) << 4);
 #pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const auto &v = a[b & 1];
-                if (b > 0 && 4 * b >= my_rows) break;
-                next_slot();
-                if (4 * b < my_rows) {
-                    auto codes = [&](int j) {
-                        return lstm_cell_codes(v[0][2 * j], v[0][2 * j + 1], v[1][2 * j], v[1][2 * j + 1], v[2][2 * j], v[2][2 * j + 1],
-                                               v[3][2 * j], v[3][2 * j + 1], make_float2(b_i, b_i), make_float2(b_f, b_f),
-                                               make_float2(b_g, b_g), make_float2(b_o, b_o), c2[e][2 * b + j]);
-                    };
-                    auto stage_codes = [&](int j, int2 h) {
-                        sts8(stage + slot + 2 * j * 128 + q * 32 + lane, h.x);
-                        sts8(stage + slot + (2 * j + 1) * 128 + q * 32 + lane, h.y);
-                    };
-                    // Both pairs side by side: two chains. The second is left out where its rows do not exist.
-                    // With the branch against without, us per step, x_down included: C = 6 7 rows per cluster 1.53 :
-                    // 1.62, 14 rows 1.67 : 1.70, 20 rows 2.25 : 2.37; C = 7 and 8 alike (7 rows 1.57 : 1.67, 1.63 :
-                    // 1.70), 10 rows 1 % slower. Two groups, 47 rows: 3.02 : 2.98, so not there. C = 2 and 3 go without:
-                    // between -5 % (7 rows 1.47 : 1.55) and +1 % (10 and 16 rows).
-                    if (G > 1 || C < 4 || 4 * b + 2 < my_rows) {
-                        const int2 h0 = codes(0), h1 = codes(1);
-                        stage_codes(0, h0);
-                        stage_codes(1, h1);
-                    } else {
-                        stage_codes(0, codes(0));
+                        for (int d = 0; d < C; d += 4) {
+                            const int m = d + (lane >> 3);
+                            int to = m + rank;            // start with a different peer in every CTA
+                            if (to >= C) to -= C;
+                            if (m < C && row < rows_of(e)) store_to_peer(map_to_rank(at, to), w, map_to_rank(bar_hh_e, to));
+                        }
                     }
                 }
-                quad_sync(1 + ug);
-                if (const uint32_t dst = ok ? hs_dst[e][b] : 0u) {
-                    const uint4 v = lds128(stage + slot + q * 128 + piece(dst) * 16);
-                    if (i + 1 < p.T) send(dst, v, &bar_h[e]);
-                    if (lane < 8) {
-                        const size_t off = size_t(m0 + r0 + 4 * b + q) * H + n0 + piece(dst) * 16;
-                        *reinterpret_cast<uint4 *>(h_out + off) = v;
-                        if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + off) = v;
-                    }
+                // ---- gates, cell update, hidden codes ----
+                ok = mbar_wait(&bar_acc[e], i & 1, abort_flag, 103);
+                FLUKE_STAMP(blockIdx.x == 0 && (warp == 2 || warp == 10) && lane == 0, i * 16 + 12 + e, clock64());
+                if (!ok) break;
+                tc_fence_after_sync();
+                Acc a[kPairs / 2];
+#pragma unroll
+                for (int b = 0; b < kPairs / 2; ++b)
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_acc + g * S + 4 * b, a[b][g]);
+                tmem_ld_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_acc_free);
+#pragma unroll
+                for (int j = 0; j < kPairs; ++j) {
+                    const int2 h = codes(a[j / 2], j & 1, c2[j]);
+                    const int row = r0 + 2 * j;
+                    if (2 * j >= my_rows) break;
+                    sts8(code + row * 128 + (((q * 2 + (lane >> 4)) ^ (row & 7)) << 4), h.x);
+                    sts8(code + (row + 1) * 128 + (((q * 2 + (lane >> 4)) ^ ((row + 1) & 7)) << 4), h.y);   // a row behind the last one is not read
                 }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_code[e]);
+                FLUKE_STAMP(blockIdx.x == 0 && (warp == 2 || warp == 10) && lane == 0, i * 16 + (e == 0 ? 15 : 11), clock64());
             }
-            FLUKE_STAMP(blockIdx.x == 0 && threadIdx.x == 64 && e == 0, i * 8 + 1, clock64());
-        };
-
-        for (; i < p.T; ++i, h_out += plane) {
-            project_epilogue(Int<0>{});
-            if constexpr (G > 1) project_epilogue(Int<1>{});
-            gate_epilogue(Int<0>{});
-            if constexpr (G > 1) gate_epilogue(Int<1>{});
+            // the last codes are the final hidden state
+            if (ok)
+                for (int row = r0; row < r0 + my_rows; ++row)
+                    p.h_state[int64_t(m0 + F.rows * e + row) * H + unit] = int8_t(lds8(code + row * 128 + (((q * 2 + (lane >> 4)) ^ (row & 7)) << 4)));
         }
 #pragma unroll
-        for (int e = 0; e < G; ++e)
-#pragma unroll
-            for (int j = 0; j < kCols / 2; ++j) {
-                float *cp = p.c + int64_t(m0 + r0_of(e) + 2 * j) * H + unit;
-                const int n = my_rows_of(e);
-                if (2 * j < n) cp[0] = c2[e][j].x;
-                if (2 * j + 1 < n) cp[H] = c2[e][j].y;
-            }
+        for (int j = 0; j < kPairs; ++j) {
+            if (2 * j < my_rows) c_at[int64_t(2 * j) * H] = c2[j].x;
+            if (2 * j + 1 < my_rows) c_at[int64_t(2 * j + 1) * H] = c2[j].y;
+        }
     }
 
     // Nobody leaves (and frees shared memory that a peer's store may still target) before every
@@ -588,51 +729,33 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 constexpr int kGMinRows = 2;  // fewer rows than this per cluster do not make a step shorter
 
 struct GroupPlan {
-    int kernel;       // index in kGroupKernels
+    int form;         // see group_form
     int rows;         // rows per cluster
     int tiles;        // clusters
 };
 
-using group_kernel_fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GroupDev);
-struct GroupKernel { int n0, n1; group_kernel_fn fn[kGMaxCtas + 1]; };
-// Rows per cluster from which two groups are the faster: see group_kernel_for.
-constexpr int group_two_from(int C) { return C == 3 ? 17 : 18 + 2 * C; }
-template <int N0, int N1, int C>
-constexpr group_kernel_fn group_kernel_fits() {
-    constexpr bool kUsed = N1 == 0 || N0 + N1 > 32 || group_two_from(C) <= N0 + N1;
-    if constexpr (kUsed && group_layout(N0, N1, C).dynamic <= kGMaxSmem) return lstm_group_kernel<N0, N1, C>;
-    else return nullptr;
-}
-template <int N0, int N1>
-constexpr GroupKernel group_kernels() {
-    return {N0, N1, {nullptr, nullptr, group_kernel_fits<N0, N1, 2>(), group_kernel_fits<N0, N1, 3>(), group_kernel_fits<N0, N1, 4>(),
-                     group_kernel_fits<N0, N1, 5>(), group_kernel_fits<N0, N1, 6>(), group_kernel_fits<N0, N1, 7>(),
-                     group_kernel_fits<N0, N1, 8>()}};
-}
-const GroupKernel kGroupKernels[] = {group_kernels<16, 0>(), group_kernels<32, 0>(), group_kernels<16, 16>(), group_kernels<16, 32>()};
+using group_kernel_fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GroupDev);
+struct GroupKernel { group_kernel_fn fn; int smem; };
+template <int V, int C>
+constexpr GroupKernel group_kernel() { return {lstm_group_kernel<V, C>, group_layout(V, C).dynamic}; }
+#define FLUKE_GROUP_KERNELS(V) \
+    {{}, {}, group_kernel<V, 2>(), group_kernel<V, 3>(), group_kernel<V, 4>(), group_kernel<V, 5>(), group_kernel<V, 6>(), \
+     group_kernel<V, 7>(), group_kernel<V, 8>()}
+const GroupKernel kGroupKernels[kGForms][kGMaxCtas + 1] = {FLUKE_GROUP_KERNELS(0), FLUKE_GROUP_KERNELS(1), FLUKE_GROUP_KERNELS(2),
+                                                            FLUKE_GROUP_KERNELS(3)};
+#undef FLUKE_GROUP_KERNELS
 
-// The kernel for `rows` rows per cluster of hidden size H, or -1. One group has the shorter chain, two hide
-// half of it: the longer the exchanges (more CTAs), the more rows it takes for two to be the faster. Step of one
-// group against two, in us: H = 256, 20 rows 2.09 : 2.16, 28 rows 2.30 : 2.22; H = 384 (one pair of CTAs
-// projects all rows), 17 rows 2.19 : 2.19, 20 rows 2.40 : 2.21; H = 512, 26 rows 2.36 : 2.35, 32 rows 2.52 : 2.36;
-// H = 768, 28 rows 2.52 : 2.56, 32 rows 2.65 : 2.56; H = 1024, 32 rows 2.75 : 2.80.
-inline int group_kernel_for(int rows, int H) {
-    const int C = H / kGUnits;
-    const int k = rows <= 16 ? 0 : rows <= 32 ? (rows < group_two_from(C) ? 1 : 2) : 3;
-    return rows <= 48 && kGroupKernels[k].fn[C] ? k : -1;
-}
-
-// Clusters of C CTAs of kernel k that the device runs at once with the largest shared memory a CTA can
+// Clusters of C CTAs of form V that the device runs at once with the largest shared memory a CTA can
 // have (0: the form is not available).
-int group_capacity(int k, int C) {
-    static int known[64][sizeof(kGroupKernels) / sizeof(kGroupKernels[0])][kGMaxCtas + 1];  // n + 1, or -1
+int group_capacity(int V, int C) {
+    static int known[64][kGForms][kGMaxCtas + 1];  // n + 1, or -1
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return 0;
-    int &slot = known[dev][k][C];
+    int &slot = known[dev][V][C];
     if (slot == 0) {
         int n = 0;
-        const void *fn = reinterpret_cast<const void *>(kGroupKernels[k].fn[C]);
+        const void *fn = reinterpret_cast<const void *>(kGroupKernels[V][C].fn);
         bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGMaxSmem) == cudaSuccess;
         if (ok) {
             cudaLaunchConfig_t cfg = {};
@@ -654,24 +777,23 @@ int group_capacity(int k, int C) {
     return slot > 0 ? slot - 1 : 0;
 }
 
-// How B rows of hidden size H are spread: as few waves of clusters as the largest row count that
-// fits shared memory allows, then evenly over all clusters of those waves.
+// How B rows of hidden size H are spread: as few waves of clusters as the largest row count allows, then
+// evenly over all clusters of those waves.
 bool group_plan(int B, int H, GroupPlan *g) {
     if (H % kGUnits) return false;
     const int C = H / kGUnits;
     if (C < 2 || C > kGMaxCtas) return false;
-    int max_rows = 48;
-    while (max_rows > 0 && (g->kernel = group_kernel_for(max_rows, H)) < 0) max_rows -= 16;
-    if (max_rows < 16) return false;
-    const int cap = group_capacity(g->kernel, C);
+    const int cap = group_capacity(kGForms - 1, C);
     if (cap < 1) return false;
-    const int waves = (B + cap * max_rows - 1) / (cap * max_rows);
+    const int per_wave = cap * group_form(kGForms - 1).most;
+    const int waves = (B + per_wave - 1) / per_wave;
     int tiles = cap * waves;
     if (tiles > (B + kGMinRows - 1) / kGMinRows) tiles = (B + kGMinRows - 1) / kGMinRows;
     g->rows = (B + tiles - 1) / tiles;
     g->tiles = (B + g->rows - 1) / g->rows;
-    g->kernel = group_kernel_for(g->rows, H);
-    return g->kernel >= 0 && group_capacity(g->kernel, C) > 0;
+    g->form = 0;
+    while (g->rows > group_form(g->form).most) ++g->form;
+    return group_capacity(g->form, C) > 0;
 }
 
 }  // namespace
@@ -685,14 +807,13 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     const int T = l->T, B = l->B, H = l->H, R = l->R;
     GroupPlan g;
     if (R != kGRank || !group_plan(B, H, &g)) return -2;
-    const GroupKernel &kn = kGroupKernels[g.kernel];
     const int C = H / kGUnits;
+    const GroupForm f = group_form(g.form);
+    const GroupKernel &kn = kGroupKernels[g.form][C];
 
     GroupDev p;
     p.T = T; p.B = B; p.reverse = l->reverse;
     p.rows = g.rows;
-    const int in_group[2] = {kn.n1 ? min(g.rows, kn.n0) : g.rows, kn.n1 ? max(g.rows - kn.n0, 0) : 0};
-    for (int e = 0; e < 2; ++e) p.n_own[e] = max((in_group[e] + C / 2 - 1) / (C / 2), 1);
     p.dn = static_cast<const int8_t *>(l->dn_hh_i8);
     p.w_up = static_cast<const __half *>(l->w_up_f16);
     p.bias = static_cast<const float *>(l->bias_f32);
@@ -702,7 +823,7 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     p.h_state = static_cast<int8_t *>(l->h_i8);
     p.trace = trace_buffer();
 
-    CUtensorMap tm_w, tm_x, tm_dn, tm_h[2];
+    CUtensorMap tm_w, tm_x, tm_dn, tm_h0, tm_o[2];
     int rc = make_tmap_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, l->w_up_f16, 4 * uint64_t(H), 2 * R, uint64_t(2 * R) * 2,
                           kGUnits, 64, true);
     if (rc) return rc;
@@ -710,24 +831,30 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
         // both K blocks of a row range in one box: the 128-byte blocks of a row are a dimension
         const uint64_t dims[4] = {64, uint64_t(B), 2, uint64_t(T)};
         const uint64_t strides[3] = {uint64_t(R) * 2, 128, uint64_t(B) * R * 2};
-        const uint32_t box[4] = {64, uint32_t(kn.n0 + kn.n1), 2, 1};
+        const uint32_t box[4] = {64, uint32_t(f.groups * f.rows), f.rows == 8 ? 1u : 2u, 1};
         rc = make_tmap_nd(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_down, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
-    rc = make_tmap_2d(&tm_dn, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, l->dn_hh_i8, R, H, H, 64, 128, true);
+    rc = make_tmap_2d(&tm_dn, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, l->dn_hh_i8, R, H, H, kGRank, 128, true);
     if (rc) return rc;
-    for (int e = 0; e < 2; ++e) {
+    {
         const uint64_t dims[3] = {128, uint64_t(B), uint64_t(C)};
         const uint64_t strides[2] = {uint64_t(H), 128};
-        const uint32_t box[3] = {128, uint32_t(group_h_rows(e && kn.n1 ? kn.n1 : kn.n0, C)), uint32_t(C)};
-        rc = make_tmap_nd(&tm_h[e], CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_i8, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+        const uint32_t box[3] = {128, uint32_t(f.rows), uint32_t(f.gather ? C : 1)};
+        rc = make_tmap_nd(&tm_h0, CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_i8, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc) return rc;
+    }
+    // boxes of exactly the rows a group has: the rows behind them are another cluster's
+    for (int e = 0; e < 2; ++e) {
+        const int box_rows = e == 0 ? min(g.rows, f.rows) : max(g.rows - f.rows, 1);
+        rc = make_tmap_3d(&tm_o[e], CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_out_i8, T, B, H, H, uint64_t(B) * H, box_rows, 128, true);
         if (rc) return rc;
     }
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.tiles * C);
     cfg.blockDim = dim3(kGThreads);
-    cfg.dynamicSmemBytes = group_layout(kn.n0, kn.n1, C).dynamic;
+    cfg.dynamicSmemBytes = kn.smem;
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -736,5 +863,5 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kn.fn[C], tm_w, tm_x, tm_dn, tm_h[0], tm_h[1], p);
+    return (int)cudaLaunchKernelEx(&cfg, kn.fn, tm_w, tm_x, tm_dn, tm_h0, tm_o[0], tm_o[1], p);
 }

@@ -415,6 +415,9 @@ __device__ __forceinline__ void tmem_ld_32x4(uint32_t taddr, uint32_t (&r)[4]) {
                  : "r"(taddr)
                  : "memory");
 }
+__device__ __forceinline__ void tmem_ld_32x2(uint32_t taddr, uint32_t &r0, uint32_t &r1) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(taddr) : "memory");
+}
 // Thread i of the warp writes columns [col, col+8) of row (lane base + i).
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, uint4 lo, uint4 hi) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"

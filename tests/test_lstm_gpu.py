@@ -470,3 +470,27 @@ def test_small_cluster_form_gives_the_bytes_of_the_l2_form(flib, H, B, T):
     flib.fluke_set_lstm_persistent(1)
     for got, want in zip(*res):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("H,B", [(256, 1), (256, 528), (256, 529), (384, 3), (384, 391), (384, 393), (512, 287), (512, 290), (640, 175), (640, 185),
+                                 (768, 2), (768, 44), (768, 175), (768, 176), (768, 177), (768, 1023), (896, 143), (896, 145), (1024, 5),
+                                 (1024, 144), (1024, 145), (1024, 577), (1024, 863)])
+@pytest.mark.parametrize("T", [1, 2, 5, 10])
+def test_small_cluster_form_of_few_rows_and_of_two_groups_gives_the_bytes_of_the_l2_form(flib, H, B, T):
+    """As above, at the row counts per cluster where the form that contracts the x rows of two steps at once ends (8 on a B200),
+    its ring of five slots (steps 4, 5 and 8, 9 reuse them), and one wave of 33 to 48 rows at H = 1024. Exact."""
+    layer, x, xs = _layer_case(T, B, H, 128, H + B, B % 2 == 1)
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, h = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale,
+                                         layer.w_up, layer.bias, c, h, reverse=layer.reverse)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, h))
+    flib.fluke_set_lstm_persistent(1)
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
