@@ -39,9 +39,10 @@
 //
 // What bounds a step (B200, H = 768, cycles). 2 rows per cluster, 2100: the chain of exchange (490 from the first
 // store to the last arrival), projection 500, its conversion 220, hh half 460, cell update and staging 450. 14 rows, 2900: the
-// same with 950 for the cell updates and 600 for the exchange. 47 rows, 4930: tensor pipe (x part 1540, hh half 1460,
-// projections 370), idle from the end of a step's contractions to the first group's codes (900: 24 rows x 128 units of
-// cell updates share the special-function units with the other group's).
+// same with 950 for the cell updates and 600 for the exchange. 47 rows, 4700: tensor pipe (x part 1540, hh half 1460,
+// projections 370), idle from the end of a step's contractions to the first group's codes (700: 24 rows x 128 units of
+// cell updates, beside the other group's) and while the partial sums travel. The cell updates live on few instructions:
+// with places in the swizzle worked out per row instead of by one exclusive or, 1024 chunks took 2.89 us, 700 2.13.
 //
 // The operand rows that are zero (see group_form) add zero times a weight to another group's or step's accumulators: with
 // finite weights nothing.
@@ -86,9 +87,9 @@ struct GroupDev {
 
 // The forms of the kernel: chunk rows per cluster up to 8, 16, 32 and 48. GATHER is one group of rows, SPLIT two. Step of the
 // kernel of one and two groups that exchanged hidden rows between pairs of CTAs and projected them there, against
-// these, in us, x_down included: H = 768 32 chunks (2 rows per cluster) 1.45 : 1.14, 170 (8 rows) 1.56 : 1.30, 300 (14 rows) 1.66 :
-// 1.61, 500 (23 rows) 2.40 : 2.05, 700 (32 rows) 2.62 : 2.13, 1024 (47 rows) 2.97 : 2.89; H = 384, 32 chunks (2 rows) 1.37 : 1.07;
-// H = 1024, where it took two waves from 577 chunks on, 700 (39 rows) 4.85 : 2.92.
+// these, in us, x_down included: H = 768 32 chunks (2 rows per cluster) 1.45 : 1.15, 170 (8 rows) 1.56 : 1.34, 300 (14 rows) 1.66 :
+// 1.61, 500 (23 rows) 2.40 : 1.96, 700 (32 rows) 2.62 : 2.04, 1024 (47 rows) 2.97 : 2.75; H = 384, 32 chunks (2 rows) 1.37 : 1.08;
+// H = 1024, where it took two waves from 577 chunks on, 700 (39 rows) 4.85 : 2.86.
 // Everything below depends on the form V and the cluster size C = H / 128, which the kernel is compiled
 // for: with operand addresses at fixed distances the issuer needs few instructions between MMAs.
 constexpr int kGForms = 4;
@@ -469,7 +470,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
             // more registers than there are.
             asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
-            constexpr int kFirstX = kTwoSteps ? 10 : kGather ? 24 : 4;
+            constexpr int kFirstX = kTwoSteps ? 10 : kGather ? 24 : 2;
             if constexpr (kGather) {
                 // Most of the x part while the hidden state is computed and travels, the rest while the
                 // projection is converted. 300 chunks, 20 / 24 / 28 of 32 in front: 1.63 / 1.60 / 1.63 us per step; 32 chunks, 8 / 10 /
@@ -485,8 +486,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
                 // what has long been there takes 100 cycles and more while the gate warps keep the units of the SM busy that
                 // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step).
-                // MMAs in front of the second projection, 1024 chunks: 2 2.88, 4 2.89, 8 2.99; 700 chunks 2.15, 2.13, 2.17.
-                // Four in front of the first as well 2.93 and 2.20.
+                // MMAs in front of the second projection, 1024 chunks: 2 2.71-2.76, 4 2.74-2.78, 8 2.79; 700 chunks 2.04, 2.04-2.08,
+                // 2.12. Four in front of the first as well 3.07-3.16 and 2.24-2.33.
                 if (!wait_x(i) || !wait_sent(both ? 2 * i : i)) break;
                 if (!project(Int<0>{}, i)) break;
                 if (!wait_acc()) break;
@@ -504,12 +505,12 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     } else {
         // ------------------------------ gates -------------------------------------------
         // thread = hidden unit. GATHER: a quarter of the rows; SPLIT: half of the rows of one group, eight warps each, so
-        // that one group's waits are the other's time (a share is even, so that rows pair up)
+        // that one group's waits are the other's time
         const int q = warp & 3;
         const int e = kGather ? 0 : (warp - 2) >> 3, part = ((warp - 2) >> 2) & (kGather ? 3 : 1);
         constexpr int kParts = kGather ? 4 : 2;
-        const int share = ((min(p.rows - F.rows * e, F.rows) + kParts - 1) / kParts + 1) & ~1;
-        const int r0 = part * share, my_rows = min(max(rows_of(e) - r0, 0), share);
+        constexpr int kShare = F.rows / kParts;
+        const int r0 = part * kShare, my_rows = min(max(rows_of(e) - r0, 0), kShare);
         const int unit = n0 + q * 32 + lane;
         const float b_i = __ldg(p.bias + unit), b_f = __ldg(p.bias + H + unit);
         const float b_g = __ldg(p.bias + 2 * H + unit), b_o = __ldg(p.bias + 3 * H + unit);
@@ -536,13 +537,18 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             const uint32_t stage = smem_u32(smem + L.stage) + part * 256;
             uint32_t slot = 0;
             // lanes 0-15 send to the CTA q behind this one, 16-31 to that q + 4 behind; the last sixteen of the four warps store
-            const int s_row = (lane >> 3) & 1, s_to = q + 4 * (lane >> 4);
+            const int s_row = (lane >> 3) & 1, s_to = q + 4 * (lane >> 4), s_piece = (lane ^ (r0 + s_row)) & 7;
             const uint32_t to = uint32_t((s_to + rank) % C);
-            const uint32_t dst = map_to_rank(smem_u32(smem + L.h) + rank * kTile + (lane & 7) * 16, to);
+            // Piece c of row r lies at place c ^ (r & 7) of the 128-byte swizzle. A share starts at a multiple of its size, a power of
+            // two, so the row j rows on has its place at exclusive or j.
+            const uint32_t dst = map_to_rank(smem_u32(smem + L.h) + rank * kTile + (r0 + s_row) * 128 + (lane & 7) * 16, to);
+            const uint32_t src = stage + s_row * 128 + s_piece * 16;
             const uint32_t dst_bar = map_to_rank(smem_u32(bar_h), to);
             const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + q * 32 + lane);   // operand order of the dequant GEMM: sa * sb
-            const uint32_t hh = smem_u32(smem + L.hh) + (q >> 1) * kHhTile + (kTwoSteps ? 1024 : 0) + (lane & 7) * 2;
-            int8_t *h_out = p.h_out + (int64_t(time_of(0)) * p.B + m0) * H + n0;
+            const uint32_t hh = smem_u32(smem + L.hh) + (q >> 1) * kHhTile + (kTwoSteps ? 1024 : 0) + r0 * 128 +
+                                (((q & 1) * 4 + (lane >> 3)) ^ (r0 & 7)) * 16 + (lane & 7) * 2;
+            const int64_t at = int64_t(m0 + r0 + s_row) * H + n0;   // plus the piece
+            int8_t *h_out = p.h_out + int64_t(time_of(0)) * p.B * H + at;
             const int64_t plane = int64_t(p.reverse ? -p.B : p.B) * H;
             // A warp whose wait ran out walks the remaining steps without waiting, sending or storing: the
             // three it shares a slot with meet it at every barrier until their own waits give up.
@@ -558,8 +564,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 #pragma unroll
                     for (int j = 0; j < 2 * kPairs; ++j)
                         if (j < my_rows)
-                            sts16(hh + (r0 + j) * 128 + ((((q & 1) * 4 + (lane >> 3)) ^ ((r0 + j) & 7)) << 4),
-                                  __half_as_ushort(__float2half_rn(float(int(v[j])) * sc)));
+                            sts16((hh ^ (j << 4)) + j * 128, __half_as_ushort(__float2half_rn(float(int(v[j])) * sc)));
                     tc_fence_before_sync();
                     fence_proxy_async_smem();
                 }
@@ -591,15 +596,13 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     sts8(stage + slot + q * 32 + lane, h.x);
                     sts8(stage + slot + 128 + q * 32 + lane, h.y);
                     quad_sync(1 + part);
-                    const int row = r0 + 2 * j + s_row;
                     if (ok && 2 * j + s_row < my_rows) {
-                        const int piece = (lane ^ row) & 7;   // that belongs at place lane & 7 of the 128-byte swizzle
-                        const uint4 v = lds128(stage + slot + s_row * 128 + piece * 16);
-                        if (s_to < C && i + 1 < p.T) store_to_peer(dst + (i & 1) * (C * kTile) + row * 128, v, dst_bar + (i & 1) * 8);
+                        const uint4 v = lds128((src ^ (j << 5)) + slot);
+                        if (s_to < C && i + 1 < p.T) store_to_peer(dst + (i & 1) * (C * kTile) + j * 256, v, dst_bar + (i & 1) * 8);
                         if (s_to == 7) {
-                            const int64_t off = int64_t(row) * H + piece * 16;
+                            const int off = 2 * j * H + ((s_piece ^ (2 * j)) << 4);
                             *reinterpret_cast<uint4 *>(h_out + off) = v;
-                            if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + int64_t(m0) * H + n0 + off) = v;
+                            if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + at + off) = v;
                         }
                     }
                 }
@@ -607,7 +610,9 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             }
         } else if (e == 0 || both) {
             // The codes go straight into the operand of the projection (128-byte swizzle), from where the issuer also stores them.
-            const uint32_t code = smem_u32(smem + L.h) + e * kTile + (lane & 15);
+            // Twelve rows on is four on in the swizzle: exclusive or 4, and exclusive or j mod 8 for the rows behind.
+            const uint32_t code = smem_u32(smem + L.h) + e * kTile + r0 * 128 + (((q * 2 + (lane >> 4)) ^ (r0 & 7)) << 4) + (lane & 15);
+            auto code_at = [&](int j) { return (code ^ ((j & 7) << 4)) + j * 128; };
             const uint32_t t_acc = t_lane + F.rows * e + r0;
             const uint32_t t_proj = t_lane + 4 * S + (kOneProj ? 0 : e * F.n) + part * 4;
             const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + q * 32 + lane);   // operand order of the dequant GEMM: sa * sb
@@ -689,11 +694,9 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (lane == 0) mbar_arrive(bar_acc_free);
 #pragma unroll
                 for (int j = 0; j < kPairs; ++j) {
-                    const int2 h = codes(a[j / 2], j & 1, c2[j]);
-                    const int row = r0 + 2 * j;
-                    if (2 * j >= my_rows) break;
-                    sts8(code + row * 128 + (((q * 2 + (lane >> 4)) ^ (row & 7)) << 4), h.x);
-                    sts8(code + (row + 1) * 128 + (((q * 2 + (lane >> 4)) ^ ((row + 1) & 7)) << 4), h.y);   // a row behind the last one is not read
+                    const int2 h = codes(a[j / 2], j & 1, c2[j]);   // of rows that the group does not have as well: nothing reads them
+                    sts8(code_at(2 * j), h.x);
+                    sts8(code_at(2 * j + 1), h.y);
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -702,8 +705,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             }
             // the last codes are the final hidden state
             if (ok)
-                for (int row = r0; row < r0 + my_rows; ++row)
-                    p.h_state[int64_t(m0 + F.rows * e + row) * H + unit] = int8_t(lds8(code + row * 128 + (((q * 2 + (lane >> 4)) ^ (row & 7)) << 4)));
+                for (int j = 0; j < my_rows; ++j) p.h_state[int64_t(m0 + F.rows * e + r0 + j) * H + unit] = int8_t(lds8(code_at(j)));
         }
 #pragma unroll
         for (int j = 0; j < kPairs; ++j) {
