@@ -389,9 +389,8 @@ extern "C" int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, 
             }
         };
         // The small clusters come first wherever they cover the shape. Step time at H = 768, against
-        // the fastest of the other forms: 16 chunks 1.5 us (5.76), 300 1.7 (5.83), 704 2.55 (5.82),
-        // 1024 2.9 (7.31), 2048 in two waves 5.7 (8.9); at H = 1024, where a wave holds 480
-        // chunks, 1024 chunks 7.2 (8.3).
+        // the fastest of the other forms: 32 chunks 1.1 us (5.76), 300 1.6 (5.83), 700 2.0 (5.82),
+        // 1024 2.7 (7.31), 2048 in two waves 5.3 (8.9).
         int order[4] = {0, 0, 0, 0};
         switch (g_lstm_persistent) {
             case 2: order[0] = 2; break;
