@@ -45,7 +45,8 @@
 // with places in the swizzle worked out per row instead of by one exclusive or, 1024 chunks took 2.89 us, 700 2.13.
 //
 // The operand rows that are zero (see group_form) add zero times a weight to another group's or step's accumulators: with
-// finite weights nothing.
+// finite weights nothing. A CTA whose recurrent gate weights are not all finite (0 x inf is NaN) issues other MMAs, see
+// issue_exact: an infinite weight reaches the rows of its unit through their own factors only.
 //
 // Arithmetic and its order are those of the other single-launch forms (x_down half first, then the
 // hh_down half in K steps of 16; int32 sums scaled by (1/127)*scale and rounded to f16): the bytes
@@ -70,6 +71,7 @@ constexpr int kGTmemCols = 512;
 constexpr int kGTmemW = 256;       // first column of the hh half of the gate weights: 4 gates x 64
 constexpr int kGWxBytes = 4 * kGUnits * 256;  // x half of the gate weights in shared memory
 constexpr int kGMaxSmem = 232448;
+constexpr int kGBars = 24;         // mbarriers of a CTA
 
 struct GroupDev {
     int T, B;
@@ -141,7 +143,7 @@ __host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
     // partial sums of the CTA's own pieces: per piece and source CTA [128 columns][4 rows] int32
     l.stage = l.recv + (f.gather ? 0 : group_own_pieces(V, C) * C * 2048);
     l.bars = l.stage + 2048;                      // GATHER: two slots x four quarters x [2 rows x 128 B]; else per warp [2 rows x 64 B]
-    l.misc = l.bars + 24 * 8;
+    l.misc = l.bars + kGBars * 8;
     l.dynamic = l.misc + 16 + 1024;               // slack for the manual 1024-byte alignment
     return l;
 }
@@ -177,11 +179,269 @@ __device__ __forceinline__ void sts16(uint32_t addr, unsigned short v) {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
 }
 
+// Adds zero times the halves of w to sum: NaN from the first that is infinite or NaN on, else zero.
+__device__ __forceinline__ void add_zero_times(__half2 &sum, uint4 w) {
+    const __half2 zero = __half2half2(__ushort_as_half(0));
+    const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum = __hfma2(*reinterpret_cast<const __half2 *>(&words[j]), zero, sum);
+}
+
 // Barrier of the four warps that share a staging slot.
 __device__ __forceinline__ void quad_sync(int id) { asm volatile("barrier.cta.sync %0, 128;" ::"r"(id) : "memory"); }
 
 template <int V>
 struct Int { static constexpr int value = V; };  // a number that a lambda receives as a type
+
+// What the kernel and its MMA issuer know at compile time.
+template <int V, int C>
+struct GroupConst {
+    static constexpr GroupForm F = group_form(V);
+    static constexpr GroupLayout L = group_layout(V, C);
+    static constexpr bool kGather = F.gather;
+    static constexpr int G = F.groups, NB = G * F.rows, S = F.stride, H = C * kGUnits;
+    static constexpr bool kTwoSteps = F.rows == 8;            // an x MMA covers two steps
+    static constexpr int kXSlots = kTwoSteps ? 4 : F.x_slots;
+    static constexpr int kTile = F.rows * 128;                // bytes of a group's hidden rows in one K block
+    static constexpr int kHhTile = (kTwoSteps ? 24 : F.n) * 128;   // and of its hh_down rows
+    static constexpr bool kZeroRows = kHhTile > kTile;        // some of which are zero
+    static constexpr int kPieces = F.rows / 4;                // pieces of a group
+    static constexpr int kPairs = kGather ? F.rows / 8 : F.rows / 4;   // pairs of rows of a gate thread
+    static constexpr int kDnTs = group_dn_ts(V, C);
+    static constexpr int kDnCol = kGTmemW - 8 * kDnTs;        // first column of the projection weights in tensor memory
+    static constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
+    static_assert(4 * S + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
+    static_assert(L.dynamic <= kGMaxSmem, "shared memory of a CTA");
+};
+// mbarriers of a CTA, as indices
+enum : int {
+    kBarOnce = 0,      // resident weights and the initial hidden rows loaded
+    kBarX = 1,         // [slots] x_down rows landed
+    kBarXFree = 5,     // [slots] the x part of the contraction has read them
+    kBarAccFree = 9,   // the gate warps have read all accumulators
+    kBarProj = 10,     // [G] projection accumulator complete
+    kBarAcc = 12,      // [G] gate accumulators complete
+    kBarHh = 14,       // [G] hh_down rows in place
+    kBarCode = 16,     // SPLIT [G]: hidden codes of this CTA's units in place
+    kBarSum = 18,      // SPLIT [G]: partial sums of the CTA's own pieces arrived
+    kBarSent = 20,     // SPLIT: the projection accumulator has been read
+    kBarStored = 21,   // SPLIT: the TMA stores have read the hidden codes
+    kBarH = 16         // GATHER [2]: hidden rows of all CTAs arrived
+};
+
+// The MMA issuer, warp 1. The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
+// K loops unrolled, so an MMA is issued every few cycles. kExact: for weights that are not finite.
+template <int V, int C, bool kExact>
+__device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupDev &p, int n_rows) {
+    using K = GroupConst<V, C>;
+    constexpr GroupForm F = K::F;
+    constexpr GroupLayout L = K::L;
+    constexpr bool kGather = K::kGather, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
+    constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
+    constexpr int kDnTs = K::kDnTs, kDnCol = K::kDnCol;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
+    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + kBarX, *bar_x_free = bars + kBarXFree, *bar_acc_free = bars + kBarAccFree;
+    uint64_t *bar_proj = bars + kBarProj, *bar_acc = bars + kBarAcc, *bar_hh = bars + kBarHh, *bar_code = bars + kBarCode;
+    uint64_t *bar_sent = bars + kBarSent, *bar_stored = bars + kBarStored, *bar_h = bars + kBarH;
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
+    [[maybe_unused]] const int lane = threadIdx.x & 31;
+    auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
+    const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
+    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, kTwoSteps ? 16 : NB);
+    constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
+    constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
+    uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
+    uint64_t d_x0 = make_smem_desc_sw128(smem_u32(smem + L.x));
+    uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
+    uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
+    uint64_t d_h0 = make_smem_desc_sw128(smem_u32(smem + L.h));
+    bool ok = mbar_wait(bar_once, 0, abort_flag, 97);
+    int i = 0;
+    // MMAs [from, to) of the x part of a step. They read their A operand from shared memory (42 cycles
+    // each, 48 with 48 columns) and the tensor pipe works in order, so they are issued in pieces for the times when it
+    // would wait. With up to 8 rows, where the 32 MMAs of a step would take longer than all of its waits, an MMA covers
+    // the rows of two steps: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
+    // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones.
+    constexpr int kX = kTwoSteps ? 16 : 32;
+    auto x_half = [&](auto from, auto to, int i, bool release = true) {
+        constexpr int first = decltype(from)::value, end = decltype(to)::value;
+        const uint64_t d_x = d_x0 + uint64_t((i & (kXSlots - 1)) * (kTwoSteps ? NB * 8 : NB * 16));
+        const int g0 = kTwoSteps ? 2 * (i & 1) : 0;
+        if (elect_one()) {
+#pragma unroll
+            for (int m = first; m < end; ++m) {
+                const int g = m >> 3, k = m & 7;
+                tc_mma<kKindF16>(tmem + (g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
+                                 d_x + uint64_t((k >> 2) * ((kTwoSteps ? 5 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+            }
+            if (end == kX && release) tc_commit(&bar_x_free[i & (kXSlots - 1)]);
+        }
+        __syncwarp();
+    };
+    auto wait_x = [&](int step) {
+        if (step < p.T) ok = ok && mbar_wait(&bar_x[step & (kXSlots - 1)], (step / kXSlots) & 1, abort_flag, 99);
+        return ok;
+    };
+    auto wait_acc = [&]() {
+        if (i > 0) ok = ok && mbar_wait(bar_acc_free, (i - 1) & 1, abort_flag, 98);
+        tc_fence_after_sync();
+        return ok;
+    };
+    // projection u overwrites what projection u - 1 left
+    auto wait_sent = [&](int u) {
+        if (kOneProj && u > 0) ok = ok && mbar_wait(bar_sent, (u - 1) & 1, abort_flag, 106);
+        return ok;
+    };
+    // projection of h_{i-1}. SPLIT: this CTA's K block for the rows of a group
+    auto project = [&](auto group, int i) {
+        constexpr int e = decltype(group)::value;
+        if (e > 0 && !both) return true;
+        if (i > 0) ok = ok && mbar_wait(&bar_code[e], (i - 1) & 1, abort_flag, 100);
+        if (!ok) return false;
+        tc_fence_after_sync();
+        FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + e, clock64());
+        if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint64_t rows = d_h0 + uint64_t(e * (kTile >> 4) + 2 * k);
+                constexpr int kTo = 4 * S + (kOneProj ? 0 : e * F.n);
+                if (k < kDnTs) tc_mma_ts<kKindI8>(tmem + kTo, tmem + kDnCol + 8 * k, rows, kIdescP, k != 0);
+                else tc_mma<kKindI8>(tmem + kTo, d_dn + uint64_t(2 * k), rows, kIdescP, k != 0);
+            }
+            tc_commit(&bar_proj[e]);
+        }
+        __syncwarp();
+        return true;
+    };
+    // GATHER: all K blocks
+    auto project_all = [&]() {
+        if (i > 0) ok = ok && mbar_wait<true>(&bar_h[(i + 1) & 1], ((i - 1) >> 1) & 1, abort_flag, 100);
+        if (!ok) return false;
+        FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 11, clock64());
+        fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
+        tc_fence_after_sync();
+        FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 0, clock64());
+        if (elect_one()) {
+            const uint64_t d_h = d_h0 + uint64_t(((i + 1) & 1) * (C * kTile >> 4));
+#pragma unroll
+            for (int kb = 0; kb < C; ++kb)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t rows = d_h + uint64_t(kb * (kTile >> 4) + 2 * k);
+                    if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + 4 * S, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdescP, (kb | k) != 0);
+                    else tc_mma<kKindI8>(tmem + 4 * S, d_dn + uint64_t((kb - kDnTs / 4) * 1024 + 2 * k), rows, kIdescP, (kb | k) != 0);
+                }
+            tc_commit(&bar_proj[0]);
+            if (i > 0 && i + 2 < p.T) mbar_arrive_expect_tx(&bar_h[(i + 1) & 1], uint32_t(n_rows) * H);  // for h_{i+1}
+        }
+        __syncwarp();
+        FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 1, clock64());
+        return true;
+    };
+    auto hh_half = [&](auto group) {
+        constexpr int e = decltype(group)::value;
+        if (e > 0 && !both) return true;
+        ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
+        if (!ok) return false;
+        if (!kGather) fence_proxy_async_smem();
+        tc_fence_after_sync();
+        FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 3 + e, clock64());
+        if (elect_one()) {
+            // two steps per MMA: the other step's columns get rows that are zero
+            const uint64_t rows[2] = {d_hh + uint64_t(kTwoSteps && !(i & 1) ? 64 : 0), d_hh + uint64_t(kTwoSteps && (i & 1) ? 64 : 0)};
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    tc_mma_ts<kKindF16>(tmem + g * S + F.rows * e, tmem + kGTmemW + g * 64 + k * 8,
+                                        rows[g >> 1] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
+            tc_commit(&bar_acc[e]);
+            if (!kGather && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+        }
+        __syncwarp();
+        return true;
+    };
+    // Two groups of 24 rows, kExact: 48 rows in three MMAs of sixteen, the middle one of the first group's last eight and the second's
+    // first eight (the distance of eight rows from the next is the descriptor's), when both groups are there.
+    auto hh_both = [&]() {
+        for (int e = 0; e < 2; ++e) ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
+        if (!ok) return false;
+        fence_proxy_async_smem();
+        tc_fence_after_sync();
+        if (elect_one()) {
+            constexpr uint32_t kIdesc = make_idesc<kKindF16>(128, 16);
+            constexpr uint64_t kGroup = 2 * kHhTile >> 4;   // from a group's rows to the other's
+            const uint64_t rows[3] = {d_hh, d_hh + 128 + ((kGroup - 128 - 64) << 32), d_hh + kGroup + 64};
+#pragma unroll 1
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma_ts<kKindF16>(tmem + g * S + 16 * b, tmem + kGTmemW + g * 64 + k * 8,
+                                            rows[b] + uint64_t((k >> 2) * (kHhTile >> 4) + 2 * (k & 3)), kIdesc, 1u);
+            for (int e = 0; e < 2; ++e) {
+                tc_commit(&bar_acc[e]);
+                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+            }
+        }
+        __syncwarp();
+        return true;
+    };
+    if constexpr (kTwoSteps) {
+        // gates 2 and 3 of step 0: as the second step of the one before it
+        if (ok) ok = mbar_wait(&bar_x[0], 0, abort_flag, 99);
+        if (ok) x_half(Int<0>{}, Int<16>{}, -1, false);
+    }
+    for (; i < p.T && ok; ++i) {
+        // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
+        // more registers than there are.
+        asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
+        constexpr int kFirstX = kTwoSteps ? 10 : kGather ? 24 : 2;
+        if constexpr (kGather) {
+            // Most of the x part while the hidden state is computed and travels, the rest while the
+            // projection is converted. 300 chunks, 20 / 24 / 28 of 32 in front: 1.63 / 1.60 / 1.63 us per step; 32 chunks, 8 / 10 /
+            // 12 of 16: 1.18 / 1.18 / 1.22.
+            if (!wait_x(kTwoSteps ? i + 1 : i) || !wait_acc()) break;
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
+            // Two steps per MMA: the zero rows of the step before have spoilt the accumulators of this step's gates that its x MMAs
+            // computed. Once more from the same slots; the step before may be gone from its, it enters columns that have been read.
+            if (kExact && kTwoSteps && i > 0) x_half(Int<0>{}, Int<kX>{}, i - 1, false);
+            x_half(Int<0>{}, Int<kFirstX>{}, i);
+            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 10, clock64());
+            if (!project_all()) break;
+            x_half(Int<kFirstX>{}, Int<kX>{}, i);
+            if (!hh_half(Int<0>{})) break;
+        } else {
+            // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
+            // what has long been there takes 100 cycles and more while the gate warps keep the units of the SM busy that
+            // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step).
+            // MMAs in front of the second projection, 1024 chunks: 2 2.71-2.76, 4 2.74-2.78, 8 2.79; 700 chunks 2.04, 2.04-2.08,
+            // 2.12. Four in front of the first as well 3.07-3.16 and 2.24-2.33.
+            if (!wait_x(i) || !wait_sent(both ? 2 * i : i)) break;
+            if (!project(Int<0>{}, i)) break;
+            if (!wait_acc()) break;
+            x_half(Int<0>{}, Int<kFirstX>{}, i);
+            if (both && !wait_sent(2 * i + 1)) break;
+            if (!project(Int<1>{}, i)) break;
+            x_half(Int<kFirstX>{}, Int<24>{}, i);
+            // the gate warps overwrite the hidden codes once the hh half is complete
+            if (i > 0) ok = ok && mbar_wait(bar_stored, (i - 1) & 1, abort_flag, 104);
+            x_half(Int<24>{}, Int<32>{}, i);
+            if (kExact && both) {
+                if (!hh_both()) break;
+                continue;
+            }
+            if (!hh_half(Int<0>{})) break;
+            if (!hh_half(Int<1>{})) break;
+        }
+    }
+}
+// Out of line: as a branch or a second loop in the kernel it cost the other weights 1 to 3 % of a step.
+template <int V, int C>
+__device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev p, int n_rows) {
+    issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows);
+}
 
 // The groups of chunk rows share the x part of the contraction (its MMAs read their A operand from shared memory, so
 // one for both) and go through the rest of the step one after the other: while one is exchanged, the other
@@ -195,39 +455,21 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                   const __grid_constant__ CUtensorMap tm_o,    // SPLIT: h_out [T, B, H], boxes of the first group's rows x 128
                   const __grid_constant__ CUtensorMap tm_ol,   // and of the second's
                   const GroupDev p) {
-    constexpr GroupForm F = group_form(V);
-    constexpr bool kGather = F.gather;
-    constexpr int G = F.groups, NB = G * F.rows, S = F.stride, H = C * kGUnits;
-    constexpr bool kTwoSteps = F.rows == 8;            // an x MMA covers two steps
-    constexpr int kXSlots = kTwoSteps ? 4 : F.x_slots;
-    constexpr int kTile = F.rows * 128;                // bytes of a group's hidden rows in one K block
-    constexpr int kHhTile = (kTwoSteps ? 24 : F.n) * 128;   // and of its hh_down rows
-    constexpr int kPieces = F.rows / 4;                // pieces of a group
-    constexpr int kPairs = kGather ? F.rows / 8 : F.rows / 4;   // pairs of rows of a gate thread
-    constexpr int kDnTs = group_dn_ts(V, C);
-    constexpr int kDnCol = kGTmemW - 8 * kDnTs;        // first column of the projection weights in tensor memory
-    constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
-    constexpr GroupLayout L = group_layout(V, C);
-    static_assert(4 * S + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
-    static_assert(L.dynamic <= kGMaxSmem, "shared memory of a CTA");
+    using K = GroupConst<V, C>;
+    constexpr GroupForm F = K::F;
+    constexpr GroupLayout L = K::L;
+    constexpr bool kGather = K::kGather, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
+    constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
+    constexpr int kPieces = K::kPieces, kPairs = K::kPairs, kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
     // shared-window offsets as this CTA's
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *bar_once = &bars[0];       // resident weights and the initial hidden rows loaded
-    uint64_t *bar_x = &bars[1];          // [slots] x_down rows landed
-    uint64_t *bar_x_free = &bars[5];     // [slots] the x part of the contraction has read them
-    uint64_t *bar_acc_free = &bars[9];   // the gate warps have read all accumulators
-    uint64_t *bar_proj = &bars[10];      // [G] projection accumulator complete
-    uint64_t *bar_acc = &bars[12];       // [G] gate accumulators complete
-    uint64_t *bar_hh = &bars[14];        // [G] hh_down rows in place
-    uint64_t *bar_code = &bars[16];      // SPLIT [G]: hidden codes of this CTA's units in place
-    uint64_t *bar_sum = &bars[18];       // SPLIT [G]: partial sums of the CTA's own pieces arrived
-    uint64_t *bar_sent = &bars[20];      // SPLIT: the projection accumulator has been read
-    uint64_t *bar_stored = &bars[21];    // SPLIT: the TMA stores have read the hidden codes
-    uint64_t *bar_h = &bars[16];         // GATHER [2]: hidden rows of all CTAs arrived
+    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + kBarX, *bar_x_free = bars + kBarXFree, *bar_acc_free = bars + kBarAccFree;
+    uint64_t *bar_proj = bars + kBarProj, *bar_acc = bars + kBarAcc, *bar_hh = bars + kBarHh, *bar_code = bars + kBarCode;
+    uint64_t *bar_sum = bars + kBarSum, *bar_sent = bars + kBarSent, *bar_stored = bars + kBarStored, *bar_h = bars + kBarH;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
 
@@ -248,7 +490,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 24; ++b) mbar_init(&bars[b], 1);
+        for (int b = 0; b < kGBars; ++b) mbar_init(&bars[b], 1);
         mbar_init(bar_acc_free, kGather || both ? kGEpiWarps : kGEpiWarps / 2);
         if (kGather) mbar_init(bar_hh, kGEpiWarps);
         else for (int e = 0; e < G; ++e) mbar_init(&bar_code[e], kGEpiWarps / 2);
@@ -265,7 +507,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             }
         }
     }
-    if (kHhTile > F.rows * 128) {   // the operand rows that are zero
+    if (K::kZeroRows) {
         for (int o = threadIdx.x * 16; o < L.dn - L.hh; o += kGThreads * 16)
             *reinterpret_cast<uint4 *>(smem + L.hh + o) = make_uint4(0, 0, 0, 0);
         fence_proxy_async_smem();
@@ -275,22 +517,33 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    bool non_finite = false;   // one of the recurrent gate weights
     if (warp >= 2) {
         // the hh half of the gate weights: warp = (lane quadrant, gate), thread = row of the block
         const int q = warp & 3, g = (warp - 2) >> 2;
         const uint4 *src = reinterpret_cast<const uint4 *>(
             p.w_up + (size_t(g) * H + n0 + q * 32 + lane) * (2 * kGRank));
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
+        __half2 zeros[2] = {__half2half2(__ushort_as_half(0)), __half2half2(__ushort_as_half(0))};
 #pragma unroll 1
-        for (int v = 0; v < 8; ++v) tmem_st_32x8(t_lane + kGTmemW + g * 64 + v * 8, __ldg(src + 2 * v), __ldg(src + 2 * v + 1));
+        for (int v = 0; v < 8; ++v) {
+            const uint4 lo = __ldg(src + 2 * v), hi = __ldg(src + 2 * v + 1);
+            tmem_st_32x8(t_lane + kGTmemW + g * 64 + v * 8, lo, hi);
+            if (K::kZeroRows) {
+                add_zero_times(zeros[0], lo);
+                add_zero_times(zeros[1], hi);
+            }
+        }
         // and K steps g, g + 4, .. of the projection rows, of all units or this CTA's
         const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(q * 32 + lane) * H + (kGather ? 0 : n0));
 #pragma unroll 1
         for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
+        const __half2 sum = __hadd2(zeros[0], zeros[1]);
+        non_finite = __hisnan(__low2half(sum)) || __hisnan(__high2half(sum));
         tmem_st_wait();
         tc_fence_before_sync();
     }
-    __syncthreads();
+    const bool finite = !__syncthreads_or(non_finite);
     tc_fence_after_sync();
     // every barrier of the cluster is initialised before any CTA may store to a peer
     cluster_sync_all();
@@ -344,164 +597,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ------------------------------ MMA issuer --------------------------------------
-        // The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
-        // K loops unrolled, so an MMA is issued every few cycles.
-        constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, kTwoSteps ? 16 : NB);
-        constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
-        constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
-        uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
-        uint64_t d_x0 = make_smem_desc_sw128(smem_u32(smem + L.x));
-        uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
-        uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
-        uint64_t d_h0 = make_smem_desc_sw128(smem_u32(smem + L.h));
-        bool ok = mbar_wait(bar_once, 0, abort_flag, 97);
-        int i = 0;
-        // MMAs [from, to) of the x part of a step. They read their A operand from shared memory (42 cycles
-        // each, 48 with 48 columns) and the tensor pipe works in order, so they are issued in pieces for the times when it
-        // would wait. With up to 8 rows, where the 32 MMAs of a step would take longer than all of its waits, an MMA covers
-        // the rows of two steps: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
-        // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones.
-        constexpr int kX = kTwoSteps ? 16 : 32;
-        auto x_half = [&](auto from, auto to, int i) {
-            constexpr int m0 = decltype(from)::value, m1 = decltype(to)::value;
-            const uint64_t d_x = d_x0 + uint64_t((i & (kXSlots - 1)) * (kTwoSteps ? NB * 8 : NB * 16));
-            const int g0 = kTwoSteps ? 2 * (i & 1) : 0;
-            if (elect_one()) {
-#pragma unroll
-                for (int m = m0; m < m1; ++m) {
-                    const int g = m >> 3, k = m & 7;
-                    tc_mma<kKindF16>(tmem + (g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                     d_x + uint64_t((k >> 2) * ((kTwoSteps ? 5 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
-                }
-                if (m1 == kX && i >= 0) tc_commit(&bar_x_free[i & (kXSlots - 1)]);
-            }
-            __syncwarp();
-        };
-        auto wait_x = [&](int step) {
-            if (step < p.T) ok = ok && mbar_wait(&bar_x[step & (kXSlots - 1)], (step / kXSlots) & 1, abort_flag, 99);
-            return ok;
-        };
-        auto wait_acc = [&]() {
-            if (i > 0) ok = ok && mbar_wait(bar_acc_free, (i - 1) & 1, abort_flag, 98);
-            tc_fence_after_sync();
-            return ok;
-        };
-        // projection u overwrites what projection u - 1 left
-        auto wait_sent = [&](int u) {
-            if (kOneProj && u > 0) ok = ok && mbar_wait(bar_sent, (u - 1) & 1, abort_flag, 106);
-            return ok;
-        };
-        // projection of h_{i-1}. SPLIT: this CTA's K block for the rows of a group
-        auto project = [&](auto group, int i) {
-            constexpr int e = decltype(group)::value;
-            if (e > 0 && !both) return true;
-            if (i > 0) ok = ok && mbar_wait(&bar_code[e], (i - 1) & 1, abort_flag, 100);
-            if (!ok) return false;
-            tc_fence_after_sync();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + e, clock64());
-            if (elect_one()) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint64_t rows = d_h0 + uint64_t(e * (kTile >> 4) + 2 * k);
-                    constexpr int kTo = 4 * S + (kOneProj ? 0 : e * F.n);
-                    if (k < kDnTs) tc_mma_ts<kKindI8>(tmem + kTo, tmem + kDnCol + 8 * k, rows, kIdescP, k != 0);
-                    else tc_mma<kKindI8>(tmem + kTo, d_dn + uint64_t(2 * k), rows, kIdescP, k != 0);
-                }
-                tc_commit(&bar_proj[e]);
-            }
-            __syncwarp();
-            return true;
-        };
-        // GATHER: all K blocks
-        auto project_all = [&]() {
-            if (i > 0) ok = ok && mbar_wait<true>(&bar_h[(i + 1) & 1], ((i - 1) >> 1) & 1, abort_flag, 100);
-            if (!ok) return false;
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 11, clock64());
-            fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
-            tc_fence_after_sync();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 0, clock64());
-            if (elect_one()) {
-                const uint64_t d_h = d_h0 + uint64_t(((i + 1) & 1) * (C * kTile >> 4));
-#pragma unroll
-                for (int kb = 0; kb < C; ++kb)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint64_t rows = d_h + uint64_t(kb * (kTile >> 4) + 2 * k);
-                        if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + 4 * S, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdescP, (kb | k) != 0);
-                        else tc_mma<kKindI8>(tmem + 4 * S, d_dn + uint64_t((kb - kDnTs / 4) * 1024 + 2 * k), rows, kIdescP, (kb | k) != 0);
-                    }
-                tc_commit(&bar_proj[0]);
-                if (i > 0 && i + 2 < p.T) mbar_arrive_expect_tx(&bar_h[(i + 1) & 1], uint32_t(n_rows) * H);  // for h_{i+1}
-            }
-            __syncwarp();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 1, clock64());
-            return true;
-        };
-        auto hh_half = [&](auto group) {
-            constexpr int e = decltype(group)::value;
-            if (e > 0 && !both) return true;
-            ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
-            if (!ok) return false;
-            if (!kGather) fence_proxy_async_smem();
-            tc_fence_after_sync();
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 3 + e, clock64());
-            if (elect_one()) {
-                // two steps per MMA: the other step's columns get rows that are zero
-                const uint64_t rows[2] = {d_hh + uint64_t(kTwoSteps && !(i & 1) ? 64 : 0), d_hh + uint64_t(kTwoSteps && (i & 1) ? 64 : 0)};
-#pragma unroll
-                for (int g = 0; g < 4; ++g)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        tc_mma_ts<kKindF16>(tmem + g * S + F.rows * e, tmem + kGTmemW + g * 64 + k * 8,
-                                            rows[g >> 1] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
-                tc_commit(&bar_acc[e]);
-                if (!kGather && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
-            }
-            __syncwarp();
-            return true;
-        };
-        if constexpr (kTwoSteps) {
-            // gates 2 and 3 of step 0: as the second step of the one before it
-            if (ok) ok = mbar_wait(&bar_x[0], 0, abort_flag, 99);
-            if (ok) x_half(Int<0>{}, Int<16>{}, -1);
-        }
-        for (; i < p.T && ok; ++i) {
-            // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
-            // more registers than there are.
-            asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
-            constexpr int kFirstX = kTwoSteps ? 10 : kGather ? 24 : 2;
-            if constexpr (kGather) {
-                // Most of the x part while the hidden state is computed and travels, the rest while the
-                // projection is converted. 300 chunks, 20 / 24 / 28 of 32 in front: 1.63 / 1.60 / 1.63 us per step; 32 chunks, 8 / 10 /
-                // 12 of 16: 1.18 / 1.18 / 1.22.
-                if (!wait_x(kTwoSteps ? i + 1 : i) || !wait_acc()) break;
-                FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
-                x_half(Int<0>{}, Int<kFirstX>{}, i);
-                FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 10, clock64());
-                if (!project_all()) break;
-                x_half(Int<kFirstX>{}, Int<kX>{}, i);
-                if (!hh_half(Int<0>{})) break;
-            } else {
-                // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
-                // what has long been there takes 100 cycles and more while the gate warps keep the units of the SM busy that
-                // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step).
-                // MMAs in front of the second projection, 1024 chunks: 2 2.71-2.76, 4 2.74-2.78, 8 2.79; 700 chunks 2.04, 2.04-2.08,
-                // 2.12. Four in front of the first as well 3.07-3.16 and 2.24-2.33.
-                if (!wait_x(i) || !wait_sent(both ? 2 * i : i)) break;
-                if (!project(Int<0>{}, i)) break;
-                if (!wait_acc()) break;
-                x_half(Int<0>{}, Int<kFirstX>{}, i);
-                if (both && !wait_sent(2 * i + 1)) break;
-                if (!project(Int<1>{}, i)) break;
-                x_half(Int<kFirstX>{}, Int<24>{}, i);
-                // the gate warps overwrite the hidden codes once the hh half is complete
-                if (i > 0) ok = ok && mbar_wait(bar_stored, (i - 1) & 1, abort_flag, 104);
-                x_half(Int<24>{}, Int<32>{}, i);
-                if (!hh_half(Int<0>{})) break;
-                if (!hh_half(Int<1>{})) break;
-            }
-        }
+        if (K::kZeroRows && !finite) issue_exact<V, C>(smem, tmem, p, n_rows);
+        else issue<V, C, false>(smem, tmem, p, n_rows);
     } else {
         // ------------------------------ gates -------------------------------------------
         // thread = hidden unit. GATHER: a quarter of the rows; SPLIT: half of the rows of one group, eight warps each, so

@@ -494,3 +494,31 @@ def test_small_cluster_form_of_few_rows_and_of_two_groups_gives_the_bytes_of_the
     flib.fluke_set_lstm_persistent(1)
     for got, want in zip(*res):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("H,B", [(768, 44), (768, 150), (768, 300), (768, 700), (768, 1000), (1024, 100), (1024, 700), (256, 400)])
+def test_infinite_gate_weights_reach_their_own_unit_and_row_only(flib, H, B):
+    """An infinite weight makes a pre-activation infinite, so the gate saturates (NaN only where the row's own factor is zero or
+    two infinities meet), whatever the other rows of the cluster are. Every number of rows per cluster from which the small-cluster
+    form has another kernel, weights of all four gates and both halves, against the L2-exchange form, which multiplies
+    every weight by the row's own values alone: the same bytes, NaN at the same places."""
+    T, R = 7, 128
+    layer, x, xs = _layer_case(T, B, H, R, H + B, False)
+    w = layer.w_up.clone()
+    for i, (unit, k) in enumerate([(3, 5), (40, 127), (H - 1, 64), (129, 0), (70, 130), (H - 100, 255)]):
+        w[(i % 4) * H + unit, k] = float("inf") if i % 2 else float("-inf")
+    w[2 * H + 17, 33] = 65504.0
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, h = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale, w, layer.bias, c, h)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, h))
+    flib.fluke_set_lstm_persistent(1)
+    (out, c, h), (out_l2, c_l2, h_l2) = res
+    assert torch.equal(torch.isnan(c), torch.isnan(c_l2)) and not torch.isnan(c).all(0).all()
+    assert torch.equal(c.nan_to_num(7.0), c_l2.nan_to_num(7.0)) and torch.equal(out, out_l2) and torch.equal(h, h_l2)
