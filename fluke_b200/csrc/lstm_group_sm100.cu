@@ -34,7 +34,8 @@
 // after its gate contraction of step t, for which every owner of rows has read its partial sums of step t; an owner
 // sends hh_{t+1} after every CTA's projection of h_t, i.e. after every CTA's contraction of step t. GATHER: a
 // CTA sends h_t after it has received h_{t-1} of every CTA, which each sent after its projection of h_{t-2}: two
-// slots of hidden rows. Nobody leaves before the final cluster barrier. Clusters never wait for one
+// slots of hidden rows. The final hidden state goes where the initial one was read: of a CTA's own units only (SPLIT), or after
+// every CTA's initial rows have landed (GATHER, before the first cluster barrier). Nobody leaves before the final cluster barrier. Clusters never wait for one
 // another, so any number of them may run in waves.
 //
 // What bounds a step (B200, H = 768, cycles). 2 rows per cluster, 2100: the chain of exchange (490 from the first
@@ -517,6 +518,19 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    if (warp == 0 && elect_one()) {
+        // what stays, and the initial hidden rows, beside the weights that go to tensor memory
+        constexpr int kDnTiles = (L.h - L.dn) / 16384;   // the last K blocks
+        mbar_arrive_expect_tx(bar_once, kGWxBytes + kDnTiles * 16384 + (kGather ? C : 1) * NB * 128);
+        for (int g = 0; g < 4; ++g)
+            for (int kb = 0; kb < 2; ++kb)
+                tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
+        for (int b = 0; b < kDnTiles; ++b)
+            tma_load_2d(smem + L.dn + b * 16384, &tm_dn, bar_once, kGather ? (kDnTs / 4 + b) * kGUnits : n0, 0);
+        // step 0 projects the layer's initial hidden state
+        for (int e = 0; e < G; ++e)
+            tma_load_3d(smem + L.h + (kGather ? C : e) * kTile, &tm_h0, bar_once, 0, m0 + F.rows * e, kGather ? 0 : rank);
+    }
     bool non_finite = false;   // one of the recurrent gate weights
     if (warp >= 2) {
         // the hh half of the gate weights: warp = (lane quadrant, gate), thread = row of the block
@@ -545,22 +559,15 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     }
     const bool finite = !__syncthreads_or(non_finite);
     tc_fence_after_sync();
+    // GATHER: a CTA loads the initial hidden rows of its peers' units too, and a layer of one step stores the final ones, of its
+    // own units and to the same place, without having heard from them: nobody passes the barrier before they have landed.
+    if (kGather) mbar_wait(bar_once, 0, abort_flag, 97);
     // every barrier of the cluster is initialised before any CTA may store to a peer
     cluster_sync_all();
 
     if (warp == 0) {
         // ------------------------------ loader (one thread) -----------------------------
         if (elect_one()) {
-            constexpr int kDnTiles = (L.h - L.dn) / 16384;   // the last K blocks
-            mbar_arrive_expect_tx(bar_once, kGWxBytes + kDnTiles * 16384 + (kGather ? C : 1) * NB * 128);
-            for (int g = 0; g < 4; ++g)
-                for (int kb = 0; kb < 2; ++kb)
-                    tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
-            for (int b = 0; b < kDnTiles; ++b)
-                tma_load_2d(smem + L.dn + b * 16384, &tm_dn, bar_once, kGather ? (kDnTs / 4 + b) * kGUnits : n0, 0);
-            // step 0 projects the layer's initial hidden state
-            for (int e = 0; e < G; ++e)
-                tma_load_3d(smem + L.h + (kGather ? C : e) * kTile, &tm_h0, bar_once, 0, m0 + F.rows * e, kGather ? 0 : rank);
             bool ok = true;
             auto load_x = [&](int i) {
                 const int s = i & (kXSlots - 1), u = i / kXSlots;
@@ -597,8 +604,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (K::kZeroRows && !finite) issue_exact<V, C>(smem, tmem, p, n_rows);
-        else issue<V, C, false>(smem, tmem, p, n_rows);
+        if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows);
+        else issue_exact<V, C>(smem, tmem, p, n_rows);
     } else {
         // ------------------------------ gates -------------------------------------------
         // thread = hidden unit. GATHER: a quarter of the rows; SPLIT: half of the rows of one group, eight warps each, so

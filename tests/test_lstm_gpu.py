@@ -522,3 +522,22 @@ def test_infinite_gate_weights_reach_their_own_unit_and_row_only(flib, H, B):
     (out, c, h), (out_l2, c_l2, h_l2) = res
     assert torch.equal(torch.isnan(c), torch.isnan(c_l2)) and not torch.isnan(c).all(0).all()
     assert torch.equal(c.nan_to_num(7.0), c_l2.nan_to_num(7.0)) and torch.equal(out, out_l2) and torch.equal(h, h_l2)
+
+
+@pytest.mark.parametrize("H,B", [(256, 600), (384, 32), (768, 44), (768, 300), (896, 144), (1024, 30), (1024, 200)])
+def test_one_timestep_per_call_gives_the_bytes_of_one_call(flib, H, B):
+    """A caller's own time loop over calls of one timestep, state carried over in place: the final hidden codes of a call are stored
+    where the cluster's CTAs load the initial ones of all units from. Rows per cluster where they do. Exact."""
+    T = 48
+    layer, x, xs = _layer_case(T, B, H, 128, H + B, False)
+    x, xs = x.to(DEV), xs.to(DEV)
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    args = (layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale, layer.w_up, layer.bias)
+    c, h = c0.clone(), h0.clone()
+    want = ops.factored_lstm_layer_i8(x, xs, *args, c, h)
+    assert flib.fluke_sm100_lstm_last_form() == 3
+    c1, h1 = c0.clone(), h0.clone()
+    got = torch.cat([ops.factored_lstm_layer_i8(x[t:t + 1], xs.view(T, B)[t], *args, c1, h1) for t in range(T)])
+    assert torch.equal(got, want) and torch.equal(c1, c) and torch.equal(h1, h)
