@@ -491,11 +491,13 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
     if (threadIdx.x == 0) {
-        for (int b = 0; b < kGBars; ++b) mbar_init(&bars[b], 1);
-        mbar_init(bar_acc_free, kGather || both ? kGEpiWarps : kGEpiWarps / 2);
-        if (kGather) mbar_init(bar_hh, kGEpiWarps);
-        else for (int e = 0; e < G; ++e) mbar_init(&bar_code[e], kGEpiWarps / 2);
-        if (!kGather) mbar_init(bar_sent, kGEpiWarps / 2);
+        auto arrivals = [&](int b) {   // warps that arrive, or one arrival with the expected bytes
+            if (b == kBarAccFree) return kGather || both ? kGEpiWarps : kGEpiWarps / 2;
+            if (kGather) return b == kBarHh ? kGEpiWarps : 1;
+            return b == kBarCode || b == kBarCode + 1 || b == kBarSent ? kGEpiWarps / 2 : 1;
+        };
+#pragma unroll
+        for (int b = 0; b < kGBars; ++b) mbar_init(&bars[b], arrivals(b));
         *abort_flag = 0;
         fence_barrier_init();
         if constexpr (kGather) {
