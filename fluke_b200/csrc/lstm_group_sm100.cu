@@ -931,7 +931,7 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     p.h_state = static_cast<int8_t *>(l->h_i8);
     p.trace = trace_buffer();
 
-    CUtensorMap tm_w, tm_x, tm_dn, tm_h0, tm_o[2];
+    CUtensorMap tm_w, tm_x, tm_dn, tm_h0, tm_o[2] = {};
     int rc = make_tmap_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, l->w_up_f16, 4 * uint64_t(H), 2 * R, uint64_t(2 * R) * 2,
                           kGUnits, 64, true);
     if (rc) return rc;
@@ -953,7 +953,7 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
         if (rc) return rc;
     }
     // boxes of exactly the rows a group has: the rows behind them are another cluster's
-    for (int e = 0; e < 2; ++e) {
+    for (int e = 0; e < 2 && !f.gather; ++e) {
         const int box_rows = e == 0 ? min(g.rows, f.rows) : max(g.rows - f.rows, 1);
         rc = make_tmap_3d(&tm_o[e], CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_out_i8, T, B, H, H, uint64_t(B) * H, box_rows, 128, true);
         if (rc) return rc;

@@ -353,8 +353,8 @@ extern "C" int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, 
         return (int)cudaErrorInvalidValue;
     if (l->workspace_bytes < fluke_sm100_lstm_layer_workspace(T, B, H, R))
         return (int)cudaErrorInvalidValue;
-    // The small-cluster and cluster forms store h_out sixteen bytes at a time and have no tensor map on it
-    // that would refuse another address, as the other forms do.
+    // The cluster form, and the small-cluster form with up to sixteen rows per cluster, store h_out sixteen bytes at a time and
+    // have no tensor map on it that would refuse another address, as the other forms do.
     if (reinterpret_cast<uintptr_t>(l->h_out_i8) & 15u) return (int)cudaErrorMisalignedAddress;
 
     uint8_t *ws = static_cast<uint8_t *>(l->workspace);
