@@ -15,7 +15,7 @@
 // cluster's rows. What is exchanged for the projection of the hidden rows depends on how many rows there are:
 //
 //   GATHER, up to 16 rows: every CTA sends the int8 codes of its units to all CTAs and projects the complete
-//   rows itself (M = 128 projection columns, K = H). One exchange per step.
+//   rows itself (M = 128 projection columns, K = H). One exchange per step. (Clusters of eight, from 9 rows on: see group_by_pair.)
 //
 //   SPLIT, two groups of up to 16 or 24 rows: a CTA projects only its own units (K = 128), so hidden codes do not
 //   leave it. Its int32 partial sums go, four rows at a time, to the CTA that adds up those rows (integer sums,
@@ -34,7 +34,8 @@
 // after its gate contraction of step t, for which every owner of rows has read its partial sums of step t; an owner
 // sends hh_{t+1} after every CTA's projection of h_t, i.e. after every CTA's contraction of step t. GATHER: a
 // CTA sends h_t after it has received h_{t-1} of every CTA, which each sent after its projection of h_{t-2}: two
-// slots of hidden rows. The final hidden state goes where the initial one was read: of a CTA's own units only (SPLIT), or after
+// slots of hidden rows. By pair: a CTA sends h_t after its contraction of step t, which needs hh_t of every pair, sent after its
+// projection of h_{t-1}; and hh the other way round. The final hidden state goes where the initial one was read: of a CTA's own units only (SPLIT), or after
 // every CTA's initial rows have landed (GATHER, before the first cluster barrier). Nobody leaves before the final cluster barrier. Clusters never wait for one
 // another, so any number of them may run in waves.
 //
@@ -126,6 +127,15 @@ __host__ __device__ constexpr int group_dn_ts(int V, int C) {
 __host__ __device__ constexpr int group_own_pieces(int V, int C) {
     return (group_form(V).groups * group_form(V).rows / 4 + C - 1) / C;
 }
+// GATHER with clusters of eight and 9 to 16 rows: rows are projected BY PAIR. Pair (2p, 2p + 1) of CTAs receives the codes of a
+// quarter of the rows, projects 64 columns per CTA (M = 64) and sends the f16 result to all: two exchanges, but half of the
+// bytes. Two such clusters share the network between the SMs of a GPC; all to all, the last code is 840 cycles old when
+// the slowest arrives, 535 where a cluster is alone in its GPC. Us per step, x_down included, all to all against by pair: 9 rows 1.89 : 1.66,
+// 12 rows 1.98 : 1.71, 14 rows 2.13 : 1.79, 16 rows 2.19 : 1.87 (the kernel of 31278fa, by pair as well: 1.76, 1.88, 1.95, 2.04).
+// Smaller clusters stay with all to all: an odd number of CTAs has no pairs, a pair of fewer than eight would own more than one
+// row per quarter of its gate warps, and there all to all was the faster against that kernel (H = 768, 14 rows 1.61 : 1.66).
+// Up to 8 rows two steps per x MMA make up for it (H = 1024, 8 rows 1.69 : 1.73 against that kernel).
+__host__ __device__ constexpr bool group_by_pair(int V, int C) { return V == 1 && C == 8; }
 struct GroupLayout {
     int x, hh, dn, h, recv, stage, bars, misc, dynamic;
 };
@@ -136,14 +146,15 @@ __host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
     l.hh = l.x + f.x_slots * f.groups * f.rows * 256;
     // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
     l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
-    // projection weights [128 x 128 B] of the K blocks that are not all in tensor memory
-    l.h = l.dn + 16384 * ((f.gather ? C : 1) - group_dn_ts(V, C) / 4);
-    // int8 hidden rows. GATHER: two slots of C K blocks [rows x 128 B]; else this CTA's units, per group [rows x 128 B].
-    // An MMA of more columns reads on behind them
-    l.recv = l.h + (f.gather ? 2 * C : f.groups) * f.rows * 128;
+    // projection weights [128 x 128 B] (by pair [64 x 128 B]) of the K blocks that are not all in tensor memory
+    l.h = l.dn + (group_by_pair(V, C) ? 8192 : 16384) * ((f.gather ? C : 1) - group_dn_ts(V, C) / 4);
+    // int8 hidden rows. GATHER: two slots of C K blocks [rows x 128 B], by pair one of [8 x 128 B]; else this CTA's units, per
+    // group [rows x 128 B]. An MMA of more columns reads on behind them
+    l.recv = l.h + (group_by_pair(V, C) ? C * 1024 : (f.gather ? 2 * C : f.groups) * f.rows * 128);
     // partial sums of the CTA's own pieces: per piece and source CTA [128 columns][4 rows] int32
     l.stage = l.recv + (f.gather ? 0 : group_own_pieces(V, C) * C * 2048);
-    l.bars = l.stage + 2048;                      // GATHER: two slots x four quarters x [2 rows x 128 B]; else per warp [2 rows x 64 B]
+    // GATHER: two slots x four quarters x [2 rows x 128 B], by pair [4 rows x 128 B]; else per warp [2 rows x 64 B]
+    l.bars = l.stage + (group_by_pair(V, C) ? 4096 : 2048);
     l.misc = l.bars + kGBars * 8;
     l.dynamic = l.misc + 16 + 1024;               // slack for the manual 1024-byte alignment
     return l;
@@ -203,9 +214,12 @@ struct GroupConst {
     static constexpr int G = F.groups, NB = G * F.rows, S = F.stride, H = C * kGUnits;
     static constexpr bool kTwoSteps = F.rows == 8;            // an x MMA covers two steps
     static constexpr int kXSlots = kTwoSteps ? 4 : F.x_slots;
-    static constexpr int kTile = F.rows * 128;                // bytes of a group's hidden rows in one K block
+    static constexpr bool kByPair = group_by_pair(V, C);
+    static constexpr bool kPeerHh = !kGather || kByPair;      // hh_down rows come from peers
+    static constexpr int kTile = (kByPair ? 8 : F.rows) * 128;     // bytes of a group's hidden rows in one K block
     static constexpr int kHhTile = (kTwoSteps ? 24 : F.n) * 128;   // and of its hh_down rows
-    static constexpr bool kZeroRows = kHhTile > kTile;        // some of which are zero
+    static constexpr bool kZeroRows = kHhTile > F.rows * 128; // some of which are zero
+    static constexpr int kDnRows = kByPair ? 64 : kGRank;     // projection columns of a CTA
     static constexpr int kPieces = F.rows / 4;                // pieces of a group
     static constexpr int kPairs = kGather ? F.rows / 8 : F.rows / 4;   // pairs of rows of a gate thread
     static constexpr int kDnTs = group_dn_ts(V, C);
@@ -213,6 +227,7 @@ struct GroupConst {
     static constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
     static_assert(4 * S + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
     static_assert(L.dynamic <= kGMaxSmem, "shared memory of a CTA");
+    static_assert(!kByPair || (C % 2 == 0 && F.rows <= 2 * C), "a pair's rows are one per quarter of the gate warps");
 };
 // mbarriers of a CTA, as indices
 enum : int {
@@ -227,17 +242,17 @@ enum : int {
     kBarSum = 18,      // SPLIT [G]: partial sums of the CTA's own pieces arrived
     kBarSent = 20,     // SPLIT: the projection accumulator has been read
     kBarStored = 21,   // SPLIT: the TMA stores have read the hidden codes
-    kBarH = 16         // GATHER [2]: hidden rows of all CTAs arrived
+    kBarH = 16         // GATHER [2], by pair [1]: hidden rows of all CTAs arrived
 };
 
 // The MMA issuer, warp 1. The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
 // K loops unrolled, so an MMA is issued every few cycles. kExact: for weights that are not finite.
 template <int V, int C, bool kExact>
-__device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupDev &p, int n_rows) {
+__device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupDev &p, int n_rows, int own_rows) {
     using K = GroupConst<V, C>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
-    constexpr bool kGather = K::kGather, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
+    constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
     constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
     constexpr int kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
@@ -314,26 +329,28 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         __syncwarp();
         return true;
     };
-    // GATHER: all K blocks
+    // GATHER: all K blocks. Hidden rows of step u are in slot u mod 2, by pair in the only one
     auto project_all = [&]() {
-        if (i > 0) ok = ok && mbar_wait<true>(&bar_h[(i + 1) & 1], ((i - 1) >> 1) & 1, abort_flag, 100);
+        if (i > 0) ok = ok && mbar_wait<true>(&bar_h[kByPair ? 0 : (i + 1) & 1], (kByPair ? i - 1 : (i - 1) >> 1) & 1, abort_flag, 100);
         if (!ok) return false;
         FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 11, clock64());
         fence_proxy_async_smem();   // the peers' stores are generic-proxy writes
         tc_fence_after_sync();
         FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 0, clock64());
         if (elect_one()) {
-            const uint64_t d_h = d_h0 + uint64_t(((i + 1) & 1) * (C * kTile >> 4));
+            const uint64_t d_h = d_h0 + uint64_t((kByPair ? 0 : (i + 1) & 1) * (C * kTile >> 4));
+            constexpr uint32_t kIdesc = make_idesc<kKindI8>(K::kDnRows, kByPair ? 8 : F.n);
 #pragma unroll
             for (int kb = 0; kb < C; ++kb)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const uint64_t rows = d_h + uint64_t(kb * (kTile >> 4) + 2 * k);
-                    if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + 4 * S, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdescP, (kb | k) != 0);
-                    else tc_mma<kKindI8>(tmem + 4 * S, d_dn + uint64_t((kb - kDnTs / 4) * 1024 + 2 * k), rows, kIdescP, (kb | k) != 0);
+                    if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + 4 * S, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdesc, (kb | k) != 0);
+                    else tc_mma<kKindI8>(tmem + 4 * S, d_dn + uint64_t((kb - kDnTs / 4) * (K::kDnRows * 8) + 2 * k), rows, kIdesc, (kb | k) != 0);
                 }
             tc_commit(&bar_proj[0]);
-            if (i > 0 && i + 2 < p.T) mbar_arrive_expect_tx(&bar_h[(i + 1) & 1], uint32_t(n_rows) * H);  // for h_{i+1}
+            if (kByPair && i > 0 && i + 1 < p.T) mbar_arrive_expect_tx(&bar_h[0], uint32_t(own_rows) * H);  // for h_i
+            if (!kByPair && i > 0 && i + 2 < p.T) mbar_arrive_expect_tx(&bar_h[(i + 1) & 1], uint32_t(n_rows) * H);  // for h_{i+1}
         }
         __syncwarp();
         FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 1, clock64());
@@ -344,7 +361,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         if (e > 0 && !both) return true;
         ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
         if (!ok) return false;
-        if (!kGather) fence_proxy_async_smem();
+        if (K::kPeerHh) fence_proxy_async_smem();
         tc_fence_after_sync();
         FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 3 + e, clock64());
         if (elect_one()) {
@@ -357,7 +374,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
                     tc_mma_ts<kKindF16>(tmem + g * S + F.rows * e, tmem + kGTmemW + g * 64 + k * 8,
                                         rows[g >> 1] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
             tc_commit(&bar_acc[e]);
-            if (!kGather && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+            if (K::kPeerHh && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
         }
         __syncwarp();
         return true;
@@ -398,7 +415,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
         // more registers than there are.
         asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
-        constexpr int kFirstX = kTwoSteps ? 10 : kGather ? 24 : 2;
+        constexpr int kFirstX = kTwoSteps ? 10 : kByPair ? 16 : kGather ? 24 : 2;
         if constexpr (kGather) {
             // Most of the x part while the hidden state is computed and travels, the rest while the
             // projection is converted. 300 chunks, 20 / 24 / 28 of 32 in front: 1.63 / 1.60 / 1.63 us per step; 32 chunks, 8 / 10 /
@@ -441,7 +458,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
 // Out of line: as a branch or a second loop in the kernel it cost the other weights 1 to 3 % of a step.
 template <int V, int C>
 __device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev p, int n_rows) {
-    issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows);
+    issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows, 0);
 }
 
 // The groups of chunk rows share the x part of the contraction (its MMAs read their A operand from shared memory, so
@@ -459,7 +476,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     using K = GroupConst<V, C>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
-    constexpr bool kGather = K::kGather, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
+    constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
     constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
     constexpr int kPieces = K::kPieces, kPairs = K::kPairs, kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     extern __shared__ uint8_t smem_raw[];
@@ -480,6 +497,10 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     const int n_rows = min(p.rows, p.B - m0);          // and how many it has
     const int n0 = rank * kGUnits;
     auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
+    // by pair: rows per pair, and those of this one
+    const int pair = rank >> 1, half = rank & 1;
+    const int per_pair = kByPair ? (p.rows + C / 2 - 1) / (C / 2) : 0;
+    const int own_rows = kByPair ? min(max(n_rows - pair * per_pair, 0), per_pair) : 0;
     // whether this CTA adds up piece k of group e, and how many pieces of the group it adds up
     auto own_piece = [&](int e, int k) { return (kPieces * e + k) % C == rank && 4 * k < rows_of(e); };
     auto own_pieces = [&](int e) {
@@ -493,14 +514,17 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     if (threadIdx.x == 0) {
         auto arrivals = [&](int b) {   // warps that arrive, or one arrival with the expected bytes
             if (b == kBarAccFree) return kGather || both ? kGEpiWarps : kGEpiWarps / 2;
-            if (kGather) return b == kBarHh ? kGEpiWarps : 1;
+            if (kGather) return !kByPair && b == kBarHh ? kGEpiWarps : 1;
             return b == kBarCode || b == kBarCode + 1 || b == kBarSent ? kGEpiWarps / 2 : 1;
         };
 #pragma unroll
         for (int b = 0; b < kGBars; ++b) mbar_init(&bars[b], arrivals(b));
         *abort_flag = 0;
         fence_barrier_init();
-        if constexpr (kGather) {
+        if constexpr (kByPair) {
+            mbar_arrive_expect_tx(&bar_hh[0], uint32_t(n_rows) * 256);
+            if (p.T > 1) mbar_arrive_expect_tx(&bar_h[0], uint32_t(own_rows) * H);
+        } else if constexpr (kGather) {
             for (int s = 0; s < 2; ++s)
                 if (s + 1 < p.T) mbar_arrive_expect_tx(&bar_h[s], uint32_t(n_rows) * H);
         } else {
@@ -522,16 +546,17 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     const uint32_t tmem = *tmem_slot;
     if (warp == 0 && elect_one()) {
         // what stays, and the initial hidden rows, beside the weights that go to tensor memory
-        constexpr int kDnTiles = (L.h - L.dn) / 16384;   // the last K blocks
-        mbar_arrive_expect_tx(bar_once, kGWxBytes + kDnTiles * 16384 + (kGather ? C : 1) * NB * 128);
+        constexpr int kDnTile = K::kDnRows * 128, kDnTiles = (L.h - L.dn) / kDnTile;   // the last K blocks
+        mbar_arrive_expect_tx(bar_once, kGWxBytes + kDnTiles * kDnTile + (kGather ? C : G) * kTile);
         for (int g = 0; g < 4; ++g)
             for (int kb = 0; kb < 2; ++kb)
                 tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
         for (int b = 0; b < kDnTiles; ++b)
-            tma_load_2d(smem + L.dn + b * 16384, &tm_dn, bar_once, kGather ? (kDnTs / 4 + b) * kGUnits : n0, 0);
+            tma_load_2d(smem + L.dn + b * kDnTile, &tm_dn, bar_once, kGather ? (kDnTs / 4 + b) * kGUnits : n0, kByPair ? half * 64 : 0);
         // step 0 projects the layer's initial hidden state
         for (int e = 0; e < G; ++e)
-            tma_load_3d(smem + L.h + (kGather ? C : e) * kTile, &tm_h0, bar_once, 0, m0 + F.rows * e, kGather ? 0 : rank);
+            tma_load_3d(smem + L.h + (kByPair ? 0 : kGather ? C : e) * kTile, &tm_h0, bar_once, 0,
+                        kByPair ? m0 + pair * per_pair : m0 + F.rows * e, kGather ? 0 : rank);
     }
     bool non_finite = false;   // one of the recurrent gate weights
     if (warp >= 2) {
@@ -551,7 +576,9 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             }
         }
         // and K steps g, g + 4, .. of the projection rows, of all units or this CTA's
-        const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(q * 32 + lane) * H + (kGather ? 0 : n0));
+        // (M = 64: row 16 q + i in lane 32 q + i)
+        const int dn_row = kByPair ? half * 64 + q * 16 + (lane & 15) : q * 32 + lane;
+        const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(dn_row) * H + (kGather ? 0 : n0));
 #pragma unroll 1
         for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
         const __half2 sum = __hadd2(zeros[0], zeros[1]);
@@ -606,7 +633,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows);
+        if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows, own_rows);
         else issue_exact<V, C>(smem, tmem, p, n_rows);
     } else {
         // ------------------------------ gates -------------------------------------------
@@ -634,7 +661,77 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                                    make_float2(b_g, b_g), make_float2(b_o, b_o), c);
         };
 
-        if constexpr (kGather) {
+        if constexpr (kByPair) {
+            // What a CTA sends leaves in rows of 128 bytes, eight lanes each (see below). The four warps of a quarter stage together, one
+            // projected row or four rows of codes, in two slots in turn: the barrier after one batch is staged also
+            // says that the slot of the batch before has been read.
+            const uint32_t stage = smem_u32(smem + L.stage) + part * 512;
+            uint32_t slot = 0;
+            // the pair's row `part` of this CTA's columns: lanes 8 j .. 8 j + 7 of warps 0 and 1 send it to the CTA 4 q + j behind this one
+            const bool projects = part < own_rows;
+            const int p_row = pair * per_pair + part;
+            const uint32_t p_to = uint32_t((4 * q + (lane >> 3) + rank) % C);
+            const uint32_t p_dst = map_to_rank(smem_u32(smem + L.hh + half * kHhTile) + p_row * 128 + (lane & 7) * 16, p_to);
+            const uint32_t p_bar = map_to_rank(smem_u32(bar_hh), p_to);
+            // codes: row q of the quarter, lanes 0-7 to the first CTA of the pair that owns it, 8-15 to the second
+            const int h_row = r0 + q, h_pair = h_row / per_pair, h_own = h_row - h_pair * per_pair;
+            const bool sends = lane < 16 && q < my_rows;
+            const uint32_t h_to = sends ? uint32_t(2 * h_pair + (lane >> 3)) : uint32_t(rank);
+            const uint32_t h_dst = map_to_rank(smem_u32(smem + L.h) + rank * kTile + h_own * 128 + (lane & 7) * 16, h_to);
+            const uint32_t h_bar = map_to_rank(smem_u32(bar_h), h_to);
+            // the piece of a staged row that belongs at a place of the 128-byte swizzle
+            const uint32_t p_src = stage + ((lane ^ p_row) & 7) * 16, h_src = stage + q * 128 + ((lane ^ h_own) & 7) * 16;
+            const int64_t at = int64_t(m0 + h_row) * H + n0 + ((lane ^ h_own) & 7) * 16;
+            const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + half * 64 + q * 16 + (lane & 15));  // operand order of the dequant GEMM: sa * sb
+            int8_t *h_out = p.h_out + int64_t(time_of(0)) * p.B * H + at;
+            const int64_t plane = int64_t(p.reverse ? -p.B : p.B) * H;
+            // A warp whose wait ran out goes on without waiting, sending or storing, as below.
+            for (int i = 0; i < p.T; ++i, h_out += plane) {
+                // ---- projection of the pair's h_{i-1}: int32 -> f16, to every CTA ----
+                if (projects) {
+                    ok = ok && mbar_wait(&bar_proj[0], i & 1, abort_flag, 102);
+                    slot ^= 2048;
+                    tc_fence_after_sync();
+                    uint32_t v, next;
+                    tmem_ld_32x2(t_lane + 4 * S + part, v, next);
+                    tmem_ld_wait();
+                    if (lane < 16) sts16(stage + slot + q * 32 + lane * 2, __half_as_ushort(__float2half_rn(float(int(v)) * sc)));
+                    tc_fence_before_sync();
+                    quad_sync(1 + part);
+                    if (ok && q < 2) store_to_peer(p_dst, lds128(p_src + slot), p_bar);
+                }
+                // ---- gates, cell update, hidden codes: all four rows, sent as soon as they are staged ----
+                ok = ok && mbar_wait(&bar_acc[0], i & 1, abort_flag, 103);
+                Acc a;
+                if (my_rows > 0) {
+                    tc_fence_after_sync();
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_lane + g * S + r0, a[g]);
+                    tmem_ld_wait();
+                    tc_fence_before_sync();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_acc_free);
+                if (my_rows == 0) continue;
+                slot ^= 2048;
+                auto stage_pair = [&](int j) {
+                    const int2 h = codes(a, j, c2[j]);
+                    sts8(stage + slot + 2 * j * 128 + q * 32 + lane, h.x);
+                    sts8(stage + slot + (2 * j + 1) * 128 + q * 32 + lane, h.y);
+                };
+                stage_pair(0);
+                if (my_rows > 2) stage_pair(kPairs - 1);
+                quad_sync(1 + part);
+                if (ok && sends) {
+                    const uint4 v = lds128(h_src + slot);
+                    if (i + 1 < p.T) store_to_peer(h_dst, v, h_bar);
+                    if (lane < 8) {
+                        *reinterpret_cast<uint4 *>(h_out) = v;
+                        if (i + 1 == p.T) *reinterpret_cast<uint4 *>(p.h_state + at) = v;
+                    }
+                }
+            }
+        } else if constexpr (kGather) {
             // Two rows at a time leave as rows of 128 bytes, eight lanes each: the network between the SMs moves 64
             // contiguous bytes to one CTA in the time of 16 (20.7 against 9.5 B per cycle and SM, measured with
             // six CTAs sending to each other). A warp holds 32 bytes of a row, so the four warps of a quarter stage
@@ -943,12 +1040,13 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
         rc = make_tmap_nd(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_down, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
-    rc = make_tmap_2d(&tm_dn, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, l->dn_hh_i8, R, H, H, kGRank, 128, true);
+    const bool by_pair = group_by_pair(g.form, C);
+    rc = make_tmap_2d(&tm_dn, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, l->dn_hh_i8, R, H, H, by_pair ? 64 : kGRank, 128, true);
     if (rc) return rc;
     {
         const uint64_t dims[3] = {128, uint64_t(B), uint64_t(C)};
         const uint64_t strides[2] = {uint64_t(H), 128};
-        const uint32_t box[3] = {128, uint32_t(f.rows), uint32_t(f.gather ? C : 1)};
+        const uint32_t box[3] = {128, by_pair ? 8u : uint32_t(f.rows), uint32_t(f.gather ? C : 1)};
         rc = make_tmap_nd(&tm_h0, CU_TENSOR_MAP_DATA_TYPE_UINT8, l->h_i8, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }

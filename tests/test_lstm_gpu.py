@@ -541,3 +541,26 @@ def test_one_timestep_per_call_gives_the_bytes_of_one_call(flib, H, B):
     c1, h1 = c0.clone(), h0.clone()
     got = torch.cat([ops.factored_lstm_layer_i8(x[t:t + 1], xs.view(T, B)[t], *args, c1, h1) for t in range(T)])
     assert torch.equal(got, want) and torch.equal(c1, c) and torch.equal(h1, h)
+
+
+@pytest.mark.parametrize("B", [120, 121, 127, 135, 136, 151, 166, 180, 181, 211, 226, 240, 241])
+@pytest.mark.parametrize("T", [1, 2, 3, 9])
+def test_rows_projected_by_pair_give_the_bytes_of_the_l2_form(flib, B, T):
+    """H = 1024, around and within the 9 to 16 rows per cluster (15 clusters on a B200) that are projected by pairs of CTAs: one to four rows
+    per pair, pairs and quarters without rows in the last cluster. Against the L2-exchange form. Exact."""
+    H = 1024
+    layer, x, xs = _layer_case(T, B, H, 128, B + T, B % 2 == 1)
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, h = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale,
+                                         layer.w_up, layer.bias, c, h, reverse=layer.reverse)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, h))
+    flib.fluke_set_lstm_persistent(1)
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
