@@ -837,7 +837,7 @@ def run_ours(args):
                     "chunks_per_launch": batches * B,
                     "traffic": None if tr is None else tr["dram_read_bytes_per_step"] * T + float(T) * batches * B * H,
                     "traffic_source": None if tr is None else
-                    f"profiles/lstm_recurrence_traffic.json: {tr['dram_read_bytes_per_step']:.0f} B read per step (ncu, T={tr['T_captured']}) "
+                    f"profiles/lstm_recurrence_traffic.json, {tr['config']}: {tr['dram_read_bytes_per_step']:.0f} B read per step (ncu, T={tr['T_captured']}) "
                     "x T, plus the h_out the launch writes (larger than L2)",
                     "flops_per_launch": batches * flops,
                     "us_per_launch": {"layer_total": round(us_layer, 3), "x_down_gemm": round(us_xdown, 3), kname: round(us_k, 3)},

@@ -35,16 +35,19 @@
 // sends hh_{t+1} after every CTA's projection of h_t, i.e. after every CTA's contraction of step t. GATHER: a
 // CTA sends h_t after it has received h_{t-1} of every CTA, which each sent after its projection of h_{t-2}: two
 // slots of hidden rows. By pair: a CTA sends h_t after its contraction of step t, which needs hh_t of every pair, sent after its
-// projection of h_{t-1}; and hh the other way round. The final hidden state goes where the initial one was read: of a CTA's own units only (SPLIT), or after
-// every CTA's initial rows have landed (GATHER, before the first cluster barrier). Nobody leaves before the final cluster barrier. Clusters never wait for one
-// another, so any number of them may run in waves.
+// projection of h_{t-1}; and hh the other way round. The final hidden state goes where the initial one was read: of a CTA's
+// own units only (SPLIT), or after every CTA's initial rows have landed (GATHER, before the first cluster barrier).
+// Nobody leaves before the final cluster barrier. Clusters never wait for one another, so any number of them may run in waves.
 //
-// What bounds a step (B200, H = 768, cycles). 2 rows per cluster, 2100: the chain of exchange (490 from the first
-// store to the last arrival), projection 500, its conversion 220, hh half 460, cell update and staging 450. 14 rows, 2900: the
-// same with 950 for the cell updates and 600 for the exchange. 47 rows, 4700: tensor pipe (x part 1540, hh half 1460,
-// projections 370), idle from the end of a step's contractions to the first group's codes (700: 24 rows x 128 units of
-// cell updates, beside the other group's) and while the partial sums travel. The cell updates live on few instructions:
-// with places in the swizzle worked out per row instead of by one exclusive or, 1024 chunks took 2.89 us, 700 2.13.
+// What bounds a step (B200, H = 768; cycles of one CTA by clock stamps, which add up to its period and lengthen it by 2 to 4 %). 2 rows
+// per cluster, 2210: the chain of projection 530, its conversion 240, hh half 470, cell update and staging 500, exchange
+// 470. 14 rows, 2930: 530, 390, 450, 1050 (the cell updates) and 510. 47 rows, 4740: first group's projection 440, its partial
+// sums on the way 860, their sum and the way back 1480, contraction 730, cell updates 930 (24 rows, eight warps), 300 until the issuer has
+// seen the last warp's codes; the second group's chain runs beside it, and the tensor pipe works 3370 of them (x part 1540,
+// hh half 1460, projections 370). Without stamps most clusters take 4600 cycles, the slowest of 22 4780, and the layer ends with those:
+// 2.60 us per step at the 1.83 GHz that the nanosecond timer gives inside the kernel (the driver reports 1965 MHz meanwhile).
+// The cell updates live on few instructions: with places in the swizzle worked out per row instead of by one exclusive or,
+// 1024 chunks took 2.89 us, 700 2.13.
 //
 // The operand rows that are zero (see group_form) add zero times a weight to another group's or step's accumulators: with
 // finite weights nothing. A CTA whose recurrent gate weights are not all finite (0 x inf is NaN) issues other MMAs, see
@@ -93,7 +96,11 @@ struct GroupDev {
 // kernel of one and two groups that exchanged hidden rows between pairs of CTAs and projected them there, against
 // these, in us, x_down included: H = 768 32 chunks (2 rows per cluster) 1.45 : 1.15, 170 (8 rows) 1.56 : 1.34, 300 (14 rows) 1.66 :
 // 1.61, 500 (23 rows) 2.40 : 1.96, 700 (32 rows) 2.62 : 2.04, 1024 (47 rows) 2.97 : 2.75; H = 384, 32 chunks (2 rows) 1.37 : 1.08;
-// H = 1024, where it took two waves from 577 chunks on, 700 (39 rows) 4.85 : 2.86.
+// H = 1024, where it took two waves from 577 chunks on, 700 (47 rows) 4.85 : 2.86. The limits are the same for every cluster size. Layers of
+// 400 steps at 32 numbers of chunks per size, that kernel against these: H = 256 594 chunks 1.48 : 1.45, 1122 1.73 : 1.54; H = 384 387 1.55 :
+// 1.48, 731 2.29 : 2.02; H = 512 288 1.52 : 1.49, 544 2.09 : 2.00; H = 640 234 1.57 : 1.54, 442 2.18 : 2.00, 858 2.87 : 2.75; H = 896 153 1.72 :
+// 1.67, 289 2.38 : 2.04, 561 3.06 : 2.67. Slower only with 48-row kernels of small clusters: H = 256 2376 chunks 2.69 : 2.75, H = 512
+// 1472 2.91 : 2.97, which no smaller form holds in one wave.
 // Everything below depends on the form V and the cluster size C = H / 128, which the kernel is compiled
 // for: with operand addresses at fixed distances the issuer needs few instructions between MMAs.
 constexpr int kGForms = 4;
@@ -418,8 +425,10 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         constexpr int kFirstX = kTwoSteps ? 10 : kByPair ? 16 : kGather ? 24 : 2;
         if constexpr (kGather) {
             // Most of the x part while the hidden state is computed and travels, the rest while the
-            // projection is converted. 300 chunks, 20 / 24 / 28 of 32 in front: 1.63 / 1.60 / 1.63 us per step; 32 chunks, 8 / 10 /
-            // 12 of 16: 1.18 / 1.18 / 1.22.
+            // projection is converted. 20 / 24 / 28 of 32 in front, us per step (x_down included): H = 768 200 chunks 1.62 / 1.57 / 1.64, 300
+            // 1.74 / 1.70 / 1.73; H = 384 600 1.58 / 1.54 / 1.63; H = 512 500 1.68 / 1.62 / 1.65; H = 896 180 1.71 / 1.70 / 1.74. 8 / 10 / 12 of 16: H = 768
+            // 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 384 200 1.19 / 1.19 / 1.20; H = 1024 60 1.42 / 1.40 / 1.44. By pair 12 / 16 /
+            // 20 of 32: 135 chunks 1.68 / 1.66 / 1.73, 240 1.86 / 1.87 / 1.88.
             if (!wait_x(kTwoSteps ? i + 1 : i) || !wait_acc()) break;
             FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
             // Two steps per MMA: the zero rows of the step before have spoilt the accumulators of this step's gates that its x MMAs
@@ -433,9 +442,11 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         } else {
             // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
             // what has long been there takes 100 cycles and more while the gate warps keep the units of the SM busy that
-            // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step).
-            // MMAs in front of the second projection, 1024 chunks: 2 2.71-2.76, 4 2.74-2.78, 8 2.79; 700 chunks 2.04, 2.04-2.08,
-            // 2.12. Four in front of the first as well 3.07-3.16 and 2.24-2.33.
+            // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step when it was done).
+            // 0 / 2 / 4 / 8 MMAs in front of the second projection, us per step (x_down included): H = 768 500 chunks 2.09 / 2.05 / 2.03 / 2.07,
+            // 700 2.14 / 2.13 / 2.13 / 2.22, 900 2.76 / 2.76 / 2.77 / 2.83, 1024 2.93 / 2.93 / 2.96 / 2.94; H = 384 900 2.07 / 2.04 / 2.05 / 2.06, 1500
+            // 2.71 / 2.71 / 2.71 / 2.71; H = 1024 300 2.17 / 2.16 / 2.16 / 2.18, 700 2.90 / 2.91 / 2.92 / 2.98. Four in front of the first as well
+            // took 0.3 us more.
             if (!wait_x(i) || !wait_sent(both ? 2 * i : i)) break;
             if (!project(Int<0>{}, i)) break;
             if (!wait_acc()) break;
