@@ -592,16 +592,20 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(dn_row) * H + (kGather ? 0 : n0));
 #pragma unroll 1
         for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
-        const __half2 sum = __hadd2(zeros[0], zeros[1]);
-        non_finite = __hisnan(__low2half(sum)) || __hisnan(__high2half(sum));
+        if constexpr (K::kZeroRows) {
+            const __half2 sum = __hadd2(zeros[0], zeros[1]);
+            non_finite = __hisnan(__low2half(sum)) || __hisnan(__high2half(sum));
+        }
         tmem_st_wait();
         tc_fence_before_sync();
     }
-    const bool finite = !__syncthreads_or(non_finite);
+    bool finite = true;
+    if constexpr (K::kZeroRows) finite = !__syncthreads_or(non_finite);
+    else __syncthreads();
     tc_fence_after_sync();
     // GATHER: a CTA loads the initial hidden rows of its peers' units too, and a layer of one step stores the final ones, of its
-    // own units and to the same place, without having heard from them: nobody passes the barrier before they have landed.
-    if (kGather) mbar_wait(bar_once, 0, abort_flag, 97);
+    // own units and to the same place, without having heard from them: no CTA passes the barrier before they have landed.
+    if (kGather && warp < 2) mbar_wait(bar_once, 0, abort_flag, 97);
     // every barrier of the cluster is initialised before any CTA may store to a peer
     cluster_sync_all();
 
