@@ -496,11 +496,11 @@ def test_small_cluster_form_of_few_rows_and_of_two_groups_gives_the_bytes_of_the
         assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("H,B", [(768, 44), (768, 150), (768, 300), (768, 700), (768, 1000), (1024, 100), (1024, 700), (256, 400)])
+@pytest.mark.parametrize("H,B", [(768, 44), (768, 150), (768, 300), (768, 700), (768, 727), (768, 1000), (1024, 100), (1024, 700), (256, 400)])
 def test_infinite_gate_weights_reach_their_own_unit_and_row_only(flib, H, B):
     """An infinite weight makes a pre-activation infinite, so the gate saturates (NaN only where the row's own factor is zero or
     two infinities meet), whatever the other rows of the cluster are. Every number of rows per cluster from which the small-cluster
-    form has another kernel, weights of all four gates and both halves, against the L2-exchange form, which multiplies
+    form has another kernel (727: nothing in the last cluster's second group), weights of all four gates and both halves, against the L2-exchange form, which multiplies
     every weight by the row's own values alone: the same bytes, NaN at the same places."""
     T, R = 7, 128
     layer, x, xs = _layer_case(T, B, H, R, H + B, False)
