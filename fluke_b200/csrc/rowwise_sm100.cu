@@ -75,6 +75,15 @@ __device__ __forceinline__ void e4m3x4_decode(uint32_t word, float2 &lo, float2 
     hi = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
 }
 
+// The same with the instruction's own results for those: NaN and -0.
+__device__ __forceinline__ void e4m3x4_to_float(uint32_t word, float2 &lo, float2 &hi) {
+    uint32_t h01, h23;
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h01) : "h"(uint16_t(word & 0xFFFFu)));
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h23) : "h"(uint16_t(word >> 16)));
+    lo = __half22float2(*reinterpret_cast<const __half2 *>(&h01));
+    hi = __half22float2(*reinterpret_cast<const __half2 *>(&h23));
+}
+
 // Two values at once with the conversion instruction. The instruction rounds to nearest even,
 // the software encoder above (the reference's) rounds half away from zero: setting the lowest
 // mantissa bit of the f32 input moves an exact tie (an even bit pattern, whatever the exponent)
@@ -111,6 +120,32 @@ __device__ __forceinline__ float2 div_by_scale2(float2 x, float s, float r) {
                        __uint_as_float((__float_as_uint(q.y) & 0x7FFFFFFFu) | (__float_as_uint(x.y) & 0x80000000u)));
 }
 
+// Sixteen quotients v / s as e4m3 codes (round half away, as the software encoder) without dividing: with r within two units
+// in the last place (u = 2^-24) of 1 / s, the products v * r(1 -+ 16 u) lie on either side of the f32 quotient and strictly so, since what is
+// rounded on the way adds up to less than 8 u. Where both convert to the same code no tie of the conversion lies between
+// them, nor at the quotient. Returns whether that holds for all sixteen (some 1 - 3e-4 of random ones; v finite). For
+// values that are not the caller divides.
+__device__ __forceinline__ bool e4m3_quotients16(const float2 (&v)[8], float r, uint4 &codes) {
+    const float lo = __fmul_rn(r, 1.0f - 0x1p-20f), hi = __fmul_rn(r, 1.0f + 0x1p-20f);
+    uint32_t c[4], differ = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        uint32_t w[2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const float2 f = make_float2(b ? hi : lo, b ? hi : lo), p0 = mul2(v[2 * j], f), p1 = mul2(v[2 * j + 1], f);
+            uint16_t h0, h1;
+            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(h0) : "f"(p0.y), "f"(p0.x));
+            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(h1) : "f"(p1.y), "f"(p1.x));
+            w[b] = uint32_t(h0) | (uint32_t(h1) << 16);
+        }
+        differ |= w[0] ^ w[1];
+        c[j] = w[0];
+    }
+    codes = make_uint4(c[0], c[1], c[2], c[3]);
+    return differ == 0;
+}
+
 // ---- launching ----------------------------------------------------------------------------
 // Every kernel here is launched as a dependent of the one before it and starts with
 // dependency_wait(). None calls dependency_trigger(): with thousands of short-lived CTAs the next
@@ -140,6 +175,12 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
     return v;
+}
+// The largest of three, NaN if any of them is.
+__device__ __forceinline__ float max_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
 }
 __device__ __forceinline__ int clamp127(int v) { return max(-127, min(127, v)); }
 
@@ -451,15 +492,15 @@ __device__ __forceinline__ uint4 int8_codes16(const float2 (&v)[8], float scale)
 }
 
 // ---- RMSNorm family, hidden_dim = 512, 32-byte aligned rows: one warp per row, sixteen consecutive
-// elements per lane (256-bit accesses). Same bits as rmsnorm_rows_kernel.
-template <int MODE>
-__global__ void __launch_bounds__(kNormWarps * 32, 16)
-rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
-                      int n_tokens, float alpha, float eps) {
-    dependency_wait();
-    const int lane = threadIdx.x & 31;
-    const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
-    if (row >= n_tokens) return;
+// elements per lane (256-bit accesses). Same bits as rmsnorm_rows_kernel. The e4m3 form is bound by its instructions: 32 of them per
+// lane and row went into dividing (now two products and two conversions per pair of values, e4m3_quotients16) and
+// as many into clearing codes in the residual; without both 128000 rows take 50.2 us instead of 58.8, 32000 13.5 instead of 14.7.
+// EXACT = false (e4m3 only) returns false, with nothing written, for a row that has a residual code or result that is
+// not finite: the decoding instruction gives NaN for the NaN codes where the reference's gives 0, which makes every result
+// of the row NaN, and quotients of such values are left to the division.
+template <int MODE, bool EXACT>
+__device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
+                                               int64_t row, int lane, float alpha, float eps) {
     const int64_t off = row * 512 + lane * 16;
 
     float2 val[8];
@@ -481,13 +522,19 @@ rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *w
                 if constexpr (MODE == kOutI8) {
                     ra = i8_pair_to_float(words[j] ^ 0x80808080u, 0x7440u, 0x7441u);
                     rb = i8_pair_to_float(words[j] ^ 0x80808080u, 0x7442u, 0x7443u);
-                } else {
+                } else if constexpr (EXACT) {
                     e4m3x4_decode(words[j], ra, rb);
+                } else {
+                    e4m3x4_to_float(words[j], ra, rb);
                 }
                 // x + (r * rs) * alpha: product, then one fused multiply-add (the form the reference's
-                // build contracts to)
-                val[2 * j] = fma2(mul2(ra, make_float2(rs, rs)), make_float2(alpha, alpha), half2_bits_to_float2(x[2 * j]));
-                val[2 * j + 1] = fma2(mul2(rb, make_float2(rs, rs)), make_float2(alpha, alpha), half2_bits_to_float2(x[2 * j + 1]));
+                // build contracts to). The code of -0 is +0 there: added to +0 its product is too.
+                auto scaled = [&](float2 r) {
+                    const float2 rs2 = make_float2(rs, rs);
+                    return MODE == kOutF8 && !EXACT ? fma2(r, rs2, make_float2(0.f, 0.f)) : mul2(r, rs2);
+                };
+                val[2 * j] = fma2(scaled(ra), make_float2(alpha, alpha), half2_bits_to_float2(x[2 * j]));
+                val[2 * j + 1] = fma2(scaled(rb), make_float2(alpha, alpha), half2_bits_to_float2(x[2 * j + 1]));
             }
         }
     }
@@ -509,16 +556,18 @@ rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *w
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         val[k] = mul2(mul2(val[k], make_float2(rms_inv, rms_inv)), half2_bits_to_float2(w[k]));
-        if constexpr (MODE != kOutF16) amax = fmaxf(amax, fmaxf(fabsf(val[k].x), fabsf(val[k].y)));
+        if constexpr (MODE == kOutF8 && !EXACT) amax = max_nan(amax, fabsf(val[k].x), fabsf(val[k].y));
+        else if constexpr (MODE != kOutF16) amax = fmaxf(amax, fmaxf(fabsf(val[k].x), fabsf(val[k].y)));
     }
     if constexpr (MODE == kOutF16) {
         uint32_t o[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) o[k] = float2_to_half2_bits(val[k]);
         store32(static_cast<__half *>(out) + off, o);
-        return;
+        return true;
     }
     amax = warp_max_nonneg(amax);
+    if (MODE == kOutF8 && !EXACT && !(amax < __int_as_float(0x7F800000))) return false;
     uint4 codes;
     if constexpr (MODE == kOutI8) {
         const float quant_scale = (amax > 0.0f) ? (127.0f / amax) : 1.0f;
@@ -527,22 +576,43 @@ rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *w
         codes = int8_codes16<false>(val, quant_scale);
     } else {
         const float fp8_scale = fmaxf(amax, 1e-12f) / 448.0f;
-        const float fp8_rcp = 1.0f / fp8_scale;
         if (lane == 0) res_scale[row] = fp8_scale;
-        uint32_t c[4];
+        if (EXACT || !e4m3_quotients16(val, __fdividef(1.0f, fp8_scale), codes)) {
+            const float fp8_rcp = 1.0f / fp8_scale;
+            uint32_t c[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            uint32_t h[2];
+            for (int j = 0; j < 4; ++j) {
+                uint32_t h[2];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float2 dv = div_by_scale2(val[2 * j + i], fp8_scale, fp8_rcp);
-                h[i] = e4m3_encode_pair(fminf(448.0f, dv.x), fminf(448.0f, dv.y));  // NaN gives 448; the conversion saturates the rest
+                for (int i = 0; i < 2; ++i) {
+                    const float2 dv = div_by_scale2(val[2 * j + i], fp8_scale, fp8_rcp);
+                    h[i] = e4m3_encode_pair(fminf(448.0f, dv.x), fminf(448.0f, dv.y));  // NaN gives 448; the conversion saturates the rest
+                }
+                c[j] = h[0] | (h[1] << 16);
             }
-            c[j] = h[0] | (h[1] << 16);
+            codes = make_uint4(c[0], c[1], c[2], c[3]);
         }
-        codes = make_uint4(c[0], c[1], c[2], c[3]);
     }
     *reinterpret_cast<uint4 *>(static_cast<uint8_t *>(out) + off) = codes;
+    return true;
+}
+
+// Out of line, so that the rows that need it take no registers from the others.
+__device__ __noinline__ void rmsnorm_row512_exact(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
+                                                  int64_t row, int lane, float alpha, float eps) {
+    rmsnorm_row512<kOutF8, true>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kNormWarps * 32, 16)
+rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
+                      int n_tokens, float alpha, float eps) {
+    dependency_wait();
+    const int lane = threadIdx.x & 31;
+    const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
+    if (row >= n_tokens) return;
+    if (!rmsnorm_row512<MODE, MODE != kOutF8>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps))
+        rmsnorm_row512_exact(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
 }
 
 // ---- RMSNorm family, any even hidden_dim <= 1024: one CTA per row, thread t owns pair t ------

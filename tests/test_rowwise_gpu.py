@@ -315,3 +315,42 @@ def test_wide_elementwise_forms_give_the_bits_of_narrow_ones(rows):
     qkv = torch.randn(n, seq, 3, 8, 64, generator=g, device=DEV).half()
     want = torch.cat([ops.rotary_qkv_(p.clone(), sin, cos, 32) for p in qkv.split(20)])
     assert torch.equal(ops.rotary_qkv_(qkv, sin, cos, 32), want) and torch.equal(qkv, want)
+
+
+@pytest.mark.parametrize("n", [1, 5, 4096])
+def test_fp8_rmsnorm_quotients_at_ties_and_not_finite(n):
+    """The 512-wide e4m3 form decides codes without dividing where it can. Against the dividing form that takes rows off a 32-byte
+    boundary: quotients within units in the last place of the conversion's ties, residual codes of NaN and -0 under an x of -0, values
+    that are infinite or NaN, rows of zeros."""
+    h = 512
+    g = torch.Generator(device=DEV).manual_seed(n)
+    # every tie of the positive codes times powers of two, in f16 exact; the row's largest value fixes the scale
+    codes = torch.arange(0, 0x7E, device=DEV, dtype=torch.int32)
+    exp, man = (codes >> 3), (codes & 7)
+    value = torch.where(exp > 0, (8 + man) * 2.0 ** (exp - 10).float(), man * 2.0 ** -9)
+    ties = (value[1:] + value[:-1]) / 2
+    pick = torch.randint(0, ties.numel(), (n, h), generator=g, device=DEV)
+    x = ties[pick] * torch.where(torch.rand(n, h, generator=g, device=DEV) < 0.5, -1.0, 1.0)
+    x[:, 0] = 448.0
+    x *= 2.0 ** torch.randint(-2, 3, (n, 1), generator=g, device=DEV).float()
+    x = x.half()
+    res = torch.zeros(n, h, dtype=torch.uint8, device=DEV)
+    if n > 1:
+        res[1:] = torch.randint(0, 256, (n - 1, h), generator=g, device=DEV, dtype=torch.uint8)   # NaN and -0 codes among them
+        res[2] &= 0x77
+        x[2::7], res[2::7] = 0.0, 0x80
+        x[2::7, ::3] = -0.0
+        x[3::7, 17] = float("inf")
+        x[4::7, 501] = float("nan")
+        x[4::14, 500] = float("-inf")
+    w = torch.ones(h, device=DEV).half()
+    scale = torch.rand(n, generator=g, device=DEV) * 1e-3
+    got = []
+    for shift in (0, 8):   # elements of the buffer in front of x
+        xb = torch.zeros(n * h + 16, dtype=torch.float16, device=DEV)
+        xs = xb[shift:shift + n * h].view(n, h)
+        xs.copy_(x)
+        q, s = res.clone(), scale.clone()
+        ops.rmsnorm_quant_fp8(xs, w, q, s, 0.5, 1e-5)
+        got.append((q, s))
+    assert same_bits(got[0][0], got[1][0]) and same_bits(got[0][1], got[1][1])
