@@ -38,6 +38,16 @@ inline int device_sm_count() {
     return cached[dev];
 }
 
+// L2 cache of the current device.
+inline int device_l2_bytes() {
+    static int cached[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrL2CacheSize, dev);
+    return cached[dev];
+}
+
 // cuTensorMapEncodeTiled with the options every map of the library shares (no interleave, unit
 // element strides, 256-byte L2 promotion, zero fill). An encoded map depends on nothing but these
 // arguments, so each host thread keeps up to kMapSlots of them, one per value of the hash. A program that calls

@@ -522,3 +522,30 @@ def test_more_columns_than_resident_weight_tiles_are_refused_for_any_number_of_r
     for m in (64, 128, 1024, 3000):
         with pytest.raises(RuntimeError):
             ops.gemm_i8(torch.zeros(m, 128, dtype=torch.int8, device=DEV), b, torch.zeros(m, device=DEV), sb)
+
+
+@pytest.mark.parametrize("kind", ["qkv", "mlp"])
+def test_outputs_larger_than_l2_equal_those_of_parts(kind):
+    """Outputs about as large as L2 are stored under another eviction policy: the bytes are those of the same rows in two calls."""
+    seq = 100
+    n = 1536 if kind == "qkv" else 2048
+    m = (140 << 20) // (2 * n) // (2 * seq) * (2 * seq)
+    g = torch.Generator().manual_seed(7)
+    gd = torch.Generator(device=DEV).manual_seed(7)
+    a = torch.randint(-127, 128, (m, 512), generator=gd, device=DEV, dtype=torch.int8)
+    sa = torch.rand(m, generator=gd, device=DEV) * 0.02 + 1e-3
+    w, sw = prep.quantize_int8_rows(torch.randn(n, 512, generator=g) * 0.02)
+    u, su = prep.quantize_int8_rows(torch.randn(n, 512, generator=g) * 0.02)
+    w, sw, u, su = (t.to(DEV) for t in (w, sw, u, su))
+    sin, cos = prep.rotary_tables(seq, 64, device=DEV)
+    be = ops.int8_select(0)
+
+    def run(lo, hi):
+        if kind == "qkv":
+            return ops.qkv_rotary_i8(be, a[lo:hi], w, sa[lo:hi], sw, sin, cos, seq)
+        return ops.gated_mlp_i8(be, a[lo:hi], w, u, sa[lo:hi], sw, su)
+
+    whole = run(0, m).view(torch.int16)
+    for lo, hi in ((0, m // 2), (m // 2, m)):
+        part = run(lo, hi).view(torch.int16)
+        assert torch.equal(whole[lo:hi].reshape(part.shape), part)
