@@ -51,8 +51,11 @@ def run_stack(layers, x_i8, x_scale, state=None, workspace=None, buffers=None):
     t, b, h = x_i8.shape
     dev = x_i8.device
     if state is None:
-        state = [(torch.zeros(b, h, dtype=torch.float32, device=dev),
-                  torch.zeros(b, h, dtype=torch.int8, device=dev)) for _ in layers]
+        # one fill for all layers, where 16-byte alignment of every part allows it
+        n = len(layers) if (b * h) % 16 == 0 else 1
+        parts = [(torch.zeros(n, b, h, dtype=torch.float32, device=dev), torch.zeros(n, b, h, dtype=torch.int8, device=dev))
+                 for _ in range(len(layers) // max(n, 1))]
+        state = [s for c, hs in parts for s in zip(c, hs)]
     if buffers is None:
         buffers = [torch.empty(t, b, h, dtype=torch.int8, device=dev) for _ in range(2)]
     cur, cur_scale = x_i8, x_scale
