@@ -611,13 +611,14 @@ __device__ __noinline__ void rmsnorm_row512_exact(const __half *in, const void *
     rmsnorm_row512<kOutF8, true>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kNormWarps * 32, 16)
+// CTAs of WARPS rows, CTAS of them per SM, which sets the registers of a thread (WARPS * CTAS * 32 of 2048 threads: 32 at 64 warps).
+template <int MODE, int WARPS, int CTAS>
+__global__ void __launch_bounds__(WARPS * 32, CTAS)
 rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
                       int n_tokens, float alpha, float eps) {
     dependency_wait();
     const int lane = threadIdx.x & 31;
-    const int64_t row = int64_t(blockIdx.x) * kNormWarps + (threadIdx.x >> 5);
+    const int64_t row = int64_t(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (row >= n_tokens) return;
     if (!rmsnorm_row512<MODE, MODE != kOutF8>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps))
         rmsnorm_row512_exact(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
@@ -727,7 +728,16 @@ int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, 
         ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weight) |
           reinterpret_cast<uintptr_t>(residual_in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
     if (hidden_dim == 512 && aligned && aligned32(in, MODE == kOutF16 ? residual_in : nullptr, MODE == kOutF16 ? out : nullptr)) {
-        rc = launch_dependent(rmsnorm_row512_kernel<MODE>, (n_tokens + kNormWarps - 1) / kNormWarps, kNormWarps * 32, 0, s, x, residual_in, w, out, res_scale, n_tokens, alpha, eps);
+        // Sixteen values and their codes do not fit 32 registers: what a thread spills or loads late lengthens its chain, fewer warps
+        // hide less of it. e4m3: 36 warps of 56 registers (us, 64 warps : these; 125 rows 1.87 : 1.49, 1803 2.38 : 2.19, 16000 8.33 : 7.64,
+        // 128000 48.3 : 45.8; with four rows per CTA 47.0). int8: 40 warps of 48 registers while all rows run at once (125 rows 1.89 : 1.62,
+        // 1803 2.32 : 2.14, 5000 3.23 : 3.09), with more of them 64 warps (9331 rows 4.98 : 5.14, 32000 11.9 : 12.9).
+        auto go = [&](auto kernel, int warps) {
+            return launch_dependent(kernel, (n_tokens + warps - 1) / warps, warps * 32, 0, s, x, residual_in, w, out, res_scale, n_tokens, alpha, eps);
+        };
+        if constexpr (MODE == kOutF8) rc = go(rmsnorm_row512_kernel<MODE, 2, 18>, 2);
+        else if (MODE == kOutI8 && n_tokens <= 4 * 10 * device_sm_count()) rc = go(rmsnorm_row512_kernel<MODE, 4, 10>, 4);
+        else rc = go(rmsnorm_row512_kernel<MODE, 4, 16>, 4);
     } else if (hidden_dim % 256 == 0 && aligned) {
         const int grid = (n_tokens + kNormWarps - 1) / kNormWarps;
         const int block = kNormWarps * 32;

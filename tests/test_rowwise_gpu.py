@@ -354,3 +354,22 @@ def test_fp8_rmsnorm_quotients_at_ties_and_not_finite(n):
         ops.rmsnorm_quant_fp8(xs, w, q, s, 0.5, 1e-5)
         got.append((q, s))
     assert same_bits(got[0][0], got[1][0]) and same_bits(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("over", [0, 1, 5])
+def test_int8_rmsnorm_around_one_wave_of_rows(over):
+    """Rows that all run at once take a kernel of more registers: the bits of the rows kernel on either side of the rule."""
+    n = 40 * torch.cuda.get_device_properties(0).multi_processor_count + over
+    g = torch.Generator(device=DEV).manual_seed(over)
+    x = torch.randn(n, 512, generator=g, device=DEV).half()
+    w = (1 + 0.1 * torch.randn(512, generator=g, device=DEV)).half()
+    res = torch.randint(-127, 128, (n, 512), generator=g, device=DEV, dtype=torch.int8)
+    scale = torch.rand(n, generator=g, device=DEV) * 0.02
+    got = []
+    for shift in (0, 8):
+        xs = torch.zeros(n * 512 + 16, dtype=torch.float16, device=DEV)[shift:shift + n * 512].view(n, 512)
+        xs.copy_(x)
+        q, s = res.clone(), scale.clone()
+        ops.rmsnorm_quant_int8(xs, w, q, s, 2.0, 1e-5)
+        got.append((q, s))
+    assert same_bits(got[0][0], got[1][0]) and same_bits(got[0][1], got[1][1])
