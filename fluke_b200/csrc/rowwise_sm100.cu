@@ -210,8 +210,9 @@ __device__ __forceinline__ void load32(const void *p, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "l"(p) : "memory");
 }
-// The same for data that is read for the last time, as the f16 input of a kernel that quantises it: its lines leave L2 first
-// (int8 layer of 7 x 1333 rows 54.6 -> 54.0 us; 32 x 1000 beside the MLP's stores that do, 138.2 -> 135.3).
+// The same for data that is read for the last time, as the f16 input of a kernel that quantises it: its lines leave L2 first. From
+// many rows on (many_rows), layers with plain loads against these, us: 7 x 1333 54.6 : 54.0, 16 x 1000 79.7 : 79.1, 32 x 1000 143.2 : 139.7,
+// 60 x 1000 261.6 : 248.9; with few rows, which L2 holds anyway, they cost 1 % (3 x 601 26.6 : 27.0).
 __device__ __forceinline__ void load32_last_use(const void *p, uint32_t (&r)[8]) {
     asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -505,7 +506,7 @@ __device__ __forceinline__ uint4 int8_codes16(const float2 (&v)[8], float scale)
 // EXACT = false (e4m3 only) returns false, with nothing written, for a row that has a residual code or result that is
 // not finite: the decoding instruction gives NaN for the NaN codes where the reference's gives 0, which makes every result
 // of the row NaN, and quotients of such values are left to the division.
-template <int MODE, bool EXACT>
+template <int MODE, bool EXACT, bool LAST_USE>
 __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
                                                int64_t row, int lane, float alpha, float eps) {
     const int64_t off = row * 512 + lane * 16;
@@ -513,8 +514,8 @@ __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *res
     float2 val[8];
     {
         uint32_t x[8];
-        if (MODE == kOutF16) load32(in + off, x);
-        else load32_last_use(in + off, x);
+        if (LAST_USE) load32_last_use(in + off, x);
+        else load32(in + off, x);
         if constexpr (MODE == kOutF16) {
             uint32_t r[8];
             load32(static_cast<const __half *>(residual_in) + off, r);
@@ -605,14 +606,17 @@ __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *res
     return true;
 }
 
-// Out of line, so that the rows that need it take no registers from the others.
+// Out of line, so that the rows that need it take no registers from the others; one for each kernel (the compiler does not
+// come through with one that two call).
+template <bool LAST_USE>
 __device__ __noinline__ void rmsnorm_row512_exact(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
                                                   int64_t row, int lane, float alpha, float eps) {
-    rmsnorm_row512<kOutF8, true>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
+    rmsnorm_row512<kOutF8, true, false>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
 }
 
 // CTAs of WARPS rows, CTAS of them per SM, which sets the registers of a thread (WARPS * CTAS * 32 of 2048 threads: 32 at 64 warps).
-template <int MODE, int WARPS, int CTAS>
+// LAST_USE: see load32_last_use.
+template <int MODE, int WARPS, int CTAS, bool LAST_USE>
 __global__ void __launch_bounds__(WARPS * 32, CTAS)
 rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
                       int n_tokens, float alpha, float eps) {
@@ -620,8 +624,8 @@ rmsnorm_row512_kernel(const __half *in, const void *residual_in, const __half *w
     const int lane = threadIdx.x & 31;
     const int64_t row = int64_t(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (row >= n_tokens) return;
-    if (!rmsnorm_row512<MODE, MODE != kOutF8>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps))
-        rmsnorm_row512_exact(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
+    if (!rmsnorm_row512<MODE, MODE != kOutF8, LAST_USE>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps))
+        rmsnorm_row512_exact<LAST_USE>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
 }
 
 // ---- RMSNorm family, any even hidden_dim <= 1024: one CTA per row, thread t owns pair t ------
@@ -717,6 +721,9 @@ __global__ void rmsnorm_generic_kernel(const __half * in, const void *residual_i
     }
 }
 
+// More rows than 40 warps on every SM hold at once.
+inline bool many_rows(int n_tokens) { return n_tokens > 40 * device_sm_count(); }
+
 template <int MODE>
 int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, void *out,
                    float *res_scale, int n_tokens, int hidden_dim, float alpha, float eps,
@@ -735,9 +742,9 @@ int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, 
         auto go = [&](auto kernel, int warps) {
             return launch_dependent(kernel, (n_tokens + warps - 1) / warps, warps * 32, 0, s, x, residual_in, w, out, res_scale, n_tokens, alpha, eps);
         };
-        if constexpr (MODE == kOutF8) rc = go(rmsnorm_row512_kernel<MODE, 2, 18>, 2);
-        else if (MODE == kOutI8 && n_tokens <= 4 * 10 * device_sm_count()) rc = go(rmsnorm_row512_kernel<MODE, 4, 10>, 4);
-        else rc = go(rmsnorm_row512_kernel<MODE, 4, 16>, 4);
+        if constexpr (MODE == kOutF8) rc = many_rows(n_tokens) ? go(rmsnorm_row512_kernel<MODE, 2, 18, true>, 2) : go(rmsnorm_row512_kernel<MODE, 2, 18, false>, 2);
+        else if constexpr (MODE == kOutI8) rc = many_rows(n_tokens) ? go(rmsnorm_row512_kernel<MODE, 4, 16, true>, 4) : go(rmsnorm_row512_kernel<MODE, 4, 10, false>, 4);
+        else rc = go(rmsnorm_row512_kernel<MODE, 4, 16, false>, 4);
     } else if (hidden_dim % 256 == 0 && aligned) {
         const int grid = (n_tokens + kNormWarps - 1) / kNormWarps;
         const int block = kNormWarps * 32;
@@ -810,7 +817,7 @@ quant_rows_reg_kernel(const __half * in, uint8_t * out,
 }
 
 // The same for hidden_dim = 512 and 32-byte aligned rows: sixteen consecutive elements per lane.
-template <bool FP8>
+template <bool FP8, bool LAST_USE>
 __global__ void __launch_bounds__(kNormWarps * 32, 16)
 quant_row512_kernel(const __half *in, uint8_t *out, float *scale, int n_tokens) {
     dependency_wait();
@@ -819,7 +826,8 @@ quant_row512_kernel(const __half *in, uint8_t *out, float *scale, int n_tokens) 
     if (row >= n_tokens) return;
     const int64_t off = row * 512 + lane * 16;
     uint32_t x[8];
-    load32_last_use(in + off, x);
+    if (LAST_USE) load32_last_use(in + off, x);
+    else load32(in + off, x);
     float2 val[8];
     float amax = 0.f;
 #pragma unroll
@@ -1220,7 +1228,9 @@ static int launch_quant(const void *in, void *out, void *scale, int n_tokens, in
                        ((reinterpret_cast<uintptr_t>(in) & 15u) == 0) &&
                        ((reinterpret_cast<uintptr_t>(out) & 7u) == 0);
     if (vec_ok && hidden_dim == 512 && aligned32(in) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
-        auto kernel = fp8 ? quant_row512_kernel<true> : quant_row512_kernel<false>;
+        const bool many = many_rows(n_tokens);
+        auto kernel = fp8 ? (many ? quant_row512_kernel<true, true> : quant_row512_kernel<true, false>)
+                          : (many ? quant_row512_kernel<false, true> : quant_row512_kernel<false, false>);
         return launch_dependent(kernel, (n_tokens + kNormWarps - 1) / kNormWarps, kNormWarps * 32, 0, s, static_cast<const __half *>(in),
                                 static_cast<uint8_t *>(out), static_cast<float *>(scale), n_tokens);
     }
