@@ -76,7 +76,7 @@ constexpr int kGTmemCols = 512;
 constexpr int kGTmemW = 256;       // first column of the hh half of the gate weights: 4 gates x 64
 constexpr int kGWxBytes = 4 * kGUnits * 256;  // x half of the gate weights in shared memory
 constexpr int kGMaxSmem = 232448;
-constexpr int kGBars = 24;         // mbarriers of a CTA
+constexpr int kGBars = 32;         // mbarriers of a CTA
 
 struct GroupDev {
     int T, B;
@@ -238,7 +238,7 @@ struct GroupConst {
 };
 // mbarriers of a CTA, as indices
 enum : int {
-    kBarOnce = 0,      // resident weights and the initial hidden rows loaded
+    kBarOnce = 0,      // x half of the gate weights loaded
     kBarX = 1,         // [slots] x_down rows landed
     kBarXFree = 5,     // [slots] the x part of the contraction has read them
     kBarAccFree = 9,   // the gate warps have read all accumulators
@@ -249,7 +249,10 @@ enum : int {
     kBarSum = 18,      // SPLIT [G]: partial sums of the CTA's own pieces arrived
     kBarSent = 20,     // SPLIT: the projection accumulator has been read
     kBarStored = 21,   // SPLIT: the TMA stores have read the hidden codes
-    kBarH = 16         // GATHER [2], by pair [1]: hidden rows of all CTAs arrived
+    kBarStart = 22,    // resident projection weights and the initial hidden rows loaded
+    kBarH = 16,        // GATHER [2], by pair [1]: hidden rows of all CTAs arrived
+    kBarW = 24,        // set-up [4]: recurrent weights of a gate landed in shared memory
+    kBarWRead = 28     // set-up [4]: and have been read from there
 };
 
 // The MMA issuer, warp 1. The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
@@ -278,7 +281,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     uint64_t d_hh = make_smem_desc_sw128(smem_u32(smem + L.hh));
     uint64_t d_dn = make_smem_desc_sw128(smem_u32(smem + L.dn));
     uint64_t d_h0 = make_smem_desc_sw128(smem_u32(smem + L.h));
-    bool ok = mbar_wait(bar_once, 0, abort_flag, 97);
+    bool ok = mbar_wait(bars + kBarStart, 0, abort_flag, 97) && mbar_wait(bar_once, 0, abort_flag, 97);
     int i = 0;
     // MMAs [from, to) of the x part of a step. They read their A operand from shared memory (42 cycles
     // each, 48 with 48 columns) and the tensor pipe works in order, so they are issued in pieces for the times when it
@@ -525,6 +528,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     if (threadIdx.x == 0) {
         auto arrivals = [&](int b) {   // warps that arrive, or one arrival with the expected bytes
             if (b == kBarAccFree) return kGather || both ? kGEpiWarps : kGEpiWarps / 2;
+            if (b >= kBarWRead) return 4;
             if (kGather) return !kByPair && b == kBarHh ? kGEpiWarps : 1;
             return b == kBarCode || b == kBarCode + 1 || b == kBarSent ? kGEpiWarps / 2 : 1;
         };
@@ -555,43 +559,58 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    uint64_t *bar_w = bars + kBarW, *bar_w_read = bars + kBarWRead, *bar_start = bars + kBarStart;
     if (warp == 0 && elect_one()) {
-        // what stays, and the initial hidden rows, beside the weights that go to tensor memory
+        // The recurrent half of the gate weights comes by way of the places of the x half: read by the threads from global memory,
+        // one row per lane, every load touched 32 lines. Layer of one step, us, x_down included, that against this: H = 384 32 chunks 16.7 : 14.6,
+        // H = 768 300 20.7 : 17.1, 500 18.7 : 15.1, 1024 19.5 : 16.6, H = 1024 200 20.6 : 16.6.
+        for (int g = 0; g < 4; ++g) {
+            mbar_arrive_expect_tx(&bar_w[g], 32768);
+            for (int kb = 0; kb < 2; ++kb) tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, &bar_w[g], kb * 64, g * H + n0);
+        }
+        // what stays, and the initial hidden rows
         constexpr int kDnTile = K::kDnRows * 128, kDnTiles = (L.h - L.dn) / kDnTile;   // the last K blocks
-        mbar_arrive_expect_tx(bar_once, kGWxBytes + kDnTiles * kDnTile + (kGather ? C : G) * kTile);
-        for (int g = 0; g < 4; ++g)
-            for (int kb = 0; kb < 2; ++kb)
-                tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
+        mbar_arrive_expect_tx(bar_once, kGWxBytes);
+        mbar_arrive_expect_tx(bar_start, kDnTiles * kDnTile + (kGather ? C : G) * kTile);
         for (int b = 0; b < kDnTiles; ++b)
-            tma_load_2d(smem + L.dn + b * kDnTile, &tm_dn, bar_once, kGather ? (kDnTs / 4 + b) * kGUnits : n0, kByPair ? half * 64 : 0);
+            tma_load_2d(smem + L.dn + b * kDnTile, &tm_dn, bar_start, kGather ? (kDnTs / 4 + b) * kGUnits : n0, kByPair ? half * 64 : 0);
         // step 0 projects the layer's initial hidden state
         for (int e = 0; e < G; ++e)
-            tma_load_3d(smem + L.h + (kByPair ? 0 : kGather ? C : e) * kTile, &tm_h0, bar_once, 0,
+            tma_load_3d(smem + L.h + (kByPair ? 0 : kGather ? C : e) * kTile, &tm_h0, bar_start, 0,
                         kByPair ? m0 + pair * per_pair : m0 + F.rows * e, kGather ? 0 : rank);
+        for (int g = 0; g < 4; ++g) {
+            if (!mbar_wait(&bar_w_read[g], 0, abort_flag, 108)) break;
+            for (int kb = 0; kb < 2; ++kb)
+                tma_load_2d(smem + (g * 2 + kb) * 16384, &tm_w, bar_once, kGRank + kb * 64, g * H + n0);
+        }
     }
     bool non_finite = false;   // one of the recurrent gate weights
     if (warp >= 2) {
-        // the hh half of the gate weights: warp = (lane quadrant, gate), thread = row of the block
+        // warp = (lane quadrant, gate), thread = row of the block: first projection weights, then the hh half of the gate weights
         const int q = warp & 3, g = (warp - 2) >> 2;
-        const uint4 *src = reinterpret_cast<const uint4 *>(
-            p.w_up + (size_t(g) * H + n0 + q * 32 + lane) * (2 * kGRank));
         const uint32_t t_lane = tmem + (uint32_t(q * 32) << 16);
-        __half2 zeros[2] = {__half2half2(__ushort_as_half(0)), __half2half2(__ushort_as_half(0))};
-#pragma unroll 1
-        for (int v = 0; v < 8; ++v) {
-            const uint4 lo = __ldg(src + 2 * v), hi = __ldg(src + 2 * v + 1);
-            tmem_st_32x8(t_lane + kGTmemW + g * 64 + v * 8, lo, hi);
-            if (K::kZeroRows) {
-                add_zero_times(zeros[0], lo);
-                add_zero_times(zeros[1], hi);
-            }
-        }
-        // and K steps g, g + 4, .. of the projection rows, of all units or this CTA's
+        // K steps g, g + 4, .. of the projection rows, of all units or this CTA's
         // (M = 64: row 16 q + i in lane 32 q + i)
         const int dn_row = kByPair ? half * 64 + q * 16 + (lane & 15) : q * 32 + lane;
         const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(dn_row) * H + (kGather ? 0 : n0));
 #pragma unroll 1
         for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
+        __half2 zeros[2] = {__half2half2(__ushort_as_half(0)), __half2half2(__ushort_as_half(0))};
+        if (__all_sync(0xffffffffu, mbar_wait(&bar_w[g], 0, abort_flag, 109))) {
+            const uint32_t row = smem_u32(smem) + g * 32768 + (q * 32 + lane) * 128;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                const uint32_t at = row + (v >> 2) * 16384;
+                const uint4 lo = lds128(at + (((2 * (v & 3)) ^ (lane & 7)) << 4)), hi = lds128(at + (((2 * (v & 3) + 1) ^ (lane & 7)) << 4));
+                tmem_st_32x8(t_lane + kGTmemW + g * 64 + v * 8, lo, hi);
+                if (K::kZeroRows) {
+                    add_zero_times(zeros[0], lo);
+                    add_zero_times(zeros[1], hi);
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_w_read[g]);
         if constexpr (K::kZeroRows) {
             const __half2 sum = __hadd2(zeros[0], zeros[1]);
             non_finite = __hisnan(__low2half(sum)) || __hisnan(__high2half(sum));
@@ -605,7 +624,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     tc_fence_after_sync();
     // GATHER: a CTA loads the initial hidden rows of its peers' units too, and a layer of one step stores the final ones, of its
     // own units and to the same place, without having heard from them: no CTA passes the barrier before they have landed.
-    if (kGather && warp < 2) mbar_wait(bar_once, 0, abort_flag, 97);
+    if (kGather && warp < 2) mbar_wait(bar_start, 0, abort_flag, 97);
     // every barrier of the cluster is initialised before any CTA may store to a peer
     cluster_sync_all();
 
