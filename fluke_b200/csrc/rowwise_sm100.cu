@@ -614,7 +614,7 @@ __device__ __noinline__ void rmsnorm_row512_exact(const __half *in, const void *
     rmsnorm_row512<kOutF8, true, false>(in, residual_in, weight, out, res_scale, row, lane, alpha, eps);
 }
 
-// CTAs of WARPS rows, CTAS of them per SM, which sets the registers of a thread (WARPS * CTAS * 32 of 2048 threads: 32 at 64 warps).
+// CTAs of WARPS rows, at least CTAS of them per SM, which bounds the registers of a thread (32 at 64 warps, 56 at 36).
 // LAST_USE: see load32_last_use.
 template <int MODE, int WARPS, int CTAS, bool LAST_USE>
 __global__ void __launch_bounds__(WARPS * 32, CTAS)
@@ -736,7 +736,7 @@ int launch_rmsnorm(const void *in, const void *residual_in, const void *weight, 
           reinterpret_cast<uintptr_t>(residual_in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
     if (hidden_dim == 512 && aligned && aligned32(in, MODE == kOutF16 ? residual_in : nullptr, MODE == kOutF16 ? out : nullptr)) {
         // Sixteen values and their codes do not fit 32 registers: what a thread spills or loads late lengthens its chain, fewer warps
-        // hide less of it. e4m3: 36 warps of 56 registers (us, 64 warps : these; 125 rows 1.87 : 1.49, 1803 2.38 : 2.19, 16000 8.33 : 7.64,
+        // hide less of it. e4m3: compiled for 36 warps, 48 registers (us, 64 warps : these; 125 rows 1.87 : 1.49, 1803 2.38 : 2.19, 16000 8.33 : 7.64,
         // 128000 48.3 : 45.8; with four rows per CTA 47.0). int8: 40 warps of 48 registers while all rows run at once (125 rows 1.89 : 1.62,
         // 1803 2.32 : 2.14, 5000 3.23 : 3.09), with more of them 64 warps (9331 rows 4.98 : 5.14, 32000 11.9 : 12.9).
         auto go = [&](auto kernel, int warps) {
