@@ -503,8 +503,8 @@ __device__ __forceinline__ uint4 int8_codes16(const float2 (&v)[8], float scale)
 // elements per lane (256-bit accesses). Same bits as rmsnorm_rows_kernel. The e4m3 form is bound by its instructions: 32 of them per
 // lane and row went into dividing (now two products and two conversions per pair of values, e4m3_quotients16) and
 // as many into clearing codes in the residual; without both 128000 rows take 50.2 us instead of 58.8, 32000 13.5 instead of 14.7.
-// EXACT = false (e4m3 only) returns false, with nothing written, for a row that has a residual code or result that is
-// not finite: the decoding instruction gives NaN for the NaN codes where the reference's gives 0, which makes every result
+// EXACT = false (e4m3 only) returns false, with nothing written, for a row whose scale is not positive (the sign of zeros) or
+// that has a residual code or result that is not finite: the decoding instruction gives NaN for the NaN codes where the reference's gives 0, which makes every result
 // of the row NaN, and quotients of such values are left to the division.
 template <int MODE, bool EXACT, bool LAST_USE>
 __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
@@ -523,7 +523,8 @@ __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *res
             for (int k = 0; k < 8; ++k) val[k] = fma2(half2_bits_to_float2(r[k]), make_float2(alpha, alpha), half2_bits_to_float2(x[k]));
         } else {
             const uint4 raw = load16(static_cast<const uint8_t *>(residual_in) + off);
-            const float rs = res_scale[row];
+            const float stored = res_scale[row];
+            const float rs = MODE != kOutF8 || EXACT || stored > 0.f ? stored : __int_as_float(0x7FC00000);   // makes all results NaN
             const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -537,7 +538,7 @@ __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *res
                     e4m3x4_to_float(words[j], ra, rb);
                 }
                 // x + (r * rs) * alpha: product, then one fused multiply-add (the form the reference's
-                // build contracts to). The code of -0 is +0 there: added to +0 its product is too.
+                // build contracts to). The code of -0 is +0 there: added to +0 its product is too (with rs > 0).
                 auto scaled = [&](float2 r) {
                     const float2 rs2 = make_float2(rs, rs);
                     return MODE == kOutF8 && !EXACT ? fma2(r, rs2, make_float2(0.f, 0.f)) : mul2(r, rs2);

@@ -321,7 +321,7 @@ def test_wide_elementwise_forms_give_the_bits_of_narrow_ones(rows):
 def test_fp8_rmsnorm_quotients_at_ties_and_not_finite(n):
     """The 512-wide e4m3 form decides codes without dividing where it can. Against the dividing form that takes rows off a 32-byte
     boundary: quotients within units in the last place of the conversion's ties, residual codes of NaN and -0 under an x of -0, values
-    that are infinite or NaN, rows of zeros."""
+    that are infinite or NaN, rows of zeros, scales that are not positive."""
     h = 512
     g = torch.Generator(device=DEV).manual_seed(n)
     # every tie of the positive codes times powers of two, in f16 exact; the row's largest value fixes the scale
@@ -345,6 +345,9 @@ def test_fp8_rmsnorm_quotients_at_ties_and_not_finite(n):
         x[4::14, 500] = float("-inf")
     w = torch.ones(h, device=DEV).half()
     scale = torch.rand(n, generator=g, device=DEV) * 1e-3
+    if n > 1:   # scales that no kernel writes, under zeros of x of either sign
+        x[1::9, ::2] = -0.0
+        scale[1::9] = torch.tensor([0.0, -0.0, -1e-3, float("nan"), float("inf")], device=DEV).repeat(n)[:scale[1::9].numel()]
     got = []
     for shift in (0, 8):   # elements of the buffer in front of x
         xb = torch.zeros(n * h + 16, dtype=torch.float16, device=DEV)
