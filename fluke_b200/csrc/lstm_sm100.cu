@@ -371,7 +371,7 @@ extern "C" int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, 
         g.a = l->x_i8; g.b = l->dn_ih_i8; g.out = x_down; g.ld_out = R;
         g.scale_a = static_cast<const float *>(l->x_scale); g.const_scale_a = kHScale;
         g.scale_b = static_cast<const float *>(l->dn_ih_scale);
-        rc = launch<kKindI8, FLUKE_SM100_EPI_DEQUANT, kPlainBN, kPlainStages>(&g, stream);
+        rc = dispatch<kKindI8>(&g, stream);
         if (rc) return rc;
     }
 
