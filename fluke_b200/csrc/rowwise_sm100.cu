@@ -1031,6 +1031,46 @@ __device__ __forceinline__ void split_index(int64_t idx, int64_t total, int per_
 }
 
 // ---- SiLU-multiply (nn_kernel_cuda.h:71-90) -----------------------------------------------------
+// g / (1 + exp(-g)) for f16 values g >= -69 without the division's checks: one correction of the product with the approximate
+// reciprocal gives the correctly rounded quotient for every one of them (all 53329 compared with the division; without it 9347 differ);
+// the sign is g's own where the quotient is a zero. The divisions were most of what the kernel
+// issued: [32000, 4096] 67.8 -> 59.0 us (1.02 of the copy bandwidth), 128000 rows 284 -> 242, 2000 6.4 -> 5.3, 125 1.73 -> 1.39.
+__device__ __forceinline__ float2 silu2(float2 g) {
+    const float2 b = make_float2(1.0f + __expf(-g.x), 1.0f + __expf(-g.y));
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(b.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(b.y));
+    float2 q = mul2(g, r);
+    q = fma2(fma2(make_float2(-b.x, -b.y), q, g), r, q);
+    return make_float2(__uint_as_float((__float_as_uint(q.x) & 0x7FFFFFFFu) | (__float_as_uint(g.x) & 0x80000000u)),
+                       __uint_as_float((__float_as_uint(q.y) & 0x7FFFFFFFu) | (__float_as_uint(g.y) & 0x80000000u)));
+}
+__device__ __forceinline__ float2 silu2_any(float2 g) {
+    return make_float2(g.x / (1.0f + __expf(-g.x)), g.y / (1.0f + __expf(-g.y)));
+}
+// Whether silu2 takes all of N pairs: none below -69 or infinite (NaN gives NaN in either).
+template <int N>
+__device__ __forceinline__ bool silu2_takes(const uint32_t (&g)[N]) {
+    __half2 lo = *reinterpret_cast<const __half2 *>(&g[0]), hi = lo;
+#pragma unroll
+    for (int j = 1; j < N; ++j) {
+        lo = __hmin2(lo, *reinterpret_cast<const __half2 *>(&g[j]));
+        hi = __hmax2(hi, *reinterpret_cast<const __half2 *>(&g[j]));
+    }
+    return __hbge2(lo, __float2half2_rn(-69.f)) && __hble2(hi, __float2half2_rn(65504.f));
+}
+// N pairs of outputs from the words of both halves.
+template <int N>
+__device__ __forceinline__ void silu_mul_pairs(const uint32_t (&y)[N], const uint32_t (&g)[N], uint32_t (&o)[N]) {
+    if (silu2_takes(g)) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) o[j] = float2_to_half2_bits(mul2(silu2(half2_bits_to_float2(g[j])), half2_bits_to_float2(y[j])));
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) o[j] = float2_to_half2_bits(mul2(silu2_any(half2_bits_to_float2(g[j])), half2_bits_to_float2(y[j])));
+    }
+}
+
 template <int VEC>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __half * in, __half * out, int64_t total_vec,
@@ -1050,22 +1090,14 @@ silu_mul_kernel(const __half * in, __half * out, int64_t total_vec,
         uint32_t yr[8], gr[8], o8[8];
         load32(y, yr);
         load32(g, gr);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float2 yf = half2_bits_to_float2(yr[j]), gf = half2_bits_to_float2(gr[j]);
-            o8[j] = float2_to_half2_bits(make_float2((gf.x / (1.0f + __expf(-gf.x))) * yf.x, (gf.y / (1.0f + __expf(-gf.y))) * yf.y));
-        }
+        silu_mul_pairs(yr, gr, o8);
         store32(o, o8);
     } else if constexpr (VEC == 8) {
-        float2 yf[4], gf[4], of[4];
-        unpack8(*(reinterpret_cast<const uint4 *>(y)), yf);
-        unpack8(*(reinterpret_cast<const uint4 *>(g)), gf);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            of[j].x = (gf[j].x / (1.0f + __expf(-gf[j].x))) * yf[j].x;
-            of[j].y = (gf[j].y / (1.0f + __expf(-gf[j].y))) * yf[j].y;
-        }
-        *reinterpret_cast<uint4 *>(o) = pack8(of);
+        const uint4 yv = *reinterpret_cast<const uint4 *>(y), gv = *reinterpret_cast<const uint4 *>(g);
+        const uint32_t yr[4] = {yv.x, yv.y, yv.z, yv.w}, gr[4] = {gv.x, gv.y, gv.z, gv.w};
+        uint32_t o4[4];
+        silu_mul_pairs(yr, gr, o4);
+        *reinterpret_cast<uint4 *>(o) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
     } else {
         const float gv = __half2float(*g);
         const float silu = gv / (1.0f + __expf(-gv));

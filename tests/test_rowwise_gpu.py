@@ -376,3 +376,26 @@ def test_int8_rmsnorm_around_one_wave_of_rows(over):
         ops.rmsnorm_quant_int8(xs, w, q, s, 2.0, 1e-5)
         got.append((q, s))
     assert same_bits(got[0][0], got[1][0]) and same_bits(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("rows", [20, 2368])
+def test_silu_mul_of_every_f16_gate_equals_the_dividing_form(rows):
+    """All 65536 bit patterns as gates, eight (few rows) and sixteen (many) elements per thread: the bits of the form that takes tensors
+    off a 16-byte boundary, one element per thread with a division. Values in order, so that threads have only gates that need no division, and
+    shuffled among those that do."""
+    h = 4096
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    gate = torch.arange(65536, device=DEV, dtype=torch.int32).to(torch.int16)
+    gate = torch.cat([gate, gate[torch.randperm(65536, generator=g, device=DEV)]]).repeat(rows * h // 131072 + 1)[:rows * h]
+    y = torch.randn(rows, h, generator=g, device=DEV).half()
+    y[:, 3::64] = 0.0
+    y[1::2, 5::64] = float("inf")
+    y[:, 7::64] = -0.0
+    y[:, 9::64] = 1.0
+    y[::3, 11::64] = float("nan")
+    x = torch.cat([y, gate.view(rows, h).view(torch.float16)], dim=1).contiguous()
+    raw = torch.empty(x.numel() + 16, dtype=torch.float16, device=DEV)
+    odd = raw[1:1 + x.numel()].view(x.shape)
+    odd.copy_(x)
+    assert odd.data_ptr() % 16 == 2
+    assert same_bits(ops.silu_mul(x), ops.silu_mul(odd))
