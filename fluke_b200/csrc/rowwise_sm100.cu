@@ -210,9 +210,11 @@ __device__ __forceinline__ void load32(const void *p, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "l"(p) : "memory");
 }
-// The same for data that is read for the last time, as the f16 input of a kernel that quantises it: its lines leave L2 first. From
-// many rows on (many_rows), layers with plain loads against these, us: 7 x 1333 54.6 : 54.0, 16 x 1000 79.7 : 79.1, 32 x 1000 143.2 : 139.7,
-// 60 x 1000 261.6 : 248.9; with few rows, which L2 holds anyway, they cost 1 % (3 x 601 26.6 : 27.0).
+// The same for data whose lines leave L2 first: the f16 input of a norm, which adds it to the residual and is as a rule its last reader. From
+// many rows on (many_rows), layers with plain loads in the norms against these, us: 7 x 1333 54.6 : 54.7, 16 x 1000 78.6 : 77.7, 32 x 1000 138.4 : 136.4,
+// 60 x 1000 254.8 : 245.3, e4m3 32 x 1000 144.4 : 143.0, 60 x 1000 263.2 : 253.7; norms back to back with themselves lose up to 1.5 % (int8 32000 rows
+// 12.3 : 12.5); with few rows, which L2 holds anyway, a layer loses that (3 x 601 26.6 : 27.0). Not in the quantisers, whose caller may well read its tensor
+// again: back to back 8.65 : 8.97 (32000 rows), 29.9 : 31.0 (128000), for 0 to 1 % of a layer (7 x 1333 54.7 : 54.1, 32 x 1000 136.4 : 137.4, 60 x 1000 245.3 : 244.3).
 __device__ __forceinline__ void load32_last_use(const void *p, uint32_t (&r)[8]) {
     asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -818,7 +820,7 @@ quant_rows_reg_kernel(const __half * in, uint8_t * out,
 }
 
 // The same for hidden_dim = 512 and 32-byte aligned rows: sixteen consecutive elements per lane.
-template <bool FP8, bool LAST_USE>
+template <bool FP8>
 __global__ void __launch_bounds__(kNormWarps * 32, 16)
 quant_row512_kernel(const __half *in, uint8_t *out, float *scale, int n_tokens) {
     dependency_wait();
@@ -827,8 +829,7 @@ quant_row512_kernel(const __half *in, uint8_t *out, float *scale, int n_tokens) 
     if (row >= n_tokens) return;
     const int64_t off = row * 512 + lane * 16;
     uint32_t x[8];
-    if (LAST_USE) load32_last_use(in + off, x);
-    else load32(in + off, x);
+    load32(in + off, x);
     float2 val[8];
     float amax = 0.f;
 #pragma unroll
@@ -1261,9 +1262,7 @@ static int launch_quant(const void *in, void *out, void *scale, int n_tokens, in
                        ((reinterpret_cast<uintptr_t>(in) & 15u) == 0) &&
                        ((reinterpret_cast<uintptr_t>(out) & 7u) == 0);
     if (vec_ok && hidden_dim == 512 && aligned32(in) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
-        const bool many = many_rows(n_tokens);
-        auto kernel = fp8 ? (many ? quant_row512_kernel<true, true> : quant_row512_kernel<true, false>)
-                          : (many ? quant_row512_kernel<false, true> : quant_row512_kernel<false, false>);
+        auto kernel = fp8 ? quant_row512_kernel<true> : quant_row512_kernel<false>;
         return launch_dependent(kernel, (n_tokens + kNormWarps - 1) / kNormWarps, kNormWarps * 32, 0, s, static_cast<const __half *>(in),
                                 static_cast<uint8_t *>(out), static_cast<float *>(scale), n_tokens);
     }
