@@ -399,3 +399,45 @@ def test_silu_mul_of_every_f16_gate_equals_the_dividing_form(rows):
     odd.copy_(x)
     assert odd.data_ptr() % 16 == 2
     assert same_bits(ops.silu_mul(x), ops.silu_mul(odd))
+
+
+@pytest.mark.parametrize("over", [0, 1, 5, 6000])
+def test_quantising_kernels_around_one_wave_of_rows(over):
+    """The 512-wide e4m3 norm on either side of the row count from which another instance of it (and of the function for its exceptional
+    rows) runs, and the quantisers of the same rows, against the forms that take rows off a 32-byte boundary. Most rows are
+    decided without dividing: quotients at the conversion's ties under many row scales (no residual), ordinary rows, residuals of any
+    finite code. Every eighth row has one NaN code, every eighth a value or a scale that is not finite or not positive."""
+    n, h = 40 * torch.cuda.get_device_properties(0).multi_processor_count + over, 512
+    g = torch.Generator(device=DEV).manual_seed(over)
+    codes = torch.arange(0, 0x7F, device=DEV, dtype=torch.uint8)
+    value = codes.view(torch.float8_e4m3fn).float()
+    ties = (value[1:] + value[:-1]) / 2
+    kind = torch.arange(n, device=DEV) % 8
+    x = torch.randn(n, h, generator=g, device=DEV)
+    tied = ties[torch.randint(0, ties.numel(), (n, h), generator=g, device=DEV)] * x.sign()
+    tied[:, 0] = 448.0
+    # odd multiples of powers of two: all ties stay exact in f16 and every row has a scale of its own
+    tied *= (1 + 2 * torch.randint(0, 4, (n, 1), generator=g, device=DEV).float()) * 2.0 ** torch.randint(-6, 2, (n, 1), generator=g, device=DEV).float()
+    x = torch.where((kind < 4)[:, None], tied, x).half()
+    assert torch.isfinite(x).all()
+    res = torch.randint(0, 256, (n, h), generator=g, device=DEV, dtype=torch.uint8)
+    res = torch.where((res & 0x7F) == 0x7F, res ^ 1, res)          # no NaN codes; -0 among them
+    res[kind < 4] = 0
+    rows = torch.nonzero(kind == 6).flatten()
+    res[rows, torch.randint(0, h, (len(rows),), generator=g, device=DEV)] = 0xFF
+    scale = torch.rand(n, generator=g, device=DEV) * 1e-3 + 1e-6
+    odd = torch.nonzero(kind == 7).flatten()
+    x[odd[0::4], 17], x[odd[1::4], 501] = float("inf"), float("nan")
+    x[odd[2::4], ::2] = -0.0
+    scale[odd[2::4]] = torch.tensor([0.0, -1e-3, float("nan"), float("inf")], device=DEV).repeat(n)[:len(odd[2::4])]
+    x[odd[3::4]] = 0.0
+    w = torch.ones(h, device=DEV).half()
+    got = []
+    for shift in (0, 8):
+        xs = torch.zeros(n * h + 16, dtype=torch.float16, device=DEV)[shift:shift + n * h].view(n, h)
+        xs.copy_(x)
+        q, s = res.clone(), scale.clone()
+        ops.rmsnorm_quant_fp8(xs, w, q, s, 0.5, 1e-5)
+        got.append((q, s) + tuple(ops.quant_fp8(xs)) + tuple(ops.quant_int8(xs)))
+    for a, b in zip(*got):
+        assert same_bits(a, b)
