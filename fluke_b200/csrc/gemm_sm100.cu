@@ -74,7 +74,7 @@ struct GemmDev {
     int seq_tiles;  // 0: plain tiling, tile t covers rows [128 t, 128 t + 128)
     int n_seq;
     int items_per_cta;
-    int passes_by;  // the output is larger than what L2 can keep: its lines go first
+    int passes_by;  // SILU: the output is larger than what L2 can keep, its lines go first
 };
 
 struct TrueTag { static constexpr bool value = true; };
@@ -341,7 +341,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
         TileCursor it(p, m_first);
         int local = 0;
         bool ok = true;
-        const uint64_t policy = l2_policy(p.passes_by);
 
         // row scales of the thread's four rows of the tile that starts at row m0
         auto load_sa = [&](int m0, float (&sa)[4]) {
@@ -509,7 +508,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
-                        tma_store_2d(&tm_out, staging, n0 + c0, m0 + q * 32, policy);
+                        tma_store_2d(&tm_out, staging, n0 + c0, m0 + q * 32);
                         tma_store_commit();
                     }
                 };
@@ -541,6 +540,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                     sc_up[j] = cols_ok ? *reinterpret_cast<const float2 *>(p.scale_b2 + col) : make_float2(0.f, 0.f);
                 }
             }
+            const uint64_t evict_first = kDual ? l2_evict_first() : 0;
             float sa_next[4];
             if (it.valid()) load_sa(it.row, sa_next);
             for (; it.valid() && ok; ++local) {
@@ -610,7 +610,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_2d(&tm_out, staging, n0 + c0, m0 + q * 32, policy);
+                    // The policy only where it applies: as an operand of every store (the ordinary one elsewhere) it cost 1 to 2 % (gated MLP,
+                    // us, with : without: 16000 rows 32.0 : 31.6, e4m3 4500 11.8 : 11.5, 9331 21.4 : 20.9).
+                    if (kDual && p.passes_by) tma_store_2d(&tm_out, staging, n0 + c0, m0 + q * 32, evict_first);
+                    else tma_store_2d(&tm_out, staging, n0 + c0, m0 + q * 32);
                     tma_store_commit();
                 }
             }
@@ -658,14 +661,15 @@ int configure_smem(int bytes) {
     return 0;
 }
 
-// Whether the output's lines leave L2 first. Of an output about as large as L2 hardly anything is found there by whoever reads it
-// next, but on its way it drives out the residual stream and what else the layer's next kernels read. Where it fits, its reader
-// needs it: gated MLP and a reader of its output, us, ordinary stores against these: 33 MB 22.6 : 25.3, 66 MB 40.7 : 46.3,
-// 82 MB 55.2 : 57.2, 98 MB 68.4 : 68.5, 131 MB 97.4 : 97.5. Int8 layer of 32 x 1000 rows (131 MB from the MLP) 142.5 -> 135.8 us,
-// e4m3 153.1 -> 145.8, 60 x 1000 257.6 -> 245.7; with 128 x 1000 rows, where the residual alone is half of L2, no difference.
+// Whether the lines of the gated MLP's output leave L2 first. Of an output about as large as L2 hardly anything is found there by whoever reads it
+// next, but on its way it drives out the residual stream and what else the layer's next kernels read. Layers with the norms' loads as they are, us,
+// ordinary stores : these: int8 32 x 1000 rows (131 MB from the MLP) 141.0 : 137.4, 44 x 1000 188.1 : 181.9, 60 x 1000 249.0 : 244.3, e4m3 32 x 1000
+// 145.3 : 143.6, 60 x 1000 256.2 : 253.4; 128 x 1000, where the residual alone is half of L2, no difference. Where the output fits, its reader needs it: MLP and a
+// reader of its output, 82 MB 56.2 : 58.2, 94 66.5 : 66.9, 106 77.0 : 77.5, 115 83.3 : 83.3, 127 92.1 : 92.1, 164 109.4 : 110.1, 258 181.1 : 181.2, 520
+// 364.3 : 364.0; the line is between, at 7/8 of L2. QKV + rotary stays with ordinary stores: its reader is the very next kernel (46 MB 24.5 : 28.1, 80 44.1 :
+// 46.1, 95 53.8 : 55.0, 129 72.2 : 73.0, 261 144.9 : 145.7, 390 211.7 : 212.2) and the layer does not gain (60 x 1000 243 : 244).
 bool passes_by(const fluke_sm100_gemm_t *g) {
-    if (g->epilogue != FLUKE_SM100_EPI_ROTARY && g->epilogue != FLUKE_SM100_EPI_SILU) return false;
-    return int64_t(g->M) * g->N * 2 > device_l2_bytes() / 8 * 7;
+    return g->epilogue == FLUKE_SM100_EPI_SILU && int64_t(g->M) * g->N * 2 > device_l2_bytes() / 8 * 7;
 }
 
 // `a_planes` > 1 describes A as [a_planes, M, K] (plane stride M*K bytes).

@@ -257,12 +257,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *m, const void *s
                  ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "l"(policy)
                  : "memory");
 }
-// L2 eviction policy of a store: lines that go first, or the ordinary ones.
-__device__ __forceinline__ uint64_t l2_policy(bool evict_first) {
-    uint64_t first, normal;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
-    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
-    return evict_first ? first : normal;
+// L2 eviction policy: lines that go first.
+__device__ __forceinline__ uint64_t l2_evict_first() {
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    return policy;
 }
 __device__ __forceinline__ void tma_store_commit() {
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");

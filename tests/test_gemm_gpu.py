@@ -549,3 +549,35 @@ def test_outputs_larger_than_l2_equal_those_of_parts(kind):
     for lo, hi in ((0, m // 2), (m // 2, m)):
         part = run(lo, hi).view(torch.int16)
         assert torch.equal(whole[lo:hi].reshape(part.shape), part)
+
+
+@pytest.mark.parametrize("kind,fp8", [("qkv", False), ("qkv", True), ("mlp", True)])
+def test_outputs_larger_than_l2_equal_those_of_parts_whole_sequences_and_fp8(kind, fp8):
+    """As above with e4m3 operands and with sequences of 1000 positions, to which the rotary tiles are aligned: 147 MB of
+    output in one call and in two."""
+    seq, n = 1000, 1536 if kind == "qkv" else 2048
+    m = (147 << 20) // (2 * n) // (2 * seq) * (2 * seq)
+    gd = torch.Generator(device=DEV).manual_seed(11)
+
+    def operand(rows, scale):
+        t = torch.randn(rows, 512, generator=gd, device=DEV) * scale
+        q, s = prep.quantize_fp8_rows(t) if fp8 else prep.quantize_int8_rows(t)
+        return (q.view(torch.uint8) if fp8 else q).contiguous(), s.contiguous()
+
+    a, sa = operand(m, 1.0)
+    w, sw = operand(n, 0.02)
+    u, su = operand(n, 0.02)
+    sin, cos = prep.rotary_tables(seq, 64, device=DEV)
+    be = ops.fp8_select(0) if fp8 else ops.int8_select(0)
+    plain = {"plain": True} if fp8 else {}
+    qkv, mlp = (ops.qkv_rotary_fp8, ops.gated_mlp_fp8) if fp8 else (ops.qkv_rotary_i8, ops.gated_mlp_i8)
+
+    def run(lo, hi):
+        if kind == "qkv":
+            return qkv(be, a[lo:hi], w, sa[lo:hi], sw, sin, cos, seq, **plain)
+        return mlp(be, a[lo:hi], w, u, sa[lo:hi], sw, su, **plain)
+
+    whole = run(0, m).view(torch.int16)
+    for lo, hi in ((0, m // 2), (m // 2, m)):
+        part = run(lo, hi).view(torch.int16)
+        assert torch.equal(whole[lo:hi].reshape(part.shape), part)
