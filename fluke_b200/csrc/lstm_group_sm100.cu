@@ -475,6 +475,29 @@ __device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev 
     issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows, 0);
 }
 
+// A row of the recurrent weights of a gate from its place in shared memory (two K blocks of 64 in the 128-byte swizzle) to its lane of tensor
+// memory; returns whether one of them is not finite, where that matters. All eight loads go ahead of the stores: unrolled once the set-up of a layer
+// with few rows takes 0.5 us more. Out of line because it runs once: in the kernel either form of the loop moved the code of the steps, and each made another form
+// of them 0.6 to 1.6 % slower (us per step, unrolled 8 : 1 : this; H = 384 32 chunks 1.163 : 1.179 : 1.155, H = 768 300 1.757 : 1.743 : 1.738, H = 1024 240
+// 1.892 : 1.863 : 1.861; the largest losses of this one 256 64 1.126 : 1.146 : 1.143, 768 170 1.441 : 1.440 : 1.455).
+template <int V, int C>
+__device__ __noinline__ bool recurrent_weights(uint32_t row, uint32_t t_w, int lane) {
+    using K = GroupConst<V, C>;
+    __half2 zeros[2] = {__half2half2(__ushort_as_half(0)), __half2half2(__ushort_as_half(0))};
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+        const uint32_t at = row + (v >> 2) * 16384;
+        const uint4 lo = lds128(at + (((2 * (v & 3)) ^ (lane & 7)) << 4)), hi = lds128(at + (((2 * (v & 3) + 1) ^ (lane & 7)) << 4));
+        tmem_st_32x8(t_w + v * 8, lo, hi);
+        if (K::kZeroRows) {
+            add_zero_times(zeros[0], lo);
+            add_zero_times(zeros[1], hi);
+        }
+    }
+    const __half2 sum = __hadd2(zeros[0], zeros[1]);
+    return K::kZeroRows && (__hisnan(__low2half(sum)) || __hisnan(__high2half(sum)));
+}
+
 // The groups of chunk rows share the x part of the contraction (its MMAs read their A operand from shared memory, so
 // one for both) and go through the rest of the step one after the other: while one is exchanged, the other
 // is projected or computed.
@@ -595,29 +618,10 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         const uint4 *dn = reinterpret_cast<const uint4 *>(p.dn + size_t(dn_row) * H + (kGather ? 0 : n0));
 #pragma unroll 1
         for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
-        __half2 zeros[2] = {__half2half2(__ushort_as_half(0)), __half2half2(__ushort_as_half(0))};
-        if (__all_sync(0xffffffffu, mbar_wait(&bar_w[g], 0, abort_flag, 109))) {
-            const uint32_t row = smem_u32(smem) + g * 32768 + (q * 32 + lane) * 128;
-            // Unrolled or not moves the code of the steps behind it, by which they differ: up to 8 rows a step is 1.6 % faster behind the
-            // long form (H = 384, 32 chunks), from 9 rows on up to 1.5 % behind the short one (H = 1024 200 chunks, H = 768 300 0.7 %).
-            constexpr int kUnroll = V == 0 ? 8 : 1;
-#pragma unroll kUnroll
-            for (int v = 0; v < 8; ++v) {
-                const uint32_t at = row + (v >> 2) * 16384;
-                const uint4 lo = lds128(at + (((2 * (v & 3)) ^ (lane & 7)) << 4)), hi = lds128(at + (((2 * (v & 3) + 1) ^ (lane & 7)) << 4));
-                tmem_st_32x8(t_lane + kGTmemW + g * 64 + v * 8, lo, hi);
-                if (K::kZeroRows) {
-                    add_zero_times(zeros[0], lo);
-                    add_zero_times(zeros[1], hi);
-                }
-            }
-        }
+        if (__all_sync(0xffffffffu, mbar_wait(&bar_w[g], 0, abort_flag, 109)))
+            non_finite = recurrent_weights<V, C>(smem_u32(smem) + g * 32768 + (q * 32 + lane) * 128, t_lane + kGTmemW + g * 64, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_w_read[g]);
-        if constexpr (K::kZeroRows) {
-            const __half2 sum = __hadd2(zeros[0], zeros[1]);
-            non_finite = __hisnan(__low2half(sum)) || __hisnan(__high2half(sum));
-        }
         tmem_st_wait();
         tc_fence_before_sync();
     }
