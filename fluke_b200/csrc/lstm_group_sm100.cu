@@ -83,7 +83,6 @@ struct GroupDev {
     int reverse;
     int rows;                  // chunk rows per cluster (the last one may have fewer)
     const int8_t *dn;          // [R, H]
-    const __half *w_up;        // [4H, 2R]
     const float *bias;         // [4H]
     const float *dn_scale;     // [R]
     float *c;                  // [B,H]
@@ -1061,7 +1060,6 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     p.T = T; p.B = B; p.reverse = l->reverse;
     p.rows = g.rows;
     p.dn = static_cast<const int8_t *>(l->dn_hh_i8);
-    p.w_up = static_cast<const __half *>(l->w_up_f16);
     p.bias = static_cast<const float *>(l->bias_f32);
     p.dn_scale = static_cast<const float *>(l->dn_hh_scale);
     p.c = static_cast<float *>(l->c_f32);
