@@ -46,16 +46,17 @@ class FactoredLstmLayer:
 
 def run_stack(layers, x_i8, x_scale, state=None, workspace=None, buffers=None):
     """x_i8 [T,B,H] int8 with per-row scales x_scale [T*B]. Returns (h_out of the last layer
-    [T,B,H] int8 @1/127, state) where state is a list of (c f32 [B,H], h int8 [B,H]) per layer.
+    [T,B,H] int8 @1/127, state) where state is a list of (c f32 [B,H], h int8 [B,H]) per layer. Without `state` all
+    layers start from zero; what is returned then are views of one tensor of cell and one of hidden states, so a caller
+    who keeps a single layer's beyond the pass clones it.
     `buffers` may hold two reusable [T,B,H] int8 outputs."""
     t, b, h = x_i8.shape
     dev = x_i8.device
     if state is None:
-        # one fill for all layers, where 16-byte alignment of every part allows it
-        n = len(layers) if (b * h) % 16 == 0 else 1
-        parts = [(torch.zeros(n, b, h, dtype=torch.float32, device=dev), torch.zeros(n, b, h, dtype=torch.int8, device=dev))
-                 for _ in range(len(layers) // max(n, 1))]
-        state = [s for c, hs in parts for s in zip(c, hs)]
+        # one fill per kind for all layers
+        c = torch.zeros(len(layers), b, h, dtype=torch.float32, device=dev)
+        hs = torch.zeros(len(layers), b, h, dtype=torch.int8, device=dev)
+        state = list(zip(c, hs))
     if buffers is None:
         buffers = [torch.empty(t, b, h, dtype=torch.int8, device=dev) for _ in range(2)]
     cur, cur_scale = x_i8, x_scale
