@@ -248,6 +248,8 @@ inline int tile_smem(int K, int rows_b) { return (K / 128 + 1) / 2 * 2 * (128 + 
 template <int KIND, int EPI, int BN>
 int tile_launch(const fluke_sm100_gemm_t *g, cudaStream_t stream) {
     constexpr bool kDual = EPI == FLUKE_SM100_EPI_SILU;
+    constexpr int kMaxK = EPI == FLUKE_SM100_EPI_SILU || EPI == FLUKE_SM100_EPI_ROTARY ? 512 : 1024;   // as the persistent kernel
+    if (g->K > kMaxK) return (int)cudaErrorInvalidValue;
     GemmTileDev p;
     p.M = g->M; p.N = g->N; p.ld_out = g->ld_out;
     p.nkb = g->K / 128; p.half_kb = (p.nkb + 1) / 2;
@@ -271,7 +273,6 @@ int tile_launch(const fluke_sm100_gemm_t *g, cudaStream_t stream) {
         if (rc) return rc;
     }
     constexpr int kRowsB = kDual ? 2 * BN : BN;
-    constexpr int kMaxK = EPI == FLUKE_SM100_EPI_SILU || EPI == FLUKE_SM100_EPI_ROTARY ? 512 : 1024;
     rc = configure_smem<gemm_tile_kernel<KIND, EPI, BN>>(tile_smem(kMaxK, kRowsB));
     if (rc) return rc;
     return launch_dependent(gemm_tile_kernel<KIND, EPI, BN>, dim3(g->N / BN, (g->M + 127) / 128), kTileThreads, tile_smem(g->K, kRowsB), stream,

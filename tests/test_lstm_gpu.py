@@ -564,3 +564,38 @@ def test_rows_projected_by_pair_give_the_bytes_of_the_l2_form(flib, B, T):
     flib.fluke_set_lstm_persistent(1)
     for got, want in zip(*res):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("h", [1088, 1152, 1280, 2048])
+@pytest.mark.parametrize("b", [16, 3000])
+def test_layers_of_more_than_1024_units_are_refused_without_a_launch(flib, h, b):
+    """The down-projection's contraction is limited to 1024; a layer beyond it is refused by the library's own check whichever kernel
+    its number of rows would take, also during a stream capture, which goes on."""
+    t = 2
+    layer = FactoredLstmLayer.random(h, 128, False, torch.Generator().manual_seed(h), DEV)
+    x = torch.zeros(t, b, h, dtype=torch.int8, device=DEV)
+    c, hs = torch.ones(b, h, device=DEV), torch.ones(b, h, dtype=torch.int8, device=DEV)
+    out = torch.full_like(x, 5)
+    ws = torch.empty(flib.fluke_factored_lstm_layer_workspace(t, b, h, 128), dtype=torch.uint8, device=DEV)
+
+    def layer_is_refused():
+        with pytest.raises(RuntimeError):
+            ops.factored_lstm_layer_i8(x, None, layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale, layer.w_up,
+                                       layer.bias, c, hs, h_out=out, workspace=ws)
+
+    layer_is_refused()
+    y = torch.randn(40, 512, device=DEV).half()
+    want = ops.silu_mul(y)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        ops.set_stream(stream)
+        try:
+            layer_is_refused()
+            got = ops.silu_mul(y)
+        finally:
+            ops.set_stream(None)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    assert bool((c == 1).all()) and bool((hs == 1).all()) and bool((out == 5).all())
