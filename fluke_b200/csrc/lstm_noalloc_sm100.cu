@@ -21,8 +21,9 @@
 //  * First call per device. It looks up the device address of the array (the array's name in
 //    host code is only a host-side handle, not something a kernel can dereference) and caches
 //    it, and the kernels it launches are configured on their first use. Make the first call on
-//    a device -- with the layer shape (B, H, R) and the fluke_set_lstm_persistent mode that later
-//    calls will use, since those choose the kernels -- before any stream capture begins, with the
+//    a device -- with the layer shape (T, B, H, R) and the fluke_set_lstm_persistent mode that later
+//    calls will use, since those choose the kernels (T as well: the down-projection of all T * B rows takes another
+//    one for few rows than for many) -- before any stream capture begins, with the
 //    device current.
 //  * One layer at a time per device. All calls share the one array; it still holds the previous
 //    call's intermediates when the next call starts. That is harmless -- every element a layer
