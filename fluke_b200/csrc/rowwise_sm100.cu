@@ -504,7 +504,8 @@ __device__ __forceinline__ uint4 int8_codes16(const float2 (&v)[8], float scale)
 // ---- RMSNorm family, hidden_dim = 512, 32-byte aligned rows: one warp per row, sixteen consecutive
 // elements per lane (256-bit accesses). Same bits as rmsnorm_rows_kernel. The e4m3 form is bound by its instructions: 32 of them per
 // lane and row went into dividing (now two products and two conversions per pair of values, e4m3_quotients16) and
-// as many into clearing codes in the residual; without both 128000 rows take 50.2 us instead of 58.8, 32000 13.5 instead of 14.7.
+// as many into clearing codes in the residual. With both, and in 32 registers, 128000 rows took 62.0 us and 32000 15.7; without, and with the registers of
+// launch_rmsnorm, 49.4 and 13.3.
 // EXACT = false (e4m3 only) returns false, with nothing written, for a row whose scale is not positive (the sign of zeros) or
 // that has a residual code or result that is not finite: the decoding instruction gives NaN for the NaN codes where the reference's gives 0, which makes every result
 // of the row NaN, and quotients of such values are left to the division.
@@ -609,8 +610,8 @@ __device__ __forceinline__ bool rmsnorm_row512(const __half *in, const void *res
     return true;
 }
 
-// Out of line, so that the rows that need it take no registers from the others; one for each kernel (the compiler does not
-// come through with one that two call).
+// Out of line, so that the rows that need it take no registers from the others. LAST_USE selects nothing in it: nvcc 12.9 ends with a
+// segmentation fault where two kernels call the same such function, so each of the two e4m3 kernels has its own.
 template <bool LAST_USE>
 __device__ __noinline__ void rmsnorm_row512_exact(const __half *in, const void *residual_in, const __half *weight, void *out, float *res_scale,
                                                   int64_t row, int lane, float alpha, float eps) {
@@ -1032,8 +1033,8 @@ __device__ __forceinline__ void split_index(int64_t idx, int64_t total, int per_
 }
 
 // ---- SiLU-multiply (nn_kernel_cuda.h:71-90) -----------------------------------------------------
-// g / (1 + exp(-g)) for f16 values g >= -69 without the division's checks: one correction of the product with the approximate
-// reciprocal gives the correctly rounded quotient for every one of them (all 53329 compared with the division; without it 9347 differ);
+// g / (1 + exp(-g)) for f16 values g >= -69 without the division's checks: one correction by the exact residual (Markstein, as in
+// div_by_scale) of the product with the approximate reciprocal gives the correctly rounded quotient for every one of them (all 53329 compared with the division; without it 9347 differ);
 // the sign is g's own where the quotient is a zero. The divisions were most of what the kernel
 // issued: [32000, 4096] 67.8 -> 59.0 us (1.02 of the copy bandwidth), 128000 rows 284 -> 242, 2000 6.4 -> 5.3, 125 1.73 -> 1.39.
 __device__ __forceinline__ float2 silu2(float2 g) {
@@ -1365,9 +1366,8 @@ extern "C" int fluke_sm100_silu_mul(const void *in, void *out, int n_tokens, int
     int rc;
     const bool vec = (hidden_dim % 8 == 0) &&
                      (((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0);
-    // Sixteen elements per thread once those threads fill the device ([32000, 4096]: 72.8 -> 62.8 us, 0.95 of
-    // the copy bandwidth); below that twice as many threads with eight each finish sooner (125 rows:
-    // 1.84 against 2.27 us, 1803 rows 4.85 against 5.0).
+    // Sixteen elements per thread once those threads fill the device, below that twice as many threads with eight each. us of rows
+    // of 4096, eight : sixteen: 125 rows 1.49 : 1.66, 500 2.01 : 2.11, 2000 5.40 : 5.42, 9331 19.6 : 18.0, 32000 65.3 : 58.5, 128000 266 : 232.
     if (vec && hidden_dim % 16 == 0 && aligned32(in, out) && int64_t(n_tokens) * (hidden_dim / 16) >= full_device_threads()) {
         const int64_t total = int64_t(n_tokens) * (hidden_dim / 16);
         rc = launch_dependent(silu_mul_kernel<16>, grid_for(total, 256), 256, 0, s, static_cast<const __half *>(in), static_cast<__half *>(out), total, hidden_dim);
