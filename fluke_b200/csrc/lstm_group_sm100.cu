@@ -76,7 +76,7 @@ constexpr int kGTmemCols = 512;
 constexpr int kGTmemW = 256;       // first column of the hh half of the gate weights: 4 gates x 64
 constexpr int kGWxBytes = 4 * kGUnits * 256;  // x half of the gate weights in shared memory
 constexpr int kGMaxSmem = 232448;
-constexpr int kGBars = 32;         // mbarriers of a CTA
+constexpr int kGBars = 48;         // mbarriers of a CTA
 
 struct GroupDev {
     int T, B;
@@ -112,20 +112,29 @@ struct GroupForm {
     int proj;           // columns of projection accumulators
     int x_slots;        // steps whose x_down rows are in shared memory
 };
-// 8 rows: the sixteen columns that an MMA has at least are two steps' rows, see x_half. Two groups of 24 rows: an MMA of
+// 8 rows: the columns of an x MMA are two or four steps' rows, see x_half. Two groups of 24 rows: an MMA of
 // the first group also covers the first columns of the second, with operand rows that are zero, before that
 // group's own MMAs; the second group's covers unused columns. They take turns with one projection accumulator.
 __host__ __device__ constexpr GroupForm group_form(int V) {
-    return V == 0   ? GroupForm{8, true, 1, 8, 16, 16, 16, 5}
+    return V == 0   ? GroupForm{8, true, 1, 8, 16, 16, 16, 5}   // four steps: group_stride, 11 slots
            : V == 1 ? GroupForm{16, true, 1, 16, 16, 16, 16, 2}
            : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32, 2}
                     : GroupForm{48, false, 2, 24, 32, 56, 32, 2};
 }
+// Up to 8 rows: steps whose x part one MMA covers. MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
+// sixteen that there are at least (42), and what is issued of them before the hidden codes arrive holds the issuer up: with 16 such MMAs per step
+// it saw codes that had travelled for 200 cycles after 430. Four steps per MMA are 8 per step, and twice the accumulators, which clusters of
+// two and three have the tensor memory for beside all projection weights. Two steps against four, us per step, x_down included: H = 384 32 chunks 1.156 :
+// 1.044, 120 1.186 : 1.078, 172 1.188 : 1.088, 250 1.200 : 1.160, 344 1.235 : 1.238; H = 256 32 1.137 : 1.027, 300 1.182 : 1.109, 528 1.222 : 1.202. With
+// more CTAs some projection weights have to give way: H = 512 32 chunks 1.166 : 1.125, but 200 1.269 : 1.339; H = 640 200 1.366 : 1.467.
+__host__ __device__ constexpr int group_x_steps(int V, int C) { return V != 0 ? 1 : C <= 3 ? 4 : 2; }
+// Accumulator columns from gate to gate.
+__host__ __device__ constexpr int group_stride(int V, int C) { return group_x_steps(V, C) == 4 ? 32 : group_form(V).stride; }
 // K steps (32 units, 8 columns) of the projection weights that fit in tensor memory beside the gate weights, the gate
 // accumulators and the projections.
 __host__ __device__ constexpr int group_dn_ts(int V, int C) {
     const GroupForm f = group_form(V);
-    const int fit = (kGTmemW - 4 * f.stride - f.proj) / 8, all = f.gather ? 4 * C : 4;
+    const int fit = (kGTmemW - 4 * group_stride(V, C) - f.proj) / 8, all = f.gather ? 4 * C : 4;
     return fit < all ? fit : all;
 }
 // Four rows of a group are projected as one piece (16 bytes per projection column). The pieces of all groups are dealt to
@@ -149,7 +158,7 @@ __host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
     const GroupForm f = group_form(V);
     GroupLayout l = {};
     l.x = kGWxBytes;                              // x_down rows, see x_half
-    l.hh = l.x + f.x_slots * f.groups * f.rows * 256;
+    l.hh = l.x + (group_x_steps(V, C) == 4 ? 11 : f.x_slots) * f.groups * f.rows * 256;
     // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
     l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
     // projection weights [128 x 128 B] (by pair [64 x 128 B]) of the K blocks that are not all in tensor memory
@@ -217,13 +226,16 @@ struct GroupConst {
     static constexpr GroupForm F = group_form(V);
     static constexpr GroupLayout L = group_layout(V, C);
     static constexpr bool kGather = F.gather;
-    static constexpr int G = F.groups, NB = G * F.rows, S = F.stride, H = C * kGUnits;
-    static constexpr bool kTwoSteps = F.rows == 8;            // an x MMA covers two steps
-    static constexpr int kXSlots = kTwoSteps ? 4 : F.x_slots;
+    static constexpr int G = F.groups, NB = G * F.rows, S = group_stride(V, C), H = C * kGUnits;
+    static constexpr bool kTwoSteps = group_x_steps(V, C) == 2;    // an x MMA covers two steps
+    static constexpr bool kFourSteps = group_x_steps(V, C) == 4;   // or four
+    static constexpr int kXSlots = kFourSteps ? 8 : kTwoSteps ? 4 : F.x_slots;
+    static constexpr int kXRing = kFourSteps ? 11 : 5;        // slots of 8 rows when an x MMA covers several steps
+    static constexpr int kFirstBarX = kFourSteps ? 32 : 1;
     static constexpr bool kByPair = group_by_pair(V, C);
     static constexpr bool kPeerHh = !kGather || kByPair;      // hh_down rows come from peers
     static constexpr int kTile = (kByPair ? 8 : F.rows) * 128;     // bytes of a group's hidden rows in one K block
-    static constexpr int kHhTile = (kTwoSteps ? 24 : F.n) * 128;   // and of its hh_down rows
+    static constexpr int kHhTile = (F.rows == 8 ? 24 : F.n) * 128;   // and of its hh_down rows
     static constexpr bool kZeroRows = kHhTile > F.rows * 128; // some of which are zero
     static constexpr int kDnRows = kByPair ? 64 : kGRank;     // projection columns of a CTA
     static constexpr int kPieces = F.rows / 4;                // pieces of a group
@@ -261,18 +273,18 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     using K = GroupConst<V, C>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
-    constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
+    constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kFourSteps = K::kFourSteps, kOneProj = K::kOneProj;
     constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
     constexpr int kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + kBarX, *bar_x_free = bars + kBarXFree, *bar_acc_free = bars + kBarAccFree;
+    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + K::kFirstBarX, *bar_x_free = bar_x + (kFourSteps ? 8 : 4), *bar_acc_free = bars + kBarAccFree;
     uint64_t *bar_proj = bars + kBarProj, *bar_acc = bars + kBarAcc, *bar_hh = bars + kBarHh, *bar_code = bars + kBarCode;
     uint64_t *bar_sent = bars + kBarSent, *bar_stored = bars + kBarStored, *bar_h = bars + kBarH;
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
     [[maybe_unused]] const int lane = threadIdx.x & 31;
     auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
-    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, kTwoSteps ? 16 : NB);
+    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, kFourSteps ? 32 : kTwoSteps ? 16 : NB);
     constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
     constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
     uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
@@ -285,21 +297,23 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     // MMAs [from, to) of the x part of a step. They read their A operand from shared memory (42 cycles
     // each, 48 with 48 columns) and the tensor pipe works in order, so they are issued in pieces for the times when it
     // would wait. With up to 8 rows, where the 32 MMAs of a step would take longer than all of its waits, an MMA covers
-    // the rows of two steps: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
-    // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones.
-    constexpr int kX = kTwoSteps ? 16 : 32;
-    auto x_half = [&](auto from, auto to, int i, bool release = true) {
+    // the rows of two or four steps. Two: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
+    // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones. Four: step i computes gate
+    // i mod 4 of itself and the next three, whose rows are contiguous in a ring of eight slots of which the first three are repeated behind it.
+    constexpr int kX = kFourSteps ? 8 : kTwoSteps ? 16 : 32;
+    auto x_half = [&](auto from, auto to, int i, bool release = true, int gate = 0) {
         constexpr int first = decltype(from)::value, end = decltype(to)::value;
-        const uint64_t d_x = d_x0 + uint64_t((i & (kXSlots - 1)) * (kTwoSteps ? NB * 8 : NB * 16));
-        const int g0 = kTwoSteps ? 2 * (i & 1) : 0;
+        const int slot = i & (kXSlots - 1);
+        const uint64_t d_x = d_x0 + uint64_t(slot * (kTwoSteps || kFourSteps ? NB * 8 : NB * 16));
+        const int g0 = kFourSteps ? (kExact ? gate : i & 3) : kTwoSteps ? 2 * (i & 1) : 0;
         if (elect_one()) {
 #pragma unroll
             for (int m = first; m < end; ++m) {
                 const int g = m >> 3, k = m & 7;
                 tc_mma<kKindF16>(tmem + (g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                 d_x + uint64_t((k >> 2) * ((kTwoSteps ? 5 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+                                 d_x + uint64_t((k >> 2) * ((kTwoSteps || kFourSteps ? K::kXRing : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
             }
-            if (end == kX && release) tc_commit(&bar_x_free[i & (kXSlots - 1)]);
+            if (end == kX && release) tc_commit(&bar_x_free[slot]);
         }
         __syncwarp();
     };
@@ -368,20 +382,33 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     auto hh_half = [&](auto group) {
         constexpr int e = decltype(group)::value;
         if (e > 0 && !both) return true;
+        // Several steps per x MMA: neighbouring steps' columns get rows that are zero. All of it is worked out in front of the wait.
+        uint64_t rows[4];
+        uint32_t cols[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            rows[g] = d_hh;
+            cols[g] = tmem + g * S + F.rows * e;
+            if (kTwoSteps) rows[g] += (i ^ (g >> 1)) & 1 ? 0 : 64;
+            if (kFourSteps) {
+                const int at = kExact ? 0 : (i - g) & 3;
+                rows[g] += at < 3 ? 64 : 0;
+                cols[g] += at < 3 ? 8 * at : 16;
+                asm volatile("" : "+l"(rows[g]), "+r"(cols[g]));
+            }
+        }
         ok = ok && mbar_wait<true>(&bar_hh[e], i & 1, abort_flag, 101);
         if (!ok) return false;
         if (K::kPeerHh) fence_proxy_async_smem();
         tc_fence_after_sync();
         FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 3 + e, clock64());
         if (elect_one()) {
-            // two steps per MMA: the other step's columns get rows that are zero
-            const uint64_t rows[2] = {d_hh + uint64_t(kTwoSteps && !(i & 1) ? 64 : 0), d_hh + uint64_t(kTwoSteps && (i & 1) ? 64 : 0)};
 #pragma unroll
             for (int g = 0; g < 4; ++g)
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    tc_mma_ts<kKindF16>(tmem + g * S + F.rows * e, tmem + kGTmemW + g * 64 + k * 8,
-                                        rows[g >> 1] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
+                    tc_mma_ts<kKindF16>(cols[g], tmem + kGTmemW + g * 64 + k * 8,
+                                        rows[g] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
             tc_commit(&bar_acc[e]);
             if (K::kPeerHh && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
         }
@@ -420,26 +447,36 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         if (ok) ok = mbar_wait(&bar_x[0], 0, abort_flag, 99);
         if (ok) x_half(Int<0>{}, Int<16>{}, -1, false);
     }
+    if constexpr (kFourSteps) {
+        // gates 1, 2 and 3 of the first steps, as of steps before them: whatever is in the slots enters columns that nothing reads
+        for (int w = -3; w < 0 && wait_x(w + 3); ++w) x_half(Int<0>{}, Int<kX>{}, w, false, w & 3);
+    }
     for (; i < p.T && ok; ++i) {
         // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
         // more registers than there are.
         asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
-        constexpr int kFirstX = kTwoSteps ? 10 : kByPair ? 16 : kGather ? 24 : 2;
+        constexpr int kFirstX = kFourSteps ? 4 : kTwoSteps ? 10 : kByPair ? 16 : kGather ? 24 : 2;
         if constexpr (kGather) {
             // Most of the x part while the hidden state is computed and travels, the rest while the
             // projection is converted. 20 / 24 / 28 of 32 in front, us per step (x_down included): H = 768 200 chunks 1.62 / 1.57 / 1.64, 300
             // 1.74 / 1.70 / 1.73; H = 384 600 1.58 / 1.54 / 1.63; H = 512 500 1.68 / 1.62 / 1.65; H = 896 180 1.71 / 1.70 / 1.74. 8 / 10 / 12 of 16: H = 768
-            // 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 384 200 1.19 / 1.19 / 1.20; H = 1024 60 1.42 / 1.40 / 1.44. By pair 12 / 16 /
+            // 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 1024 60 1.42 / 1.40 / 1.44. 3 / 4 / 5 of 8 within 1 % of each other. By pair 12 / 16 /
             // 20 of 32: 135 chunks 1.68 / 1.66 / 1.73, 240 1.86 / 1.87 / 1.88.
-            if (!wait_x(kTwoSteps ? i + 1 : i) || !wait_acc()) break;
+            if (!wait_x(kFourSteps ? i + 3 : kTwoSteps ? i + 1 : i) || !wait_acc()) break;
             FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
             // Two steps per MMA: the zero rows of the step before have spoilt the accumulators of this step's gates that its x MMAs
             // computed. Once more from the same slots; the step before may be gone from its, it enters columns that have been read.
             if (kExact && kTwoSteps && i > 0) x_half(Int<0>{}, Int<kX>{}, i - 1, false);
-            x_half(Int<0>{}, Int<kFirstX>{}, i);
-            FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 10, clock64());
-            if (!project_all()) break;
-            x_half(Int<kFirstX>{}, Int<kX>{}, i);
+            if constexpr (kExact && kFourSteps) {
+                // all gates of this step from this step's window: what the zero rows spoil is never used
+                for (int g = 0; g < 4; ++g) x_half(Int<0>{}, Int<kX>{}, i, g == 3, g);
+                if (!project_all()) break;
+            } else {
+                x_half(Int<0>{}, Int<kFirstX>{}, i);
+                FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 10, clock64());
+                if (!project_all()) break;
+                x_half(Int<kFirstX>{}, Int<kX>{}, i);
+            }
             if (!hh_half(Int<0>{})) break;
         } else {
             // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
@@ -512,7 +549,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     using K = GroupConst<V, C>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
-    constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kOneProj = K::kOneProj;
+    constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kFourSteps = K::kFourSteps, kOneProj = K::kOneProj;
     constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
     constexpr int kPieces = K::kPieces, kPairs = K::kPairs, kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     extern __shared__ uint8_t smem_raw[];
@@ -521,7 +558,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + kBarX, *bar_x_free = bars + kBarXFree, *bar_acc_free = bars + kBarAccFree;
+    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + K::kFirstBarX, *bar_x_free = bar_x + (kFourSteps ? 8 : 4), *bar_acc_free = bars + kBarAccFree;
     uint64_t *bar_proj = bars + kBarProj, *bar_acc = bars + kBarAcc, *bar_hh = bars + kBarHh, *bar_code = bars + kBarCode;
     uint64_t *bar_sum = bars + kBarSum, *bar_sent = bars + kBarSent, *bar_stored = bars + kBarStored, *bar_h = bars + kBarH;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.misc);
@@ -550,7 +587,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     if (threadIdx.x == 0) {
         auto arrivals = [&](int b) {   // warps that arrive, or one arrival with the expected bytes
             if (b == kBarAccFree) return kGather || both ? kGEpiWarps : kGEpiWarps / 2;
-            if (b >= kBarWRead) return 4;
+            if (b >= kBarWRead && b < kBarWRead + 4) return 4;
+            if (b >= kBarWRead) return 1;
             if (kGather) return !kByPair && b == kBarHh ? kGEpiWarps : 1;
             return b == kBarCode || b == kBarCode + 1 || b == kBarSent ? kGEpiWarps / 2 : 1;
         };
@@ -642,12 +680,12 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 const int s = i & (kXSlots - 1), u = i / kXSlots;
                 if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
                 if (!ok) return;
-                if constexpr (kTwoSteps) {
-                    const bool twice = s == 0;   // the fifth slot repeats the first
+                if constexpr (kTwoSteps || kFourSteps) {
+                    const bool twice = s < K::kXRing - kXSlots;   // the last slots repeat the first
                     mbar_arrive_expect_tx(&bar_x[s], NB * 256 * (twice ? 2 : 1));
                     for (int kb = 0; kb < 2; ++kb)
                         for (int n = 0; n < (twice ? 2 : 1); ++n)
-                            tma_load_4d(smem + L.x + (kb * 5 + s + 4 * n) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
+                            tma_load_4d(smem + L.x + (kb * K::kXRing + s + kXSlots * n) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
                 } else {
                     mbar_arrive_expect_tx(&bar_x[s], NB * 256);
                     tma_load_4d(smem + L.x + s * (NB * 256), &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
@@ -788,7 +826,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             const uint32_t src = stage + s_row * 128 + s_piece * 16;
             const uint32_t dst_bar = map_to_rank(smem_u32(bar_h), to);
             const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + q * 32 + lane);   // operand order of the dequant GEMM: sa * sb
-            const uint32_t hh = smem_u32(smem + L.hh) + (q >> 1) * kHhTile + (kTwoSteps ? 1024 : 0) + r0 * 128 +
+            const uint32_t hh = smem_u32(smem + L.hh) + (q >> 1) * kHhTile + (F.rows == 8 ? 1024 : 0) + r0 * 128 +
                                 (((q & 1) * 4 + (lane >> 3)) ^ (r0 & 7)) * 16 + (lane & 7) * 2;
             const int64_t at = int64_t(m0 + r0 + s_row) * H + n0;   // plus the piece
             int8_t *h_out = p.h_out + int64_t(time_of(0)) * p.B * H + at;
@@ -815,6 +853,15 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (lane == 0) mbar_arrive(bar_hh);
                 FLUKE_STAMP(blockIdx.x == 0 && warp == 2 && lane == 0, i * 16 + 7, clock64());
                 // ---- gates, cell update, hidden codes ----
+                uint32_t cols[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    cols[g] = t_lane + g * S + r0 + (kTwoSteps ? ((i ^ (g >> 1)) & 1) * 8 : 0);
+                    if (kFourSteps) {
+                        cols[g] += 8 * (finite ? (i - g) & 3 : 0);
+                        asm volatile("" : "+r"(cols[g]));   // worked out in front of the wait
+                    }
+                }
                 ok = ok && mbar_wait(&bar_acc[0], i & 1, abort_flag, 103);
                 FLUKE_STAMP(blockIdx.x == 0 && warp == 2 && lane == 0, i * 16 + 12, clock64());
                 Acc a;
@@ -822,9 +869,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     tc_fence_after_sync();
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
-                        const uint32_t col = t_lane + g * S + r0 + (kTwoSteps ? ((i ^ (g >> 1)) & 1) * 8 : 0);
-                        if (kPairs > 1) tmem_ld_32x4(col, a[g]);
-                        else tmem_ld_32x2(col, a[g][0], a[g][1]);
+                        if (kPairs > 1) tmem_ld_32x4(cols[g], a[g]);
+                        else tmem_ld_32x2(cols[g], a[g][0], a[g][1]);
                     }
                     tmem_ld_wait();
                     tc_fence_before_sync();

@@ -543,6 +543,37 @@ def test_one_timestep_per_call_gives_the_bytes_of_one_call(flib, H, B):
     assert torch.equal(got, want) and torch.equal(c1, c) and torch.equal(h1, h)
 
 
+@pytest.mark.parametrize("H,B", [(256, 3), (256, 64), (256, 527), (256, 528), (384, 32), (384, 130), (384, 343), (384, 344), (384, 345)])
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 8, 9, 17])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_four_steps_per_contraction_give_the_bytes_of_the_l2_form(flib, H, B, T, infinite):
+    """Clusters of two and three with up to 8 rows each (528 and 344 chunks on a B200) contract the x rows of four steps at once, from a
+    ring of eight slots: fewer steps than that, the ring's wrap, both directions, ragged last clusters; and weights that are not finite, for
+    which every step contracts its own. Against the L2-exchange form. Exact."""
+    layer, x, xs = _layer_case(T, B, H, 128, H + B + T, T % 2 == 1)
+    w = layer.w_up.clone()
+    if infinite:
+        for i, (unit, k) in enumerate([(3, 5), (40, 127), (H - 1, 64), (129, 0), (70, 130), (H - 100, 255)]):
+            w[(i % 4) * H + unit, k] = float("inf") if i % 2 else float("-inf")
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, h = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale, w, layer.bias,
+                                         c, h, reverse=layer.reverse)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, h))
+    flib.fluke_set_lstm_persistent(1)
+    for got, want in zip(*res):
+        if got.is_floating_point():
+            assert torch.equal(torch.isnan(got), torch.isnan(want))
+            got, want = got.nan_to_num(7.0), want.nan_to_num(7.0)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("B", [120, 121, 127, 135, 136, 151, 166, 180, 181, 211, 226, 240, 241])
 @pytest.mark.parametrize("T", [1, 2, 3, 9])
 def test_rows_projected_by_pair_give_the_bytes_of_the_l2_form(flib, B, T):
