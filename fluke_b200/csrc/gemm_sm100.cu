@@ -70,10 +70,14 @@ struct GemmDev {
     // ROTARY with whole sequences (M = n_seq * seqlen, seqlen >= 128): tiles are aligned to the
     // sequences (seq_tiles per sequence, the last one shifted up to end at the sequence end) and a
     // CTA takes a contiguous run of the list ordered by (tile-in-sequence, sequence), so the rows
-    // of successive tiles keep their positions and their sin/cos values stay in registers.
+    // of successive tiles keep their positions and their sin/cos values stay in registers. Where that takes no more items per CTA, a run is
+    // of one tile-in-sequence: a change of positions is 64 loads per thread in front of the tile's arithmetic, and with runs that cross
+    // from one to the next nearly every CTA had one. Us, runs of the whole list : of one tile-in-sequence, 7 x 1333 rows 13.06 : 11.77, 5 x 900 8.87 : 7.77, 16 x
+    // 1000 17.16 : 16.19, 32 x 1000 28.15 : 27.40; the others, whose runs did not cross, 1 to 3 % faster with the start below.
     int seq_tiles;  // 0: plain tiling, tile t covers rows [128 t, 128 t + 128)
     int n_seq;
     int items_per_cta;
+    int ctas_per_s;  // CTAs that share a tile-in-sequence; 0: runs of the whole list
     int passes_by;  // SILU: the output is larger than what L2 can keep, its lines go first
 };
 
@@ -88,10 +92,16 @@ struct TileCursor {
     int seq, s;      // sequence and tile in the sequence (whole sequences only)
     __device__ __forceinline__ TileCursor(const GemmDev &p, int m_first) {
         if (p.seq_tiles > 0) {
-            const int w = m_first * p.items_per_cta;
-            left = min(p.seq_tiles * p.n_seq - w, p.items_per_cta);
-            s = w / p.n_seq;
-            seq = w - s * p.n_seq;
+            if (p.ctas_per_s > 0) {
+                s = m_first / p.ctas_per_s;
+                seq = (m_first - s * p.ctas_per_s) * p.items_per_cta;
+                left = min(p.n_seq - seq, p.items_per_cta);
+            } else {
+                const int w = m_first * p.items_per_cta;
+                left = min(p.seq_tiles * p.n_seq - w, p.items_per_cta);
+                s = w / p.n_seq;
+                seq = w - s * p.n_seq;
+            }
             row = seq * p.seqlen + seq_pos0(p);
         } else {
             left = (p.num_m_tiles - m_first + p.ctas_per_n - 1) / p.ctas_per_n;
@@ -728,7 +738,7 @@ int plan_build(const fluke_sm100_gemm_t *g, int a_planes, GemmPlan *plan) {
     if (p.num_n_tiles > sms || p.num_k_blocks > SmemLayout<EPI, BN_MMA, STAGES>::kMaxKBlocks)
         return (int)cudaErrorInvalidValue;  // N tile count / K beyond what one resident tile covers
     p.passes_by = passes_by(g);
-    p.seq_tiles = 0; p.n_seq = 0; p.items_per_cta = 0;
+    p.seq_tiles = 0; p.n_seq = 0; p.items_per_cta = 0; p.ctas_per_s = 0;
     int items = p.num_m_tiles;
     if (EPI == FLUKE_SM100_EPI_ROTARY && p.seqlen >= kBlockM && g->M % p.seqlen == 0) {
         p.seq_tiles = (p.seqlen + kBlockM - 1) / kBlockM;
@@ -740,7 +750,14 @@ int plan_build(const fluke_sm100_gemm_t *g, int a_planes, GemmPlan *plan) {
     if (per_n < 1) per_n = 1;
     if (p.seq_tiles > 0) {
         p.items_per_cta = (items + per_n - 1) / per_n;
-        per_n = (items + p.items_per_cta - 1) / p.items_per_cta;  // no CTA without work
+        const int share = per_n / p.seq_tiles;
+        if (share > 0 && p.n_seq <= share * p.items_per_cta) {
+            p.items_per_cta = (p.n_seq + share - 1) / share;
+            p.ctas_per_s = (p.n_seq + p.items_per_cta - 1) / p.items_per_cta;  // no CTA without work
+            per_n = p.ctas_per_s * p.seq_tiles;
+        } else {
+            per_n = (items + p.items_per_cta - 1) / p.items_per_cta;
+        }
     }
     p.ctas_per_n = per_n;
     plan->grid = p.num_m_tiles > 0 ? per_n * p.num_n_tiles : 0;

@@ -153,6 +153,28 @@ def test_qkv_rotary_golden_from_reference_test(be, golden_tests):
     assert (got.float().cpu() - torch.from_numpy(g["rot_expected"].astype(np.float32))).abs().max() < 0.05  # cute/test_rotary.py ABS_TOL
 
 
+@pytest.mark.parametrize("batch,seqlen", [(7, 1333), (5, 900), (40, 129), (13, 255), (25, 384), (3, 1600), (9, 777), (24, 128), (17, 1000)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_qkv_rotary_of_many_chunks_equals_chunk_by_chunk(be, batch, seqlen, fp8):
+    """Runs of one tile-in-sequence or of the whole list of tiles (3 x 1600: no more CTAs than tiles in a sequence), last tiles of a sequence shifted
+    up, CTAs with fewer chunks than others, against one call per chunk, which the one-tile kernel or runs of a single chunk compute. Exact."""
+    m = batch * seqlen
+    g = torch.Generator().manual_seed(m)
+    quantise = prep.quantize_fp8_rows if fp8 else prep.quantize_int8_rows
+    (a, sa), (w, sb) = ([t.to(DEV).contiguous() for t in quantise(torch.randn(n, 512, generator=g) * s)] for n, s in ((m, 1.0), (1536, 0.02)))
+    sin, cos = (t.to(DEV) for t in prep.rotary_tables(seqlen, 64))
+    if fp8:
+        backend = ops.fp8_select(0, max_seq=2048)
+        a, w = a.view(torch.uint8), w.view(torch.uint8)
+        call = lambda x, s: ops.qkv_rotary_fp8(backend, x, w, s, sb, sin, cos, seqlen, plain=True)
+    else:
+        call = lambda x, s: ops.qkv_rotary_i8(be, x, w, s, sb, sin, cos, seqlen)
+    got = call(a, sa)
+    for i in range(batch):
+        rows = slice(i * seqlen, (i + 1) * seqlen)
+        assert torch.equal(got[rows].view(torch.int16), call(a[rows].contiguous(), sa[rows].contiguous()).view(torch.int16))
+
+
 def test_qkv_rotary_full_size_sampled_rows_and_v_passthrough(be):
     m, seqlen = 32000, 1000
     a, sa, w, sb = _qkv_inputs(m, torch.Generator().manual_seed(0))
