@@ -22,7 +22,8 @@
 //   exact in any order), which sends the f16 result to all. Projecting complete rows takes 24 MMAs per group
 //   at H = 768 and 96 KB of weights, this 4 and 16 KB; what one group waits for is the other's time.
 //
-// All exchanges are 16-byte st.async stores that complete on an mbarrier of the receiver.
+// All exchanges between CTAs are 16-byte st.async stores that complete on an mbarrier of the receiver; SPLIT: what stays in the CTA
+// is stored there and announced by an arrival per warp.
 //
 //   warp 0       loader: resident weights, x_down rows of every step; SPLIT: also the TMA stores of h_out
 //   warp 1       MMA issuer
@@ -194,6 +195,9 @@ __device__ __forceinline__ int2 lds64(uint32_t addr) {
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ int lds8(uint32_t addr) {
     int v;
     asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -269,7 +273,7 @@ enum : int {
 // The MMA issuer, warp 1. The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
 // K loops unrolled, so an MMA is issued every few cycles. kExact: for weights that are not finite.
 template <int V, int C, bool kExact>
-__device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupDev &p, int n_rows, int own_rows) {
+__device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupDev &p, int n_rows, int own_rows, uint32_t hh_bytes0, uint32_t hh_bytes1) {
     using K = GroupConst<V, C>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
@@ -410,7 +414,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
                     tc_mma_ts<kKindF16>(cols[g], tmem + kGTmemW + g * 64 + k * 8,
                                         rows[g] + uint64_t((2 * e + (k >> 2)) * (kHhTile >> 4) + 2 * (k & 3)), kIdescHh, 1u);
             tc_commit(&bar_acc[e]);
-            if (K::kPeerHh && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+            if (K::kPeerHh && i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], kGather ? uint32_t(n_rows) * 256 : e == 0 ? hh_bytes0 : hh_bytes1);
         }
         __syncwarp();
         return true;
@@ -436,7 +440,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
                                             rows[b] + uint64_t((k >> 2) * (kHhTile >> 4) + 2 * (k & 3)), kIdesc, 1u);
             for (int e = 0; e < 2; ++e) {
                 tc_commit(&bar_acc[e]);
-                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
+                if (i + 1 < p.T) mbar_arrive_expect_tx(&bar_hh[e], e == 0 ? hh_bytes0 : hh_bytes1);
             }
         }
         __syncwarp();
@@ -507,8 +511,8 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
 }
 // Out of line: as a branch or a second loop in the kernel it cost the other weights 1 to 3 % of a step.
 template <int V, int C>
-__device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev p, int n_rows) {
-    issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows, 0);
+__device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev p, int n_rows, uint32_t hh_bytes0, uint32_t hh_bytes1) {
+    issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows, 0, hh_bytes0, hh_bytes1);
 }
 
 // A row of the recurrent weights of a gate from its place in shared memory (two K blocks of 64 in the 128-byte swizzle) to its lane of tensor
@@ -582,12 +586,22 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         for (int k = 0; k < kPieces; ++k) n += own_piece(e, k);
         return n;
     };
+    // bytes of hh_down rows that a group receives from peers
+    auto hh_bytes = [&](int e) {
+        int n = rows_of(e);
+#pragma unroll
+        for (int k = 0; k < kPieces; ++k)
+            if (own_piece(e, k)) n -= min(4, rows_of(e) - 4 * k);
+        return uint32_t(n) * 256;
+    };
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
     if (threadIdx.x == 0) {
         auto arrivals = [&](int b) {   // warps that arrive, or one arrival with the expected bytes
             if (b == kBarAccFree) return kGather || both ? kGEpiWarps : kGEpiWarps / 2;
             if (b >= kBarWRead && b < kBarWRead + 4) return 4;
+            if (!kGather && (b == kBarSum || b == kBarSum + 1)) return 1 + 4 * own_pieces(b - kBarSum);
+            if (!kGather && (b == kBarHh || b == kBarHh + 1)) return 1 + (kGEpiWarps / 2) * own_pieces(b - kBarHh);
             if (b >= kBarWRead) return 1;
             if (kGather) return !kByPair && b == kBarHh ? kGEpiWarps : 1;
             return b == kBarCode || b == kBarCode + 1 || b == kBarSent ? kGEpiWarps / 2 : 1;
@@ -604,8 +618,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (s + 1 < p.T) mbar_arrive_expect_tx(&bar_h[s], uint32_t(n_rows) * H);
         } else {
             for (int e = 0; e < (both ? 2 : 1); ++e) {
-                mbar_arrive_expect_tx(&bar_hh[e], uint32_t(rows_of(e)) * 256);
-                if (const int n = own_pieces(e)) mbar_arrive_expect_tx(&bar_sum[e], uint32_t(n) * C * 2048);
+                mbar_arrive_expect_tx(&bar_hh[e], hh_bytes(e));
+                if (const int n = own_pieces(e)) mbar_arrive_expect_tx(&bar_sum[e], uint32_t(n) * (C - 1) * 2048);
             }
         }
     }
@@ -711,8 +725,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows, own_rows);
-        else issue_exact<V, C>(smem, tmem, p, n_rows);
+        if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows, own_rows, hh_bytes(0), hh_bytes(1));
+        else issue_exact<V, C>(smem, tmem, p, n_rows, hh_bytes(0), hh_bytes(1));
     } else {
         // ------------------------------ gates -------------------------------------------
         // thread = hidden unit. GATHER: a quarter of the rows; SPLIT: half of the rows of one group, eight warps each, so
@@ -911,11 +925,35 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             const uint32_t hh = smem_u32(smem + L.hh) + (2 * e + (q >> 1)) * kHhTile;
             const int s_row = 2 * part + ((lane >> 2) & 1), s_piece = (q & 1) * 4 + (lane & 3);
             const int own = own_pieces(e);
+            // Where the projected pieces and the rows of hh_down go. What stays in the CTA is stored there by itself: st.async takes it through the
+            // network like the rest, whose bytes bound the step where several clusters share a GPC (clusters of 1024 chunks had periods of 4520 to 5080
+            // cycles). Us per step, with : without, H = 768 700 chunks 2.138 : 2.114, 900 2.801 : 2.673, 1024 2.942 : 2.716; H = 1024 500 2.776 : 2.657, 700 2.911 :
+            // 2.823; H = 384 900 2.041 : 2.074, 1500 2.685 : 2.615; H = 512 1400 2.863 : 2.728. Up to 16 rows (GATHER) it costs 2 to 8 %: 300 chunks 1.730 : 1.814.
+            uint32_t p_to[kPieces / 2], p_bar[kPieces / 2];
+            int p_own = 0;   // one bit per piece that the CTA adds up itself
+#pragma unroll
+            for (int k = 0; k < kPieces / 2; ++k) {
+                const uint32_t n = uint32_t(kPieces * e + 2 * k + part), to = n % C;
+                p_to[k] = map_to_rank(recv + ((n / C) * C + rank) * 2048, to);
+                if (to == rank) p_own |= 1 << k, p_to[k] = recv + ((n / C) * C + rank) * 2048;
+                p_bar[k] = map_to_rank(bar_sum_e, to);
+            }
             // Every other eight columns' pieces have rows 2 and 3 in front: what a warp reads of them, two rows of 32 columns, then lies in all banks instead
             // of half of them. The sums stood 440 to 600 cycles behind their arrival, now 380 (us per step: H = 768 400 chunks 2.076 -> 2.052, 900 2.827 ->
             // 2.793; H = 384 1500 2.738 -> 2.689; H = 512 1400 2.960 -> 2.813; H = 768 1024 2.954 -> 2.959).
             const bool swap = lane & 8;
-            const uint32_t mine = recv + ((part ^ (swap ? 1 : 0)) * 8);
+            // the first of the group's pieces that this CTA adds up
+            const int k_first = (rank + C * ((kPieces * e + C - 1 - rank) / C)) - kPieces * e, rows_e = rows_of(e);
+            const uint32_t mine_first = recv + ((part ^ (swap ? 1 : 0)) * 8) + ((kPieces * e + k_first) / C) * C * 2048;
+            uint32_t hh_to[(C + 3) / 4], bar_to[(C + 3) / 4];
+#pragma unroll
+            for (int d = 0; d < C; d += 4) {
+                int to = d + (lane >> 3) + rank;            // start with a different peer in every CTA
+                if (to >= C) to -= C;
+                if (to >= C) to = 0;
+                hh_to[d / 4] = map_to_rank(hh, to);
+                bar_to[d / 4] = map_to_rank(bar_hh_e, to);
+            }
             for (int i = 0; i < p.T && ok; ++i) {
                 // ---- projection of this CTA's h_{i-1}: every other piece to its owner ----
                 ok = mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
@@ -933,26 +971,30 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 FLUKE_STAMP(blockIdx.x == 0 && (warp == 2 || warp == 10) && lane == 0, i * 16 + 6 + e, clock64());
 #pragma unroll
                 for (int k = 0; k < kPieces / 2; ++k) {
-                    const uint32_t n = uint32_t(kPieces * e + 2 * k + part), to = n % C;
-                    if (4 * (2 * k + part) < rows_of(e))
-                        store_to_peer(map_to_rank(recv + ((n / C) * C + rank) * 2048, to), make_uint4(swap ? v[k][2] : v[k][0], swap ? v[k][3] : v[k][1], swap ? v[k][0] : v[k][2], swap ? v[k][1] : v[k][3]),
-                                      map_to_rank(bar_sum_e, to));
+                    if (4 * (2 * k + part) >= rows_of(e)) continue;
+                    const uint4 w = make_uint4(swap ? v[k][2] : v[k][0], swap ? v[k][3] : v[k][1], swap ? v[k][0] : v[k][2], swap ? v[k][1] : v[k][3]);
+                    if (p_own >> k & 1) {
+                        sts128(p_to[k], w);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bar_sum[e]);
+                    } else {
+                        store_to_peer(p_to[k], w, p_bar[k]);
+                    }
                 }
                 // ---- the CTA's own pieces: summed, converted, to every CTA (two of the four rows) ----
                 if (own > 0) {
                     ok = mbar_wait<true>(&bar_sum[e], i & 1, abort_flag, 105);
                     if (!ok) break;
                     if (q == 0 && part == 0 && lane == 0 && i + 1 < p.T)   // for the next step
-                        mbar_arrive_expect_tx(&bar_sum[e], uint32_t(own) * C * 2048);
+                        mbar_arrive_expect_tx(&bar_sum[e], uint32_t(own) * (C - 1) * 2048);
                     FLUKE_STAMP(blockIdx.x == 0 && (warp == 2 || warp == 10) && lane == 0, i * 16 + 9 + e, clock64());
+                    uint32_t at_mine = mine_first;
 #pragma unroll 1
-                    for (int n = rank; n < kPieces * G; n += C) {
-                        const int k = n - kPieces * e;
-                        if (k < 0 || k >= kPieces || 4 * k >= rows_of(e)) continue;
+                    for (int k = k_first; 4 * k < rows_e; k += C, at_mine += C * 2048) {
                         int s0 = 0, s1 = 0;
 #pragma unroll
                         for (int j = 0; j < C; ++j) {
-                            const int2 w = lds64(mine + ((n / C) * C + j) * 2048);
+                            const int2 w = lds64(at_mine + j * 2048);
                             s0 += w.x;
                             s1 += w.y;
                         }
@@ -962,14 +1004,15 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                         __syncwarp();
                         const uint4 w = lds128(stage + (lane & 7) * 16);
                         const int row = 4 * k + s_row;
-                        const uint32_t at = hh + row * 128 + ((s_piece ^ (row & 7)) << 4);
+                        const uint32_t at = row * 128 + ((s_piece ^ (row & 7)) << 4);
 #pragma unroll
-                        for (int d = 0; d < C; d += 4) {
-                            const int m = d + (lane >> 3);
-                            int to = m + rank;            // start with a different peer in every CTA
-                            if (to >= C) to -= C;
-                            if (m < C && row < rows_of(e)) store_to_peer(map_to_rank(at, to), w, map_to_rank(bar_hh_e, to));
-                        }
+                        for (int d = 0; d < C; d += 4)
+                            if (d + (lane >> 3) < C && row < rows_e) {
+                                if (d == 0 && lane < 8) sts128(hh + at, w);
+                                else store_to_peer(hh_to[d / 4] + at, w, bar_to[d / 4]);
+                            }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bar_hh[e]);
                     }
                 }
                 // ---- gates, cell update, hidden codes ----
