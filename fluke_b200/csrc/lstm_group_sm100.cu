@@ -195,6 +195,10 @@ __device__ __forceinline__ int2 lds64(uint32_t addr) {
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
     return v;
 }
+// n arrivals at once
+__device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, int n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
 __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -938,6 +942,10 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (to == rank) p_own |= 1 << k, p_to[k] = recv + ((n / C) * C + rank) * 2048;
                 p_bar[k] = map_to_rank(bar_sum_e, to);
             }
+            int p_arrivals = 0;   // of those that there are
+#pragma unroll
+            for (int k = 0; k < kPieces / 2; ++k) p_arrivals += (p_own >> k & 1) && 4 * (2 * k + part) < rows_of(e);
+            if (p_arrivals == 0) p_own = 0;
             // Every other eight columns' pieces have rows 2 and 3 in front: what a warp reads of them, two rows of 32 columns, then lies in all banks instead
             // of half of them. The sums stood 440 to 600 cycles behind their arrival, now 380 (us per step: H = 768 400 chunks 2.076 -> 2.052, 900 2.827 ->
             // 2.793; H = 384 1500 2.738 -> 2.689; H = 512 1400 2.960 -> 2.813; H = 768 1024 2.954 -> 2.959).
@@ -973,13 +981,14 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 for (int k = 0; k < kPieces / 2; ++k) {
                     if (4 * (2 * k + part) >= rows_of(e)) continue;
                     const uint4 w = make_uint4(swap ? v[k][2] : v[k][0], swap ? v[k][3] : v[k][1], swap ? v[k][0] : v[k][2], swap ? v[k][1] : v[k][3]);
-                    if (p_own >> k & 1) {
-                        sts128(p_to[k], w);
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&bar_sum[e]);
-                    } else {
-                        store_to_peer(p_to[k], w, p_bar[k]);
-                    }
+                    if (p_own >> k & 1) sts128(p_to[k], w);
+                    else store_to_peer(p_to[k], w, p_bar[k]);
+                }
+                // announced behind the last of the pieces: in between it held the others up (H = 768 900 chunks 2.659 -> 2.621, 1024 2.706 -> 2.682; H = 384
+                // 1500 2.600 -> 2.633, others the same)
+                if (p_own) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_n(&bar_sum[e], p_arrivals);
                 }
                 // ---- the CTA's own pieces: summed, converted, to every CTA (two of the four rows) ----
                 if (own > 0) {
