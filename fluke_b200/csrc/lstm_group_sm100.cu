@@ -122,20 +122,25 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
            : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32, 2}
                     : GroupForm{48, false, 2, 24, 32, 56, 32, 2};
 }
-// Up to 8 rows: steps whose x part one MMA covers. MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
+// Steps whose x part one MMA covers, up to 8 rows and (two) from 17 to 32. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
 // sixteen that there are at least (42), and what is issued of them before the hidden codes arrive holds the issuer up: with 16 such MMAs per step
 // it saw codes that had travelled for 200 cycles after 430. Four steps per MMA are 8 per step, and twice the accumulators, which clusters of
 // two and three have the tensor memory for beside all projection weights. Two steps against four, us per step, x_down included: H = 384 32 chunks 1.156 :
 // 1.044, 120 1.186 : 1.078, 172 1.188 : 1.088, 250 1.200 : 1.160, 344 1.235 : 1.238; H = 256 32 1.137 : 1.027, 300 1.182 : 1.109, 528 1.222 : 1.202. With
 // more CTAs some projection weights have to give way: H = 512 32 chunks 1.166 : 1.125, but 200 1.269 : 1.339; H = 640 200 1.366 : 1.467.
-__host__ __device__ constexpr int group_x_steps(int V, int C) { return V != 0 ? 1 : C <= 3 ? 4 : 2; }
+// 17 to 32 rows: an MMA of 64 columns takes 48 cycles, one of 32 takes 44, and while they run little else gets at the shared memory (a step without any x part takes
+// 10 % less at H = 768, 15 % at H = 512). One step against two: H = 768 360 chunks 2.031 : 1.941, 500 2.063 : 1.989, 700 2.103 : 2.037; H = 384 900 2.062 : 1.934; H =
+// 256 1200 2.045 : 1.827; H = 512 700 2.047 : 1.835; H = 640 600 2.063 : 1.885; H = 896 400 2.060 : 2.050; clusters of eight 300 2.089 : 2.138.
+__host__ __device__ constexpr int group_x_steps(int V, int C) { return V == 2 ? (C <= 7 ? 2 : 1) : V != 0 ? 1 : C <= 3 ? 4 : 2; }
 // Accumulator columns from gate to gate.
 __host__ __device__ constexpr int group_stride(int V, int C) { return group_x_steps(V, C) == 4 ? 32 : group_form(V).stride; }
+// Columns of all gate accumulators. Two steps of 17 to 32 rows: six places of 32 columns hold the four gates of a step and two of the next.
+__host__ __device__ constexpr int group_acc_cols(int V, int C) { return (V == 2 && group_x_steps(V, C) == 2 ? 6 : 4) * group_stride(V, C); }
 // K steps (32 units, 8 columns) of the projection weights that fit in tensor memory beside the gate weights, the gate
 // accumulators and the projections.
 __host__ __device__ constexpr int group_dn_ts(int V, int C) {
     const GroupForm f = group_form(V);
-    const int fit = (kGTmemW - 4 * group_stride(V, C) - f.proj) / 8, all = f.gather ? 4 * C : 4;
+    const int fit = (kGTmemW - group_acc_cols(V, C) - f.proj) / 8, all = f.gather ? 4 * C : 4;
     return fit < all ? fit : all;
 }
 // Four rows of a group are projected as one piece (16 bytes per projection column). The pieces of all groups are dealt to
@@ -159,7 +164,7 @@ __host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
     const GroupForm f = group_form(V);
     GroupLayout l = {};
     l.x = kGWxBytes;                              // x_down rows, see x_half
-    l.hh = l.x + (group_x_steps(V, C) == 4 ? 11 : f.x_slots) * f.groups * f.rows * 256;
+    l.hh = l.x + (group_x_steps(V, C) == 4 ? 11 : V == 2 && group_x_steps(V, C) == 2 ? 4 : f.x_slots) * f.groups * f.rows * 256;
     // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
     l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
     // projection weights [128 x 128 B] (by pair [64 x 128 B]) of the K blocks that are not all in tensor memory
@@ -235,8 +240,10 @@ struct GroupConst {
     static constexpr GroupLayout L = group_layout(V, C);
     static constexpr bool kGather = F.gather;
     static constexpr int G = F.groups, NB = G * F.rows, S = group_stride(V, C), H = C * kGUnits;
-    static constexpr bool kTwoSteps = group_x_steps(V, C) == 2;    // an x MMA covers two steps
+    static constexpr bool kTwoSteps = kGather && group_x_steps(V, C) == 2;    // an x MMA covers two steps
     static constexpr bool kFourSteps = group_x_steps(V, C) == 4;   // or four
+    static constexpr bool kTwoStepsSplit = !kGather && group_x_steps(V, C) == 2;   // SPLIT: two steps, see x_half
+    static constexpr int kAcc = group_acc_cols(V, C);         // columns of the gate accumulators; the projections' follow
     static constexpr int kXSlots = kFourSteps ? 8 : kTwoSteps ? 4 : F.x_slots;
     static constexpr int kXRing = kFourSteps ? 11 : 5;        // slots of 8 rows when an x MMA covers several steps
     static constexpr int kFirstBarX = kFourSteps ? 32 : 1;
@@ -251,7 +258,7 @@ struct GroupConst {
     static constexpr int kDnTs = group_dn_ts(V, C);
     static constexpr int kDnCol = kGTmemW - 8 * kDnTs;        // first column of the projection weights in tensor memory
     static constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
-    static_assert(4 * S + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
+    static_assert(kAcc + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
     static_assert(L.dynamic <= kGMaxSmem, "shared memory of a CTA");
     static_assert(!kByPair || (C % 2 == 0 && F.rows <= 2 * C), "a pair's rows are one per quarter of the gate warps");
 };
@@ -292,7 +299,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     [[maybe_unused]] const int lane = threadIdx.x & 31;
     auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
-    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, kFourSteps ? 32 : kTwoSteps ? 16 : NB);
+    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, K::kTwoStepsSplit ? 2 * NB : kFourSteps ? 32 : kTwoSteps ? 16 : NB);
     constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
     constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
     uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
@@ -308,25 +315,29 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     // the rows of two or four steps. Two: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
     // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones. Four: step i computes gate
     // i mod 4 of itself and the next three, whose rows are contiguous in a ring of eight slots of which the first three are repeated behind it.
-    constexpr int kX = kFourSteps ? 8 : kTwoSteps ? 16 : 32;
+    // 17 to 32 rows, two steps: step i computes gates 0 and 1 (i even) or 2 and 3 of itself and the next, 64 columns each. What has been read makes room for them
+    // if even steps lie behind the odd ones of their window: gates 0 and 1 in places 0, 1 and 3, 4 of the six, 2 and 3 in 1, 2 and 4, 5, so that gate g of step i
+    // is at place 3 (g mod 2) + g / 2 + (1 if i is even). A window is loaded as one tile of 64 rows per K block, each step twice.
+    constexpr int kX = kFourSteps ? 8 : kTwoSteps || K::kTwoStepsSplit ? 16 : 32;
     auto x_half = [&](auto from, auto to, int i, bool release = true, int gate = 0) {
         constexpr int first = decltype(from)::value, end = decltype(to)::value;
-        const int slot = i & (kXSlots - 1);
-        const uint64_t d_x = d_x0 + uint64_t(slot * (kTwoSteps || kFourSteps ? NB * 8 : NB * 16));
-        const int g0 = kFourSteps ? (kExact ? gate : i & 3) : kTwoSteps ? 2 * (i & 1) : 0;
+        const int slot = (K::kTwoStepsSplit ? i + 1 : i) & (kXSlots - 1);
+        const uint64_t d_x = d_x0 + uint64_t(slot * (K::kTwoStepsSplit ? NB * 32 : kTwoSteps || kFourSteps ? NB * 8 : NB * 16));
+        const int g0 = kFourSteps ? (kExact ? gate : i & 3) : kTwoSteps || K::kTwoStepsSplit ? 2 * (i & 1) : 0;
         if (elect_one()) {
 #pragma unroll
             for (int m = first; m < end; ++m) {
                 const int g = m >> 3, k = m & 7;
-                tc_mma<kKindF16>(tmem + (g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                 d_x + uint64_t((k >> 2) * ((kTwoSteps || kFourSteps ? K::kXRing : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+                tc_mma<kKindF16>(tmem + (K::kTwoStepsSplit ? 3 * g + (i & 1) : g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
+                                 d_x + uint64_t((k >> 2) * ((kTwoSteps || kFourSteps ? K::kXRing : K::kTwoStepsSplit ? 2 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
             }
             if (end == kX && release) tc_commit(&bar_x_free[slot]);
         }
         __syncwarp();
     };
     auto wait_x = [&](int step) {
-        if (step < p.T) ok = ok && mbar_wait(&bar_x[step & (kXSlots - 1)], (step / kXSlots) & 1, abort_flag, 99);
+        const int n = K::kTwoStepsSplit ? step + 1 : step;
+        if (step < p.T) ok = ok && mbar_wait(&bar_x[n & (kXSlots - 1)], (n / kXSlots) & 1, abort_flag, 99);
         return ok;
     };
     auto wait_acc = [&]() {
@@ -351,7 +362,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint64_t rows = d_h0 + uint64_t(e * (kTile >> 4) + 2 * k);
-                constexpr int kTo = 4 * S + (kOneProj ? 0 : e * F.n);
+                constexpr int kTo = K::kAcc + (kOneProj ? 0 : e * F.n);
                 if (k < kDnTs) tc_mma_ts<kKindI8>(tmem + kTo, tmem + kDnCol + 8 * k, rows, kIdescP, k != 0);
                 else tc_mma<kKindI8>(tmem + kTo, d_dn + uint64_t(2 * k), rows, kIdescP, k != 0);
             }
@@ -376,8 +387,8 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const uint64_t rows = d_h + uint64_t(kb * (kTile >> 4) + 2 * k);
-                    if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + 4 * S, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdesc, (kb | k) != 0);
-                    else tc_mma<kKindI8>(tmem + 4 * S, d_dn + uint64_t((kb - kDnTs / 4) * (K::kDnRows * 8) + 2 * k), rows, kIdesc, (kb | k) != 0);
+                    if (4 * kb + k < kDnTs) tc_mma_ts<kKindI8>(tmem + K::kAcc, tmem + kDnCol + 8 * (4 * kb + k), rows, kIdesc, (kb | k) != 0);
+                    else tc_mma<kKindI8>(tmem + K::kAcc, d_dn + uint64_t((kb - kDnTs / 4) * (K::kDnRows * 8) + 2 * k), rows, kIdesc, (kb | k) != 0);
                 }
             tc_commit(&bar_proj[0]);
             if (kByPair && i > 0 && i + 1 < p.T) mbar_arrive_expect_tx(&bar_h[0], uint32_t(own_rows) * H);  // for h_i
@@ -396,7 +407,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             rows[g] = d_hh;
-            cols[g] = tmem + g * S + F.rows * e;
+            cols[g] = tmem + (K::kTwoStepsSplit ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + F.rows * e;
             if (kTwoSteps) rows[g] += (i ^ (g >> 1)) & 1 ? 0 : 64;
             if (kFourSteps) {
                 const int at = kExact ? 0 : (i - g) & 3;
@@ -455,6 +466,10 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         if (ok) ok = mbar_wait(&bar_x[0], 0, abort_flag, 99);
         if (ok) x_half(Int<0>{}, Int<16>{}, -1, false);
     }
+    if constexpr (K::kTwoStepsSplit) {
+        // gates 2 and 3 of step 0: as the second step of a window that begins before it
+        if (wait_x(-1)) x_half(Int<0>{}, Int<kX>{}, -1);
+    }
     if constexpr (kFourSteps) {
         // gates 1, 2 and 3 of the first steps, as of steps before them: whatever is in the slots enters columns that nothing reads
         for (int w = -3; w < 0 && wait_x(w + 3); ++w) x_half(Int<0>{}, Int<kX>{}, w, false, w & 3);
@@ -500,10 +515,11 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
             x_half(Int<0>{}, Int<kFirstX>{}, i);
             if (both && !wait_sent(2 * i + 1)) break;
             if (!project(Int<1>{}, i)) break;
-            x_half(Int<kFirstX>{}, Int<24>{}, i);
+            constexpr int kLastX = kX - kX / 4;
+            x_half(Int<kFirstX>{}, Int<kLastX>{}, i);
             // the gate warps overwrite the hidden codes once the hh half is complete
             if (i > 0) ok = ok && mbar_wait(bar_stored, (i - 1) & 1, abort_flag, 104);
-            x_half(Int<24>{}, Int<32>{}, i);
+            x_half(Int<kLastX>{}, Int<kX>{}, i);
             if (kExact && both) {
                 if (!hh_both()) break;
                 continue;
@@ -695,7 +711,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         if (elect_one()) {
             bool ok = true;
             auto load_x = [&](int i) {
-                const int s = i & (kXSlots - 1), u = i / kXSlots;
+                const int s = (K::kTwoStepsSplit ? i + 1 : i) & (kXSlots - 1), u = (K::kTwoStepsSplit ? i + 1 : i) / kXSlots;
                 if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
                 if (!ok) return;
                 if constexpr (kTwoSteps || kFourSteps) {
@@ -704,6 +720,13 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     for (int kb = 0; kb < 2; ++kb)
                         for (int n = 0; n < (twice ? 2 : 1); ++n)
                             tma_load_4d(smem + L.x + (kb * K::kXRing + s + kXSlots * n) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
+                } else if constexpr (K::kTwoStepsSplit) {
+                    // steps i and i + 1, the odd one in front
+                    const int from = max(i, 0), to = min(i + 2, p.T);
+                    mbar_arrive_expect_tx(&bar_x[s], NB * 256 * (to - from));
+                    for (int t = from; t < to; ++t)
+                        for (int kb = 0; kb < 2; ++kb)
+                            tma_load_4d(smem + L.x + s * (NB * 512) + (kb * 2 + 1 - (t & 1)) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(t));
                 } else {
                     mbar_arrive_expect_tx(&bar_x[s], NB * 256);
                     tma_load_4d(smem + L.x + s * (NB * 256), &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
@@ -713,14 +736,16 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 for (int i = 0; i < p.T && ok; ++i) load_x(i);
             } else {
                 // between the loads the stores of the hidden rows
-                for (int i = 0; i < min(p.T, kXSlots); ++i) load_x(i);
+                constexpr int kEarly = K::kTwoStepsSplit ? 1 : 0;   // windows that begin before step 0
+                for (int i = -kEarly; i < min(p.T, kXSlots - kEarly); ++i) load_x(i);
                 for (int i = 0; i < p.T && ok; ++i) {
+                    if (K::kTwoStepsSplit && i + 1 < p.T) load_x(i + 1);   // of two tiles, the other one is in use
                     for (int e = 0; e < (both ? 2 : 1) && ok; ++e) {
                         ok = mbar_wait(&bar_code[e], i & 1, abort_flag, 107);
                         if (ok) tma_store_3d(e > 0 ? &tm_ol : &tm_o, smem + L.h + e * kTile, n0, m0 + F.rows * e, time_of(i));
                     }
                     tma_store_commit();
-                    if (i + kXSlots < p.T) load_x(i + kXSlots);
+                    if (!K::kTwoStepsSplit && i + kXSlots < p.T) load_x(i + kXSlots);
                     tma_store_wait_read<0>();
                     mbar_arrive(bar_stored);
                 }
@@ -789,7 +814,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     slot ^= 2048;
                     tc_fence_after_sync();
                     uint32_t v, next;
-                    tmem_ld_32x2(t_lane + 4 * S + part, v, next);
+                    tmem_ld_32x2(t_lane + K::kAcc + part, v, next);
                     tmem_ld_wait();
                     if (lane < 16) sts16(stage + slot + q * 32 + lane * 2, __half_as_ushort(__float2half_rn(float(int(v)) * sc)));
                     tc_fence_before_sync();
@@ -858,7 +883,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (my_rows > 0) {
                     tc_fence_after_sync();
                     uint32_t v[4];
-                    tmem_ld_32x4(t_lane + 4 * S + r0, v);
+                    tmem_ld_32x4(t_lane + K::kAcc + r0, v);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 2 * kPairs; ++j)
@@ -921,7 +946,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             const uint32_t code = smem_u32(smem + L.h) + e * kTile + r0 * 128 + (((q * 2 + (lane >> 4)) ^ (r0 & 7)) << 4) + (lane & 15);
             auto code_at = [&](int j) { return (code ^ ((j & 7) << 4)) + j * 128; };
             const uint32_t t_acc = t_lane + F.rows * e + r0;
-            const uint32_t t_proj = t_lane + 4 * S + (kOneProj ? 0 : e * F.n) + part * 4;
+            const uint32_t t_proj = t_lane + K::kAcc + (kOneProj ? 0 : e * F.n) + part * 4;
             const float sc = (1.0f / 127.0f) * __ldg(p.dn_scale + q * 32 + lane);   // operand order of the dequant GEMM: sa * sb
             const uint32_t recv = smem_u32(smem + L.recv) + uint32_t(q * 32 + lane) * 16;
             const uint32_t bar_sum_e = smem_u32(&bar_sum[e]), bar_hh_e = smem_u32(&bar_hh[e]);
@@ -1033,7 +1058,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 #pragma unroll
                 for (int b = 0; b < kPairs / 2; ++b)
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) tmem_ld_32x4(t_acc + g * S + 4 * b, a[b][g]);
+                    for (int g = 0; g < 4; ++g)
+                        tmem_ld_32x4(t_acc + (K::kTwoStepsSplit ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + 4 * b, a[b][g]);
                 tmem_ld_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -1178,7 +1204,7 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
         // both K blocks of a row range in one box: the 128-byte blocks of a row are a dimension
         const uint64_t dims[4] = {64, uint64_t(B), 2, uint64_t(T)};
         const uint64_t strides[3] = {uint64_t(R) * 2, 128, uint64_t(B) * R * 2};
-        const uint32_t box[4] = {64, uint32_t(f.groups * f.rows), f.rows == 8 ? 1u : 2u, 1};
+        const uint32_t box[4] = {64, uint32_t(f.groups * f.rows), group_x_steps(g.form, C) > 1 ? 1u : 2u, 1};
         rc = make_tmap_nd(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_down, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }

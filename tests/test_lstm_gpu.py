@@ -574,6 +574,29 @@ def test_four_steps_per_contraction_give_the_bytes_of_the_l2_form(flib, H, B, T,
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("H,B", [(256, 1057), (256, 2112), (384, 689), (384, 1376), (512, 513), (512, 1024), (640, 443), (640, 832), (768, 353), (768, 704),
+                                 (896, 289), (896, 544), (1024, 300)])
+@pytest.mark.parametrize("T", [1, 2, 3, 6, 7])
+def test_two_groups_of_sixteen_rows_give_the_bytes_of_the_l2_form(flib, H, B, T):
+    """17 to 32 rows per cluster on a B200, the fewest and the most at each cluster size: two steps' x rows per contraction (up to clusters of seven), windows that
+    begin before the first step and end behind the last, both parities and directions; pieces that stay in a CTA. Against the L2-exchange form. Exact."""
+    layer, x, xs = _layer_case(T, B, H, 128, H + B + T, T % 2 == 0)
+    g = torch.Generator().manual_seed(B)
+    c0 = (torch.randn(B, H, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-128, 128, (B, H), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, h = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale,
+                                         layer.w_up, layer.bias, c, h, reverse=layer.reverse)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, h))
+    flib.fluke_set_lstm_persistent(1)
+    for got, want in zip(*res):
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("B", [120, 121, 127, 135, 136, 151, 166, 180, 181, 211, 226, 240, 241])
 @pytest.mark.parametrize("T", [1, 2, 3, 9])
 def test_rows_projected_by_pair_give_the_bytes_of_the_l2_form(flib, B, T):
