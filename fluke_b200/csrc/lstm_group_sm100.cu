@@ -122,7 +122,7 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
            : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32, 2}
                     : GroupForm{48, false, 2, 24, 32, 56, 32, 2};
 }
-// Steps whose x part one MMA covers, up to 8 rows and (two) from 17 to 32. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
+// Steps whose x part one MMA covers. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
 // sixteen that there are at least (42), and what is issued of them before the hidden codes arrive holds the issuer up: with 16 such MMAs per step
 // it saw codes that had travelled for 200 cycles after 430. Four steps per MMA are 8 per step, and twice the accumulators, which clusters of
 // two and three have the tensor memory for beside all projection weights. Two steps against four, us per step, x_down included: H = 384 32 chunks 1.156 :
@@ -131,11 +131,13 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
 // 17 to 32 rows: an MMA of 64 columns takes 48 cycles, one of 32 takes 44, and while they run little else gets at the shared memory (a step without any x part takes
 // 10 % less at H = 768, 15 % at H = 512). One step against two: H = 768 360 chunks 2.031 : 1.941, 500 2.063 : 1.989, 700 2.103 : 2.037; H = 384 900 2.062 : 1.934; H =
 // 256 1200 2.045 : 1.827; H = 512 700 2.047 : 1.835; H = 640 600 2.063 : 1.885; H = 896 400 2.060 : 2.050; clusters of eight 300 2.089 : 2.138.
-__host__ __device__ constexpr int group_x_steps(int V, int C) { return V == 2 ? (C <= 7 ? 2 : 1) : V != 0 ? 1 : C <= 3 ? 4 : 2; }
+// 9 to 16 rows, where the larger accumulators leave tensor memory for all projection weights: H = 256 600 chunks 1.455 : 1.369, 1000 1.545 : 1.507; H = 384 400
+// 1.485 : 1.395, 600 1.569 : 1.547, 680 1.589 : 1.593; H = 512 300 1.494 : 1.462, 500 1.657 : 1.654. Without: H = 768 200 1.606 : 1.667, 300 1.758 : 1.842.
+__host__ __device__ constexpr int group_x_steps(int V, int C) { return V == 2 ? (C <= 7 ? 2 : 1) : V == 1 ? (C <= 4 ? 2 : 1) : V != 0 ? 1 : C <= 3 ? 4 : 2; }
 // Accumulator columns from gate to gate.
 __host__ __device__ constexpr int group_stride(int V, int C) { return group_x_steps(V, C) == 4 ? 32 : group_form(V).stride; }
-// Columns of all gate accumulators. Two steps of 17 to 32 rows: six places of 32 columns hold the four gates of a step and two of the next.
-__host__ __device__ constexpr int group_acc_cols(int V, int C) { return (V == 2 && group_x_steps(V, C) == 2 ? 6 : 4) * group_stride(V, C); }
+// Columns of all gate accumulators. Two steps of more than 8 rows: six places of a gate's columns hold the four gates of a step and two of the next.
+__host__ __device__ constexpr int group_acc_cols(int V, int C) { return (V > 0 && group_x_steps(V, C) == 2 ? 6 : 4) * group_stride(V, C); }
 // K steps (32 units, 8 columns) of the projection weights that fit in tensor memory beside the gate weights, the gate
 // accumulators and the projections.
 __host__ __device__ constexpr int group_dn_ts(int V, int C) {
@@ -164,7 +166,7 @@ __host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
     const GroupForm f = group_form(V);
     GroupLayout l = {};
     l.x = kGWxBytes;                              // x_down rows, see x_half
-    l.hh = l.x + (group_x_steps(V, C) == 4 ? 11 : V == 2 && group_x_steps(V, C) == 2 ? 4 : f.x_slots) * f.groups * f.rows * 256;
+    l.hh = l.x + (group_x_steps(V, C) == 4 ? 11 : V > 0 && group_x_steps(V, C) == 2 ? 4 : f.x_slots) * f.groups * f.rows * 256;
     // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
     l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
     // projection weights [128 x 128 B] (by pair [64 x 128 B]) of the K blocks that are not all in tensor memory
@@ -240,9 +242,9 @@ struct GroupConst {
     static constexpr GroupLayout L = group_layout(V, C);
     static constexpr bool kGather = F.gather;
     static constexpr int G = F.groups, NB = G * F.rows, S = group_stride(V, C), H = C * kGUnits;
-    static constexpr bool kTwoSteps = kGather && group_x_steps(V, C) == 2;    // an x MMA covers two steps
+    static constexpr bool kTwoSteps = V == 0 && group_x_steps(V, C) == 2;    // an x MMA covers two steps
     static constexpr bool kFourSteps = group_x_steps(V, C) == 4;   // or four
-    static constexpr bool kTwoStepsSplit = !kGather && group_x_steps(V, C) == 2;   // SPLIT: two steps, see x_half
+    static constexpr bool kTwoStepsWide = V > 0 && group_x_steps(V, C) == 2;   // two steps of more than 8 rows, see x_half
     static constexpr int kAcc = group_acc_cols(V, C);         // columns of the gate accumulators; the projections' follow
     static constexpr int kXSlots = kFourSteps ? 8 : kTwoSteps ? 4 : F.x_slots;
     static constexpr int kXRing = kFourSteps ? 11 : 5;        // slots of 8 rows when an x MMA covers several steps
@@ -299,7 +301,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     [[maybe_unused]] const int lane = threadIdx.x & 31;
     auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
-    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, K::kTwoStepsSplit ? 2 * NB : kFourSteps ? 32 : kTwoSteps ? 16 : NB);
+    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, K::kTwoStepsWide ? 2 * NB : kFourSteps ? 32 : kTwoSteps ? 16 : NB);
     constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
     constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
     uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
@@ -315,28 +317,28 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     // the rows of two or four steps. Two: even steps compute gates 0 and 1 of themselves and the next, odd ones gates 2 and
     // 3. Slot s of five holds step s mod 4, so that a step's rows and the next one's are sixteen contiguous ones. Four: step i computes gate
     // i mod 4 of itself and the next three, whose rows are contiguous in a ring of eight slots of which the first three are repeated behind it.
-    // 17 to 32 rows, two steps: step i computes gates 0 and 1 (i even) or 2 and 3 of itself and the next, 64 columns each. What has been read makes room for them
+    // More than 8 rows, two steps: step i computes gates 0 and 1 (i even) or 2 and 3 of itself and the next, side by side. What has been read makes room for them
     // if even steps lie behind the odd ones of their window: gates 0 and 1 in places 0, 1 and 3, 4 of the six, 2 and 3 in 1, 2 and 4, 5, so that gate g of step i
-    // is at place 3 (g mod 2) + g / 2 + (1 if i is even). A window is loaded as one tile of 64 rows per K block, each step twice.
-    constexpr int kX = kFourSteps ? 8 : kTwoSteps || K::kTwoStepsSplit ? 16 : 32;
+    // is at place 3 (g mod 2) + g / 2 + (1 if i is even). A window is loaded as one tile of both steps' rows per K block, each step twice.
+    constexpr int kX = kFourSteps ? 8 : kTwoSteps || K::kTwoStepsWide ? 16 : 32;
     auto x_half = [&](auto from, auto to, int i, bool release = true, int gate = 0) {
         constexpr int first = decltype(from)::value, end = decltype(to)::value;
-        const int slot = (K::kTwoStepsSplit ? i + 1 : i) & (kXSlots - 1);
-        const uint64_t d_x = d_x0 + uint64_t(slot * (K::kTwoStepsSplit ? NB * 32 : kTwoSteps || kFourSteps ? NB * 8 : NB * 16));
-        const int g0 = kFourSteps ? (kExact ? gate : i & 3) : kTwoSteps || K::kTwoStepsSplit ? 2 * (i & 1) : 0;
+        const int slot = (K::kTwoStepsWide ? i + 1 : i) & (kXSlots - 1);
+        const uint64_t d_x = d_x0 + uint64_t(slot * (K::kTwoStepsWide ? NB * 32 : kTwoSteps || kFourSteps ? NB * 8 : NB * 16));
+        const int g0 = kFourSteps ? (kExact ? gate : i & 3) : kTwoSteps || K::kTwoStepsWide ? 2 * (i & 1) : 0;
         if (elect_one()) {
 #pragma unroll
             for (int m = first; m < end; ++m) {
                 const int g = m >> 3, k = m & 7;
-                tc_mma<kKindF16>(tmem + (K::kTwoStepsSplit ? 3 * g + (i & 1) : g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                 d_x + uint64_t((k >> 2) * ((kTwoSteps || kFourSteps ? K::kXRing : K::kTwoStepsSplit ? 2 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+                tc_mma<kKindF16>(tmem + (K::kTwoStepsWide ? 3 * g + (i & 1) : g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
+                                 d_x + uint64_t((k >> 2) * ((kTwoSteps || kFourSteps ? K::kXRing : K::kTwoStepsWide ? 2 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
             }
             if (end == kX && release) tc_commit(&bar_x_free[slot]);
         }
         __syncwarp();
     };
     auto wait_x = [&](int step) {
-        const int n = K::kTwoStepsSplit ? step + 1 : step;
+        const int n = K::kTwoStepsWide ? step + 1 : step;
         if (step < p.T) ok = ok && mbar_wait(&bar_x[n & (kXSlots - 1)], (n / kXSlots) & 1, abort_flag, 99);
         return ok;
     };
@@ -407,7 +409,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             rows[g] = d_hh;
-            cols[g] = tmem + (K::kTwoStepsSplit ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + F.rows * e;
+            cols[g] = tmem + (K::kTwoStepsWide ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + F.rows * e;
             if (kTwoSteps) rows[g] += (i ^ (g >> 1)) & 1 ? 0 : 64;
             if (kFourSteps) {
                 const int at = kExact ? 0 : (i - g) & 3;
@@ -466,7 +468,7 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         if (ok) ok = mbar_wait(&bar_x[0], 0, abort_flag, 99);
         if (ok) x_half(Int<0>{}, Int<16>{}, -1, false);
     }
-    if constexpr (K::kTwoStepsSplit) {
+    if constexpr (K::kTwoStepsWide) {
         // gates 2 and 3 of step 0: as the second step of a window that begins before it
         if (wait_x(-1)) x_half(Int<0>{}, Int<kX>{}, -1);
     }
@@ -478,12 +480,12 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         // Fresh values in every step: hoisted out of the loop, the operands of its MMAs would fill
         // more registers than there are.
         asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
-        constexpr int kFirstX = kFourSteps ? 4 : kTwoSteps ? 10 : kByPair ? 16 : kGather ? 24 : 2;
+        constexpr int kFirstX = kFourSteps ? 4 : kTwoSteps ? 10 : kByPair ? 16 : kGather ? (K::kTwoStepsWide ? 12 : 24) : 2;
         if constexpr (kGather) {
             // Most of the x part while the hidden state is computed and travels, the rest while the
             // projection is converted. 20 / 24 / 28 of 32 in front, us per step (x_down included): H = 768 200 chunks 1.62 / 1.57 / 1.64, 300
             // 1.74 / 1.70 / 1.73; H = 384 600 1.58 / 1.54 / 1.63; H = 512 500 1.68 / 1.62 / 1.65; H = 896 180 1.71 / 1.70 / 1.74. 8 / 10 / 12 of 16: H = 768
-            // 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 1024 60 1.42 / 1.40 / 1.44. 3 / 4 / 5 of 8 within 1 % of each other. By pair 12 / 16 /
+            // 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 1024 60 1.42 / 1.40 / 1.44. 10 / 12 of 16 for more rows: H = 384 600 1.559 / 1.547. 3 / 4 / 5 of 8 within 1 % of each other. By pair 12 / 16 /
             // 20 of 32: 135 chunks 1.68 / 1.66 / 1.73, 240 1.86 / 1.87 / 1.88.
             if (!wait_x(kFourSteps ? i + 3 : kTwoSteps ? i + 1 : i) || !wait_acc()) break;
             FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
@@ -711,7 +713,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         if (elect_one()) {
             bool ok = true;
             auto load_x = [&](int i) {
-                const int s = (K::kTwoStepsSplit ? i + 1 : i) & (kXSlots - 1), u = (K::kTwoStepsSplit ? i + 1 : i) / kXSlots;
+                const int s = (K::kTwoStepsWide ? i + 1 : i) & (kXSlots - 1), u = (K::kTwoStepsWide ? i + 1 : i) / kXSlots;
                 if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
                 if (!ok) return;
                 if constexpr (kTwoSteps || kFourSteps) {
@@ -720,7 +722,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                     for (int kb = 0; kb < 2; ++kb)
                         for (int n = 0; n < (twice ? 2 : 1); ++n)
                             tma_load_4d(smem + L.x + (kb * K::kXRing + s + kXSlots * n) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
-                } else if constexpr (K::kTwoStepsSplit) {
+                } else if constexpr (K::kTwoStepsWide) {
                     // steps i and i + 1, the odd one in front
                     const int from = max(i, 0), to = min(i + 2, p.T);
                     mbar_arrive_expect_tx(&bar_x[s], NB * 256 * (to - from));
@@ -733,19 +735,19 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 }
             };
             if constexpr (kGather) {
-                for (int i = 0; i < p.T && ok; ++i) load_x(i);
+                for (int i = K::kTwoStepsWide ? -1 : 0; i < p.T && ok; ++i) load_x(i);
             } else {
                 // between the loads the stores of the hidden rows
-                constexpr int kEarly = K::kTwoStepsSplit ? 1 : 0;   // windows that begin before step 0
+                constexpr int kEarly = K::kTwoStepsWide ? 1 : 0;   // windows that begin before step 0
                 for (int i = -kEarly; i < min(p.T, kXSlots - kEarly); ++i) load_x(i);
                 for (int i = 0; i < p.T && ok; ++i) {
-                    if (K::kTwoStepsSplit && i + 1 < p.T) load_x(i + 1);   // of two tiles, the other one is in use
+                    if (K::kTwoStepsWide && i + 1 < p.T) load_x(i + 1);   // of two tiles, the other one is in use
                     for (int e = 0; e < (both ? 2 : 1) && ok; ++e) {
                         ok = mbar_wait(&bar_code[e], i & 1, abort_flag, 107);
                         if (ok) tma_store_3d(e > 0 ? &tm_ol : &tm_o, smem + L.h + e * kTile, n0, m0 + F.rows * e, time_of(i));
                     }
                     tma_store_commit();
-                    if (!K::kTwoStepsSplit && i + kXSlots < p.T) load_x(i + kXSlots);
+                    if (!K::kTwoStepsWide && i + kXSlots < p.T) load_x(i + kXSlots);
                     tma_store_wait_read<0>();
                     mbar_arrive(bar_stored);
                 }
@@ -899,7 +901,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 uint32_t cols[4];
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
-                    cols[g] = t_lane + g * S + r0 + (kTwoSteps ? ((i ^ (g >> 1)) & 1) * 8 : 0);
+                    cols[g] = t_lane + (K::kTwoStepsWide ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + r0 + (kTwoSteps ? ((i ^ (g >> 1)) & 1) * 8 : 0);
                     if (kFourSteps) {
                         cols[g] += 8 * (finite ? (i - g) & 3 : 0);
                         asm volatile("" : "+r"(cols[g]));   // worked out in front of the wait
@@ -1059,7 +1061,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 for (int b = 0; b < kPairs / 2; ++b)
 #pragma unroll
                     for (int g = 0; g < 4; ++g)
-                        tmem_ld_32x4(t_acc + (K::kTwoStepsSplit ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + 4 * b, a[b][g]);
+                        tmem_ld_32x4(t_acc + (K::kTwoStepsWide ? 3 * (g & 1) + (g >> 1) + 1 - (i & 1) : g) * S + 4 * b, a[b][g]);
                 tmem_ld_wait();
                 tc_fence_before_sync();
                 __syncwarp();

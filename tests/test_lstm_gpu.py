@@ -575,10 +575,10 @@ def test_four_steps_per_contraction_give_the_bytes_of_the_l2_form(flib, H, B, T,
 
 
 @pytest.mark.parametrize("H,B", [(256, 1057), (256, 2112), (384, 689), (384, 1376), (512, 513), (512, 1024), (640, 443), (640, 832), (768, 353), (768, 704),
-                                 (896, 289), (896, 544), (1024, 300)])
+                                 (896, 289), (896, 544), (1024, 300), (256, 1056), (384, 345), (384, 688), (512, 257), (512, 512)])
 @pytest.mark.parametrize("T", [1, 2, 3, 6, 7])
-def test_two_groups_of_sixteen_rows_give_the_bytes_of_the_l2_form(flib, H, B, T):
-    """17 to 32 rows per cluster on a B200, the fewest and the most at each cluster size: two steps' x rows per contraction (up to clusters of seven), windows that
+def test_two_steps_per_contraction_of_more_than_eight_rows_give_the_bytes_of_the_l2_form(flib, H, B, T):
+    """17 to 32 rows per cluster on a B200 (clusters of up to seven) and 9 to 16 (up to four), the fewest and the most: two steps' x rows per contraction, windows that
     begin before the first step and end behind the last, both parities and directions; pieces that stay in a CTA. Against the L2-exchange form. Exact."""
     layer, x, xs = _layer_case(T, B, H, 128, H + B + T, T % 2 == 0)
     g = torch.Generator().manual_seed(B)
