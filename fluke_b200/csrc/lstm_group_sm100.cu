@@ -41,12 +41,12 @@
 // Nobody leaves before the final cluster barrier. Clusters never wait for one another, so any number of them may run in waves.
 //
 // What bounds a step (B200, H = 768; cycles of one CTA by clock stamps, which add up to its period and lengthen it by 2 to 4 %). 2 rows
-// per cluster, 2210: the chain of projection 530, its conversion 240, hh half 470, cell update and staging 500, exchange
-// 470. 14 rows, 2930: 530, 390, 450, 1050 (the cell updates) and 510. 47 rows, 4740: first group's projection 440, its partial
-// sums on the way 860, their sum and the way back 1480, contraction 730, cell updates 930 (24 rows, eight warps), 300 until the issuer has
-// seen the last warp's codes; the second group's chain runs beside it, and the tensor pipe works 3370 of them (x part 1540,
-// hh half 1460, projections 370). Without stamps most clusters take 4600 cycles, the slowest of 22 4780, and the layer ends with those:
-// 2.60 us per step at the 1.83 GHz that the nanosecond timer gives inside the kernel (the driver reports 1965 MHz meanwhile).
+// per cluster, 2160 (1820 at H = 384): the chain of projection 500, its conversion 140, 110 until the issuer sees it, hh half 470, cell update and staging
+// 490, exchange 430 (200 at H = 384). 14 rows, 2850: 500, 270, 130, 450, 1040 (the cell updates) and 440. 47 rows, 4500: first group's projection 460, its partial
+// sums sent 310, on the way 480 to 800, read and added up 300, converted and sent 300 to 430, on the way 490, contraction 720, cell updates 950 (24 rows, eight
+// warps), 230 until the issuer has seen the last warp's codes; the second group's chain runs beside it, and the tensor pipe works 3370 of them (x part 1540,
+// hh half 1460, projections 370). The layer ends with the slowest cluster: 1024 chunks 2.67 us per step, x_down included (2.88 before own shares stayed out of the
+// network), at the 1.83 GHz that the nanosecond timer gives inside the kernel (the driver reports 1965 MHz meanwhile).
 // The cell updates live on few instructions: with places in the swizzle worked out per row instead of by one exclusive or,
 // 1024 chunks took 2.89 us, 700 2.13.
 //
