@@ -77,7 +77,6 @@ constexpr int kGTmemCols = 512;
 constexpr int kGTmemW = 256;       // first column of the hh half of the gate weights: 4 gates x 64
 constexpr int kGWxBytes = 4 * kGUnits * 256;  // x half of the gate weights in shared memory
 constexpr int kGMaxSmem = 232448;
-constexpr int kGBars = 48;         // mbarriers of a CTA
 
 struct GroupDev {
     int T, B;
@@ -109,18 +108,17 @@ struct GroupForm {
     bool gather;
     int groups, rows;   // groups, and chunk rows of each at most
     int n;              // columns of the MMAs of one group: M = 128 takes multiples of 16
-    int stride;         // accumulator columns from gate to gate
+    int acc;            // accumulator columns of a gate in a step
     int proj;           // columns of projection accumulators
-    int x_slots;        // steps whose x_down rows are in shared memory
 };
 // 8 rows: the columns of an x MMA are two or four steps' rows, see x_half. Two groups of 24 rows: an MMA of
 // the first group also covers the first columns of the second, with operand rows that are zero, before that
 // group's own MMAs; the second group's covers unused columns. They take turns with one projection accumulator.
 __host__ __device__ constexpr GroupForm group_form(int V) {
-    return V == 0   ? GroupForm{8, true, 1, 8, 16, 16, 16, 5}   // four steps: group_stride, 11 slots
-           : V == 1 ? GroupForm{16, true, 1, 16, 16, 16, 16, 2}
-           : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32, 2}
-                    : GroupForm{48, false, 2, 24, 32, 56, 32, 2};
+    return V == 0   ? GroupForm{8, true, 1, 8, 16, 8, 16}
+           : V == 1 ? GroupForm{16, true, 1, 16, 16, 16, 16}
+           : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32}
+                    : GroupForm{48, false, 2, 24, 32, 56, 32};
 }
 // Steps whose x part one MMA covers. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
 // sixteen that there are at least (42), and what is issued of them before the hidden codes arrive holds the issuer up: with 16 such MMAs per step
@@ -134,8 +132,27 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
 // 9 to 16 rows, where the larger accumulators leave tensor memory for all projection weights: H = 256 600 chunks 1.455 : 1.369, 1000 1.545 : 1.507; H = 384 400
 // 1.485 : 1.395, 600 1.569 : 1.547, 680 1.589 : 1.593; H = 512 300 1.494 : 1.462, 500 1.657 : 1.654. Without: H = 768 200 1.606 : 1.667, 300 1.758 : 1.842.
 __host__ __device__ constexpr int group_x_steps(int V, int C) { return V == 2 ? (C <= 7 ? 2 : 1) : V == 1 ? (C <= 4 ? 2 : 1) : V != 0 ? 1 : C <= 3 ? 4 : 2; }
+// The x_down rows of a cluster in shared memory. A tile is the rows of one step in one of the two K blocks of 64. Up to 8 rows: per K block a ring of
+// tiles, of which the first steps - 1 are repeated behind it, so that the rows of a window of steps are contiguous wherever it begins. More rows, two
+// steps: two windows of two tiles per K block. Else: two steps.
+struct GroupX {
+    int steps;          // that an x MMA covers
+    int slots;          // windows (with one step: steps) that are loaded ahead, a power of two
+    int tile;           // bytes
+    int slot;           // from a slot to the next
+    int kb;             // from the first K block to the second
+    int bytes;          // all of it
+};
+__host__ __device__ constexpr GroupX group_x(int V, int C) {
+    const int steps = group_x_steps(V, C), tile = group_form(V).groups * group_form(V).rows * 128;
+    if (V == 0) {
+        const int slots = 2 * steps, ring = slots + steps - 1;
+        return GroupX{steps, slots, tile, tile, ring * tile, 2 * ring * tile};
+    }
+    return GroupX{steps, 2, tile, 2 * steps * tile, steps * tile, 2 * 2 * steps * tile};
+}
 // Accumulator columns from gate to gate.
-__host__ __device__ constexpr int group_stride(int V, int C) { return group_x_steps(V, C) == 4 ? 32 : group_form(V).stride; }
+__host__ __device__ constexpr int group_stride(int V, int C) { return group_form(V).acc * (V == 0 ? group_x_steps(V, C) : 1); }
 // Columns of all gate accumulators. Two steps of more than 8 rows: six places of a gate's columns hold the four gates of a step and two of the next.
 __host__ __device__ constexpr int group_acc_cols(int V, int C) { return (V > 0 && group_x_steps(V, C) == 2 ? 6 : 4) * group_stride(V, C); }
 // K steps (32 units, 8 columns) of the projection weights that fit in tensor memory beside the gate weights, the gate
@@ -159,6 +176,28 @@ __host__ __device__ constexpr int group_own_pieces(int V, int C) {
 // row per quarter of its gate warps, and there all to all was the faster against that kernel (H = 768, 14 rows 1.61 : 1.66).
 // Up to 8 rows two steps per x MMA make up for it (H = 1024, 8 rows 1.69 : 1.73 against that kernel).
 __host__ __device__ constexpr bool group_by_pair(int V, int C) { return V == 1 && C == 8; }
+// mbarriers of a CTA, as indices
+enum : int {
+    kBarOnce = 0,      // x half of the gate weights loaded
+    kBarX = 1,         // [slots] x_down rows landed
+    kBarXFree = 5,     // [slots] the x part of the contraction has read them
+    kBarAccFree = 9,   // the gate warps have read all accumulators
+    kBarProj = 10,     // [G] projection accumulator complete
+    kBarAcc = 12,      // [G] gate accumulators complete
+    kBarHh = 14,       // [G] hh_down rows in place
+    kBarCode = 16,     // SPLIT [G]: hidden codes of this CTA's units in place
+    kBarSum = 18,      // SPLIT [G]: partial sums of the CTA's own pieces arrived
+    kBarSent = 20,     // SPLIT: the projection accumulator has been read
+    kBarStored = 21,   // SPLIT: the TMA stores have read the hidden codes
+    kBarStart = 22,    // resident projection weights and the initial hidden rows loaded
+    kBarH = 16,        // GATHER [2], by pair [1]: hidden rows of all CTAs arrived
+    kBarW = 24,        // set-up [4]: recurrent weights of a gate landed in shared memory
+    kBarWRead = 28,    // set-up [4]: and have been read from there
+    kBarX4 = 32,       // up to 8 rows, four steps per x MMA [8]: in place of kBarX
+    kBarX4Free = 40,   // and of kBarXFree
+    kGBars = 48
+};
+
 struct GroupLayout {
     int x, hh, dn, h, recv, stage, bars, misc, dynamic;
 };
@@ -166,7 +205,7 @@ __host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
     const GroupForm f = group_form(V);
     GroupLayout l = {};
     l.x = kGWxBytes;                              // x_down rows, see x_half
-    l.hh = l.x + (group_x_steps(V, C) == 4 ? 11 : V > 0 && group_x_steps(V, C) == 2 ? 4 : f.x_slots) * f.groups * f.rows * 256;
+    l.hh = l.x + group_x(V, C).bytes;
     // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
     l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
     // projection weights [128 x 128 B] (by pair [64 x 128 B]) of the K blocks that are not all in tensor memory
@@ -246,9 +285,9 @@ struct GroupConst {
     static constexpr bool kFourSteps = group_x_steps(V, C) == 4;   // or four
     static constexpr bool kTwoStepsWide = V > 0 && group_x_steps(V, C) == 2;   // two steps of more than 8 rows, see x_half
     static constexpr int kAcc = group_acc_cols(V, C);         // columns of the gate accumulators; the projections' follow
-    static constexpr int kXSlots = kFourSteps ? 8 : kTwoSteps ? 4 : F.x_slots;
-    static constexpr int kXRing = kFourSteps ? 11 : 5;        // slots of 8 rows when an x MMA covers several steps
-    static constexpr int kFirstBarX = kFourSteps ? 32 : 1;
+    static constexpr GroupX X = group_x(V, C);
+    static constexpr int kXSlots = X.slots;
+    static constexpr int kBarXAt = kFourSteps ? kBarX4 : kBarX, kBarXFreeAt = kFourSteps ? kBarX4Free : kBarXFree;
     static constexpr bool kByPair = group_by_pair(V, C);
     static constexpr bool kPeerHh = !kGather || kByPair;      // hh_down rows come from peers
     static constexpr int kTile = (kByPair ? 8 : F.rows) * 128;     // bytes of a group's hidden rows in one K block
@@ -262,27 +301,14 @@ struct GroupConst {
     static constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
     static_assert(kAcc + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
     static_assert(L.dynamic <= kGMaxSmem, "shared memory of a CTA");
+    static_assert((kXSlots & (kXSlots - 1)) == 0 && X.tile == NB * 128, "slots by masks, tiles as the tensor map loads them");
+    static_assert(V != 0 || X.kb == (kXSlots + X.steps - 1) * X.slot, "a window of the ring ends in front of the other K block");
+    static_assert(V == 0 || (X.kb == X.steps * X.tile && X.slot == 2 * X.kb), "a window's K blocks in front of the next window");
+    static_assert(L.hh - L.x == (V == 0 ? 2 * X.kb : kXSlots * X.slot), "x_down rows end where the hh_down rows begin");
+    static_assert(kXSlots <= kBarXFreeAt - kBarXAt && kXSlots <= (kFourSteps ? kGBars : kBarAccFree) - kBarXFreeAt, "a barrier per slot");
+    static_assert(kBarX4 >= kBarWRead + 4 && L.misc - L.bars == kGBars * 8, "barriers one after the other");
     static_assert(!kByPair || (C % 2 == 0 && F.rows <= 2 * C), "a pair's rows are one per quarter of the gate warps");
 };
-// mbarriers of a CTA, as indices
-enum : int {
-    kBarOnce = 0,      // x half of the gate weights loaded
-    kBarX = 1,         // [slots] x_down rows landed
-    kBarXFree = 5,     // [slots] the x part of the contraction has read them
-    kBarAccFree = 9,   // the gate warps have read all accumulators
-    kBarProj = 10,     // [G] projection accumulator complete
-    kBarAcc = 12,      // [G] gate accumulators complete
-    kBarHh = 14,       // [G] hh_down rows in place
-    kBarCode = 16,     // SPLIT [G]: hidden codes of this CTA's units in place
-    kBarSum = 18,      // SPLIT [G]: partial sums of the CTA's own pieces arrived
-    kBarSent = 20,     // SPLIT: the projection accumulator has been read
-    kBarStored = 21,   // SPLIT: the TMA stores have read the hidden codes
-    kBarStart = 22,    // resident projection weights and the initial hidden rows loaded
-    kBarH = 16,        // GATHER [2], by pair [1]: hidden rows of all CTAs arrived
-    kBarW = 24,        // set-up [4]: recurrent weights of a gate landed in shared memory
-    kBarWRead = 28     // set-up [4]: and have been read from there
-};
-
 // The MMA issuer, warp 1. The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
 // K loops unrolled, so an MMA is issued every few cycles. kExact: for weights that are not finite.
 template <int V, int C, bool kExact>
@@ -294,14 +320,14 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
     constexpr int kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + K::kFirstBarX, *bar_x_free = bar_x + (kFourSteps ? 8 : 4), *bar_acc_free = bars + kBarAccFree;
+    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + K::kBarXAt, *bar_x_free = bars + K::kBarXFreeAt, *bar_acc_free = bars + kBarAccFree;
     uint64_t *bar_proj = bars + kBarProj, *bar_acc = bars + kBarAcc, *bar_hh = bars + kBarHh, *bar_code = bars + kBarCode;
     uint64_t *bar_sent = bars + kBarSent, *bar_stored = bars + kBarStored, *bar_h = bars + kBarH;
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L.misc + 4);
     [[maybe_unused]] const int lane = threadIdx.x & 31;
     auto rows_of = [&](int e) { return min(max(n_rows - F.rows * e, 0), F.rows); };
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
-    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, K::kTwoStepsWide ? 2 * NB : kFourSteps ? 32 : kTwoSteps ? 16 : NB);
+    constexpr uint32_t kIdescX = make_idesc<kKindF16>(128, K::X.steps * NB);
     constexpr uint32_t kIdescHh = make_idesc<kKindF16>(128, F.n);
     constexpr uint32_t kIdescP = make_idesc<kKindI8>(128, F.n);
     uint64_t d_wx = make_smem_desc_sw128(smem_u32(smem));
@@ -324,14 +350,14 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     auto x_half = [&](auto from, auto to, int i, bool release = true, int gate = 0) {
         constexpr int first = decltype(from)::value, end = decltype(to)::value;
         const int slot = (K::kTwoStepsWide ? i + 1 : i) & (kXSlots - 1);
-        const uint64_t d_x = d_x0 + uint64_t(slot * (K::kTwoStepsWide ? NB * 32 : kTwoSteps || kFourSteps ? NB * 8 : NB * 16));
+        const uint64_t d_x = d_x0 + uint64_t(slot * (K::X.slot >> 4));
         const int g0 = kFourSteps ? (kExact ? gate : i & 3) : kTwoSteps || K::kTwoStepsWide ? 2 * (i & 1) : 0;
         if (elect_one()) {
 #pragma unroll
             for (int m = first; m < end; ++m) {
                 const int g = m >> 3, k = m & 7;
                 tc_mma<kKindF16>(tmem + (K::kTwoStepsWide ? 3 * g + (i & 1) : g0 + g) * S, d_wx + uint64_t(((g0 + g) * 2 + (k >> 2)) * 1024 + 2 * (k & 3)),
-                                 d_x + uint64_t((k >> 2) * ((kTwoSteps || kFourSteps ? K::kXRing : K::kTwoStepsWide ? 2 : 1) * NB * 8) + 2 * (k & 3)), kIdescX, k != 0);
+                                 d_x + uint64_t((k >> 2) * (K::X.kb >> 4) + 2 * (k & 3)), kIdescX, k != 0);
             }
             if (end == kX && release) tc_commit(&bar_x_free[slot]);
         }
@@ -576,7 +602,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
     constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kFourSteps = K::kFourSteps, kOneProj = K::kOneProj;
-    constexpr int G = K::G, NB = K::NB, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
+    constexpr int G = K::G, S = K::S, H = K::H, kXSlots = K::kXSlots, kTile = K::kTile, kHhTile = K::kHhTile;
     constexpr int kPieces = K::kPieces, kPairs = K::kPairs, kDnTs = K::kDnTs, kDnCol = K::kDnCol;
     extern __shared__ uint8_t smem_raw[];
     // every CTA of the cluster computes the same offset, so peers' buffers are at the same
@@ -584,7 +610,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + K::kFirstBarX, *bar_x_free = bar_x + (kFourSteps ? 8 : 4), *bar_acc_free = bars + kBarAccFree;
+    uint64_t *bar_once = bars + kBarOnce, *bar_x = bars + K::kBarXAt, *bar_x_free = bars + K::kBarXFreeAt, *bar_acc_free = bars + kBarAccFree;
     uint64_t *bar_proj = bars + kBarProj, *bar_acc = bars + kBarAcc, *bar_hh = bars + kBarHh, *bar_code = bars + kBarCode;
     uint64_t *bar_sum = bars + kBarSum, *bar_sent = bars + kBarSent, *bar_stored = bars + kBarStored, *bar_h = bars + kBarH;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.misc);
@@ -717,21 +743,21 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
                 if (!ok) return;
                 if constexpr (kTwoSteps || kFourSteps) {
-                    const bool twice = s < K::kXRing - kXSlots;   // the last slots repeat the first
-                    mbar_arrive_expect_tx(&bar_x[s], NB * 256 * (twice ? 2 : 1));
+                    const bool twice = s < K::X.steps - 1;   // the last slots repeat the first
+                    mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile * (twice ? 2 : 1));
                     for (int kb = 0; kb < 2; ++kb)
                         for (int n = 0; n < (twice ? 2 : 1); ++n)
-                            tma_load_4d(smem + L.x + (kb * K::kXRing + s + kXSlots * n) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
+                            tma_load_4d(smem + L.x + kb * K::X.kb + (s + kXSlots * n) * K::X.slot, &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
                 } else if constexpr (K::kTwoStepsWide) {
                     // steps i and i + 1, the odd one in front
                     const int from = max(i, 0), to = min(i + 2, p.T);
-                    mbar_arrive_expect_tx(&bar_x[s], NB * 256 * (to - from));
+                    mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile * (to - from));
                     for (int t = from; t < to; ++t)
                         for (int kb = 0; kb < 2; ++kb)
-                            tma_load_4d(smem + L.x + s * (NB * 512) + (kb * 2 + 1 - (t & 1)) * (NB * 128), &tm_x, &bar_x[s], 0, m0, kb, time_of(t));
+                            tma_load_4d(smem + L.x + s * K::X.slot + kb * K::X.kb + (1 - (t & 1)) * K::X.tile, &tm_x, &bar_x[s], 0, m0, kb, time_of(t));
                 } else {
-                    mbar_arrive_expect_tx(&bar_x[s], NB * 256);
-                    tma_load_4d(smem + L.x + s * (NB * 256), &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
+                    mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile);
+                    tma_load_4d(smem + L.x + s * K::X.slot, &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
                 }
             };
             if constexpr (kGather) {
