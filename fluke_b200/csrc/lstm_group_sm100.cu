@@ -626,21 +626,14 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     const int pair = rank >> 1, half = rank & 1;
     const int per_pair = kByPair ? (p.rows + C / 2 - 1) / (C / 2) : 0;
     const int own_rows = kByPair ? min(max(n_rows - pair * per_pair, 0), per_pair) : 0;
-    // whether this CTA adds up piece k of group e, and how many pieces of the group it adds up
-    auto own_piece = [&](int e, int k) { return (kPieces * e + k) % C == rank && 4 * k < rows_of(e); };
-    auto own_pieces = [&](int e) {
-        int n = 0;
-#pragma unroll
-        for (int k = 0; k < kPieces; ++k) n += own_piece(e, k);
-        return n;
-    };
-    // bytes of hh_down rows that a group receives from peers
+    // pieces of a group that this CTA adds up, and bytes of hh_down rows that the group receives from peers
+    auto pieces_below = [&](unsigned n) { return (n + unsigned(C - 1 - rank)) / C; };   // own ones among the first n of all groups
+    auto pieces_of = [&](int e) { return (unsigned(rows_of(e)) + 3) / 4; };
+    auto own_pieces = [&](int e) { return int(pieces_below(kPieces * e + pieces_of(e)) - pieces_below(kPieces * e)); };
     auto hh_bytes = [&](int e) {
-        int n = rows_of(e);
-#pragma unroll
-        for (int k = 0; k < kPieces; ++k)
-            if (own_piece(e, k)) n -= min(4, rows_of(e) - 4 * k);
-        return uint32_t(n) * 256;
+        const unsigned rows = rows_of(e), pieces = pieces_of(e);
+        const bool owns_last = pieces > 0 && (kPieces * e + pieces - 1) % C == unsigned(rank);   // which may have fewer than four rows
+        return (rows - 4 * own_pieces(e) + (owns_last ? 4 * pieces - rows : 0)) * 256;
     };
     const bool both = G > 1 && n_rows > F.rows;        // the last cluster may have nothing in its second group
     auto time_of = [&](int i) { return p.reverse ? p.T - 1 - i : i; };
@@ -648,14 +641,13 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         auto arrivals = [&](int b) {   // warps that arrive, or one arrival with the expected bytes
             if (b == kBarAccFree) return kGather || both ? kGEpiWarps : kGEpiWarps / 2;
             if (b >= kBarWRead && b < kBarWRead + 4) return 4;
-            if (!kGather && (b == kBarSum || b == kBarSum + 1)) return 1 + 4 * own_pieces(b - kBarSum);
-            if (!kGather && (b == kBarHh || b == kBarHh + 1)) return 1 + (kGEpiWarps / 2) * own_pieces(b - kBarHh);
             if (b >= kBarWRead) return 1;
             if (kGather) return !kByPair && b == kBarHh ? kGEpiWarps : 1;
             return b == kBarCode || b == kBarCode + 1 || b == kBarSent ? kGEpiWarps / 2 : 1;
         };
 #pragma unroll
-        for (int b = 0; b < kGBars; ++b) mbar_init(&bars[b], arrivals(b));
+        for (int b = 0; b < (kFourSteps ? kGBars : kBarX4); ++b)
+            if (kGather || (b / 2 != kBarSum / 2 && b / 2 != kBarHh / 2)) mbar_init(&bars[b], arrivals(b));
         *abort_flag = 0;
         fence_barrier_init();
         if constexpr (kByPair) {
@@ -664,11 +656,19 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         } else if constexpr (kGather) {
             for (int s = 0; s < 2; ++s)
                 if (s + 1 < p.T) mbar_arrive_expect_tx(&bar_h[s], uint32_t(n_rows) * H);
-        } else {
-            for (int e = 0; e < (both ? 2 : 1); ++e) {
-                mbar_arrive_expect_tx(&bar_hh[e], hh_bytes(e));
-                if (const int n = own_pieces(e)) mbar_arrive_expect_tx(&bar_sum[e], uint32_t(n) * (C - 1) * 2048);
-            }
+        }
+    }
+    // SPLIT: the barriers whose counts are those of the CTA's own pieces, by a second thread. Code that runs once costs its instruction fetches, and all
+    // that the first thread does stands in front of the loads of the weights (pieces counted one by one by that thread: 330 cycles later).
+    if (!kGather && threadIdx.x == 64) {
+        for (int e = 0; e < 2; ++e) {
+            const int n = own_pieces(e);
+            mbar_init(&bar_hh[e], 1 + (kGEpiWarps / 2) * n);
+            mbar_init(&bar_sum[e], 1 + 4 * n);
+            fence_barrier_init();
+            if (e > 0 && !both) break;
+            mbar_arrive_expect_tx(&bar_hh[e], hh_bytes(e));
+            if (n > 0) mbar_arrive_expect_tx(&bar_sum[e], uint32_t(n) * (C - 1) * 2048);
         }
     }
     if (K::kZeroRows) {
@@ -731,41 +731,47 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
     // GATHER: a CTA loads the initial hidden rows of its peers' units too, and a layer of one step stores the final ones, of its
     // own units and to the same place, without having heard from them: no CTA passes the barrier before they have landed.
     if (kGather && warp < 2) mbar_wait(bar_start, 0, abort_flag, 97);
-    // every barrier of the cluster is initialised before any CTA may store to a peer
-    cluster_sync_all();
+    // Every barrier of the cluster is initialised before any CTA may store to a peer: each warp passes this once. SPLIT: what a role prepares without
+    // its peers stands in front of it, where there is time: behind it the set-up of sixteen warps held the issuer up for 900 cycles. (GATHER, which has
+    // less of it: no gain, and steps up to 1 % slower from where the code then lies.)
+    auto peers_ready = [&]() { cluster_sync_all(); };
+    if (kGather) peers_ready();
 
     if (warp == 0) {
         // ------------------------------ loader (one thread) -----------------------------
-        if (elect_one()) {
-            bool ok = true;
-            auto load_x = [&](int i) {
-                const int s = (K::kTwoStepsWide ? i + 1 : i) & (kXSlots - 1), u = (K::kTwoStepsWide ? i + 1 : i) / kXSlots;
-                if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
-                if (!ok) return;
-                if constexpr (kTwoSteps || kFourSteps) {
-                    const bool twice = s < K::X.steps - 1;   // the last slots repeat the first
-                    mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile * (twice ? 2 : 1));
+        bool ok = true;
+        auto load_x = [&](int i) {
+            const int s = (K::kTwoStepsWide ? i + 1 : i) & (kXSlots - 1), u = (K::kTwoStepsWide ? i + 1 : i) / kXSlots;
+            if (u > 0) ok = ok && mbar_wait(&bar_x_free[s], (u - 1) & 1, abort_flag, 96);
+            if (!ok) return;
+            if constexpr (kTwoSteps || kFourSteps) {
+                const bool twice = s < K::X.steps - 1;   // the last slots repeat the first
+                mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile * (twice ? 2 : 1));
+                for (int kb = 0; kb < 2; ++kb)
+                    for (int n = 0; n < (twice ? 2 : 1); ++n)
+                        tma_load_4d(smem + L.x + kb * K::X.kb + (s + kXSlots * n) * K::X.slot, &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
+            } else if constexpr (K::kTwoStepsWide) {
+                // steps i and i + 1, the odd one in front
+                const int from = max(i, 0), to = min(i + 2, p.T);
+                mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile * (to - from));
+                for (int t = from; t < to; ++t)
                     for (int kb = 0; kb < 2; ++kb)
-                        for (int n = 0; n < (twice ? 2 : 1); ++n)
-                            tma_load_4d(smem + L.x + kb * K::X.kb + (s + kXSlots * n) * K::X.slot, &tm_x, &bar_x[s], 0, m0, kb, time_of(i));
-                } else if constexpr (K::kTwoStepsWide) {
-                    // steps i and i + 1, the odd one in front
-                    const int from = max(i, 0), to = min(i + 2, p.T);
-                    mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile * (to - from));
-                    for (int t = from; t < to; ++t)
-                        for (int kb = 0; kb < 2; ++kb)
-                            tma_load_4d(smem + L.x + s * K::X.slot + kb * K::X.kb + (1 - (t & 1)) * K::X.tile, &tm_x, &bar_x[s], 0, m0, kb, time_of(t));
-                } else {
-                    mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile);
-                    tma_load_4d(smem + L.x + s * K::X.slot, &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
-                }
-            };
+                        tma_load_4d(smem + L.x + s * K::X.slot + kb * K::X.kb + (1 - (t & 1)) * K::X.tile, &tm_x, &bar_x[s], 0, m0, kb, time_of(t));
+            } else {
+                mbar_arrive_expect_tx(&bar_x[s], 2 * K::X.tile);
+                tma_load_4d(smem + L.x + s * K::X.slot, &tm_x, &bar_x[s], 0, m0, 0, time_of(i));
+            }
+        };
+        constexpr int kEarly = K::kTwoStepsWide ? 1 : 0;   // windows that begin before step 0
+        if (!kGather && elect_one())
+            for (int i = -kEarly; i < min(p.T, kXSlots - kEarly); ++i) load_x(i);
+        __syncwarp();
+        if (!kGather) peers_ready();
+        if (elect_one()) {
             if constexpr (kGather) {
-                for (int i = K::kTwoStepsWide ? -1 : 0; i < p.T && ok; ++i) load_x(i);
+                for (int i = -kEarly; i < p.T && ok; ++i) load_x(i);
             } else {
                 // between the loads the stores of the hidden rows
-                constexpr int kEarly = K::kTwoStepsWide ? 1 : 0;   // windows that begin before step 0
-                for (int i = -kEarly; i < min(p.T, kXSlots - kEarly); ++i) load_x(i);
                 for (int i = 0; i < p.T && ok; ++i) {
                     if (K::kTwoStepsWide && i + 1 < p.T) load_x(i + 1);   // of two tiles, the other one is in use
                     for (int e = 0; e < (both ? 2 : 1) && ok; ++e) {
@@ -782,6 +788,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         }
         __syncwarp();
     } else if (warp == 1) {
+        if (!kGather) peers_ready();
         if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows, own_rows, hh_bytes(0), hh_bytes(1));
         else issue_exact<V, C>(smem, tmem, p, n_rows, hh_bytes(0), hh_bytes(1));
     } else {
@@ -1015,6 +1022,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                 hh_to[d / 4] = map_to_rank(hh, to);
                 bar_to[d / 4] = map_to_rank(bar_hh_e, to);
             }
+            peers_ready();
             for (int i = 0; i < p.T && ok; ++i) {
                 // ---- projection of this CTA's h_{i-1}: every other piece to its owner ----
                 ok = mbar_wait(&bar_proj[e], i & 1, abort_flag, 102);
@@ -1106,6 +1114,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             // the last codes are the final hidden state
             if (ok)
                 for (int j = 0; j < my_rows; ++j) p.h_state[int64_t(m0 + F.rows * e + r0 + j) * H + unit] = int8_t(lds8(code_at(j)));
+        } else {
+            peers_ready();
         }
 #pragma unroll
         for (int j = 0; j < kPairs; ++j) {
