@@ -157,6 +157,9 @@ void fluke_sm100_set_lstm_wide(int mode);
 /* Which form the last whole-layer call used: 3 small clusters, 1 cluster exchange, 2 L2 exchange,
  * 0 per step. */
 int fluke_sm100_lstm_last_form(void);
+/* How the small-cluster form spreads T steps of B chunks of hidden size H: chunk rows per cluster (0: shape or device not covered), and in
+ * *x_steps (may be null) the steps whose x_down rows one contraction covers. For tests and measurements; launches nothing. */
+int fluke_sm100_lstm_small_clusters(int T, int B, int H, int *x_steps);
 /* Row tiles (clusters) of the cluster form that run at once for hidden size H; 0 = unavailable. */
 int fluke_sm100_lstm_cluster_capacity(int H);
 

@@ -1211,6 +1211,14 @@ bool group_plan(int B, int H, GroupPlan *g) {
 }  // namespace
 }  // namespace fluke_sm100
 
+extern "C" int fluke_sm100_lstm_small_clusters(int T, int B, int H, int *x_steps) {
+    using namespace fluke_sm100;
+    GroupPlan g;
+    if (T < 1 || B < 1 || H < 1 || !group_plan(B, H, &g)) return 0;
+    if (x_steps) *x_steps = group_x_steps(g.form, H / kGUnits);
+    return g.rows;
+}
+
 // Runs the recurrence of one layer (x_down already computed) with the batch spread over small
 // clusters, and writes the final hidden state. Returns -2 when the shape or the device is not covered.
 extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_down, void *stream) {

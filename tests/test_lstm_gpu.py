@@ -5,6 +5,8 @@ Bar (f16 tensor-core contraction, f32 accumulate in an unspecified order): cell 
 bar holds per step while the fraction of differing codes stays small. Batch shards reproduce
 the unsharded result bit for bit.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -29,6 +31,13 @@ def lstm_mode(request, flib):
     launches per step."""
     flib.fluke_set_lstm_persistent(LSTM_MODES[request.param][0])
     yield request.param
+    flib.fluke_set_lstm_persistent(1)
+
+
+@pytest.fixture(autouse=True)
+def _default_form_afterwards(flib):
+    """A test that fails between two forms leaves the next one the default."""
+    yield
     flib.fluke_set_lstm_persistent(1)
 
 
@@ -653,3 +662,60 @@ def test_layers_of_more_than_1024_units_are_refused_without_a_launch(flib, h, b)
     torch.cuda.synchronize()
     assert torch.equal(got, want)
     assert bool((c == 1).all()) and bool((hs == 1).all()) and bool((out == 5).all())
+
+
+def _small_clusters(flib, t, b, h):
+    """(chunk rows per cluster, steps whose x rows one contraction covers) of the small-cluster form on this device."""
+    steps = ctypes.c_int(0)
+    return flib.fluke_sm100_lstm_small_clusters(t, b, h, ctypes.byref(steps)), steps.value
+
+
+def _chunk_counts(flib, h, rows):
+    """So many rows in every cluster that the device runs at once, and as few as the last one can have beside them."""
+    per_cluster = lambda b: _small_clusters(flib, 1, b, h)[0]
+    clusters = next(n for n in range(1, 256) if per_cluster(48 * n) == 48 and per_cluster(48 * n + 1) < 48)
+    return clusters * rows, clusters * rows - min(rows, clusters) + 1
+
+
+def _assert_default_form_gives_the_bytes_of_the_l2_form(flib, t, b, h, infinite):
+    """Of both directions' layers from a non-zero state; infinite: weights of all gates and both halves, as above. Exact, NaN at the same places."""
+    layer, x, xs = _layer_case(t, b, h, 128, h + b + t, (t + b) % 2 == 1)
+    w = layer.w_up.clone()
+    if infinite:
+        for i, (unit, k) in enumerate([(3, 5), (40, 127), (h - 1, 64), (129, 0), (70, 130), (h - 100, 255)]):
+            w[(i % 4) * h + unit, k] = float("inf") if i % 2 else float("-inf")
+    g = torch.Generator().manual_seed(b)
+    c0 = (torch.randn(b, h, generator=g) * 0.3).to(DEV)
+    h0 = torch.randint(-127, 128, (b, h), generator=g, dtype=torch.int8).to(DEV)
+    res = []
+    for mode, form in ((1, 3), (2, 2)):
+        flib.fluke_set_lstm_persistent(mode)
+        c, hs = c0.clone(), h0.clone()
+        out = ops.factored_lstm_layer_i8(x.to(DEV), xs.to(DEV), layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale, w, layer.bias,
+                                         c, hs, reverse=layer.reverse)
+        assert flib.fluke_sm100_lstm_last_form() == form
+        res.append((out, c, hs))
+    (out, c, hs), (out_l2, c_l2, hs_l2) = res
+    assert torch.equal(torch.isnan(c), torch.isnan(c_l2)) and torch.equal(c.nan_to_num(7.0), c_l2.nan_to_num(7.0))
+    assert torch.equal(out, out_l2) and torch.equal(hs, hs_l2)
+
+
+@pytest.mark.parametrize("h,rows,steps", [(256, 8, 4), (384, 6, 4), (512, 8, 2), (256, 9, 2), (256, 16, 2), (384, 14, 2), (512, 12, 2), (640, 16, 1), (1024, 16, 1),
+                                          (256, 17, 2), (512, 32, 2), (896, 24, 2), (1024, 32, 1), (768, 33, 1)])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_every_kernel_of_the_small_clusters_gives_the_bytes_of_the_l2_form(flib, h, rows, steps, infinite):
+    """Rows per cluster on this device, and the steps per contraction of the kernel they take, are asked for and asserted. All clusters full, and the
+    last one short of rows; also weights that are not finite in windows of two steps of more than 8 rows."""
+    t = 18
+    for b in _chunk_counts(flib, h, rows):
+        assert _small_clusters(flib, t, b, h) == (rows, steps)
+        _assert_default_form_gives_the_bytes_of_the_l2_form(flib, t, b, h, infinite)
+
+
+@pytest.mark.parametrize("h,rows", [(256, 33), (384, 40), (512, 47), (640, 33), (768, 47), (896, 36), (1024, 33), (1024, 48)])
+@pytest.mark.parametrize("t", [1, 2, 3])
+def test_infinite_gate_weights_in_layers_of_few_steps(flib, h, rows, t):
+    """Two groups of 24 rows, whose MMAs for such weights are others: one step (no barrier is armed again) to three; an empty second group in the last cluster."""
+    for b in _chunk_counts(flib, h, rows):
+        assert _small_clusters(flib, t, b, h) == (rows, 1)
+        _assert_default_form_gives_the_bytes_of_the_l2_form(flib, t, b, h, True)
