@@ -120,7 +120,7 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
            : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32}
                     : GroupForm{48, false, 2, 24, 32, 56, 32};
 }
-// Steps whose x part one MMA covers. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
+// Steps whose x part one MMA covers: for each form and cluster size a kernel of the fewest and, where it pays, one of more. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
 // sixteen that there are at least (42), and what is issued of them before the hidden codes arrive holds the issuer up: with 16 such MMAs per step
 // it saw codes that had travelled for 200 cycles after 430. Four steps per MMA are 8 per step, and twice the accumulators, which clusters of
 // two and three have the tensor memory for beside all projection weights. Two steps against four, us per step, x_down included: H = 384 32 chunks 1.156 :
@@ -131,7 +131,19 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
 // 256 1200 2.045 : 1.827; H = 512 700 2.047 : 1.835; H = 640 600 2.063 : 1.885; H = 896 400 2.060 : 2.050; clusters of eight 300 2.089 : 2.138.
 // 9 to 16 rows, where the larger accumulators leave tensor memory for all projection weights: H = 256 600 chunks 1.455 : 1.369, 1000 1.545 : 1.507; H = 384 400
 // 1.485 : 1.395, 600 1.569 : 1.547, 680 1.589 : 1.593; H = 512 300 1.494 : 1.462, 500 1.657 : 1.654. Without: H = 768 200 1.606 : 1.667, 300 1.758 : 1.842.
-__host__ __device__ constexpr int group_x_steps(int V, int C) { return V == 2 ? (C <= 7 ? 2 : 1) : V == 1 ? (C <= 4 ? 2 : 1) : V != 0 ? 1 : C <= 3 ? 4 : 2; }
+constexpr int group_x_steps(int V, int C, bool most) { return V == 0 ? (most && C <= 3 ? 4 : 2) : most && ((V == 1 && C <= 4) || (V == 2 && C <= 7)) ? 2 : 1; }
+// Which of the two. Windows of several steps begin before the first one or end behind the last, so a layer of few steps pays for more than its
+// own; and with many rows in its form the wider accumulators cost more than they save. Fewest : most, us of a layer, x_down included.
+// Up to 8 rows, H = 384 86 chunks (2 rows) 1 step 12.4 : 12.7, H = 256 132 8 steps 19.6 : 19.2; H = 384 301 chunks (7 rows) 100 steps 127.2 : 127.3, 344 (8) 400 steps 485 : 492.
+// 9 to 16 rows, H = 512 448 chunks (14) 1 step 13.2 : 13.7; H = 384 602 (14) 10 steps 26.1 : 26.5, 24 steps 46.3 : 46.5 and in long layers 0.7 % less; H = 256 924 (14) 16 steps
+// 34.3 : 34.1; H = 512 384 (12) 48 steps 80.4 : 80.1, 448 (14) 400 steps 627 : 634; H = 384 688 (16) 400 steps 612 : 619. 17 to 32 rows, H = 256 2112 chunks 1 step 12.5 : 13.0, 1848 8
+// steps 27.0 : 26.4; H = 640 700 8 steps 26.7 : 26.4; H = 768 704 1 step 12.7 : 13.3, 8 steps 26.7 : 27.0, 20 steps 50.6 : 50.4; H = 896 448 20 steps 49.0 : 50.1, 100 to 400 steps
+// within 1 % of each other.
+bool group_most_x_steps(int T, int rows, int V, int C) {
+    if (V == 1) return T >= 16 && rows <= (C == 2 ? 16 : C == 3 ? 14 : 12);
+    if (V == 2) return T >= (C <= 5 ? 8 : 16);
+    return T >= 8 && rows <= (C == 2 ? 8 : 6);
+}
 // The x_down rows of a cluster in shared memory. A tile is the rows of one step in one of the two K blocks of 64. Up to 8 rows: per K block a ring of
 // tiles, of which the first steps - 1 are repeated behind it, so that the rows of a window of steps are contiguous wherever it begins. More rows, two
 // steps: two windows of two tiles per K block. Else: two steps.
@@ -143,8 +155,8 @@ struct GroupX {
     int kb;             // from the first K block to the second
     int bytes;          // all of it
 };
-__host__ __device__ constexpr GroupX group_x(int V, int C) {
-    const int steps = group_x_steps(V, C), tile = group_form(V).groups * group_form(V).rows * 128;
+__host__ __device__ constexpr GroupX group_x(int V, int steps) {
+    const int tile = group_form(V).groups * group_form(V).rows * 128;
     if (V == 0) {
         const int slots = 2 * steps, ring = slots + steps - 1;
         return GroupX{steps, slots, tile, tile, ring * tile, 2 * ring * tile};
@@ -152,14 +164,14 @@ __host__ __device__ constexpr GroupX group_x(int V, int C) {
     return GroupX{steps, 2, tile, 2 * steps * tile, steps * tile, 2 * 2 * steps * tile};
 }
 // Accumulator columns from gate to gate.
-__host__ __device__ constexpr int group_stride(int V, int C) { return group_form(V).acc * (V == 0 ? group_x_steps(V, C) : 1); }
+__host__ __device__ constexpr int group_stride(int V, int X) { return group_form(V).acc * (V == 0 ? X : 1); }
 // Columns of all gate accumulators. Two steps of more than 8 rows: six places of a gate's columns hold the four gates of a step and two of the next.
-__host__ __device__ constexpr int group_acc_cols(int V, int C) { return (V > 0 && group_x_steps(V, C) == 2 ? 6 : 4) * group_stride(V, C); }
+__host__ __device__ constexpr int group_acc_cols(int V, int X) { return (V > 0 && X == 2 ? 6 : 4) * group_stride(V, X); }
 // K steps (32 units, 8 columns) of the projection weights that fit in tensor memory beside the gate weights, the gate
 // accumulators and the projections.
-__host__ __device__ constexpr int group_dn_ts(int V, int C) {
+__host__ __device__ constexpr int group_dn_ts(int V, int C, int X) {
     const GroupForm f = group_form(V);
-    const int fit = (kGTmemW - group_acc_cols(V, C) - f.proj) / 8, all = f.gather ? 4 * C : 4;
+    const int fit = (kGTmemW - group_acc_cols(V, X) - f.proj) / 8, all = f.gather ? 4 * C : 4;
     return fit < all ? fit : all;
 }
 // Four rows of a group are projected as one piece (16 bytes per projection column). The pieces of all groups are dealt to
@@ -201,15 +213,15 @@ enum : int {
 struct GroupLayout {
     int x, hh, dn, h, recv, stage, bars, misc, dynamic;
 };
-__host__ __device__ constexpr GroupLayout group_layout(int V, int C) {
+__host__ __device__ constexpr GroupLayout group_layout(int V, int C, int X) {
     const GroupForm f = group_form(V);
     GroupLayout l = {};
     l.x = kGWxBytes;                              // x_down rows, see x_half
-    l.hh = l.x + group_x(V, C).bytes;
+    l.hh = l.x + group_x(V, X).bytes;
     // hh_down rows: per group 2 K blocks [n x 128 B]; 8 rows: [24 x 128 B], the rows in front and behind are zero
     l.dn = l.hh + (f.rows == 8 ? 24 : f.groups * f.n) * 256;
     // projection weights [128 x 128 B] (by pair [64 x 128 B]) of the K blocks that are not all in tensor memory
-    l.h = l.dn + (group_by_pair(V, C) ? 8192 : 16384) * ((f.gather ? C : 1) - group_dn_ts(V, C) / 4);
+    l.h = l.dn + (group_by_pair(V, C) ? 8192 : 16384) * ((f.gather ? C : 1) - group_dn_ts(V, C, X) / 4);
     // int8 hidden rows. GATHER: two slots of C K blocks [rows x 128 B], by pair one of [8 x 128 B]; else this CTA's units, per
     // group [rows x 128 B]. An MMA of more columns reads on behind them
     l.recv = l.h + (group_by_pair(V, C) ? C * 1024 : (f.gather ? 2 * C : f.groups) * f.rows * 128);
@@ -275,17 +287,17 @@ template <int V>
 struct Int { static constexpr int value = V; };  // a number that a lambda receives as a type
 
 // What the kernel and its MMA issuer know at compile time.
-template <int V, int C>
+template <int V, int C, int STEPS>
 struct GroupConst {
     static constexpr GroupForm F = group_form(V);
-    static constexpr GroupLayout L = group_layout(V, C);
+    static constexpr GroupLayout L = group_layout(V, C, STEPS);
     static constexpr bool kGather = F.gather;
-    static constexpr int G = F.groups, NB = G * F.rows, S = group_stride(V, C), H = C * kGUnits;
-    static constexpr bool kTwoSteps = V == 0 && group_x_steps(V, C) == 2;    // an x MMA covers two steps
-    static constexpr bool kFourSteps = group_x_steps(V, C) == 4;   // or four
-    static constexpr bool kTwoStepsWide = V > 0 && group_x_steps(V, C) == 2;   // two steps of more than 8 rows, see x_half
-    static constexpr int kAcc = group_acc_cols(V, C);         // columns of the gate accumulators; the projections' follow
-    static constexpr GroupX X = group_x(V, C);
+    static constexpr int G = F.groups, NB = G * F.rows, S = group_stride(V, STEPS), H = C * kGUnits;
+    static constexpr bool kTwoSteps = V == 0 && STEPS == 2;    // an x MMA covers two steps
+    static constexpr bool kFourSteps = STEPS == 4;   // or four
+    static constexpr bool kTwoStepsWide = V > 0 && STEPS == 2;   // two steps of more than 8 rows, see x_half
+    static constexpr int kAcc = group_acc_cols(V, STEPS);         // columns of the gate accumulators; the projections' follow
+    static constexpr GroupX X = group_x(V, STEPS);
     static constexpr int kXSlots = X.slots;
     static constexpr int kBarXAt = kFourSteps ? kBarX4 : kBarX, kBarXFreeAt = kFourSteps ? kBarX4Free : kBarXFree;
     static constexpr bool kByPair = group_by_pair(V, C);
@@ -296,7 +308,7 @@ struct GroupConst {
     static constexpr int kDnRows = kByPair ? 64 : kGRank;     // projection columns of a CTA
     static constexpr int kPieces = F.rows / 4;                // pieces of a group
     static constexpr int kPairs = kGather ? F.rows / 8 : F.rows / 4;   // pairs of rows of a gate thread
-    static constexpr int kDnTs = group_dn_ts(V, C);
+    static constexpr int kDnTs = group_dn_ts(V, C, STEPS);
     static constexpr int kDnCol = kGTmemW - 8 * kDnTs;        // first column of the projection weights in tensor memory
     static constexpr bool kOneProj = F.proj < G * F.n;        // the groups share the projection accumulator
     static_assert(kAcc + F.proj + 8 * kDnTs <= kGTmemW, "accumulators beside the weights in tensor memory");
@@ -311,9 +323,9 @@ struct GroupConst {
 };
 // The MMA issuer, warp 1. The whole warp walks the loop; one elected lane issues. Descriptors are uniform and the
 // K loops unrolled, so an MMA is issued every few cycles. kExact: for weights that are not finite.
-template <int V, int C, bool kExact>
+template <int V, int C, int STEPS, bool kExact>
 __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupDev &p, int n_rows, int own_rows, uint32_t hh_bytes0, uint32_t hh_bytes1) {
-    using K = GroupConst<V, C>;
+    using K = GroupConst<V, C, STEPS>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
     constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kFourSteps = K::kFourSteps, kOneProj = K::kOneProj;
@@ -558,9 +570,9 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
     }
 }
 // Out of line: as a branch or a second loop in the kernel it cost the other weights 1 to 3 % of a step.
-template <int V, int C>
+template <int V, int C, int STEPS>
 __device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev p, int n_rows, uint32_t hh_bytes0, uint32_t hh_bytes1) {
-    issue<V, C, GroupConst<V, C>::kZeroRows>(smem, tmem, p, n_rows, 0, hh_bytes0, hh_bytes1);
+    issue<V, C, STEPS, GroupConst<V, C, STEPS>::kZeroRows>(smem, tmem, p, n_rows, 0, hh_bytes0, hh_bytes1);
 }
 
 // A row of the recurrent weights of a gate from its place in shared memory (two K blocks of 64 in the 128-byte swizzle) to its lane of tensor
@@ -568,9 +580,9 @@ __device__ __noinline__ void issue_exact(uint8_t *smem, uint32_t tmem, GroupDev 
 // with few rows takes 0.5 us more. Out of line because it runs once: in the kernel either form of the loop moved the code of the steps, and each made another form
 // of them 0.6 to 1.6 % slower (us per step, unrolled 8 : 1 : this; H = 384 32 chunks 1.163 : 1.179 : 1.155, H = 768 300 1.757 : 1.743 : 1.738, H = 1024 240
 // 1.892 : 1.863 : 1.861; the largest losses of this one 256 64 1.126 : 1.146 : 1.143, 768 170 1.441 : 1.440 : 1.455).
-template <int V, int C>
+template <int V, int C, int STEPS>
 __device__ __noinline__ bool recurrent_weights(uint32_t row, uint32_t t_w, int lane) {
-    using K = GroupConst<V, C>;
+    using K = GroupConst<V, C, STEPS>;
     __half2 zeros[2] = {__half2half2(__ushort_as_half(0)), __half2half2(__ushort_as_half(0))};
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
@@ -589,7 +601,7 @@ __device__ __noinline__ bool recurrent_weights(uint32_t row, uint32_t t_w, int l
 // The groups of chunk rows share the x part of the contraction (its MMAs read their A operand from shared memory, so
 // one for both) and go through the rest of the step one after the other: while one is exchanged, the other
 // is projected or computed.
-template <int V, int C>
+template <int V, int C, int STEPS>
 __global__ void __launch_bounds__(kGThreads, 1)
 lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] f16, boxes 128 x 64
                   const __grid_constant__ CUtensorMap tm_x,    // x_down [T, 2, B, 64] f16, boxes of all rows
@@ -598,7 +610,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
                   const __grid_constant__ CUtensorMap tm_o,    // SPLIT: h_out [T, B, H], boxes of the first group's rows x 128
                   const __grid_constant__ CUtensorMap tm_ol,   // and of the second's
                   const GroupDev p) {
-    using K = GroupConst<V, C>;
+    using K = GroupConst<V, C, STEPS>;
     constexpr GroupForm F = K::F;
     constexpr GroupLayout L = K::L;
     constexpr bool kGather = K::kGather, kByPair = K::kByPair, kTwoSteps = K::kTwoSteps, kFourSteps = K::kFourSteps, kOneProj = K::kOneProj;
@@ -718,7 +730,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
 #pragma unroll 1
         for (int s = g; s < kDnTs; s += 4) tmem_st_32x8(t_lane + kDnCol + s * 8, __ldg(dn + 2 * s), __ldg(dn + 2 * s + 1));
         if (__all_sync(0xffffffffu, mbar_wait(&bar_w[g], 0, abort_flag, 109)))
-            non_finite = recurrent_weights<V, C>(smem_u32(smem) + g * 32768 + (q * 32 + lane) * 128, t_lane + kGTmemW + g * 64, lane);
+            non_finite = recurrent_weights<V, C, STEPS>(smem_u32(smem) + g * 32768 + (q * 32 + lane) * 128, t_lane + kGTmemW + g * 64, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_w_read[g]);
         tmem_st_wait();
@@ -789,8 +801,8 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
         __syncwarp();
     } else if (warp == 1) {
         if (!kGather) peers_ready();
-        if (!K::kZeroRows || finite) issue<V, C, false>(smem, tmem, p, n_rows, own_rows, hh_bytes(0), hh_bytes(1));
-        else issue_exact<V, C>(smem, tmem, p, n_rows, hh_bytes(0), hh_bytes(1));
+        if (!K::kZeroRows || finite) issue<V, C, STEPS, false>(smem, tmem, p, n_rows, own_rows, hh_bytes(0), hh_bytes(1));
+        else issue_exact<V, C, STEPS>(smem, tmem, p, n_rows, hh_bytes(0), hh_bytes(1));
     } else {
         // ------------------------------ gates -------------------------------------------
         // thread = hidden unit. GATHER: a quarter of the rows; SPLIT: half of the rows of one group, eight warps each, so
@@ -1144,17 +1156,23 @@ struct GroupPlan {
     int form;         // see group_form
     int rows;         // rows per cluster
     int tiles;        // clusters
+    bool most;        // the kernel of most steps per x MMA
 };
 
 using group_kernel_fn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GroupDev);
 struct GroupKernel { group_kernel_fn fn; int smem; };
-template <int V, int C>
-constexpr GroupKernel group_kernel() { return {lstm_group_kernel<V, C>, group_layout(V, C).dynamic}; }
-#define FLUKE_GROUP_KERNELS(V) \
-    {{}, {}, group_kernel<V, 2>(), group_kernel<V, 3>(), group_kernel<V, 4>(), group_kernel<V, 5>(), group_kernel<V, 6>(), \
-     group_kernel<V, 7>(), group_kernel<V, 8>()}
-const GroupKernel kGroupKernels[kGForms][kGMaxCtas + 1] = {FLUKE_GROUP_KERNELS(0), FLUKE_GROUP_KERNELS(1), FLUKE_GROUP_KERNELS(2),
-                                                            FLUKE_GROUP_KERNELS(3)};
+template <int V, int C, bool MOST>
+constexpr GroupKernel group_kernel() {
+    constexpr int steps = group_x_steps(V, C, MOST);
+    return {lstm_group_kernel<V, C, steps>, group_layout(V, C, steps).dynamic};
+}
+#define FLUKE_GROUP_KERNELS(V, MOST) \
+    {{}, {}, group_kernel<V, 2, MOST>(), group_kernel<V, 3, MOST>(), group_kernel<V, 4, MOST>(), group_kernel<V, 5, MOST>(), group_kernel<V, 6, MOST>(), \
+     group_kernel<V, 7, MOST>(), group_kernel<V, 8, MOST>()}
+#define FLUKE_GROUP_FORMS(MOST) \
+    {FLUKE_GROUP_KERNELS(0, MOST), FLUKE_GROUP_KERNELS(1, MOST), FLUKE_GROUP_KERNELS(2, MOST), FLUKE_GROUP_KERNELS(3, MOST)}
+const GroupKernel kGroupKernels[2][kGForms][kGMaxCtas + 1] = {FLUKE_GROUP_FORMS(false), FLUKE_GROUP_FORMS(true)};
+#undef FLUKE_GROUP_FORMS
 #undef FLUKE_GROUP_KERNELS
 
 // Clusters of C CTAs of form V that the device runs at once with the largest shared memory a CTA can
@@ -1167,8 +1185,13 @@ int group_capacity(int V, int C) {
     int &slot = known[dev][V][C];
     if (slot == 0) {
         int n = 0;
-        const void *fn = reinterpret_cast<const void *>(kGroupKernels[V][C].fn);
-        bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGMaxSmem) == cudaSuccess;
+        // both kernels of the form at once: a caller that has run a long layer may capture a short one
+        const void *fn = nullptr;
+        bool ok = true;
+        for (int most = 0; most < 2 && ok; ++most) {
+            fn = reinterpret_cast<const void *>(kGroupKernels[most][V][C].fn);
+            ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGMaxSmem) == cudaSuccess;
+        }
         if (ok) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(C);
@@ -1189,9 +1212,9 @@ int group_capacity(int V, int C) {
     return slot > 0 ? slot - 1 : 0;
 }
 
-// How B rows of hidden size H are spread: as few waves of clusters as the largest row count allows, then
+// How B rows of hidden size H are spread over clusters for T steps: as few waves of clusters as the largest row count allows, then
 // evenly over all clusters of those waves.
-bool group_plan(int B, int H, GroupPlan *g) {
+bool group_plan(int T, int B, int H, GroupPlan *g) {
     if (H % kGUnits) return false;
     const int C = H / kGUnits;
     if (C < 2 || C > kGMaxCtas) return false;
@@ -1205,6 +1228,7 @@ bool group_plan(int B, int H, GroupPlan *g) {
     g->tiles = (B + g->rows - 1) / g->rows;
     g->form = 0;
     while (g->rows > group_form(g->form).most) ++g->form;
+    g->most = group_most_x_steps(T, g->rows, g->form, C);
     return group_capacity(g->form, C) > 0;
 }
 
@@ -1214,8 +1238,8 @@ bool group_plan(int B, int H, GroupPlan *g) {
 extern "C" int fluke_sm100_lstm_small_clusters(int T, int B, int H, int *x_steps) {
     using namespace fluke_sm100;
     GroupPlan g;
-    if (T < 1 || B < 1 || H < 1 || !group_plan(B, H, &g)) return 0;
-    if (x_steps) *x_steps = group_x_steps(g.form, H / kGUnits);
+    if (T < 1 || B < 1 || H < 1 || !group_plan(T, B, H, &g)) return 0;
+    if (x_steps) *x_steps = group_x_steps(g.form, H / kGUnits, g.most);
     return g.rows;
 }
 
@@ -1226,10 +1250,10 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
     const fluke_flstm_layer_t *l = static_cast<const fluke_flstm_layer_t *>(layer);
     const int T = l->T, B = l->B, H = l->H, R = l->R;
     GroupPlan g;
-    if (R != kGRank || !group_plan(B, H, &g)) return -2;
+    if (R != kGRank || !group_plan(T, B, H, &g)) return -2;
     const int C = H / kGUnits;
     const GroupForm f = group_form(g.form);
-    const GroupKernel &kn = kGroupKernels[g.form][C];
+    const GroupKernel &kn = kGroupKernels[g.most][g.form][C];
 
     GroupDev p;
     p.T = T; p.B = B; p.reverse = l->reverse;
@@ -1250,7 +1274,7 @@ extern "C" int fluke_sm100_lstm_layer_group(const void *layer, const void *x_dow
         // both K blocks of a row range in one box: the 128-byte blocks of a row are a dimension
         const uint64_t dims[4] = {64, uint64_t(B), 2, uint64_t(T)};
         const uint64_t strides[3] = {uint64_t(R) * 2, 128, uint64_t(B) * R * 2};
-        const uint32_t box[4] = {64, uint32_t(f.groups * f.rows), group_x_steps(g.form, C) > 1 ? 1u : 2u, 1};
+        const uint32_t box[4] = {64, uint32_t(f.groups * f.rows), group_x_steps(g.form, C, g.most) > 1 ? 1u : 2u, 1};
         rc = make_tmap_nd(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x_down, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }

@@ -719,3 +719,45 @@ def test_infinite_gate_weights_in_layers_of_few_steps(flib, h, rows, t):
     for b in _chunk_counts(flib, h, rows):
         assert _small_clusters(flib, t, b, h) == (rows, 1)
         _assert_default_form_gives_the_bytes_of_the_l2_form(flib, t, b, h, True)
+
+
+@pytest.mark.parametrize("h,rows,few,enough", [(256, 8, 7, 8), (384, 6, 7, 8), (384, 7, 18, None), (256, 16, 15, 16), (384, 14, 15, 16), (384, 15, 18, None), (512, 12, 15, 16),
+                                               (512, 13, 18, None), (256, 17, 7, 8), (640, 32, 7, 8), (896, 32, 15, 16)])
+def test_layers_of_few_steps_take_the_kernel_of_fewer_steps_per_contraction(flib, h, rows, few, enough):
+    """On either side of the numbers of timesteps (and of rows: None) from which a contraction covers more of them. Exact."""
+    b = _chunk_counts(flib, h, rows)[1]
+    fewest = 2 if rows <= 8 else 1
+    for t in range(max(1, few - 1), few + 1):
+        assert _small_clusters(flib, t, b, h) == (rows, fewest)
+        _assert_default_form_gives_the_bytes_of_the_l2_form(flib, t, b, h, False)
+    if enough:
+        assert _small_clusters(flib, enough, b, h) == (rows, 2 * fewest)
+        _assert_default_form_gives_the_bytes_of_the_l2_form(flib, enough, b, h, False)
+
+
+def test_a_short_layer_is_captured_after_a_long_one_has_run(flib):
+    """The kernel of a layer of few steps is another one than that of a longer layer; it is configured with it, in front of the capture."""
+    h, rows, t = 640, 20, 9
+    b = _chunk_counts(flib, h, rows)[0]
+    assert _small_clusters(flib, t, b, h)[1] != _small_clusters(flib, 3, b, h)[1]
+    layer, x, xs = _layer_case(t, b, h, 128, 5, False)
+    x, xs = x.to(DEV), xs.to(DEV)
+    args = (layer.dn_ih, layer.dn_ih_scale, layer.dn_hh, layer.dn_hh_scale, layer.w_up, layer.bias)
+    state = lambda: (torch.zeros(b, h, device=DEV), torch.zeros(b, h, dtype=torch.int8, device=DEV))
+    ws = torch.empty(flib.fluke_factored_lstm_layer_workspace(t, b, h, 128), dtype=torch.uint8, device=DEV)
+    ops.factored_lstm_layer_i8(x, xs, *args, *state(), workspace=ws)
+    c, hs = state()
+    out = torch.empty(3, b, h, dtype=torch.int8, device=DEV)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        ops.set_stream(stream)
+        try:
+            ops.factored_lstm_layer_i8(x[:3], xs[:3 * b], *args, c, hs, h_out=out, workspace=ws)
+        finally:
+            ops.set_stream(None)
+    graph.replay()
+    torch.cuda.synchronize()
+    c2, hs2 = state()
+    want = ops.factored_lstm_layer_i8(x[:3], xs[:3 * b], *args, c2, hs2)
+    assert torch.equal(out, want) and torch.equal(c, c2) and torch.equal(hs, hs2)
