@@ -175,6 +175,35 @@ def test_qkv_rotary_of_many_chunks_equals_chunk_by_chunk(be, batch, seqlen, fp8)
         assert torch.equal(got[rows].view(torch.int16), call(a[rows].contiguous(), sa[rows].contiguous()).view(torch.int16))
 
 
+def _runs_that_cross(batch, seqlen):
+    """Of the CTAs of an N tile, how many take a run of the whole list of tiles that goes from one tile-in-sequence to the next; None where runs keep
+    to one: if the CTAs, shared out to the tiles-in-sequence first, would have no more tiles each."""
+    tiles = -(-seqlen // 128)
+    per_n = min(torch.cuda.get_device_properties(0).multi_processor_count // 6, tiles * batch)   # 1536 columns in six N tiles
+    most = -(-tiles * batch // per_n)
+    if per_n // tiles > 0 and batch <= per_n // tiles * most:
+        return None
+    return sum(first // batch != (min(first + most, tiles * batch) - 1) // batch for first in range(0, tiles * batch, most))
+
+
+@pytest.mark.parametrize("seqlen", [640, 777, 1333, 1600, 1999])
+@pytest.mark.parametrize("crossings", [2, 4, 8])
+def test_qkv_rotary_runs_of_the_whole_list_equal_chunk_by_chunk(be, seqlen, crossings):
+    """The numbers of chunks, found for this device, whose tiles are not shared out by tile-in-sequence: at least so many runs change their
+    positions on the way. Against one call per chunk. Exact."""
+    batch = next((n for n in range(3, 64) if (_runs_that_cross(n, seqlen) or 0) >= crossings), None)
+    if batch is None:
+        pytest.skip("no such number of chunks on this device")
+    m = batch * seqlen
+    a, sa, w, sb = (t.to(DEV).contiguous() for t in _qkv_inputs(m, torch.Generator().manual_seed(m)))
+    sin, cos = (t.to(DEV) for t in prep.rotary_tables(seqlen, 64))
+    got = ops.qkv_rotary_i8(be, a, w, sa, sb, sin, cos, seqlen)
+    for i in range(batch):
+        rows = slice(i * seqlen, (i + 1) * seqlen)
+        want = ops.qkv_rotary_i8(be, a[rows].contiguous(), w, sa[rows].contiguous(), sb, sin, cos, seqlen)
+        assert torch.equal(got[rows].view(torch.int16), want.view(torch.int16))
+
+
 def test_qkv_rotary_full_size_sampled_rows_and_v_passthrough(be):
     m, seqlen = 32000, 1000
     a, sa, w, sb = _qkv_inputs(m, torch.Generator().manual_seed(0))
