@@ -775,10 +775,12 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             }
         };
         constexpr int kEarly = K::kTwoStepsWide ? 1 : 0;   // windows that begin before step 0
-        if (!kGather && elect_one())
-            for (int i = -kEarly; i < min(p.T, kXSlots - kEarly); ++i) load_x(i);
-        __syncwarp();
-        if (!kGather) peers_ready();
+        if constexpr (!kGather) {
+            if (elect_one())
+                for (int i = -kEarly; i < min(p.T, kXSlots - kEarly); ++i) load_x(i);
+            __syncwarp();
+            peers_ready();
+        }
         if (elect_one()) {
             if constexpr (kGather) {
                 for (int i = -kEarly; i < p.T && ok; ++i) load_x(i);
