@@ -72,8 +72,9 @@ struct GemmDev {
     // CTA takes a contiguous run of the list ordered by (tile-in-sequence, sequence), so the rows
     // of successive tiles keep their positions and their sin/cos values stay in registers. Where that takes no more items per CTA, a run is
     // of one tile-in-sequence: a change of positions is 64 loads per thread in front of the tile's arithmetic, and with runs that cross
-    // from one to the next nearly every CTA had one. Us, runs of the whole list : of one tile-in-sequence, 7 x 1333 rows 13.06 : 11.77, 5 x 900 8.87 : 7.77, 16 x
-    // 1000 17.16 : 16.19, 32 x 1000 28.15 : 27.40; the others, whose runs did not cross, 1 to 3 % faster with the start below.
+    // from one to the next nearly every CTA had one. Us, runs of the whole list and a start that each role works out : these, with the start below,
+    // 7 x 1333 rows 13.06 : 11.81, 5 x 900 8.88 : 7.77, 16 x 1000 17.08 : 15.95, 30 x 700 21.02 : 20.22, 32 x 1000 28.61 : 27.78; 3 x 1600, which keeps runs of the whole
+    // list, 9.04 : 9.05.
     int seq_tiles;  // 0: plain tiling, tile t covers rows [128 t, 128 t + 128)
     int n_seq;
     int items_per_cta;
@@ -213,7 +214,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
     const int m_first = blockIdx.x / p.num_n_tiles;
     const int n0 = n_tile * BN_OUT;
     // Where every role begins. Its divisions are done once, by an idle warp and while the kernel before this one still runs, instead of by
-    // each role behind the wait for that kernel: QKV + rotary 1803 rows 5.97 -> 5.71 us, 9216 10.33 -> 10.17, gated MLP 9331 17.06 -> 16.91.
+    // each role behind the wait for that kernel: QKV + rotary 1803 rows 5.96 -> 5.73 us, gated MLP 4800 rows 11.45 -> 11.21, 10000 17.79 -> 17.64, 16000 26.80 -> 26.74 (its
+    // epilogue spills 88 bytes a thread with it, 80 without).
     TileCursor *start = reinterpret_cast<TileCursor *>(smem + L::kOffMisc + 16);
 
     if (threadIdx.x == 0) {

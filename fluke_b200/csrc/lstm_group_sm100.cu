@@ -45,10 +45,11 @@
 // 490, exchange 430 (200 at H = 384). 14 rows, 2850: 500, 270, 130, 450, 1040 (the cell updates) and 440. 47 rows, 4500: first group's projection 460, its partial
 // sums sent 310, on the way 480 to 800, read and added up 300, converted and sent 300 to 430, on the way 490, contraction 720, cell updates 950 (24 rows, eight
 // warps), 230 until the issuer has seen the last warp's codes; the second group's chain runs beside it, and the tensor pipe works 3370 of them (x part 1540,
-// hh half 1460, projections 370). The layer ends with the slowest cluster: 1024 chunks 2.67 us per step, x_down included (2.88 before own shares stayed out of the
-// network), at the 1.83 GHz that the nanosecond timer gives inside the kernel (the driver reports 1965 MHz meanwhile).
-// The cell updates live on few instructions: with places in the swizzle worked out per row instead of by one exclusive or,
-// 1024 chunks took 2.89 us, 700 2.13.
+// hh half 1460, projections 370). The layer ends with the slowest cluster: 1024 chunks 2.66 us per step, x_down included, in layers of 400 steps (2.86 at commit
+// f537a30, before own shares stayed out of the network), at the 1.83 GHz that the nanosecond timer gives inside the kernel (the driver reports 1965 MHz
+// meanwhile). That is below the power limit: in a loop of seconds the gain is 5 % instead of 7 (five layers of 1000 steps 15.15 -> 14.37 ms).
+// The cell updates live on few instructions: when places in the swizzle were worked out per row instead of by one exclusive or, 1024 chunks took 0.14 us
+// more, 700 0.09.
 //
 // The operand rows that are zero (see group_form) add zero times a weight to another group's or step's accumulators: with
 // finite weights nothing. A CTA whose recurrent gate weights are not all finite (0 x inf is NaN) issues other MMAs, see
@@ -91,15 +92,13 @@ struct GroupDev {
     long long *trace;          // trace builds only: [T][16] SM-clock stamps of CTA 0
 };
 
-// The forms of the kernel: chunk rows per cluster up to 8, 16, 32 and 48. GATHER is one group of rows, SPLIT two. Step of the
-// kernel of one and two groups that exchanged hidden rows between pairs of CTAs and projected them there, against
-// these, in us, x_down included: H = 768 32 chunks (2 rows per cluster) 1.45 : 1.15, 170 (8 rows) 1.56 : 1.34, 300 (14 rows) 1.66 :
-// 1.61, 500 (23 rows) 2.40 : 1.96, 700 (32 rows) 2.62 : 2.04, 1024 (47 rows) 2.97 : 2.75; H = 384, 32 chunks (2 rows) 1.37 : 1.08;
-// H = 1024, where it took two waves from 577 chunks on, 700 (47 rows) 4.85 : 2.86. The limits are the same for every cluster size. Layers of
-// 400 steps at 32 numbers of chunks per size, that kernel against these: H = 256 594 chunks 1.48 : 1.45, 1122 1.73 : 1.54; H = 384 387 1.55 :
-// 1.48, 731 2.29 : 2.02; H = 512 288 1.52 : 1.49, 544 2.09 : 2.00; H = 640 234 1.57 : 1.54, 442 2.18 : 2.00, 858 2.87 : 2.75; H = 896 153 1.72 :
-// 1.67, 289 2.38 : 2.04, 561 3.06 : 2.67. Slower only with 48-row kernels of small clusters: H = 256 2376 chunks 2.69 : 2.75, H = 512
-// 1472 2.91 : 2.97, which no smaller form holds in one wave.
+// The forms of the kernel: chunk rows per cluster up to 8, 16, 32 and 48. GATHER is one group of rows, SPLIT two. Step of the kernel of commit 31278fa, of one and
+// two groups, which exchanged hidden rows between pairs of CTAs and projected them there, against these as they are now, us, x_down included, layers of 400 steps:
+// H = 768 32 chunks (2 rows per cluster) 1.45 : 1.23, 170 (8) 1.56 : 1.44, 300 (14) 1.66 : 1.72, 500 (23) 2.40 : 1.96, 700 (32) 2.62 : 2.02, 1024 (47) 2.97 : 2.66; H = 384 32
+// (2) 1.37 : 1.04, 387 (9) 1.55 : 1.39, 731 (17) 2.29 : 1.90; H = 256 594 (9) 1.48 : 1.37, 1122 (17) 1.73 : 1.54, 2376 (36) 2.69 : 2.64; H = 512 288 (9) 1.52 : 1.46, 544 (17) 2.09 : 1.79,
+// 1472 (46) 2.91 : 2.72; H = 640 234 1.57 : 1.53, 442 2.18 : 1.83, 858 2.87 : 2.58; H = 896 153 1.72 : 1.68, 289 2.38 : 1.99, 561 3.06 : 2.55; H = 1024 700 (47), where it took two waves from
+// 577 chunks on, 4.85 : 2.70. The left figures are of its own day, those in front of the first semicolon of longer layers, whose set-up is less per step (300 chunks of 777
+// steps take 1.68 now). The limits are the same for every cluster size.
 // Everything below depends on the form V and the cluster size C = H / 128, which the kernel is compiled
 // for: with operand addresses at fixed distances the issuer needs few instructions between MMAs.
 constexpr int kGForms = 4;
@@ -120,9 +119,9 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
            : V == 2 ? GroupForm{32, false, 2, 16, 16, 32, 32}
                     : GroupForm{48, false, 2, 24, 32, 56, 32};
 }
-// Steps whose x part one MMA covers: for each form and cluster size a kernel of the fewest and, where it pays, one of more. Up to 8 rows: MMAs of an A operand in shared memory take as long for 32 columns (44 cycles) as for the
-// sixteen that there are at least (42), and what is issued of them before the hidden codes arrive holds the issuer up: with 16 such MMAs per step
-// it saw codes that had travelled for 200 cycles after 430. Four steps per MMA are 8 per step, and twice the accumulators, which clusters of
+// Steps whose x part one MMA covers: for each form and cluster size a kernel of the fewest and, where it pays, one of more. Up to 8 rows: MMAs of an
+// A operand in shared memory take as long for 32 columns (44 cycles) as for the sixteen that there are at least (42), and what is issued of them before
+// the hidden codes arrive holds the issuer up: with 16 such MMAs per step it saw codes that had travelled for 200 cycles after 430. Four steps per MMA are 8 per step, and twice the accumulators, which clusters of
 // two and three have the tensor memory for beside all projection weights. Two steps against four, us per step, x_down included: H = 384 32 chunks 1.156 :
 // 1.044, 120 1.186 : 1.078, 172 1.188 : 1.088, 250 1.200 : 1.160, 344 1.235 : 1.238; H = 256 32 1.137 : 1.027, 300 1.182 : 1.109, 528 1.222 : 1.202. With
 // more CTAs some projection weights have to give way: H = 512 32 chunks 1.166 : 1.125, but 200 1.269 : 1.339; H = 640 200 1.366 : 1.467.
@@ -130,8 +129,13 @@ __host__ __device__ constexpr GroupForm group_form(int V) {
 // 10 % less at H = 768, 15 % at H = 512). One step against two: H = 768 360 chunks 2.031 : 1.941, 500 2.063 : 1.989, 700 2.103 : 2.037; H = 384 900 2.062 : 1.934; H =
 // 256 1200 2.045 : 1.827; H = 512 700 2.047 : 1.835; H = 640 600 2.063 : 1.885; H = 896 400 2.060 : 2.050; clusters of eight 300 2.089 : 2.138.
 // 9 to 16 rows, where the larger accumulators leave tensor memory for all projection weights: H = 256 600 chunks 1.455 : 1.369, 1000 1.545 : 1.507; H = 384 400
-// 1.485 : 1.395, 600 1.569 : 1.547, 680 1.589 : 1.593; H = 512 300 1.494 : 1.462, 500 1.657 : 1.654. Without: H = 768 200 1.606 : 1.667, 300 1.758 : 1.842.
-constexpr int group_x_steps(int V, int C, bool most) { return V == 0 ? (most && C <= 3 ? 4 : 2) : most && ((V == 1 && C <= 4) || (V == 2 && C <= 7)) ? 2 : 1; }
+// 1.485 : 1.395, 600 1.569 : 1.547, 680 1.589 : 1.593; H = 512 300 1.494 : 1.462, 500 1.657 : 1.654. Without: H = 640 230 1.547 : 1.546, 260 1.555 : 1.569, 300 1.569 : 1.621, 400
+// 1.685 : 1.772; H = 768 200 1.606 : 1.667, 300 1.758 : 1.842; clusters of seven lack the shared memory for the weights that would go there. (All pairs in layers of
+// 400 steps, each as it was measured when it was chosen.)
+constexpr int group_x_steps(int V, int C, bool most) {
+    if (V == 0) return most && C <= 3 ? 4 : 2;
+    return most && ((V == 1 && C <= 4) || (V == 2 && C <= 7)) ? 2 : 1;
+}
 // Which of the two. Windows of several steps begin before the first one or end behind the last, so a layer of few steps pays for more than its
 // own; and with many rows in its form the wider accumulators cost more than they save. Fewest : most, us of a layer, x_down included.
 // Up to 8 rows, H = 384 86 chunks (2 rows) 1 step 12.4 : 12.7, H = 256 132 8 steps 19.6 : 19.2; H = 384 301 chunks (7 rows) 100 steps 127.2 : 127.3, 344 (8) 400 steps 485 : 492.
@@ -520,11 +524,11 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
         asm volatile("" : "+l"(d_wx), "+l"(d_x0), "+l"(d_hh), "+l"(d_dn), "+l"(d_h0));
         constexpr int kFirstX = kFourSteps ? 4 : kTwoSteps ? 10 : kByPair ? 16 : kGather ? (K::kTwoStepsWide ? 12 : 24) : 2;
         if constexpr (kGather) {
-            // Most of the x part while the hidden state is computed and travels, the rest while the
-            // projection is converted. 20 / 24 / 28 of 32 in front, us per step (x_down included): H = 768 200 chunks 1.62 / 1.57 / 1.64, 300
-            // 1.74 / 1.70 / 1.73; H = 384 600 1.58 / 1.54 / 1.63; H = 512 500 1.68 / 1.62 / 1.65; H = 896 180 1.71 / 1.70 / 1.74. 8 / 10 / 12 of 16: H = 768
-            // 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 1024 60 1.42 / 1.40 / 1.44. 10 / 12 of 16 for more rows: H = 384 600 1.559 / 1.547. 3 / 4 / 5 of 8 within 1 % of each other. By pair 12 / 16 /
-            // 20 of 32: 135 chunks 1.68 / 1.66 / 1.73, 240 1.86 / 1.87 / 1.88.
+            // Most of the x part while the hidden state is computed and travels, the rest while the projection is converted. Us per step (x_down
+            // included). One step per MMA, 20 / 24 / 28 of 32 in front: H = 768 200 chunks 1.62 / 1.57 / 1.64, 300 1.74 / 1.70 / 1.73; H = 896 180 1.71 / 1.70 / 1.74. Two
+            // steps, up to 8 rows, 8 / 10 / 12 of 16: H = 768 32 chunks 1.19 / 1.19 / 1.23, 100 1.29 / 1.27 / 1.30; H = 1024 60 1.42 / 1.40 / 1.44; more rows, 10 / 12 / 14
+            // of 16: H = 384 600 1.533 / 1.529 / 1.525; H = 256 600 1.363 / 1.361 / 1.354, 1000 1.486 / 1.494 / 1.474; H = 512 300 1.480 / 1.479 / 1.482, 500 1.645 / 1.642 / 1.639. Four
+            // steps, 3 / 4 / 5 of 8 within 1 % of each other. By pair 12 / 16 / 20 of 32: 135 chunks 1.68 / 1.66 / 1.73, 240 1.86 / 1.87 / 1.88.
             if (!wait_x(kFourSteps ? i + 3 : kTwoSteps ? i + 1 : i) || !wait_acc()) break;
             FLUKE_STAMP(blockIdx.x == 0 && lane == 0, i * 16 + 15, clock64());
             // Two steps per MMA: the zero rows of the step before have spoilt the accumulators of this step's gates that its x MMAs
@@ -545,10 +549,11 @@ __device__ __forceinline__ void issue(uint8_t *smem, uint32_t tmem, const GroupD
             // A group's projection as soon as its codes are there, pieces of the x part in between. A wait for
             // what has long been there takes 100 cycles and more while the gate warps keep the units of the SM busy that
             // serve both, so such waits stand where the issuer has time (1024 chunks 3.07 -> 2.89 us per step when it was done).
-            // 0 / 2 / 4 / 8 MMAs in front of the second projection, us per step (x_down included): H = 768 500 chunks 2.09 / 2.05 / 2.03 / 2.07,
-            // 700 2.14 / 2.13 / 2.13 / 2.22, 900 2.76 / 2.76 / 2.77 / 2.83, 1024 2.93 / 2.93 / 2.96 / 2.94; H = 384 900 2.07 / 2.04 / 2.05 / 2.06, 1500
-            // 2.71 / 2.71 / 2.71 / 2.71; H = 1024 300 2.17 / 2.16 / 2.16 / 2.18, 700 2.90 / 2.91 / 2.92 / 2.98. Four in front of the first as well
-            // took 0.3 us more.
+            // MMAs in front of the second projection, us per step (x_down included). One step per MMA, 0 / 2 / 4 / 8, before own shares stayed in the CTA: H = 768 900
+            // chunks 2.76 / 2.76 / 2.77 / 2.83, 1024 2.93 / 2.93 / 2.96 / 2.94; H = 384 1500 2.71 / 2.71 / 2.71 / 2.71; H = 1024 300 2.17 / 2.16 / 2.16 / 2.18, 700 2.90 / 2.91 / 2.92 /
+            // 2.98. Four in front of the first as well took 0.3 us more. Two steps per MMA, 0 / 1 / 2 / 4 of 16: H = 768 500 1.958 / 1.960 / 1.964 / 1.966, 700 2.022 / 2.023 / 2.017 /
+            // 2.037; H = 384 900 1.912 / 1.908 / 1.923 / 1.918; H = 512 700 1.850 / 1.857 / 1.841 / 1.843; H = 640 600 1.888 / 1.878 / 1.883 / 1.902; H = 256 1200 1.824 / 1.833 / 1.816 / 1.829. The
+            // last quarter behind the wait for the stores, of 16 from 8 / 12 / 14 on: H = 768 700 2.032 / 2.017 / 2.033; H = 256 1200 1.836 / 1.816 / 1.818; others within 0.8 %.
             if (!wait_x(i) || !wait_sent(both ? 2 * i : i)) break;
             if (!project(Int<0>{}, i)) break;
             if (!wait_acc()) break;
@@ -1005,7 +1010,7 @@ lstm_group_kernel(const __grid_constant__ CUtensorMap tm_w,    // w_up [4H, 2R] 
             const int own = own_pieces(e);
             // Where the projected pieces and the rows of hh_down go. What stays in the CTA is stored there by itself: st.async takes it through the
             // network like the rest, whose bytes bound the step where several clusters share a GPC (clusters of 1024 chunks had periods of 4520 to 5080
-            // cycles). Us per step, with : without, H = 768 700 chunks 2.138 : 2.114, 900 2.801 : 2.673, 1024 2.942 : 2.716; H = 1024 500 2.776 : 2.657, 700 2.911 :
+            // cycles). Us per step of short runs, below the power limit, in the network : kept out, H = 768 700 chunks 2.138 : 2.114, 900 2.801 : 2.673, 1024 2.942 : 2.716; H = 1024 500 2.776 : 2.657, 700 2.911 :
             // 2.823; H = 384 900 2.041 : 2.074, 1500 2.685 : 2.615; H = 512 1400 2.863 : 2.728. Up to 16 rows (GATHER) it costs 2 to 8 %: 300 chunks 1.730 : 1.814.
             uint32_t p_to[kPieces / 2], p_bar[kPieces / 2];
             int p_own = 0;   // one bit per piece that the CTA adds up itself

@@ -388,9 +388,9 @@ extern "C" int fluke_sm100_lstm_layer_phases(const void *layer, int phase_mask, 
                 default: return -2;
             }
         };
-        // The small clusters come first wherever they cover the shape. Step time at H = 768, against
-        // the fastest of the other forms: 32 chunks 1.1 us (5.76), 300 1.6 (5.83), 700 2.0 (5.82),
-        // 1024 2.7 (7.31), 2048 in two waves 5.3 (8.9).
+        // The small clusters come first wherever they cover the shape. Step time at H = 768, x_down included, against
+        // the fastest of the other forms: 32 chunks 1.2 us (5.76), 300 1.7 (5.83), 700 2.0 (5.82),
+        // 1024 2.7 (7.31), 2048 in two waves 5.2 (8.9).
         int order[4] = {0, 0, 0, 0};
         switch (g_lstm_persistent) {
             case 2: order[0] = 2; break;
