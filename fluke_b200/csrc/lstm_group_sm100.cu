@@ -99,7 +99,7 @@ struct GroupDev {
 // 1472 (46) 2.91 : 2.72; H = 640 234 1.57 : 1.53, 442 2.18 : 1.83, 858 2.87 : 2.58; H = 896 153 1.72 : 1.68, 289 2.38 : 1.99, 561 3.06 : 2.55; H = 1024 700 (47), where it took two waves from
 // 577 chunks on, 4.85 : 2.70. The left figures are of its own day, those in front of the first semicolon of longer layers, whose set-up is less per step (300 chunks of 777
 // steps take 1.68 now). The limits are the same for every cluster size.
-// Everything below depends on the form V and the cluster size C = H / 128, which the kernel is compiled
+// Everything below depends on the form V, the cluster size C = H / 128 and the steps per x MMA, which the kernel is compiled
 // for: with operand addresses at fixed distances the issuer needs few instructions between MMAs.
 constexpr int kGForms = 4;
 struct GroupForm {
